@@ -6,69 +6,170 @@
 // (llm-core/src/backends/candle.rs:1276-1340: weight [out, in], used transposed,
 // optional bias added after).
 #include "common.cuh"
+#include "mma_util.cuh"
 
-constexpr int GF_BM = 64, GF_BN = 64, GF_BK = 16, GF_THREADS = 256;
-
-template <typename TX>
-__global__ void __launch_bounds__(GF_THREADS)
+// A block owns a tile of BM rows x BN features and walks K in steps of BK through NS stages of shared memory, filled by
+// asynchronous copies NS - 1 steps ahead. Both operands stay in rows along K as they come, a row padded by 16 bytes so that
+// neighbouring rows' 16-byte reads fall into different banks; a thread reads four values of K of its TM rows and TN
+// features at a time and adds them in order of K. An output is ONE chain of fused multiply-adds whatever the tile, which
+// keeps its bits the same in every batch, and is why no tile splits K: a product of few rows is bound by that chain and by
+// the latency of its stages (K = 3,072 into 1,024 features, one row: 19 us, 236 before with one synchronous stage of 16
+// values), one of many features by the stream of its weights (1,024 into 32,000: 42 us, 3.1 TB/s; 185 before), one of many
+// rows by the FMA units (2,048 rows of 4,096 x 4,096: 1,867 us, 36.8 TFLOP/s; 2,711 before).
+template <typename TX, int BM, int BN, int TM, int TN, int BK, int NS, int U, bool VEC>
+__global__ void __launch_bounds__((BM / TM) * (BN / TN))
 gemm_f32_kernel(const TX* __restrict__ x, const float* __restrict__ w, const float* __restrict__ bias,
                 float* __restrict__ out, int M, int N, int K, long long x_stride, long long out_stride) {
-  __shared__ float As[GF_BK][GF_BM + 4];
-  __shared__ float Bs[GF_BK][GF_BN + 4];
-  const int tid = threadIdx.x;
-  const int m0 = blockIdx.y * GF_BM, n0 = blockIdx.x * GF_BN;
-  const int tr = tid / 16, tc = tid % 16;  // this thread's 4x4 block: rows tr*4.., cols tc*4..
-  float acc[4][4];
-#pragma unroll
-  for (int i = 0; i < 4; ++i)
-#pragma unroll
-    for (int j = 0; j < 4; ++j) acc[i][j] = 0.f;
-
-  // Each thread loads 4 consecutive k of one row of each tile.
-  const int lrow = tid / 4, lk = (tid % 4) * 4;
-  for (int k0 = 0; k0 < K; k0 += GF_BK) {
-#pragma unroll
-    for (int e = 0; e < 4; ++e) {
-      const int k = k0 + lk + e;
-      const int m = m0 + lrow, n = n0 + lrow;
-      As[lk + e][lrow] = (m < M && k < K) ? to_float(x[(size_t)m * x_stride + k]) : 0.f;
-      Bs[lk + e][lrow] = (n < N && k < K) ? w[(size_t)n * K + k] : 0.f;
+  constexpr int THREADS = (BM / TM) * (BN / TN), CN = BN / TN, RM = BM / TM;
+  constexpr int XS = BK + 16 / (int)sizeof(TX), WS = BK + 4;      // elements a row of a stage takes
+  extern __shared__ __align__(16) unsigned char gf_raw[];
+  float* ws = reinterpret_cast<float*>(gf_raw);                   // [NS][BN][WS]
+  TX* xs = reinterpret_cast<TX*>(gf_raw + sizeof(float) * NS * BN * WS);      // [NS][BM][XS]
+  const int tid = threadIdx.x, tx = tid % CN, ty = tid / CN;
+  const int m0 = blockIdx.y * BM, n0 = blockIdx.x * BN;
+  auto load = [&](int stage, int k0) {
+    float* wd = ws + stage * BN * WS;
+    TX* xd = xs + stage * BM * XS;
+    if constexpr (VEC) {      // K, the strides and the bases are multiples of four values: a piece lies inside a row or outside
+      for (int e = tid; e < BN * (BK / 4); e += THREADS) {
+        const int r = e / (BK / 4), c = e % (BK / 4) * 4;
+        const bool in = n0 + r < N && k0 + c < K;
+        cp_async_16(wd + r * WS + c, in ? w + (size_t)(n0 + r) * K + k0 + c : w, in ? 16 : 0);
+      }
+      for (int e = tid; e < BM * (BK / 4); e += THREADS) {
+        const int r = e / (BK / 4), c = e % (BK / 4) * 4;
+        const bool in = m0 + r < M && k0 + c < K;
+        const TX* src = in ? x + (size_t)(m0 + r) * x_stride + k0 + c : x;
+        if constexpr (sizeof(TX) == 4) cp_async_16(xd + r * XS + c, src, in ? 16 : 0);
+        else cp_async_8(xd + r * XS + c, src, in ? 8 : 0);
+      }
+    } else {
+      for (int e = tid; e < BN * BK; e += THREADS) {
+        const int r = e / BK, c = e % BK;
+        wd[r * WS + c] = (n0 + r < N && k0 + c < K) ? w[(size_t)(n0 + r) * K + k0 + c] : 0.f;
+      }
+      for (int e = tid; e < BM * BK; e += THREADS) {
+        const int r = e / BK, c = e % BK;
+        xd[r * XS + c] = (m0 + r < M && k0 + c < K) ? x[(size_t)(m0 + r) * x_stride + k0 + c] : TX(0.f);
+      }
     }
-    __syncthreads();
+    cp_async_commit();
+  };
+  float acc[TM][TN];
 #pragma unroll
-    for (int kk = 0; kk < GF_BK; ++kk) {
-      float a[4], b[4];
+  for (int i = 0; i < TM; ++i)
 #pragma unroll
-      for (int i = 0; i < 4; ++i) a[i] = As[kk][tr * 4 + i];
+    for (int j = 0; j < TN; ++j) acc[i][j] = 0.f;
+  const int steps = (K + BK - 1) / BK;
 #pragma unroll
-      for (int j = 0; j < 4; ++j) b[j] = Bs[kk][tc * 4 + j];
+  for (int s = 0; s < NS - 1; ++s) {
+    if (s < steps) load(s, s * BK);
+    else cp_async_commit();
+  }
+  for (int it = 0; it < steps; ++it) {
+    cp_async_wait<NS - 2>();
+    __syncthreads();      // stage `it` is there for everyone, and everyone is done with the stage that is filled next
+    if (it + NS - 1 < steps) load((it + NS - 1) % NS, (it + NS - 1) * BK);
+    else cp_async_commit();
+    const float* wr = ws + (it % NS) * BN * WS;
+    const TX* xr = xs + (it % NS) * BM * XS;
+    // The next U pieces are read while the present ones are added: a warp alone on its scheduler would otherwise wait
+    // for shared memory in every step of its chains.
+    float4 av[2][U][TM], bv[2][U][TN];
+    auto fetch = [&](int buf, int k0) {
 #pragma unroll
-      for (int i = 0; i < 4; ++i)
+      for (int u = 0; u < U; ++u) {
 #pragma unroll
-        for (int j = 0; j < 4; ++j) acc[i][j] = fmaf(a[i], b[j], acc[i][j]);
+        for (int i = 0; i < TM; ++i) {
+          const TX* p = xr + (ty + i * RM) * XS + k0 + 4 * u;
+          if constexpr (sizeof(TX) == 4) {
+            av[buf][u][i] = *reinterpret_cast<const float4*>(p);
+          } else {
+            const float2 lo = __bfloat1622float2(*reinterpret_cast<const __nv_bfloat162*>(p));
+            const float2 hi = __bfloat1622float2(*reinterpret_cast<const __nv_bfloat162*>(p + 2));
+            av[buf][u][i] = make_float4(lo.x, lo.y, hi.x, hi.y);
+          }
+        }
+#pragma unroll
+        for (int j = 0; j < TN; ++j)
+          bv[buf][u][j] = *reinterpret_cast<const float4*>(wr + (tx + j * CN) * WS + k0 + 4 * u);
+      }
+    };
+    fetch(0, 0);
+#pragma unroll
+    for (int k = 0; k < BK; k += 4 * U) {
+      const int cur = (k / (4 * U)) & 1;
+      if (k + 4 * U < BK) fetch(cur ^ 1, k + 4 * U);
+#pragma unroll
+      for (int u = 0; u < U; ++u)
+#pragma unroll
+        for (int i = 0; i < TM; ++i)
+#pragma unroll
+          for (int j = 0; j < TN; ++j) {
+            const float4 a = av[cur][u][i], b = bv[cur][u][j];
+            acc[i][j] = fmaf(a.w, b.w, fmaf(a.z, b.z, fmaf(a.y, b.y, fmaf(a.x, b.x, acc[i][j]))));
+          }
     }
-    __syncthreads();
   }
 #pragma unroll
-  for (int i = 0; i < 4; ++i) {
-    const int m = m0 + tr * 4 + i;
+  for (int i = 0; i < TM; ++i) {
+    const int m = m0 + ty + i * RM;
     if (m >= M) continue;
 #pragma unroll
-    for (int j = 0; j < 4; ++j) {
-      const int n = n0 + tc * 4 + j;
+    for (int j = 0; j < TN; ++j) {
+      const int n = n0 + tx + j * CN;
       if (n < N) out[(size_t)m * out_stride + n] = acc[i][j] + (bias ? bias[n] : 0.f);
     }
   }
 }
 
-LLMRS_API int llmrs_gemm_f32(const float* x, long long x_stride, const float* w, const float* bias, float* out,
-                             long long out_stride, int M, int N, int K, cudaStream_t stream) {
+template <typename TX, int BM, int BN, int TM, int TN, int BK, int NS, int U>
+static int launch_gemm_f32(bool vec, const TX* x, long long x_stride, const float* w, const float* bias, float* out,
+                           long long out_stride, int M, int N, int K, cudaStream_t stream) {
+  constexpr size_t smem = (size_t)NS * (BN * (BK + 4) * sizeof(float) + BM * (BK * sizeof(TX) + 16));
+  constexpr int threads = (BM / TM) * (BN / TN);
+  const dim3 grid((N + BN - 1) / BN, (M + BM - 1) / BM);
+  LLMRS_REQUIRE(grid.y <= 65535, "gemm_f32: M=%d is too large", M);
+  auto go = [&](auto kernel) {
+    if (smem > 48 * 1024) {
+      cudaError_t e = cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
+      if (e != cudaSuccess) return llmrs_fail("gemm_f32: shared memory %zu: %s", smem, cudaGetErrorString(e));
+    }
+    kernel<<<grid, threads, smem, stream>>>(x, w, bias, out, M, N, K, x_stride, out_stride);
+    return llmrs_launch_status("gemm_f32");
+  };
+  return vec ? go(gemm_f32_kernel<TX, BM, BN, TM, TN, BK, NS, U, true>) : go(gemm_f32_kernel<TX, BM, BN, TM, TN, BK, NS, U, false>);
+}
+
+// The largest tile of which there are enough blocks for the SMs: larger tiles read the operands less often, smaller ones
+// spread a short product over the device, and no tile has more rows than the product would half fill. Both sides of the
+// line, measured: 16 rows of 2,048 into 6,144 features 43 us in tiles of 16 x 32, 72 in tiles of 32 x 32 whose second half
+// is empty; 37 rows of 1,024 into 6,144 features 48 us in 384 tiles of 32 x 32, 80 in 96 tiles of 64 x 64 (as before).
+template <typename TX>
+static int gemm_f32_any(const TX* x, long long x_stride, const float* w, const float* bias, float* out,
+                        long long out_stride, int M, int N, int K, cudaStream_t stream) {
   LLMRS_REQUIRE(M >= 0 && N > 0 && K > 0, "gemm_f32: bad sizes M=%d N=%d K=%d", M, N, K);
   if (M == 0) return 0;
-  dim3 grid((N + GF_BN - 1) / GF_BN, (M + GF_BM - 1) / GF_BM);
-  LLMRS_REQUIRE(grid.y <= 65535, "gemm_f32: M=%d is too large", M);
-  gemm_f32_kernel<float><<<grid, GF_THREADS, 0, stream>>>(x, w, bias, out, M, N, K, x_stride, out_stride);
-  return llmrs_launch_status("gemm_f32");
+  // Pieces of four values by one asynchronous copy each: every row of both operands must start on such a piece.
+  const bool vec = K % 4 == 0 && x_stride % 4 == 0 && ((uintptr_t)w & 15) == 0 && ((uintptr_t)x & (4 * sizeof(TX) - 1)) == 0;
+  auto blocks = [&](int bm, int bn) { return (long long)((M + bm - 1) / bm) * ((N + bn - 1) / bn); };
+  constexpr int ENOUGH = 148;
+#define LLMRS_GF(BM, BN, TM, TN, BK, NS, U) \
+  return launch_gemm_f32<TX, BM, BN, TM, TN, BK, NS, U>(vec, x, x_stride, w, bias, out, out_stride, M, N, K, stream)
+  if (M > 64 && blocks(128, 128) >= ENOUGH) LLMRS_GF(128, 128, 8, 8, 16, 4, 1);
+  if (M > 32 && blocks(64, 64) >= ENOUGH) LLMRS_GF(64, 64, 4, 8, 32, 4, 1);
+  if (M > 16 && blocks(32, 32) >= ENOUGH) LLMRS_GF(32, 32, 2, 4, 32, 4, 1);
+  if (M > 8 && blocks(16, 32) >= ENOUGH) LLMRS_GF(16, 32, 2, 2, 64, 4, 2);
+  if (M > 4 && blocks(8, 32) >= ENOUGH) LLMRS_GF(8, 32, 2, 1, 64, 4, 4);
+  if (M > 4) LLMRS_GF(8, 16, 1, 1, 64, 4, 4);
+  if (blocks(4, 32) >= 2 * ENOUGH) LLMRS_GF(4, 32, 1, 1, 64, 4, 4);
+  LLMRS_GF(4, 8, 1, 1, 128, 4, 4);
+#undef LLMRS_GF
+}
+
+LLMRS_API int llmrs_gemm_f32(const float* x, long long x_stride, const float* w, const float* bias, float* out,
+                             long long out_stride, int M, int N, int K, cudaStream_t stream) {
+  return gemm_f32_any<float>(x, x_stride, w, bias, out, out_stride, M, N, K, stream);
 }
 
 // The same product for rows stored in bfloat16 (activations of the bfloat16 path whose product must not be rounded:
@@ -76,13 +177,7 @@ LLMRS_API int llmrs_gemm_f32(const float* x, long long x_stride, const float* w,
 // are float32.
 LLMRS_API int llmrs_gemm_f32_bf16_rows(const void* x, long long x_stride, const float* w, const float* bias, float* out,
                                        long long out_stride, int M, int N, int K, cudaStream_t stream) {
-  LLMRS_REQUIRE(M >= 0 && N > 0 && K > 0, "gemm_f32: bad sizes M=%d N=%d K=%d", M, N, K);
-  if (M == 0) return 0;
-  dim3 grid((N + GF_BN - 1) / GF_BN, (M + GF_BM - 1) / GF_BM);
-  LLMRS_REQUIRE(grid.y <= 65535, "gemm_f32: M=%d is too large", M);
-  gemm_f32_kernel<__nv_bfloat16><<<grid, GF_THREADS, 0, stream>>>((const __nv_bfloat16*)x, w, bias, out, M, N, K,
-                                                                  x_stride, out_stride);
-  return llmrs_launch_status("gemm_f32 (bfloat16 rows)");
+  return gemm_f32_any<__nv_bfloat16>((const __nv_bfloat16*)x, x_stride, w, bias, out, out_stride, M, N, K, stream);
 }
 
 // ---------------------------------------------------------------------------------

@@ -94,6 +94,24 @@ def test_gemm_f32_is_true_float32(M, N, K):
         assert torch.equal(ops.gemm_f32(x[3:4].contiguous(), w, b)[0], got[3])
 
 
+@pytest.mark.parametrize("rows_dtype", [torch.float32, torch.bfloat16])
+@pytest.mark.parametrize("N,K,pad", [(300, 128, 0), (300, 132, 8), (1184, 68, 0), (1200, 100, 4), (4800, 36, 0), (301, 67, 1),
+                                     (2368, 260, 3)])
+def test_gemm_f32_tiles(N, K, pad, rows_dtype):
+    """Every tile of the float32 product at its edges (rows, features and K that fill no tile, rows with a stride, rows
+    that no sixteen-byte copy can take), against float64, and every row's bits the same in every batch. An output is one
+    chain of K fused multiply-adds: its error is at most K half ulps of the sum of the products' magnitudes."""
+    ops = _ops()
+    torch.manual_seed(N + K)
+    x = torch.randn(700, K + pad, device=DEV).to(rows_dtype)[:, :K]
+    w, b = torch.randn(N, K, device=DEV), torch.randn(N, device=DEV)
+    whole = ops.gemm_f32(x, w, b)
+    bound = ((x.double().abs() @ w.double().abs().t() + b.double().abs()) * (K + 1) * 2.0 ** -24)
+    assert bool(((whole.double() - (x.double() @ w.double().t() + b.double())).abs() <= bound).all())
+    for M in (1, 3, 4, 5, 8, 9, 16, 17, 31, 33, 64, 65, 129):
+        assert torch.equal(ops.gemm_f32(x[:M], w, b), whole[:M]), M
+
+
 # -- norm + rotation + cache write ---------------------------------------------------------
 def _paged_setup(lens, new, n_kv, d, page, dtype, seed=0):
     """Random cache with scattered pages; returns tensors for kernels and dense copies for the reference."""
