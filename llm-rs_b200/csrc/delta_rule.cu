@@ -11,6 +11,8 @@
 // Two kernels and a small third:
 //   prepare     a warp per (token, head), all tokens at once: decay, removal rate times unit key, unit key, and r, k, v
 //               widened, as six float32 rows [tokens, heads * d];
+//   (portions of eight tokens and more take `turns` and the walk in turns of four tokens instead of these two: state_walk.cuh;
+//   2,048 tokens of 32 heads of 64 x 64: 816 us walked one by one, 246 in turns; their rows 56 us where `prepare` takes 38)
 //   recurrence  one block per (request, head, slice of 16 value columns) walks the request's tokens of the step in
 //               order: a column of S depends on no other column, so the slices run side by side. Four adjacent lanes
 //               share a column, each keeping a quarter of its key channels in registers; u^T S and S^T r are summed
@@ -21,6 +23,7 @@
 //   output      a warp per (token, head): divides by the head's root mean square, applies the weight and the gate.
 #include "common.cuh"
 #include "mma_util.cuh"
+#include "state_walk.cuh"
 
 __device__ __forceinline__ float sigmoidf_(float x) { return 1.0f / (1.0f + expf(-x)); }
 
@@ -53,6 +56,120 @@ __global__ void delta_prepare_kernel(const TA* __restrict__ r, const TA* __restr
     prep[DR_K * plane + out0 + i] = kv;
     prep[DR_R * plane + out0 + i] = to_float(r[in0 + i]);
     prep[DR_V * plane + out0 + i] = to_float(v[in0 + i]);
+  }
+}
+
+// What the walk in turns of four tokens reads (state_walk.cuh), a warp per (turn, head): r and u decayed from the turn's start
+// (r with the token's own decay, u without: it meets the state before the token), k and the removal -a u decayed from the
+// token to the turn's end, the whole turn's decay, v widened, and the coefficients between the turn's tokens. rows: r, u, k,
+// -a u and v, each [tokens, heads * d]. vec, vec_f: the inputs' and the float32 rows' pieces of four (two with CPL 2) channels
+// start on their own boundaries.
+template <typename TA, int CPL>
+__global__ void __launch_bounds__(128)
+delta_turns_kernel(const TA* __restrict__ r, const TA* __restrict__ k, const TA* __restrict__ v, const TA* __restrict__ a_raw,
+                   long long in_stride, const float* __restrict__ decay_raw, const float* __restrict__ decay_bias,
+                   const float* __restrict__ a_bias, const int* __restrict__ q_start, const int* __restrict__ n_new,
+                   float* __restrict__ rows, float* __restrict__ w, float* __restrict__ tables, int n_tokens, int n_requests,
+                   int n_heads, int d, float decay_scale, float key_eps, bool vec, bool vec_f) {
+  const int place = blockIdx.x, h = blockIdx.y * 4 + (threadIdx.x >> 5), lane = threadIdx.x & 31;
+  if (h >= n_heads) return;
+  const int req = walk_request(q_start, n_requests, place), t_req = q_start[req];
+  const int first = (place - walk_place(t_req, req)) * WALK_TURN, have = min(WALK_TURN, n_new[req] - first);
+  if (first < 0 || have <= 0) return;
+  const size_t t0 = (size_t)(t_req + first), width = (size_t)n_heads * d, plane = (size_t)n_tokens * width;
+  float rv[4][CPL], kv[4][CPL], au[4][CPL], dec[4][CPL], bias_d[CPL], bias_a[CPL];
+  walk_load<CPL>(decay_bias + (size_t)h * d, lane, d, true, false, bias_d);
+  walk_load<CPL>(a_bias + (size_t)h * d, lane, d, true, false, bias_a);
+#pragma unroll
+  for (int t = 0; t < 4; ++t) {
+    const size_t in = (t0 + t) * in_stride + (size_t)h * d, at = (t0 + t) * width + (size_t)h * d;
+    walk_load<CPL>(k + in, lane, d, t < have, vec, kv[t]);
+    walk_load<CPL>(r + in, lane, d, t < have, vec, rv[t]);
+    walk_load<CPL>(a_raw + in, lane, d, t < have, vec, au[t]);
+    walk_load<CPL>(decay_raw + at, lane, d, t < have, vec_f, dec[t]);
+    float value[CPL];
+    walk_load<CPL>(v + in, lane, d, t < have, vec, value);
+    if (t < have) walk_store<CPL>(rows + 4 * plane + at, lane, d, vec_f, value);
+  }
+  float u[4][CPL];
+#pragma unroll
+  for (int t = 0; t < 4; ++t) {
+    float ss = 0.f;
+#pragma unroll
+    for (int m = 0; m < CPL; ++m) ss = fmaf(kv[t][m], kv[t][m], ss);
+    const float inv = 1.0f / sqrtf(warp_sum(ss) + key_eps);
+#pragma unroll
+    for (int m = 0; m < CPL; ++m) {
+      u[t][m] = kv[t][m] * inv;
+      au[t][m] = -sigmoidf_(au[t][m] + bias_a[m]) * u[t][m];
+      dec[t][m] = t < have ? expf(-decay_scale * sigmoidf_(dec[t][m] + bias_d[m])) : 1.f;
+    }
+  }
+  // A (u_i . a_j) at 0, B (u_i . k_j) at 6, for j < i at i (i - 1) / 2 + j; R (r_i . k_j) at 12, Q (r_i . a_j) at 22, for
+  // j <= i at i (i + 1) / 2 + j: 32 sums, a lane each.
+  float sums[32];
+#pragma unroll
+  for (int e = 0; e < 32; ++e) sums[e] = 0.f;
+#pragma unroll
+  for (int m = 0; m < CPL; ++m)
+#pragma unroll
+    for (int j = 0; j < 4; ++j) {
+      float kj = kv[j][m], aj = au[j][m];      // what token j wrote, decayed up to and with token t below
+      sums[12 + j * (j + 1) / 2 + j] = fmaf(rv[j][m], kj, sums[12 + j * (j + 1) / 2 + j]);
+      sums[22 + j * (j + 1) / 2 + j] = fmaf(rv[j][m], aj, sums[22 + j * (j + 1) / 2 + j]);
+#pragma unroll
+      for (int t = j + 1; t < 4; ++t) {
+        const int e = t * (t - 1) / 2 + j, f = t * (t + 1) / 2 + j;
+        sums[e] = fmaf(u[t][m], aj, sums[e]);
+        sums[6 + e] = fmaf(u[t][m], kj, sums[6 + e]);
+        kj *= dec[t][m];
+        aj *= dec[t][m];
+        sums[12 + f] = fmaf(rv[t][m], kj, sums[12 + f]);
+        sums[22 + f] = fmaf(rv[t][m], aj, sums[22 + f]);
+      }
+    }
+  float up[CPL], down[CPL], row[CPL];
+#pragma unroll
+  for (int m = 0; m < CPL; ++m) up[m] = down[m] = 1.f;
+#pragma unroll
+  for (int t = 0; t < 4; ++t) {
+    const int e = 3 - t;
+    if (t < have) {
+      const size_t at = (t0 + t) * width + (size_t)h * d;
+#pragma unroll
+      for (int m = 0; m < CPL; ++m) row[m] = u[t][m] * up[m];
+      walk_store<CPL>(rows + plane + at, lane, d, vec_f, row);
+#pragma unroll
+      for (int m = 0; m < CPL; ++m) row[m] = rv[t][m] * (up[m] * dec[t][m]);
+      walk_store<CPL>(rows + at, lane, d, vec_f, row);
+    }
+    if (e < have) {
+      const size_t at = (t0 + e) * width + (size_t)h * d;
+#pragma unroll
+      for (int m = 0; m < CPL; ++m) row[m] = kv[e][m] * down[m];
+      walk_store<CPL>(rows + 2 * plane + at, lane, d, vec_f, row);
+#pragma unroll
+      for (int m = 0; m < CPL; ++m) row[m] = au[e][m] * down[m];
+      walk_store<CPL>(rows + 3 * plane + at, lane, d, vec_f, row);
+    }
+#pragma unroll
+    for (int m = 0; m < CPL; ++m) {
+      up[m] *= dec[t][m];
+      down[m] *= dec[e][m];
+    }
+  }
+  walk_store<CPL>(w + ((size_t)place * n_heads + h) * d, lane, d, vec_f, up);
+  float* to = tables + ((size_t)place * n_heads + h) * 48;
+  const float sum = walk_sum_all<32>(sums, lane);
+  if (lane < 12) {
+    to[lane < 6 ? WALK_GA + lane : WALK_GB + lane - 6] = sum;
+  } else {
+    const int f = lane < 22 ? lane - 12 : lane - 22, i = f < 1 ? 0 : (f < 3 ? 1 : (f < 6 ? 2 : 3));
+    to[(lane < 22 ? WALK_GR : WALK_GQ) + 4 * i + f - i * (i + 1) / 2] = sum;
+  }
+  if (lane < 12) {      // above the diagonals
+    const int e = lane % 6;
+    to[(lane < 6 ? WALK_GR : WALK_GQ) + (e < 3 ? 1 + e : (e < 5 ? 3 + e : 11))] = 0.f;
   }
 }
 
@@ -181,10 +298,44 @@ static int launch_delta(int dmax, dim3 grid, cudaStream_t stream, const void* r,
                         const void* gate, const void* a_raw, long long in_stride, const float* decay_raw,
                         const float* decay_bias, const float* a_bias, const float* norm_w, float* state,
                         const int* q_start, const int* n_new, const int* slot_ids, float* work, void* out,
-                        int n_tokens, int n_heads, int d, float decay_scale, float key_eps, float norm_eps) {
+                        int n_tokens, int n_requests, int n_heads, int d, float decay_scale, float key_eps,
+                        float norm_eps) {
   const int rows = n_tokens * n_heads;
   float* prep = work;
   float* o_raw = work + (size_t)DR_ROWS * rows * d;
+  if (n_tokens - n_requests + 1 >= WALK_MIN_PORTION) {      // some request may bring a portion
+    auto up4 = [](size_t v) { return (v + 3) & ~(size_t)3; };
+    const size_t places = (size_t)walk_places(n_tokens, n_requests), plane = (size_t)rows * d;
+    float* w = work + up4((size_t)(DR_ROWS + 1) * rows * d);
+    float* tables = w + up4(places * n_heads * d);
+    const dim3 grid_t((unsigned)places, (n_heads + 3) / 4);
+    const int piece = d <= 64 ? 2 : 4;
+    auto starts = [&](const void* p, size_t size) { return ((uintptr_t)p & (piece * size - 1)) == 0; };
+    const bool vec_f = d % piece == 0 && starts(decay_raw, 4);
+    const bool vec = d % piece == 0 && in_stride % piece == 0 && starts(r, sizeof(TA)) && starts(k, sizeof(TA)) &&
+                     starts(v, sizeof(TA)) && starts(a_raw, sizeof(TA));
+#define LLMRS_DR_TURNS(CPL)                                                                                               \
+  delta_turns_kernel<TA, CPL><<<grid_t, 128, 0, stream>>>((const TA*)r, (const TA*)k, (const TA*)v, (const TA*)a_raw, in_stride, \
+                                                          decay_raw, decay_bias, a_bias, q_start, n_new, prep, w, tables, \
+                                                          n_tokens, n_requests, n_heads, d, decay_scale, key_eps, vec, vec_f)
+    if (d <= 64) LLMRS_DR_TURNS(2);
+    else if (d <= 128) LLMRS_DR_TURNS(4);
+    else LLMRS_DR_TURNS(8);
+#undef LLMRS_DR_TURNS
+    int rc = llmrs_launch_status("delta_rule (turns)");
+    if (rc != 0) return rc;
+    WalkArgs a = {};
+    a.q = prep; a.k = prep + plane; a.kb = prep + 2 * plane; a.ab = prep + 3 * plane; a.v = prep + 4 * plane; a.w = w;
+    a.q_stride = a.k_stride = a.b_stride = (long long)n_heads * d;
+    a.tables = tables; a.state = state; a.o_raw = o_raw;
+    a.q_start = q_start; a.n_new = n_new; a.slot_ids = slot_ids;
+    a.n_heads = a.n_groups = n_heads; a.d = a.dv = d;
+    rc = launch_state_walk<WALK_GENERAL>(a, n_requests, d, stream);
+    if (rc != 0) return rc;
+    delta_out_kernel<TA><<<(rows + 3) / 4, 128, 0, stream>>>(o_raw, (const TA*)gate, in_stride, norm_w, (TA*)out, rows,
+                                                             n_heads, d, norm_eps);
+    return llmrs_launch_status("delta_rule (norm and gate)");
+  }
   delta_prepare_kernel<TA><<<(rows + 3) / 4, 128, 0, stream>>>((const TA*)r, (const TA*)k, (const TA*)v,
                                                                (const TA*)a_raw, in_stride, decay_raw, decay_bias,
                                                                a_bias, prep, n_tokens, n_heads, d, decay_scale, key_eps);
@@ -202,8 +353,9 @@ static int launch_delta(int dmax, dim3 grid, cudaStream_t stream, const void* r,
 }
 
 // Float32 workspace the three kernels share, in floats.
-LLMRS_API long long llmrs_delta_rule_work_floats(int n_tokens, int n_heads, int d) {
-  return (long long)(DR_ROWS + 1) * n_tokens * n_heads * d;
+LLMRS_API long long llmrs_delta_rule_work_floats(int n_tokens, int n_requests, int n_heads, int d) {
+  return (long long)(DR_ROWS + 1) * n_tokens * n_heads * d + 16 +
+         walk_places(n_tokens, n_requests) * n_heads * (d + walk_table(WALK_GENERAL));
 }
 
 // r, k, v, gate, a_raw: [tokens, ...] of the activation type, rows `in_stride` elements apart, each pointing at its
@@ -224,11 +376,11 @@ LLMRS_API int llmrs_delta_rule(const void* r, const void* k, const void* v, cons
   dim3 grid(n_requests, n_heads, (d + DR_COLS - 1) / DR_COLS);
   if (dtype == LLMRS_F32)
     return launch_delta<float>(dmax, grid, stream, r, k, v, gate, a_raw, in_stride, decay_raw, decay_bias, a_bias,
-                               norm_w, state, q_start, n_new, slot_ids, work, out, n_tokens, n_heads, d, decay_scale,
-                               key_eps, norm_eps);
+                               norm_w, state, q_start, n_new, slot_ids, work, out, n_tokens, n_requests, n_heads, d,
+                               decay_scale, key_eps, norm_eps);
   if (dtype == LLMRS_BF16)
     return launch_delta<__nv_bfloat16>(dmax, grid, stream, r, k, v, gate, a_raw, in_stride, decay_raw, decay_bias,
-                                       a_bias, norm_w, state, q_start, n_new, slot_ids, work, out, n_tokens, n_heads,
-                                       d, decay_scale, key_eps, norm_eps);
+                                       a_bias, norm_w, state, q_start, n_new, slot_ids, work, out, n_tokens, n_requests,
+                                       n_heads, d, decay_scale, key_eps, norm_eps);
   return llmrs_fail("delta_rule: unknown dtype %d", dtype);
 }

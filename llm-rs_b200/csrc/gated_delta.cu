@@ -18,14 +18,16 @@
 //
 //   prepare      a block per token: convolutions + SiLU, unit q and k, g and beta, as float32 rows
 //   conv state   a block per request, after prepare: the request's last K - 1 convolution inputs
-//   recurrence   a block per (request, head, slice of 16 value columns) walks the request's tokens in order; four
+//   recurrence   of portions of eight tokens and more: the coefficients of turns of four tokens, then the walk in turns
+//                (state_walk.cuh). Of single tokens and shorter portions: a block per (request, head, slice of 16 value
+//                columns) walks the request's tokens one by one; four
 //                neighbouring lanes share a column, each with a quarter of the key channels in registers (lane p of the
 //                four holds channels 4 (p + 4 j) .. 4 (p + 4 j) + 3, so that the four read neighbouring 16-byte pieces
 //                of a row in shared memory, not pieces a bank's stride apart); k^T S and q^T S are summed over the four
 //                by two shuffles. Rows come in chunks through two shared-memory buffers.
 //   output       a warp per (token, head): norm, weight, gate
 //
-// Long portions take the recurrence in CHUNKS of 32 tokens instead (the same numbers up to float32 rounding, all of it
+// Long portions may take the recurrence in CHUNKS of 32 tokens instead (the same numbers up to float32 rounding, all of it
 // float32 FMA). Within a chunk that starts from the state S_0, with L_t the sum of log g up to and including token t:
 //
 //   u_t = beta_t (v_t - e^{L_t} S_0^T k_t - sum_{s<t} A[t,s] u_s),     A[t,s] = e^{L_t - L_s} (k_t . k_s)
@@ -38,10 +40,11 @@
 // products per chunk over rows that arrive through two shared-memory buffers, 32 tokens per sequential step instead of
 // one. A chunk's missing tokens (a portion's end) count as k = q = v = 0, beta = 0, g = 1 and change nothing.
 // The chunked form is OFF by default (llmrs_gated_delta_chunked): its products read every operand from shared memory
-// and are bound by that, so it does not beat the walk yet.
+// and are bound by that (2,048 tokens of 16 heads of 128 x 128: some 500 us, the walk in turns 265).
 #include "common.cuh"
 #include "mma_util.cuh"
 #include "short_conv.cuh"
+#include "state_walk.cuh"
 
 // CHANNEL: a decay per key channel; ba is then unused, b (activation type) and araw (float32 [tokens, H d]) take its place
 // and pg is [tokens, H d].
@@ -91,9 +94,9 @@ constexpr int GD_COLS = 16;      // value columns of a block
 #ifndef LLMRS_GD_LANES
 #define LLMRS_GD_LANES 8
 #endif
-// With a decay per key channel a lane reads three rows a token, not two: sixteen lanes a column shorten that where a
-// step's blocks do not fill the device twice (2,048 tokens of 16 heads of 128 x 128: 813 against 896 us for the whole
-// op), eight are ahead where they do.
+// (The kernel for single tokens and portions of fewer than eight.) With a decay per key channel a lane reads three rows a
+// token, not two: sixteen lanes a column shorten that where a step's blocks do not fill the device twice (walking 2,048 tokens
+// of 16 heads of 128 x 128: 813 against 896 us for the whole op), eight are ahead where they do.
 constexpr int GD_WIDE_MAX_BLOCKS = 296;
 
 // LANES: neighbouring lanes that share a column (4, 8 or 16; at most DMAX / 4, so that a lane holds whole pieces of
@@ -228,6 +231,94 @@ gdr_recurrence_kernel(const float* __restrict__ pq, const float* __restrict__ pk
   }
 }
 
+
+// ---- the walk in turns of four tokens (state_walk.cuh) ---------------------------------------------------------------
+// What it reads with a decay per key channel: a warp per (turn, value head) leaves the rows with their decays (qf, kf from the
+// turn's start up to and with the token, kb from the token to the turn's end), the whole turn's decay and the coefficients
+// between the turn's tokens. Products of decays, no quotients: nothing overflows.
+template <int CPL>
+__global__ void __launch_bounds__(128)
+gdr_channel_turns_kernel(const float* __restrict__ pq, const float* __restrict__ pk, const float* __restrict__ pg,
+                         const float* __restrict__ pbeta, const int* __restrict__ q_start, const int* __restrict__ n_new,
+                         float* __restrict__ qf, float* __restrict__ kf, float* __restrict__ kb, float* __restrict__ w,
+                         float* __restrict__ tables, int n_requests, int G, int H, int d) {
+  const int place = blockIdx.x, head = blockIdx.y * 4 + (threadIdx.x >> 5), lane = threadIdx.x & 31;
+  if (head >= H) return;
+  const int req = walk_request(q_start, n_requests, place), t_req = q_start[req];
+  const int first = (place - walk_place(t_req, req)) * WALK_TURN, have = min(WALK_TURN, n_new[req] - first);
+  if (first < 0 || have <= 0) return;
+  const size_t t0 = (size_t)(t_req + first);
+  const int kh = head / (H / G);
+  const bool vec = d % 4 == 0;
+  float q[4][CPL], k[4][CPL], g[4][CPL], sums[16];
+#pragma unroll
+  for (int t = 0; t < 4; ++t) {
+    walk_load<CPL>(pq + ((t0 + t) * G + kh) * d, lane, d, t < have, vec, q[t]);
+    walk_load<CPL>(pk + ((t0 + t) * G + kh) * d, lane, d, t < have, vec, k[t]);
+    walk_load<CPL>(pg + ((t0 + t) * H + head) * d, lane, d, t < have, vec, g[t]);
+    if (t >= have)
+#pragma unroll
+      for (int m = 0; m < CPL; ++m) g[t][m] = 1.f;
+  }
+  // q_i . k_j (j <= i) at i (i + 1) / 2 + j, k_i . k_j (j < i) at 10 + i (i - 1) / 2 + j, the decays after j up to and
+  // with i between them.
+#pragma unroll
+  for (int e = 0; e < 16; ++e) sums[e] = 0.f;
+#pragma unroll
+  for (int m = 0; m < CPL; ++m)
+#pragma unroll
+    for (int j = 0; j < 4; ++j) {
+      float kj = k[j][m];
+      sums[j * (j + 1) / 2 + j] = fmaf(q[j][m], kj, sums[j * (j + 1) / 2 + j]);
+#pragma unroll
+      for (int i = j + 1; i < 4; ++i) {
+        kj *= g[i][m];
+        sums[i * (i + 1) / 2 + j] = fmaf(q[i][m], kj, sums[i * (i + 1) / 2 + j]);
+        sums[10 + i * (i - 1) / 2 + j] = fmaf(k[i][m], kj, sums[10 + i * (i - 1) / 2 + j]);
+      }
+    }
+  float up[CPL], down[CPL], row[CPL];
+#pragma unroll
+  for (int m = 0; m < CPL; ++m) up[m] = down[m] = 1.f;
+#pragma unroll
+  for (int t = 0; t < 4; ++t) {
+    const int e = 3 - t;
+#pragma unroll
+    for (int m = 0; m < CPL; ++m) up[m] *= g[t][m];
+    if (t < have) {
+      const size_t at = ((t0 + t) * H + head) * d;
+#pragma unroll
+      for (int m = 0; m < CPL; ++m) row[m] = q[t][m] * up[m];
+      walk_store<CPL>(qf + at, lane, d, vec, row);
+#pragma unroll
+      for (int m = 0; m < CPL; ++m) row[m] = k[t][m] * up[m];
+      walk_store<CPL>(kf + at, lane, d, vec, row);
+    }
+    if (e < have) {
+#pragma unroll
+      for (int m = 0; m < CPL; ++m) row[m] = k[e][m] * down[m];
+      walk_store<CPL>(kb + ((t0 + e) * H + head) * d, lane, d, vec, row);
+    }
+#pragma unroll
+    for (int m = 0; m < CPL; ++m) down[m] *= g[e][m];
+  }
+  walk_store<CPL>(w + ((size_t)place * H + head) * d, lane, d, vec, up);
+  float* to = tables + ((size_t)place * H + head) * 36;
+  const float sum = walk_sum_all<16>(sums, lane);
+  if (lane < 10) {      // row i of the lower triangle begins at 0, 1, 3, 6
+    const int i = lane < 1 ? 0 : (lane < 3 ? 1 : (lane < 6 ? 2 : 3));
+    to[WALK_Q + 4 * i + lane - i * (i + 1) / 2] = sum;
+  } else if (lane < 16) {
+    to[WALK_K + lane - 10] = sum;
+  } else if (lane < 18) {
+    *reinterpret_cast<float4*>(to + (lane == 16 ? WALK_P : WALK_Z)) = make_float4(1.f, 1.f, 1.f, 1.f);
+  } else if (lane < 22) {
+    to[WALK_BETA + lane - 18] = lane - 18 < have ? pbeta[(t0 + lane - 18) * H + head] : 0.f;
+  } else if (lane < 28) {
+    const int e = lane - 22;
+    to[WALK_Q + (e < 3 ? 1 + e : (e < 5 ? 3 + e : 11))] = 0.f;
+  }
+}
 
 // ---- the recurrence in chunks ------------------------------------------------------------------------------------
 constexpr int GC_C = 32, GC_W = 16, GC_THREADS = 128, GC_TST = GC_C + 4;
@@ -506,11 +597,46 @@ static int launch_chunked(const float* pq, const float* pk, const float* pv, con
   return llmrs_launch_status("gated_delta (chunked recurrence)");
 }
 
+static int launch_turns(bool channel, const float* pq, const float* pk, const float* pv, const float* pbeta, const float* pg,
+                        float* qf, float* kf, float* kb, float* w, float* tables, float* state, const int* q_start,
+                        const int* n_new, const int* slot_ids, float* o_raw, int n_tokens, int n_requests, int G, int H, int d,
+                        int dv, cudaStream_t stream) {
+  WalkArgs a = {};
+  a.v = pv; a.tables = tables; a.state = state; a.o_raw = o_raw;
+  a.q_start = q_start; a.n_new = n_new; a.slot_ids = slot_ids;
+  a.n_heads = H; a.d = d; a.dv = dv;
+  if (channel) {
+    const dim3 grid((unsigned)walk_places(n_tokens, n_requests), (H + 3) / 4);
+    if (d <= 128)
+      gdr_channel_turns_kernel<4><<<grid, 128, 0, stream>>>(pq, pk, pg, pbeta, q_start, n_new, qf, kf, kb, w, tables,
+                                                            n_requests, G, H, d);
+    else
+      gdr_channel_turns_kernel<8><<<grid, 128, 0, stream>>>(pq, pk, pg, pbeta, q_start, n_new, qf, kf, kb, w, tables,
+                                                            n_requests, G, H, d);
+    int rc = llmrs_launch_status("gated_delta (turns)");
+    if (rc != 0) return rc;
+    a.q = qf; a.k = kf; a.kb = kb; a.w = w;
+    a.q_stride = a.k_stride = a.b_stride = (long long)H * d;
+    a.n_groups = H;
+    return launch_state_walk<WALK_CHANNEL>(a, n_requests, dv, stream);
+  }
+  int rc = launch_walk_tables<WALK_GATED>(pq, pk, (long long)G * d, pg, nullptr, pbeta, q_start, n_new, tables, n_tokens,
+                                          n_requests, H, G, d, stream);
+  if (rc != 0) return rc;
+  a.q = pq; a.k = pk;
+  a.q_stride = a.k_stride = (long long)G * d;
+  a.n_groups = G;
+  return launch_state_walk<WALK_GATED>(a, n_requests, dv, stream);
+}
+
 // Float32 workspace of the kernels, in floats: prepared q, k, v, beta, g and the raw read-outs.
 LLMRS_API long long llmrs_gated_delta_work_floats(int n_tokens, int n_requests, int G, int H, int d, int dv, int channel) {
-  if (channel) return (long long)n_tokens * (2LL * G * d + 2LL * H * dv + (long long)H * d + H) + 24;
+  const long long turns = walk_places(n_tokens, n_requests) * H;      // the walk in turns: coefficients, decays
+  if (channel)
+    return (long long)n_tokens * (2LL * G * d + 2LL * H * dv + 4LL * H * d + H) + 48 + turns * (d + walk_table(WALK_CHANNEL));
   const long long chunk_places = n_tokens / GC_C + n_requests + 1;
-  return (long long)n_tokens * (2LL * G * d + 2LL * H * dv + 3LL * H) + 24 + chunk_places * H * GC_TABLE;
+  const long long chunks = chunk_places * H * GC_TABLE, tables = turns * walk_table(WALK_GATED);
+  return (long long)n_tokens * (2LL * G * d + 2LL * H * dv + 3LL * H) + 24 + (chunks > tables ? chunks : tables);
 }
 
 static int g_gd_chunked = 0;
@@ -554,6 +680,11 @@ LLMRS_API int llmrs_gated_delta(const void* x, long long x_stride, const void* g
   const bool chunked = g_gd_chunked && !channel && n_tokens - n_requests + 1 >= 2 * GC_C && d % 4 == 0 && dv % 4 == 0 &&
                        (size_t)gc_smem_floats(d) * sizeof(float) <= 200 * 1024;
   const int max_chunks = (n_tokens - n_requests + 1 + GC_C - 1) / GC_C;
+  const bool turns = !chunked && n_tokens - n_requests + 1 >= WALK_MIN_PORTION;      // some request may bring a portion
+  // The walk's rows with a decay per key channel follow o_raw; its tables lie where the chunked form's would.
+  const size_t hd = up4((size_t)n_tokens * H * d);
+  float *qf = tables, *kf = qf + hd, *kb = kf + hd, *turn_w = kb + hd;
+  if (channel) tables = turn_w + up4((size_t)walk_places(n_tokens, n_requests) * H * d);
   const size_t smem = (size_t)C * sizeof(float);
   const int dmax = d <= 32 ? 32 : (d <= 64 ? 64 : (d <= 128 ? 128 : 256));
   dim3 grid(n_requests, H, (dv + GD_COLS - 1) / GD_COLS);
@@ -592,6 +723,10 @@ LLMRS_API int llmrs_gated_delta(const void* x, long long x_stride, const void* g
     if (chunked) {                                                                                                     \
       rc = launch_chunked(pq, pk, pv, pbeta, plg, tables, state, q_start, n_new, slot_ids, o_raw, n_requests,          \
                           max_chunks, G, H, d, dv, stream);                                                            \
+      if (rc != 0) return rc;                                                                                          \
+    } else if (turns) {                                                                                                \
+      rc = launch_turns(channel, pq, pk, pv, pbeta, pg, qf, kf, kb, turn_w, tables, state, q_start, n_new, slot_ids,   \
+                        o_raw, n_tokens, n_requests, G, H, d, dv, stream);                                             \
       if (rc != 0) return rc;                                                                                          \
     } else if (channel && (long long)grid.x * grid.y * grid.z <= GD_WIDE_MAX_BLOCKS) LLMRS_GD_REC_ALL(true, 16);       \
     else if (channel) LLMRS_GD_REC_ALL(true, 8);                                                                       \

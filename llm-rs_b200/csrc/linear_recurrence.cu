@@ -17,6 +17,7 @@
 //                a_t = exp(f_t + m_(t-1) - m_t), b_t = exp(i_t - m_t), floor_t = exp(-m_t); m is kept per slot;
 //   prepare      q, k, v of all tokens widened to float32 (optional SiLU, optional rotation of the first channels of every
 //                head of q and k by halves, q and k scaled, k multiplied by its gain);
+//   (portions of eight tokens and more: the coefficients of turns of four tokens, then the walk in turns, state_walk.cuh)
 //   recurrence   a block per (request, head, 16 value columns) walks the tokens in order; four or eight adjacent lanes
 //                share a column, each holding its part of the column's key channels in registers; rows arrive through two
 //                shared-memory buffers by 16-byte asynchronous copies. A step of one token and a prompt's portion
@@ -26,6 +27,7 @@
 #include "common.cuh"
 #include "mma_util.cuh"
 #include "short_conv.cuh"
+#include "state_walk.cuh"
 
 __device__ __forceinline__ float lr_logsigmoid(float x) { return fminf(x, 0.f) - log1pf(expf(-fabsf(x))); }
 
@@ -269,12 +271,12 @@ linear_recurrence_kernel(const float* __restrict__ Q, const float* __restrict__ 
 // [tokens, heads] or null (then head_decay [heads], or 1 when that is null too); v_gain [tokens, heads] or null (1)
 // multiplies the value that enters the state; skip [heads] or null (0): o += skip * value (without its gain);
 // S [slots, heads, dk, dv]; N [slots, heads, dk] or null (no normaliser: nq is not written; with one, v_gain and skip must
-// be null); o_raw float32 [tokens, heads * dv]; nq float32 [tokens, heads].
+// be null); tables: workspace of llmrs_linear_recurrence_table_floats; o_raw float32 [tokens, heads * dv]; nq float32 [tokens, heads].
 LLMRS_API int llmrs_linear_recurrence_planes(const float* Q, const float* K, const float* V, const float* decay,
                                              const float* head_decay, const float* v_gain, const float* skip, float* S,
                                              float* N, const int* q_start, const int* n_new, const int* slot_ids,
-                                             float* o_raw, float* nq, int n_tokens, int n_requests, int n_heads,
-                                             int n_groups, int dk, int dv, cudaStream_t stream) {
+                                             float* tables, float* o_raw, float* nq, int n_tokens, int n_requests,
+                                             int n_heads, int n_groups, int dk, int dv, cudaStream_t stream) {
   LLMRS_REQUIRE(n_requests >= 0 && n_tokens >= 0 && n_heads > 0 && dk > 0 && dv > 0, "linear_recurrence: bad sizes");
   LLMRS_REQUIRE(n_groups > 0 && n_heads % n_groups == 0, "linear_recurrence: %d heads are no multiple of %d groups",
                 n_heads, n_groups);
@@ -285,6 +287,20 @@ LLMRS_API int llmrs_linear_recurrence_planes(const float* Q, const float* K, con
   LLMRS_REQUIRE((((uintptr_t)Q | (uintptr_t)K) & 15) == 0, "linear_recurrence: planes must be 16-byte aligned");
   if (n_requests == 0 || n_tokens == 0) return 0;
   const int cols = dv + (N != nullptr ? 1 : 0);
+  if (n_tokens - n_requests + 1 >= WALK_MIN_PORTION) {      // some request may bring a portion
+    LLMRS_REQUIRE(((uintptr_t)tables & 15) == 0 && tables != nullptr, "linear_recurrence: no workspace for a portion");
+    LLMRS_REQUIRE(((uintptr_t)V & 15) == 0, "linear_recurrence: planes must be 16-byte aligned");
+    const long long stride = (long long)n_groups * dk;
+    int rc = launch_walk_tables<WALK_LINEAR>(Q, K, stride, decay, head_decay, v_gain, q_start, n_new, tables, n_tokens,
+                                             n_requests, n_heads, n_groups, dk, stream);
+    if (rc != 0) return rc;
+    WalkArgs a = {};
+    a.q = Q; a.k = K; a.q_stride = a.k_stride = stride; a.v = V; a.tables = tables; a.skip = skip;
+    a.state = S; a.norm_state = N; a.o_raw = o_raw; a.nq = nq;
+    a.q_start = q_start; a.n_new = n_new; a.slot_ids = slot_ids;
+    a.n_heads = n_heads; a.n_groups = n_groups; a.d = dk; a.dv = dv;
+    return launch_state_walk<WALK_LINEAR>(a, n_requests, cols, stream);
+  }
   dim3 grid(n_requests, n_heads, (cols + LR_COLS - 1) / LR_COLS);
 #define LLMRS_LR_LAUNCH(D, L)                                                                                     \
   linear_recurrence_kernel<D, L><<<grid, LR_COLS * L, 0, stream>>>(Q, K, V, decay, head_decay, v_gain, skip, S, N, \
@@ -298,9 +314,15 @@ LLMRS_API int llmrs_linear_recurrence_planes(const float* Q, const float* K, con
   return llmrs_launch_status("linear_recurrence");
 }
 
-// Floats of workspace for llmrs_linear_recurrence: the three prepared planes.
-LLMRS_API long long llmrs_linear_recurrence_work_floats(int n_tokens, int n_heads, int dk, int dv) {
-  return (long long)n_tokens * n_heads * (2LL * dk + dv) + 8;
+// Floats of the workspace `tables` of llmrs_linear_recurrence_planes: the coefficients of a portion's turns.
+LLMRS_API long long llmrs_linear_recurrence_table_floats(int n_tokens, int n_requests, int n_heads) {
+  return walk_places(n_tokens, n_requests) * n_heads * walk_table(WALK_LINEAR);
+}
+
+// Floats of workspace for llmrs_linear_recurrence: the three prepared planes and the tables.
+LLMRS_API long long llmrs_linear_recurrence_work_floats(int n_tokens, int n_requests, int n_heads, int dk, int dv) {
+  return (long long)n_tokens * n_heads * (2LL * dk + dv) + 12 +
+         llmrs_linear_recurrence_table_floats(n_tokens, n_requests, n_heads);
 }
 
 // q, k, v: [tokens, ...] of the activation type with their row strides, head h's channels at h * dk (h * dv);
@@ -326,6 +348,7 @@ LLMRS_API int llmrs_linear_recurrence(const void* q, const void* k, const void* 
   float* Q = work;
   float* K = Q + nk;
   float* V = K + nk;
+  float* tables = V + ((size_t)n_tokens * n_heads * dv + 3) / 4 * 4;
   const int threads = n_heads * dk >= 1024 ? 256 : 128;
   const size_t smem = (size_t)rot_dims * sizeof(float);
 #define LLMRS_LR_PREPARE(T)                                                                                       \
@@ -339,7 +362,7 @@ LLMRS_API int llmrs_linear_recurrence(const void* q, const void* k, const void* 
   int rc = llmrs_launch_status("linear_recurrence (prepare)");
   if (rc != 0) return rc;
   return llmrs_linear_recurrence_planes(Q, K, V, decay, head_decay, nullptr, nullptr, S, N, q_start, n_new, slot_ids,
-                                        o_raw, nq, n_tokens, n_requests, n_heads, n_heads, dk, dv, stream);
+                                        tables, o_raw, nq, n_tokens, n_requests, n_heads, n_heads, dk, dv, stream);
 }
 
 // ---------------------------------------------------------------------------------

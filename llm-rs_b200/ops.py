@@ -925,7 +925,8 @@ def delta_rule(r, k, v, gate, a_raw, decay_raw, decay_bias, a_bias, norm_w, stat
     _need(decay_raw, "decay_raw", torch.float32)
     _need(state, "state", torch.float32)
     out = torch.empty((r.size(0), n_heads * d), dtype=r.dtype, device=r.device)
-    work = torch.empty((7 * r.size(0) * n_heads * d,), dtype=torch.float32, device=r.device)     # six prepared rows and o
+    work = torch.empty((int(_lib_ll("llmrs_delta_rule_work_floats")(r.size(0), ctx.n_requests, n_heads, d)),),
+                       dtype=torch.float32, device=r.device)
     _check(_lib().llmrs_delta_rule(
         _ptr(r), _ptr(k), _ptr(v), _ptr(gate), _ptr(a_raw), _LL(stride), dtype_code(r.dtype), _ptr(decay_raw),
         _ptr(decay_bias), _ptr(a_bias), _ptr(norm_w), _ptr(state), _ptr(ctx.q_start), _ptr(ctx.n_new),
@@ -1160,7 +1161,7 @@ def linear_recurrence(q, k, v, gate, norm_w, state, ctx, n_heads: int, dk: int, 
     if (normaliser is None) != (floor is None):
         raise KernelError("linear_recurrence: normaliser and floor come together")
     dev = q.device
-    work = torch.empty((int(_lib_ll("llmrs_linear_recurrence_work_floats")(n, n_heads, dk, dv)),), dtype=torch.float32,
+    work = torch.empty((int(_lib_ll("llmrs_linear_recurrence_work_floats")(n, ctx.n_requests, n_heads, dk, dv)),), dtype=torch.float32,
                        device=dev)
     o_raw = torch.empty((n, n_heads * dv), dtype=torch.float32, device=dev)
     nq = torch.empty((n, n_heads), dtype=torch.float32, device=dev) if normaliser is not None else None
@@ -1204,6 +1205,8 @@ def ssd(xbc: torch.Tensor, z: torch.Tensor, dt_raw: torch.Tensor, taps: torch.Te
     _need(out, "out", xbc.dtype, contiguous=False)
     empty = lambda width: torch.empty((n, width), dtype=torch.float32, device=xbc.device)
     X, B, Cq, decay, step, y = empty(inner), empty(wk), empty(wk), empty(n_heads), empty(n_heads), empty(inner)
+    tables = torch.empty((int(_lib_ll("llmrs_linear_recurrence_table_floats")(n, ctx.n_requests, n_heads)),),
+                         dtype=torch.float32, device=xbc.device)
     _check(_lib().llmrs_ssd_prepare(
         _ptr(xbc), _LL(_row_stride(xbc, "xbc")), _ptr(dt_raw), _LL(_row_stride(dt_raw, "dt_raw")), dtype_code(xbc.dtype),
         _ptr(taps), _ptr(conv_bias), _ptr(dt_bias), _ptr(a_log), _ptr(conv_state), _ptr(ctx.token_req), _ptr(ctx.q_start),
@@ -1211,7 +1214,7 @@ def ssd(xbc: torch.Tensor, z: torch.Tensor, dt_raw: torch.Tensor, taps: torch.Te
         inner, n_groups, n_state, n_heads, K, _stream()), "ssd_prepare", 2 if K > 1 else 1)
     _check(_lib().llmrs_linear_recurrence_planes(
         _ptr(Cq), _ptr(B), _ptr(X), _ptr(decay), None, _ptr(step), _ptr(skip), _ptr(state), None, _ptr(ctx.q_start),
-        _ptr(ctx.n_new), _ptr(ctx.slot_ids), _ptr(y), None, n, ctx.n_requests, n_heads, n_groups, n_state, vdim,
+        _ptr(ctx.n_new), _ptr(ctx.slot_ids), _ptr(tables), _ptr(y), None, n, ctx.n_requests, n_heads, n_groups, n_state, vdim,
         _stream()), "linear_recurrence_planes")
     _check(_lib().llmrs_ssd_output(
         _ptr(y), _ptr(z), _LL(_row_stride(z, "z")), dtype_code(xbc.dtype), _ptr(norm_w), _ptr(out),

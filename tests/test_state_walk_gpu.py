@@ -1,0 +1,62 @@
+"""Portions of eight tokens and more take the recurrences with a matrix state in turns of four tokens
+(csrc/state_walk.cuh), single tokens one by one: the same outputs and states from either, at the edges of turns, stages and
+copies, for many requests in one step. Both are float32 evaluations of one recurrence, each some 1e-6 from 64 bits in the
+2-norm at these sizes; single elements may lie sixteen times that apart."""
+from types import SimpleNamespace
+
+import pytest
+import torch
+
+pytestmark = pytest.mark.gpu
+DEV = "cuda:0"
+
+
+def _ctx(n_new, cached):
+    i32 = lambda v: torch.tensor(v, dtype=torch.int32, device=DEV)
+    return SimpleNamespace(
+        n_tokens=sum(n_new), n_requests=len(n_new), q_start=i32([sum(n_new[:r]) for r in range(len(n_new))]), n_new=i32(n_new),
+        cached_len=i32(cached), slot_ids=i32(list(range(len(n_new)))[::-1]),
+        token_req=i32([r for r, n in enumerate(n_new) for _ in range(n)]),
+        positions=i32([c + i for c, n in zip(cached, n_new) for i in range(n)]))
+
+
+def _part(kind, d, dv):
+    from llm_rs_b200.parts.delta_rule import ChannelDelta, GatedDelta, GeneralDelta
+    from llm_rs_b200.parts.recurrent import MatrixMemory, Retention
+    from llm_rs_b200.parts.ssd import Mamba2
+    D = 40
+    return D, {"memory": lambda: MatrixMemory(D, 3, d, dv, gate_cap=9.0, prefix="m."),
+               "retention": lambda: Retention(D, 3, d, dv, [0.9, 0.0, 1.0], prefix="m."),
+               "mamba": lambda: Mamba2(D, 4, dv, d, 2, 3, norm_parts=1, prefix="m."),
+               "gated": lambda: GatedDelta(D, 4, 2, d, dv, 3, prefix="m."),
+               "channel": lambda: ChannelDelta(D, 4, 2, d, dv, 3, 8, 8, prefix="m."),
+               "general": lambda: GeneralDelta(D, 3, d, 8, prefix="m.")}[kind]()
+
+
+@pytest.mark.parametrize("kind", ["memory", "retention", "mamba", "gated", "channel", "general"])
+@pytest.mark.parametrize("d,dv,lens", [(64, 64, [8]), (128, 48, [9, 1, 13]), (30, 17, [12, 7]), (200, 20, [16, 33]),
+                                       (96, 130, [31]), (7, 3, [1, 2, 3, 4, 5, 11] * 7), (256, 16, [10, 0, 8])])
+def test_portions_in_turns_match_single_tokens(kind, d, dv, lens):
+    from llm_rs_b200.parts import Runtime
+    g = torch.Generator().manual_seed(d + dv)
+    D, part = _part(kind, d, dv)
+    w = {s.name: (torch.randn(s.shape, generator=g) * (0.5 if len(s.shape) == 1 else s.shape[-1] ** -0.5)).to(DEV)
+         for s in part.weight_specs()}
+    part.bind(w, Runtime(torch.device(DEV), torch.float32, 4096))
+    x = [torch.randn(n, D, generator=g).to(DEV) for n in lens]
+    start = {name: 0.3 * torch.randn(len(lens), *shape, generator=g).to(DEV)
+             for name, shape in part.state_need().tensors.items()}
+    whole = {k: t.clone() for k, t in start.items()}
+    got = part.forward(torch.cat(x), _ctx(lens, [0] * len(lens)), SimpleNamespace(state=whole))
+    single = {k: t.clone() for k, t in start.items()}
+    rows = [[] for _ in lens]
+    for i in range(max(lens)):
+        n_new = [int(i < n) for n in lens]
+        y = part.forward(torch.cat([a[i:i + 1] for a in x if i < a.size(0)]), _ctx(n_new, [min(i, n) for n in lens]),
+                         SimpleNamespace(state=single))
+        for r, row in zip([r for r, n in enumerate(lens) if i < n], y):
+            rows[r].append(row)
+    want = torch.stack([row for r in rows for row in r])
+    for name, a, b in [("output", got, want)] + [(k, whole[k], single[k]) for k in whole]:
+        assert torch.isfinite(a).all(), name
+        assert float((a - b).abs().max()) <= 3.2e-5 * max(1.0, float(b.abs().max())), name
