@@ -16,30 +16,11 @@
 // tile. bfloat16 operands are widened exactly; with `round_x` float32 rows of X are first rounded to bfloat16 (they
 // stand in for activations of that type).
 #include "common.cuh"
+#include "gemm_grouped.cuh"
 #include "mma_util.cuh"
 
 constexpr int GG_BM = 64, GG_BN = 64, GG_BK = 16, GG_THREADS = 256;
 
-struct GroupedGemmArgs {
-  const void* x;            // rows of X
-  long long x_stride;       // elements between rows
-  long long x_batch;        // elements between batches (batched mode)
-  const void* w;            // [groups, N, K]
-  const void* w2;           // second weights of the gated unit, or null
-  long long w_batch;        // elements between groups
-  void* out;
-  long long out_stride, out_batch;
-  int M, N, K;              // M: rows (batched mode) or total sorted rows (grouped mode)
-  const int* tiles;         // grouped mode: [tile][3] = group, first row, rows; null in batched mode
-  const int* n_tiles;       // grouped mode: number of tiles on the device
-  const int* src;           // grouped mode: sorted row -> row of X (null: the row itself)
-  int round_x;
-  int tile_rows;            // grouped mode: the most rows a tile of the list has (64 or 128)
-  GatedUnit unit;           // EPI_UNIT
-  const float* r_bias;      // EPI_GATES: [groups * N] each
-  const float* i_bias;
-  const float* rate;
-};
 enum { EPI_STORE = 0, EPI_UNIT = 1, EPI_GATES = 2 };
 
 // One element's pair of the gates epilogue: `c` is the channel over all groups, `x` the row's own number there.
@@ -348,6 +329,9 @@ static int launch_grouped_mma(const GroupedGemmArgs& a, dim3 grid, cudaStream_t 
 // 0: the CUDA-core kernel for every product (set by tests that compare the two).
 static int g_grouped_mma = 1;
 LLMRS_API void llmrs_gemm_grouped_use_mma(int on) { g_grouped_mma = on; }
+// 0: products of tiles of 128 rows stay on mma.sync (set by tests that compare the two).
+static int g_grouped_tc = 1;
+LLMRS_API void llmrs_gemm_grouped_use_tc(int on) { g_grouped_tc = on; }
 
 template <typename TX, typename TW, typename TO>
 static int launch_grouped(const GroupedGemmArgs& a, dim3 grid, cudaStream_t stream) {
@@ -360,12 +344,13 @@ static int launch_grouped(const GroupedGemmArgs& a, dim3 grid, cudaStream_t stre
 
 // Types: x_dtype / w_dtype / out_dtype are LLMRS_F32 or LLMRS_BF16. Supported: all float32; bfloat16 weights with
 // X in either type and the output in either type. `batches` > 0: batched mode; `tiles` != null: grouped mode with at
-// most `max_tiles` tiles.
+// most `max_tiles` tiles. x_rows: rows of X; groups: weight matrices; error_flag: see gemm_tcgen05.cu.
 LLMRS_API int llmrs_gemm_grouped(const void* x, int x_dtype, long long x_stride, long long x_batch, const void* w,
                                  const void* w2, int w_dtype, long long w_batch, void* out, int out_dtype,
                                  long long out_stride, long long out_batch, int M, int N, int K, int batches,
                                  const int* tiles, const int* n_tiles, int max_tiles, int tile_rows, const int* src,
-                                 int round_x, float limit, float alpha, float shift, cudaStream_t stream) {
+                                 int round_x, float limit, float alpha, float shift, int x_rows, int groups,
+                                 int* error_flag, cudaStream_t stream) {
   LLMRS_REQUIRE(M >= 0 && N > 0 && K > 0, "gemm_grouped: bad sizes M=%d N=%d K=%d", M, N, K);
   LLMRS_REQUIRE((tiles != nullptr) != (batches > 0), "gemm_grouped: either a tile list or a number of batches");
   LLMRS_REQUIRE(tiles == nullptr || n_tiles != nullptr, "gemm_grouped: a tile list needs its length");
@@ -384,6 +369,11 @@ LLMRS_API int llmrs_gemm_grouped(const void* x, int x_dtype, long long x_stride,
   if (g_grouped_mma && x_dtype == LLMRS_BF16 && w_dtype == LLMRS_BF16 && K % 8 == 0 && x_stride % 8 == 0 &&
       x_batch % 8 == 0 && ((uintptr_t)x & 15) == 0 && ((uintptr_t)w & 15) == 0 && (!w2 || ((uintptr_t)w2 & 15) == 0) &&
       (N * (long long)K) % 8 == 0) {
+    // Tiles of 128 rows go to tcgen05 where TMA can address the rows. Batches lie side by side in the rows of one tensor: a
+    // step of k past a batch's end would read the next one's numbers, so K must then be whole steps.
+    if (tile_rows == 128 && g_grouped_tc && src == nullptr && w_batch == (long long)N * K && x_stride > 0 &&
+        (tiles || (K % 64 == 0 && x_batch > 0 && (long long)(batches - 1) * x_batch + K <= 0x7fffffffLL)))
+      return launch_grouped_tc(a, out_dtype, x_rows, groups, batches, max_tiles, error_flag, stream);
     const int cols = w2 ? GmCols<true>::value : GmCols<false>::value;
     dim3 mgrid((N + cols - 1) / cols, tiles ? max_tiles : (M + tile_rows - 1) / tile_rows, grid.z);
     if (tile_rows == 128)

@@ -797,14 +797,14 @@ def tanh_slice(x: torch.Tensor, out_dtype: torch.dtype) -> torch.Tensor:
 
 
 # -- many small products in one launch ----------------------------------------------------------------
-GROUPED_TILE_ROWS = 64      # rows of a tile of the grouped product; 128 where groups have many rows (``grouped_tile_rows``)
+GROUPED_TILE_ROWS = 64      # rows of a tile of the grouped product; 128 where groups have a few rows (``grouped_tile_rows``)
 
 
 def grouped_tile_rows(n_rows: int, n_groups: int) -> int:
-    """Rows per tile for ``moe_sort`` and ``gemm_grouped``: 128 when the groups hold some hundred rows each (prompts:
-    a larger tile reads the weights half as often), else 64."""
-    return 128 if n_rows >= 96 * n_groups else GROUPED_TILE_ROWS
-
+    """Rows per tile for ``moe_sort`` and ``gemm_grouped``: 128 (the tcgen05 kernel for bfloat16) from two rows a group on, else
+    64 (mma.sync). 32 experts of 1,024 at width 2,048, both products, 64 against 128 rows a tile (us): half a row a group 65 / 72,
+    one 90 / 103, two 122 / 107, eight 123 / 107, 64 164 / 112, 256 482 / 196."""
+    return 128 if n_rows >= 2 * n_groups else GROUPED_TILE_ROWS
 
 
 def _strides3(t: torch.Tensor, name: str):
@@ -818,6 +818,13 @@ def grouped_use_tensor_cores(on: bool) -> None:
     """False: ``gemm_batched`` and ``gemm_grouped`` take the CUDA-core kernel for bfloat16 too (for tests that compare
     the two kernels). The default is True."""
     fn = _lib().llmrs_gemm_grouped_use_mma
+    fn.restype, fn.argtypes = None, [ctypes.c_int]
+    fn(1 if on else 0)
+
+
+def grouped_use_tcgen05(on: bool) -> None:
+    """False: products of tiles of 128 rows take mma.sync (for tests that compare the kernels). The default is True."""
+    fn = _lib().llmrs_gemm_grouped_use_tc
     fn.restype, fn.argtypes = None, [ctypes.c_int]
     fn(1 if on else 0)
 
@@ -838,7 +845,7 @@ def gemm_batched(x: torch.Tensor, w: torch.Tensor, out: torch.Tensor, round_x: b
     _check(_lib().llmrs_gemm_grouped(
         _ptr(x), dtype_code(x.dtype), _LL(xs), _LL(xb), _ptr(w), None, dtype_code(w.dtype), _LL(N * K), _ptr(out),
         dtype_code(out.dtype), _LL(os_), _LL(ob), M, N, K, B, None, None, 0, 0, None, int(round_x), ctypes.c_float(0),
-        ctypes.c_float(0), ctypes.c_float(0), _stream()), "gemm_batched")
+        ctypes.c_float(0), ctypes.c_float(0), M, B, _ptr(tc_error_flag(x.device)), _stream()), "gemm_batched")
     return out
 
 
@@ -859,11 +866,17 @@ def gemm_grouped(x: torch.Tensor, w: torch.Tensor, out: torch.Tensor, tiles: tor
         raise KernelError(f"gemm_grouped: x {tuple(x.shape)}, w {tuple(w.shape)}, out {tuple(out.shape)}")
     if src is not None:
         _need(src, "src", torch.int32)
+        if (tile_rows == 128 and x.dtype == w.dtype == torch.bfloat16 and K % 8 == 0 and _row_stride(x, "x") % 8 == 0
+                and x.data_ptr() % 16 == 0):      # the tcgen05 kernel reads rows as they lie
+            rows = torch.empty((out.size(0), K), dtype=torch.bfloat16, device=x.device)
+            _check(_lib().llmrs_gather_rows(_ptr(x), _LL(_row_stride(x, "x")), _ptr(src), _ptr(rows), out.size(0), K, _stream()),
+                   "gather_rows")
+            x, src = rows, None
     _check(_lib().llmrs_gemm_grouped(
         _ptr(x), dtype_code(x.dtype), _LL(_row_stride(x, "x")), _LL(0), _ptr(w), _ptr(w2), dtype_code(w.dtype),
         _LL(N * K), _ptr(out), dtype_code(out.dtype), _LL(out.stride(0)), _LL(0), out.size(0), N, K, 0, _ptr(tiles),
         _ptr(n_tiles), tiles.size(0), tile_rows, _ptr(src), int(round_x), ctypes.c_float(limit), ctypes.c_float(alpha),
-        ctypes.c_float(shift), _stream()), "gemm_grouped")
+        ctypes.c_float(shift), x.size(0), G, _ptr(tc_error_flag(x.device)), _stream()), "gemm_grouped")
     return out
 
 

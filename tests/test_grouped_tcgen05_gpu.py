@@ -1,0 +1,87 @@
+"""The grouped and batched products on tcgen05 (csrc/gemm_grouped_tc.cu) at the edges of their tiles against float64 and the
+mma.sync kernel: rows picked by an index or as they lie, groups of no, one, 128 and 129 rows, widths and depths that fill no
+tile, the gated unit, both output types; a wait that runs out. Products of bfloat16 numbers are exact in float32, so an output
+errs by at most K + 1 half ulps of the sum of the products' magnitudes, and half an ulp of its own type."""
+import pytest
+import torch
+
+pytestmark = pytest.mark.gpu
+DEV = "cuda:0"
+
+
+def _bound(x, w, out_dtype, K):
+    mag = x.double().abs() @ w.double().abs().t()
+    return mag * (K + 1) * 2.0 ** -24 + (mag * 2.0 ** -8 if out_dtype == torch.bfloat16 else 0.0) + 1e-30
+
+
+@pytest.mark.parametrize("out_dtype", [torch.float32, torch.bfloat16])
+@pytest.mark.parametrize("gather", [True, False])
+@pytest.mark.parametrize("N,K,counts", [(256, 64, [129, 0, 1, 128, 300]), (200, 72, [500, 20]), (1000, 136, [7, 257, 130]),
+                                        (64, 512, [384]), (33, 200, [128, 128, 5])])
+def test_grouped(N, K, counts, gather, out_dtype):
+    from llm_rs_b200 import ops
+    torch.manual_seed(N + K)
+    G, rows = len(counts), sum(counts)
+    w = torch.randn(G, N, K, device=DEV).bfloat16()
+    x = torch.randn(150 if gather else rows, K, device=DEV).bfloat16()
+    src = torch.randint(0, x.size(0), (rows,), device=DEV, dtype=torch.int32) if gather else None
+    starts = [sum(counts[:g]) for g in range(G)]
+    tiles = [(g, s + a, min(128, n - a)) for g, (s, n) in enumerate(zip(starts, counts)) for a in range(0, n, 128)]
+    n_tiles = torch.tensor([len(tiles)], dtype=torch.int32, device=DEV)
+    tiles = torch.tensor(tiles + [(0, 0, 0)] * 3, dtype=torch.int32, device=DEV)
+    out = torch.full((rows, N), 7.0, device=DEV, dtype=out_dtype)
+    ops.gemm_grouped(x, w, out, tiles, n_tiles, src, tile_rows=128)
+    ops.check_tc_error(DEV)
+    rows_x = x[src.long()] if gather else x
+    for g, (s, n) in enumerate(zip(starts, counts)):
+        want = rows_x[s:s + n].double() @ w[g].double().t()
+        assert bool(((out[s:s + n].double() - want).abs() <= _bound(rows_x[s:s + n], w[g], out_dtype, K)).all()), g
+    # The gated unit of two products against the other kernel's: float32 sums in another order, rounded once.
+    w2 = torch.randn(G, N, K, device=DEV).bfloat16()
+    got, other = torch.empty(rows, N, device=DEV), torch.empty(rows, N, device=DEV)
+    ops.gemm_grouped(x, w, got, tiles, n_tiles, src, w2=w2, limit=7.0, alpha=1.702, shift=1.0, tile_rows=128)
+    ops.grouped_use_tcgen05(False)
+    try:
+        ops.gemm_grouped(x, w, other, tiles, n_tiles, src, w2=w2, limit=7.0, alpha=1.702, shift=1.0, tile_rows=128)
+    finally:
+        ops.grouped_use_tcgen05(True)
+    ops.check_tc_error(DEV)
+    # gate and up each err by some 1e-6 of sqrt(K); the unit multiplies them (gate clamped at 7, up at 7 and shifted).
+    assert float((got - other).abs().max()) <= 1e-4 * max(1.0, float(other.abs().max()))
+
+
+@pytest.mark.parametrize("M,B,N,K,pad", [(128, 3, 128, 64, 0), (129, 4, 512, 128, 8), (300, 2, 40, 192, 16), (2000, 16, 128, 512, 0),
+                                         (130, 3, 96, 72, 8)])
+def test_batched(M, B, N, K, pad):
+    """(K = 72 is no whole number of steps: the mma.sync kernel keeps it.)"""
+    from llm_rs_b200 import ops
+    torch.manual_seed(M + N)
+    wide = torch.randn(M, B * (K + pad) + pad, device=DEV).bfloat16()
+    x = wide[:, : B * (K + pad)].unflatten(1, (B, K + pad))[:, :, :K]
+    wide[:, B * (K + pad):] = float("nan")      # what lies beside the batches must not be read into a sum
+    w = torch.randn(B, N, K, device=DEV).bfloat16()
+    out = torch.full((M, B, N + pad), 3.0, device=DEV, dtype=torch.bfloat16)
+    ops.gemm_batched(x, w, out[:, :, :N])
+    ops.check_tc_error(DEV)
+    for b in range(B):
+        want = x[:, b].double() @ w[b].double().t()
+        assert bool(((out[:, b, :N].double() - want).abs() <= _bound(x[:, b], w[b], torch.bfloat16, K)).all()), b
+    assert bool((out[:, :, N:] == 3.0).all())
+
+
+def test_a_wait_that_runs_out_is_reported():
+    from llm_rs_b200 import ops
+    x, w = torch.randn(256, 256, device=DEV).bfloat16(), torch.randn(1, 256, 256, device=DEV).bfloat16()
+    out = torch.empty(256, 1, 256, device=DEV, dtype=torch.bfloat16)
+    ops.set_tc_wait_limit(2000)
+    ops.test_skip_copy(gemm_k_block=2)
+    try:
+        ops.gemm_batched(x.unflatten(1, (1, 256)), w, out)
+        with pytest.raises(ops.KernelError, match="gave up waiting"):
+            ops.check_tc_error(DEV)
+    finally:
+        ops.test_skip_copy()
+        ops.set_tc_wait_limit()
+    ops.gemm_batched(x.unflatten(1, (1, 256)), w, out)
+    ops.check_tc_error(DEV)
+    assert torch.allclose(out[:, 0].float(), x.float() @ w[0].float().t(), atol=0.5, rtol=2e-2)
