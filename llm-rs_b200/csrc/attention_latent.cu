@@ -1053,3 +1053,50 @@ LLMRS_API int llmrs_latent_attention_prefill(const void* qa, long long qa_token,
   return launch_latent_prefill<1, 16>(LLMRS_LP_ARGS);
 #undef LLMRS_LP_ARGS
 }
+
+// ---------------------------------------------------------------------------------
+// The cached rows that long prompt portions see, side by side: c [rows, rank] and kr [rows, dr]. row_of [requests][2]: the row
+// of a request's first key and that key's position; a warp per row. Keys before the request's first visible one (their pages
+// may be gone) are zeros, and so are rows of requests that have none.
+// ---------------------------------------------------------------------------------
+__global__ void __launch_bounds__(256)
+latent_gather_kernel(const __nv_bfloat16* __restrict__ cache, const int* __restrict__ table, int table_width,
+                     const int* __restrict__ row_of, const int* __restrict__ n_new, const int* __restrict__ cached_len,
+                     __nv_bfloat16* __restrict__ c, __nv_bfloat16* __restrict__ kr, int n_rows, int n_requests, int rank, int dr,
+                     int page_size, int window) {
+  const int row = blockIdx.x * 8 + (threadIdx.x >> 5), lane = threadIdx.x & 31;
+  if (row >= n_rows) return;
+  int req = 0;      // the last request whose rows start at or before this one
+  for (int base = 0; base < n_requests; base += 32) {
+    const int r = base + lane;
+    const unsigned hit = __ballot_sync(0xffffffffu, r < n_requests && row_of[2 * r] <= row);
+    if (hit == 0) break;
+    req = base + 31 - __clz(hit);
+  }
+  const int key = row - row_of[2 * req] + row_of[2 * req + 1], cached = cached_len[req];
+  const bool seen = key < cached + n_new[req] && (window <= 0 || key > cached - window);
+  const uint4* src = nullptr;
+  const uint4* src_r = nullptr;
+  if (seen) {
+    const int page = LLMRS_CHECKED_PAGE(table[(size_t)req * table_width + key / page_size], 3, key), at = key % page_size;
+    const __nv_bfloat16* base = cache + (size_t)page * page_size * (rank + dr);
+    src = reinterpret_cast<const uint4*>(base + (size_t)at * rank);
+    src_r = reinterpret_cast<const uint4*>(base + (size_t)page_size * rank + (size_t)at * dr);
+  }
+  const uint4 zero = make_uint4(0u, 0u, 0u, 0u);
+  for (int e = lane; e < rank / 8; e += 32) reinterpret_cast<uint4*>(c + (size_t)row * rank)[e] = seen ? src[e] : zero;
+  for (int e = lane; e < dr / 8; e += 32) reinterpret_cast<uint4*>(kr + (size_t)row * dr)[e] = seen ? src_r[e] : zero;
+}
+
+LLMRS_API int llmrs_latent_gather(const void* cache, const int* table, int table_width, const int* row_of, const int* n_new,
+                                  const int* cached_len, void* c, void* kr, int n_rows, int n_requests, int rank, int dr,
+                                  int page_size, int window, cudaStream_t stream) {
+  LLMRS_REQUIRE(n_rows >= 0 && n_requests > 0 && rank > 0 && dr > 0 && page_size > 0, "latent_gather: bad sizes");
+  LLMRS_REQUIRE(rank % 8 == 0 && dr % 8 == 0 && (((uintptr_t)cache | (uintptr_t)c | (uintptr_t)kr) & 15) == 0,
+                "latent_gather: rows must start on 16-byte boundaries");
+  if (n_rows == 0) return 0;
+  latent_gather_kernel<<<(n_rows + 7) / 8, 256, 0, stream>>>((const __nv_bfloat16*)cache, table, table_width, row_of, n_new, cached_len,
+                                                             (__nv_bfloat16*)c, (__nv_bfloat16*)kr, n_rows, n_requests, rank, dr,
+                                                             page_size, window);
+  return llmrs_launch_status("latent_gather");
+}

@@ -39,14 +39,14 @@ typedef __nv_bfloat16 bf16;
 
 namespace {
 
-constexpr int AT_BQ = 128, AT_BK = 128, AT_D = 128, AT_THREADS = 128, AT_STAGES = 3;
+constexpr int AT_BQ = 128, AT_BK = 128, AT_D = 128, AT_THREADS = 128;
 constexpr uint32_t AT_WAIT_LIMIT = 1u << 22;
 constexpr int AT_MAX_LIST = 8192;    // entries of the tile list that a launch takes (a block notes its 128-row tiles in shared memory)
 constexpr float AT_LOG2E = 1.4426950408889634f;
-constexpr uint32_t K_BYTES = AT_BK * AT_D * 2, V_BYTES = K_BYTES, STAGE_BYTES = K_BYTES + V_BYTES;
+constexpr uint32_t V_BYTES = AT_BK * AT_D * 2;
 constexpr uint32_t HALF_BYTES = AT_BK * 128;   // one half of head_dim of a K or V tile: [128 keys][64 dims]
 // Tensor memory of a block: S twice (128 columns of float32 each; P, as bfloat16 pairs, goes over the
-// first 64 of its S), O (128 columns), Q (128 bfloat16 = 64 columns).
+// first 64 of its S), O (128 columns), Q (128 bfloat16 = 64 columns; 192 = 96 with latent keys).
 constexpr uint32_t TMEM_COLS = 512, S_COL = 0, O_COL = 256, Q_COL = 384;
 
 __device__ int g_attn_tc_error = 0;
@@ -200,15 +200,26 @@ __device__ __forceinline__ void bar_arrive(uint32_t bar) {
 // Barriers that are used every tile come in pairs, one per parity of the tile: the roles run up to
 // two tiles apart, and a wait by parity must never be a whole phase behind its barrier.
 // SCORED false: no cap, no sink, no chunks (the arguments are ignored and the code for them is not there).
-template <bool SCORED>
+// LAT > 0: keys and values do not come from pages but from rows made for the call (latent attention): keys of LAT pieces of
+// 64 channels, the last one a rotated part that all heads share (map_rot, zeros past its width), the others and the values of
+// 128 channels in one row per key, keys of all heads then values of all heads (map_kv). `rows` names per request the row of
+// its first key and that key's position. The third piece of the keys leaves room for two stages instead of three.
+struct LatentRows {
+  const int* rows;      // [requests][2]
+  int dn, dr;           // channels of a head's own key, and of the shared part
+};
+template <bool SCORED, int LAT>
 __global__ void __launch_bounds__(AT_THREADS + 96, 1)
-attn_prefill_tc_kernel(const __grid_constant__ CUtensorMap map_kv, const bf16* __restrict__ q, long long q_stride,
+attn_prefill_tc_kernel(const __grid_constant__ CUtensorMap map_kv, const __grid_constant__ CUtensorMap map_rot,
+                       const LatentRows lat, const bf16* __restrict__ q, long long q_stride,
                        bf16* __restrict__ out, long long out_stride, const int* __restrict__ tiles,
                        const int* __restrict__ q_start, const int* __restrict__ n_new,
                        const int* __restrict__ cached_len, const int* __restrict__ block_table, int table_stride,
                        int n_list, int persistent, int n_q_heads, int n_kv_heads, int page_size, int box_rows, int window, float scale,
                        float softcap_, const float* __restrict__ sink_, int chunk_, float out_scale_, int keep_,
                        const bf16* __restrict__ gate_, long long gate_stride, int* __restrict__ error_flag, uint32_t wait_limit, int test_skip_tile) {
+  constexpr int AT_STAGES = LAT == 3 ? 2 : 3, KEY_PIECES = LAT > 0 ? LAT : 2;
+  constexpr uint32_t K_BYTES = KEY_PIECES * HALF_BYTES, STAGE_BYTES = K_BYTES + V_BYTES;
   const float out_scale = SCORED ? out_scale_ : 1.0f;      // the output is multiplied by it
   const float softcap = SCORED ? softcap_ : 0.f;
   const float* sink = SCORED ? sink_ : nullptr;
@@ -252,7 +263,7 @@ attn_prefill_tc_kernel(const __grid_constant__ CUtensorMap map_kv, const bf16* _
   __syncthreads();
   const int n_valid = persistent ? *n_valid_slot : n_list;
   struct Item {
-    int rows, tok0, pos0, kv_hi, key_floor, kv_lo, n_kept, n_tiles, head, kvh;
+    int req, rows, tok0, pos0, kv_hi, key_floor, kv_lo, n_kept, n_tiles, head, kvh;
     const int* table;
   };
   const int n_lin = n_valid * n_q_heads;
@@ -265,6 +276,7 @@ attn_prefill_tc_kernel(const __grid_constant__ CUtensorMap map_kv, const bf16* _
   auto item_at = [&](int L, Item& it) {
     const int e = n_valid - 1 - L / n_q_heads, tile = persistent ? (int)valid[e] : e;
     const int req = tiles[2 * tile], q_off = tiles[2 * tile + 1];
+    it.req = req;
     it.head = L % n_q_heads;
     it.kvh = it.head / (n_q_heads / n_kv_heads);
     it.rows = min(AT_BQ, n_new[req] - q_off);
@@ -318,6 +330,37 @@ attn_prefill_tc_kernel(const __grid_constant__ CUtensorMap map_kv, const bf16* _
     // ---- the copying warps: warp 5 brings K, warp 6 V; one box per lane, and a lane's box of tile t
     // is the same part of every tile.
     const int which = warp - 5;
+    if constexpr (LAT > 0) {      // a lane for each piece of 128 keys x 64 channels
+      const int n_boxes = which ? 2 : LAT;
+      const uint32_t bar_full = which ? bar_vfull : bar_kfull, bar_free = which ? bar_vfree : bar_kfree;
+      int g0 = 0;
+      bool ok = true;
+      for (int r = 0; ok; ++r) {
+        const int L = item_index(r);
+        if (L < 0) break;
+        Item it;
+        item_at(L, it);
+        const int first_row = lat.rows[2 * it.req] - lat.rows[2 * it.req + 1];
+        const int col = which ? n_q_heads * lat.dn + it.head * AT_D + lane * 64 : it.head * lat.dn + lane * 64;
+        for (int t = 0; t < it.n_tiles; ++t) {
+          const int g = g0 + t, st = g % AT_STAGES;
+          if (g >= AT_STAGES && !wait_all(bar_free + 8 * st, ((g / AT_STAGES) - 1) & 1)) { ok = false; break; }
+          copies = g + 1;
+          if (!(which == 0 && g == test_skip_tile)) {
+            const uint32_t bar = bar_full + 8 * st, dst = sm(KV) + st * STAGE_BYTES + which * K_BYTES + lane * HALF_BYTES;
+            if (lane == 0) bar_expect(bar, (uint32_t)n_boxes * HALF_BYTES);
+            __syncwarp();
+            const int row = first_row + first_key(it, t);
+            if (lane < n_boxes) {
+              if (which == 0 && lane == LAT - 1) tma_2d(dst, &map_rot, bar, 0, row);
+              else tma_2d(dst, &map_kv, bar, col, row);
+            }
+            __syncwarp();
+          }
+        }
+        g0 += it.n_tiles;
+      }
+    } else {
     const int per_half = AT_BK / box_rows;            // boxes per half of the head: 8 or 2
     const int n_boxes = 2 * per_half;
     const int h = lane / per_half, i = lane % per_half;
@@ -364,6 +407,7 @@ attn_prefill_tc_kernel(const __grid_constant__ CUtensorMap map_kv, const bf16* _
       }
       g0 += it.n_tiles;
     }
+    }
   } else if (warp == 4) {
     // ---- the MMA warp: all lanes walk the loop together; lane 0 issues -------------------------
     // One elected lane issues, but the whole warp computes the operands of every MMA: they are then
@@ -375,8 +419,8 @@ attn_prefill_tc_kernel(const __grid_constant__ CUtensorMap map_kv, const bf16* _
       const uint32_t kbuf = sm(KV) + (g % AT_STAGES) * STAGE_BYTES;
       const uint32_t s_col = tmem + S_COL + (g & 1) * AT_BK;
 #pragma unroll
-      for (int kk = 0; kk < AT_D / 16; ++kk) {
-        const uint32_t half = kk / 4;   // head_dim 0-63 or 64-127: each half is its own swizzled tile
+      for (int kk = 0; kk < KEY_PIECES * 4; ++kk) {
+        const uint32_t half = kk / 4;   // channels 0-63, 64-127 (128-191): each piece is its own swizzled tile
         const uint64_t bd = smem_desc(kbuf + half * HALF_BYTES + (kk % 4) * 32, 16, 1024);
         if (leader) mma_ts(s_col, tmem + Q_COL + kk * 8, bd, idesc_s, kk > 0 ? 1u : 0u);
       }
@@ -462,13 +506,15 @@ attn_prefill_tc_kernel(const __grid_constant__ CUtensorMap map_kv, const bf16* _
       // A operand: shared memory then only has to feed K. (Every MMA of the item before is done: this thread
       // has waited for its last O.)
       {
-        const uint4* qrow = reinterpret_cast<const uint4*>(q + (size_t)(it.tok0 + row) * q_stride + (size_t)it.head * AT_D);
+        const uint4* qrow = reinterpret_cast<const uint4*>(q + (size_t)(it.tok0 + row) * q_stride +
+                                                           (size_t)it.head * (LAT > 0 ? lat.dn + lat.dr : AT_D));
+        const int pieces = LAT > 0 ? (lat.dn + lat.dr) / 8 : AT_D / 8;      // zeros past them
 #pragma unroll
-        for (int hlf = 0; hlf < 2; ++hlf) {
+        for (int hlf = 0; hlf < KEY_PIECES; ++hlf) {
           uint32_t rr[32];
 #pragma unroll
           for (int c = 0; c < 8; ++c) {
-            const uint4 v = row < rows ? qrow[hlf * 8 + c] : make_uint4(0u, 0u, 0u, 0u);
+            const uint4 v = row < rows && hlf * 8 + c < pieces ? qrow[hlf * 8 + c] : make_uint4(0u, 0u, 0u, 0u);
             rr[4 * c] = v.x; rr[4 * c + 1] = v.y; rr[4 * c + 2] = v.z; rr[4 * c + 3] = v.w;
           }
           tmem_st32u(lane_addr + Q_COL + hlf * 32, rr);
@@ -654,6 +700,25 @@ int make_map(CUtensorMap* map, const void* basep, long long rows, long long cols
 uint32_t g_wait_limit = AT_WAIT_LIMIT;
 int g_test_skip_tile = -1;
 
+constexpr size_t tc_smem_bytes(int stages, int key_pieces) {
+  return (size_t)stages * (key_pieces * HALF_BYTES + V_BYTES) + (4 * stages + 8) * 8 + 16 + 2 * AT_MAX_LIST;
+}
+
+template <int LAT>
+int launch_latent_tc(const CUtensorMap& map_kv, const CUtensorMap& map_rot, const LatentRows& lat, unsigned grid, int persistent,
+                     const void* q, long long q_stride, void* out, long long out_stride, const int* tiles, int n_tiles,
+                     const int* q_start, const int* n_new, const int* cached_len, int n_heads, int window, float scale,
+                     const void* gate, long long gate_stride, int* error_flag, cudaStream_t stream) {
+  constexpr size_t smem = tc_smem_bytes(LAT == 3 ? 2 : 3, LAT);
+  const cudaError_t e = cudaFuncSetAttribute(attn_prefill_tc_kernel<true, LAT>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
+  if (e != cudaSuccess) return llmrs_fail("latent_attention_tc: shared memory %zu: %s", smem, cudaGetErrorString(e));
+  attn_prefill_tc_kernel<true, LAT><<<grid, AT_THREADS + 96, smem, stream>>>(
+      map_kv, map_rot, lat, (const bf16*)q, q_stride, (bf16*)out, out_stride, tiles, q_start, n_new, cached_len, n_new, 0, n_tiles,
+      persistent, n_heads, n_heads, 16, 64, window, scale, 0.f, nullptr, 0, 1.0f, 0, (const bf16*)gate, gate_stride, error_flag,
+      g_wait_limit, g_test_skip_tile);
+  return llmrs_launch_status("latent_attention_tc");
+}
+
 }  // namespace
 
 // Polls of a barrier before a wait of the tcgen05 prefill kernel gives up (0: the default, 2^22).
@@ -714,12 +779,12 @@ int llmrs_attn_prefill_tc_scored(const void* q, long long q_stride, int n_tokens
   // One copy per page and half of the head; a page of a multiple of 64 keys is copied 64 keys at a time.
   const int box_rows = page_size % 64 == 0 ? 64 : 16;
   if ((rc = make_map(&map_kv, cache, cache_rows, AT_D, AT_D, box_rows))) return rc;
-  const size_t smem = AT_STAGES * STAGE_BYTES + (4 * AT_STAGES + 8) * 8 + 16 + 2 * AT_MAX_LIST;
+  const size_t smem = tc_smem_bytes(3, 2);
   const bool scored = softcap > 0.f || sink != nullptr || chunk > 0 || out_scale != 1.0f || keep > 0 || gate != nullptr;
   static bool configured[2] = {false, false};
   if (!configured[scored]) {
-    cudaError_t e = scored ? cudaFuncSetAttribute(attn_prefill_tc_kernel<true>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem)
-                           : cudaFuncSetAttribute(attn_prefill_tc_kernel<false>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
+    cudaError_t e = scored ? cudaFuncSetAttribute(attn_prefill_tc_kernel<true, 0>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem)
+                           : cudaFuncSetAttribute(attn_prefill_tc_kernel<false, 0>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
     if (e != cudaSuccess) return llmrs_fail("attn_prefill_tc: shared memory %zu: %s", smem, cudaGetErrorString(e));
     configured[scored] = true;
   }
@@ -740,14 +805,49 @@ int llmrs_attn_prefill_tc_scored(const void* q, long long q_stride, int n_tokens
   const int persistent = n_items > n_sm && n_items <= 16LL * n_sm ? 1 : 0;
   dim3 grid((unsigned)(persistent ? n_sm : n_lin));
   if (scored)
-    attn_prefill_tc_kernel<true><<<grid, AT_THREADS + 96, smem, stream>>>(
-        map_kv, (const bf16*)q, q_stride, (bf16*)out, out_stride, tiles, q_start, n_new, cached_len, block_table,
+    attn_prefill_tc_kernel<true, 0><<<grid, AT_THREADS + 96, smem, stream>>>(
+        map_kv, map_kv, LatentRows{}, (const bf16*)q, q_stride, (bf16*)out, out_stride, tiles, q_start, n_new, cached_len, block_table,
         table_stride, n_tiles, persistent, n_q_heads, n_kv_heads, page_size, box_rows, window, scale, softcap, sink, chunk,
         out_scale, keep, (const bf16*)gate, gate_stride, error_flag, g_wait_limit, g_test_skip_tile);
   else
-    attn_prefill_tc_kernel<false><<<grid, AT_THREADS + 96, smem, stream>>>(
-        map_kv, (const bf16*)q, q_stride, (bf16*)out, out_stride, tiles, q_start, n_new, cached_len, block_table,
+    attn_prefill_tc_kernel<false, 0><<<grid, AT_THREADS + 96, smem, stream>>>(
+        map_kv, map_kv, LatentRows{}, (const bf16*)q, q_stride, (bf16*)out, out_stride, tiles, q_start, n_new, cached_len, block_table,
         table_stride, n_tiles, persistent, n_q_heads, n_kv_heads, page_size, box_rows, window, scale, 0.f, nullptr, 0,
         1.0f, 0, nullptr, 0, error_flag, g_wait_limit, g_test_skip_tile);
   return llmrs_launch_status("attn_prefill_tc");
+}
+
+// Latent attention of long prompt portions on rows made for the call (portions of 1,700 and 300 tokens, 16 heads of 128 + 64 over
+// a window of 1,024: 62 us, and 25 for the rows; the folded form on mma.sync, with 3.4 times the multiplications, 678 and 77
+// for its products per head): kv [rows, n_heads * (dn + 128)], every head's own key
+// (dn channels), then every head's value (128); rot [rows, dr], the key part that all heads share; row_of [requests][2], the row
+// of a request's first key and that key's position (a multiple of 128). q: heads of dn + dr channels, q_stride apart; out: heads
+// of 128; tiles [n_tiles][2]: request and offset (a multiple of 128) of every 128 queries, at most AT_MAX_LIST.
+LLMRS_API int llmrs_latent_attention_tc(const void* q, long long q_stride, void* out, long long out_stride, const void* kv,
+                                        const void* rot, long long n_rows, const int* row_of, const int* tiles, int n_tiles,
+                                        const int* q_start, const int* n_new, const int* cached_len, int n_heads, int dn,
+                                        int dr, int window, float scale, const void* gate, long long gate_stride,
+                                        int* error_flag, cudaStream_t stream) {
+  LLMRS_REQUIRE((dn == 64 || dn == 128) && dr > 0 && dr <= 64 && dr % 8 == 0 && n_heads > 0, "latent_attention_tc: heads of %d + %d", dn, dr);
+  LLMRS_REQUIRE(n_tiles >= 0 && n_tiles <= AT_MAX_LIST && n_rows > 0 && scale > 0.f, "latent_attention_tc: bad sizes");
+  LLMRS_REQUIRE(q_stride % 8 == 0 && out_stride % 8 == 0 && (((uintptr_t)q | (uintptr_t)out | (uintptr_t)kv | (uintptr_t)rot) & 15) == 0,
+                "latent_attention_tc: rows must start on 16-byte boundaries");
+  if (n_tiles == 0) return 0;
+  CUtensorMap map_kv, map_rot;
+  const long long width = (long long)n_heads * (dn + AT_D);
+  int rc = make_map(&map_kv, kv, n_rows, width, width, AT_BK);
+  if (rc == 0) rc = make_map(&map_rot, rot, n_rows, dr, dr, AT_BK);
+  if (rc != 0) return rc;
+  int dev = 0, n_sm = 0;
+  cudaGetDevice(&dev);
+  cudaDeviceGetAttribute(&n_sm, cudaDevAttrMultiProcessorCount, dev);
+  const long long items = (long long)n_heads * n_tiles;
+  const int persistent = items > n_sm && items <= 16LL * n_sm ? 1 : 0;      // as above
+  LLMRS_REQUIRE(items <= 0x7fffffffLL, "latent_attention_tc: too many tiles");
+  const LatentRows lat = {row_of, dn, dr};
+  const unsigned grid = (unsigned)(persistent ? n_sm : items);
+  return dn == 128 ? launch_latent_tc<3>(map_kv, map_rot, lat, grid, persistent, q, q_stride, out, out_stride, tiles, n_tiles, q_start,
+                                         n_new, cached_len, n_heads, window, scale, gate, gate_stride, error_flag, stream)
+                   : launch_latent_tc<2>(map_kv, map_rot, lat, grid, persistent, q, q_stride, out, out_stride, tiles, n_tiles, q_start,
+                                         n_new, cached_len, n_heads, window, scale, gate, gate_stride, error_flag, stream);
 }

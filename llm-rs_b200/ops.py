@@ -1081,6 +1081,41 @@ def latent_attention_prefill(qa: torch.Tensor, q: torch.Tensor, gate: torch.Tens
     return True
 
 
+LATENT_EXPAND_BYTES = 256 << 20     # workspace that the keys and values of a step's long portions may take
+
+
+def latent_gather(cache: torch.Tensor, table: torch.Tensor, ctx, row_of: torch.Tensor, n_rows: int, rank: int, dr: int,
+                  page_size: int, window: int):
+    """The cached rows that a step's long portions see: (latents [n_rows, rank], rotated key parts [n_rows, dr]), bfloat16.
+    ``row_of`` int32 [requests, 2]: the row of a request's first key and that key's position; keys no query of the step may
+    see are zeros."""
+    _need(cache, "cache", torch.bfloat16)
+    _need(row_of, "row_of", torch.int32)
+    c = torch.empty((n_rows, rank), dtype=torch.bfloat16, device=cache.device)
+    kr = torch.empty((n_rows, dr), dtype=torch.bfloat16, device=cache.device)
+    _check(_lib().llmrs_latent_gather(_ptr(cache), _ptr(table), table.size(1), _ptr(row_of), _ptr(ctx.n_new),
+                                      _ptr(ctx.cached_len), _ptr(c), _ptr(kr), n_rows, ctx.n_requests, rank, dr, page_size,
+                                      window, _stream()), "latent_gather")
+    return c, kr
+
+
+def latent_attention_tc(q: torch.Tensor, gate: torch.Tensor, kv: torch.Tensor, kr: torch.Tensor, row_of: torch.Tensor, tiles,
+                        n_tiles: int, ctx, out: torch.Tensor, n_heads: int, dn: int, dr: int, window: int,
+                        scale: float) -> torch.Tensor:
+    """Latent attention of long prompt portions on tcgen05, over keys and values made for the step: ``kv`` [rows, heads *
+    (dn + 128)] (every head's own key, then every head's value), ``kr`` [rows, dr]; ``q`` [tokens, heads * (dn + dr)] rotated;
+    ``gate`` raw per head; ``tiles`` int32 [n_tiles, 2] = request, offset of every 128 queries; ``out`` [tokens, heads * 128],
+    of which only the tiles' rows are written."""
+    for name, t in (("q", q), ("gate", gate), ("kv", kv), ("kr", kr), ("out", out)):
+        _need(t, name, torch.bfloat16, contiguous=name in ("kv", "kr"))
+    _check(_lib().llmrs_latent_attention_tc(
+        _ptr(q), _LL(_row_stride(q, "q")), _ptr(out), _LL(_row_stride(out, "out")), _ptr(kv), _ptr(kr), _LL(kv.size(0)),
+        _ptr(row_of), _ptr(tiles), n_tiles, _ptr(ctx.q_start), _ptr(ctx.n_new), _ptr(ctx.cached_len), n_heads, dn, dr, window,
+        ctypes.c_float(scale), _ptr(gate), _LL(_row_stride(gate, "gate")), _ptr(tc_error_flag(q.device)), _stream()),
+        "latent_attention_tc")
+    return out
+
+
 # -- blocks that norm after the residual sum; small element-wise kernels -----------------------------------
 def post_norm(h: torch.Tensor, y: Optional[torch.Tensor], layer_scale: Optional[torch.Tensor], weight: torch.Tensor,
               alpha: float, eps: float, out_dtype: Optional[torch.dtype] = None) -> Optional[torch.Tensor]:

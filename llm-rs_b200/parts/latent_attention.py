@@ -3,6 +3,7 @@ from __future__ import annotations
 
 import math
 import os
+from types import SimpleNamespace
 from typing import Mapping, Optional
 
 import numpy as np
@@ -19,6 +20,14 @@ from .spec import CacheNeed, WeightSpec
 # CUDA-core kernel for everything.
 _LATENT_MMA = os.environ.get("LLMRS_LATENT_MMA", "1") != "0"
 PREFILL_MIN_TOKENS = 32
+# Portions of at least EXPAND_MIN_TOKENS tokens that see at most EXPAND_MAX_KEYS keys per token of theirs have the keys and
+# values of what they see made for the step and take the tcgen05 attention kernel: the folded form needs no keys or values but
+# 3.4 times the multiplications (a latent of 512 against heads of 192 and 128) and walks a tile's keys on mma.sync. Measured,
+# 16 heads, a whole mixer, folded against made (us): 2,000 tokens through a window of 1,024 799 / 133; 64 tokens after 4,096
+# 793 / 119, after 8,000 1,486 / 187; 32 after 2,048 418 / 77, after 256 98 / 55. Fewer tokens over more keys were not
+# measured and stay folded.
+EXPAND_MIN_TOKENS, EXPAND_MAX_KEYS = 32, 128
+EXPAND_ALIGN = 128      # keys per tile of that kernel
 
 
 def rescaled_frequencies(dims: int, base: float, scaling: Optional[Mapping] = None):
@@ -54,6 +63,18 @@ def portion_tiles(q_start, n_new, tile_tokens: int) -> np.ndarray:
     if not firsts:
         return np.zeros((0, 2), np.int32)
     return np.stack([np.concatenate(firsts), np.concatenate(counts)], axis=1).astype(np.int32)
+
+
+def expanded_rows(n_new, cached, window: int, row_bytes: int):
+    """Per request the position of the first key that is made for the step (a multiple of EXPAND_ALIGN), how many are, and
+    whether the request's portion is taken that way (``row_bytes`` a key; 0: none are; at most
+    ``ops.LATENT_EXPAND_BYTES`` together)."""
+    lo = np.maximum(0, cached - window + 1) if window > 0 else np.zeros_like(cached)
+    first = lo // EXPAND_ALIGN * EXPAND_ALIGN
+    counts = cached + n_new - first
+    is_long = (n_new >= EXPAND_MIN_TOKENS) & (counts <= EXPAND_MAX_KEYS * n_new) & (row_bytes > 0)
+    is_long &= np.cumsum(np.where(is_long, counts, 0)) * row_bytes <= ops.LATENT_EXPAND_BYTES
+    return first, np.where(is_long, counts, 0), is_long
 
 
 @register("mixer", "latent_attention")
@@ -153,6 +174,12 @@ class LatentAttention(Mixer):
         # W_uk,h transposed to [rank, dim]: the folded query is an ordinary product with it.
         self.w_uk_t = tensors[nm("uk")].view(nh, self.dim, self.rank).transpose(1, 2).contiguous()
         self.w_uv = tensors[nm("uv")].view(nh, self.vdim, self.rank).contiguous()
+        # For portions whose keys and values are made for the step: both up-projections as one product's weight.
+        self.w_expand = None
+        q_row = self.q_width if self.q_rank else self.in_proj.weight.size(0)      # the kernel reads rows of q 16 bytes at a time
+        if (q_row % 8 == 0 and runtime.act_dtype == torch.bfloat16 and self.w_uv.dtype == self.w_uk_t.dtype == torch.bfloat16 and self.dim in (64, 128)
+                and self.vdim == 128 and self.rank % 64 == 0 and self.rot_dim % 16 == 0 and 0 < self.rot_dim <= 64):
+            self.w_expand = torch.cat([tensors[nm("uk")], tensors[nm("uv")]], dim=0).contiguous()
         self.latent_norm_w = None if self.shares_cache else tensors[nm("dkv_norm")].to(torch.float32).contiguous()
         self.open_gate = torch.full((1, nh), 30.0, dtype=runtime.act_dtype, device=runtime.device)
         inv_freq, self.rot_magnitude = rescaled_frequencies(self.rot_dims, self.rot_base, self.rot_scaling)
@@ -170,28 +197,40 @@ class LatentAttention(Mixer):
             self._tile = ops.latent_prefill_tile_tokens(self.n_heads)
         return self._tile
 
+    def _expand_row_bytes(self) -> int:
+        """Bytes of workspace that a visible key takes when its keys and values are made for the step (0: never)."""
+        if not _LATENT_MMA or self.w_expand is None:
+            return 0
+        return 2 * (self.n_heads * (self.dim + self.vdim) + self.rank + self.rot_dim)
+
     def plan_key(self):
-        return ("latent_attention_tiles", self._tile_tokens())
+        return ("latent_attention_tiles", self._tile_tokens(), self.window, self._expand_row_bytes())
 
     def plan(self, step: StepInfo) -> Plan:
         """Steps that bring a prompt's portion are cut into tiles of tokens (none for steps of single tokens, which
-        the CUDA-core kernel takes with its keys cut over blocks, and which may be replayed from a graph)."""
+        the CUDA-core kernel takes with its keys cut over blocks, and which may be replayed from a graph): long portions
+        into tiles of 128 queries over rows that are made for the step (``rows``: a request's first row and the position of
+        its first key), the others into the tiles of the kernel that reads the pages."""
+        none = np.zeros((0, 2), np.int32)
         if step.for_graph or step.n_tokens < PREFILL_MIN_TOKENS or int(np.max(step.n_new, initial=0)) <= 1:
-            return Plan(arrays={"tiles": np.zeros((0, 2), np.int32)}, values={"n_tiles": 0})
-        tiles = portion_tiles(step.q_start, step.n_new, self._tile_tokens())
-        return Plan(arrays={"tiles": tiles}, values={"n_tiles": int(tiles.shape[0])})
+            return Plan(arrays={"tiles": none, "long": none, "rows": none}, values={"n_tiles": 0, "n_long": 0, "n_rows": 0})
+        n_new, cached = np.asarray(step.n_new, np.int64), np.asarray(step.cached_len, np.int64)
+        first, counts, is_long = expanded_rows(n_new, cached, self.window, self._expand_row_bytes())
+        tiles = portion_tiles(step.q_start, np.where(is_long, 0, n_new), self._tile_tokens())
+        long_tiles = [(r, a) for r in np.nonzero(is_long)[0].tolist() for a in range(0, int(n_new[r]), EXPAND_ALIGN)]
+        rows = np.stack([np.cumsum(counts) - counts, first], axis=1).astype(np.int32)
+        return Plan(arrays={"tiles": tiles, "long": np.asarray(long_tiles, np.int32).reshape(-1, 2), "rows": rows},
+                    values={"n_tiles": int(tiles.shape[0]), "n_long": len(long_tiles), "n_rows": int(counts.sum())})
 
-    def _tiles(self, ctx):
-        """(device tiles, how many) for this step; None when the step has no plan of them."""
+    def _plan_of(self, ctx):
+        """The step's plan; outside the step function (a part alone) it is made here, from the device's arrays."""
         if hasattr(ctx, "plan"):
-            view = ctx.plan(self.plan_key())
-            return (view.arrays["tiles"], view.values["n_tiles"]) if view.values["n_tiles"] else None
-        # Called outside the step function (a part alone): plan here, from the device's arrays.
-        n_new = ctx.n_new.cpu().numpy()
-        if ctx.n_tokens < PREFILL_MIN_TOKENS or int(n_new.max(initial=0)) <= 1:
-            return None
-        tiles = portion_tiles(ctx.q_start.cpu().numpy(), n_new, self._tile_tokens())
-        return torch.from_numpy(tiles).to(ctx.n_new.device), int(tiles.shape[0])
+            return ctx.plan(self.plan_key())
+        host = lambda t: t.cpu().numpy()
+        plan = self.plan(StepInfo(ctx.n_tokens, ctx.n_requests, host(ctx.q_start), host(ctx.n_new), host(ctx.cached_len),
+                                  host(ctx.slot_ids), [], [], 0, False))
+        return SimpleNamespace(arrays={k: torch.from_numpy(v).to(ctx.n_new.device) for k, v in plan.arrays.items()},
+                               values=plan.values)
 
     def forward(self, x, ctx, cache):
         nh, dn, dr, rank = self.n_heads, self.dim, self.rot_dim, self.rank
@@ -216,28 +255,41 @@ class LatentAttention(Mixer):
         ops.latent_prepare(q, dkv, self.latent_norm_w, self.inv_freq, ctx, cache.block_table,
                            None if self.shares_cache else pages, cache.page_size, nh, dn, dr, self.rot_dims, rank,
                            self.norm_eps, neighbours=self.rot_pairing == "neighbours", magnitude=self.rot_magnitude)
+        plan = self._plan_of(ctx) if _LATENT_MMA and proj.dtype == torch.bfloat16 else None
+        n_tiles, n_long = (plan.values["n_tiles"], plan.values["n_long"]) if plan is not None else (0, 0)
+        out = torch.empty((T, nh, self.vdim), dtype=proj.dtype, device=proj.device)
+        if n_long == 0 or n_tiles:
+            self._folded(q, gate, pages, cache, ctx, plan if n_tiles else None, out)
+        if n_long:      # rows of their own: what the folded form left there is overwritten
+            c, kr = ops.latent_gather(pages, cache.block_table, ctx, plan.arrays["rows"], plan.values["n_rows"], rank, dr,
+                                      cache.page_size, self.window)
+            kv = ops.gemm_bf16(c, self.w_expand)
+            ops.latent_attention_tc(q, gate, kv, kr, plan.arrays["rows"], plan.arrays["long"], n_long, ctx,
+                                    out.view(T, nh * self.vdim), nh, dn, dr, self.window, self.scale)
+        return self.o_proj.forward(out.view(T, nh * self.vdim))
+
+    def _folded(self, q, gate, pages, cache, ctx, plan, out) -> None:
+        """The attention-weighted latents through the value up-projection into ``out`` [tokens, heads, vdim]."""
+        nh, dn, dr, rank = self.n_heads, self.dim, self.rot_dim, self.rank
+        T = ctx.n_tokens
         q3 = q.unflatten(1, (nh, dn + dr))
-        qa = torch.empty((T, nh, rank), dtype=proj.dtype, device=proj.device)
+        qa = torch.empty((T, nh, rank), dtype=q.dtype, device=q.device)
         ops.gemm_batched(q3[:, :, :dn], self.w_uk_t, qa)
-        lat = torch.empty((T, nh, rank), dtype=proj.dtype, device=proj.device)
-        tiles = self._tiles(ctx) if _LATENT_MMA and proj.dtype == torch.bfloat16 else None
-        if tiles is not None and ops.latent_attention_prefill(
-                qa, q, gate, pages, cache.block_table, ctx, tiles[0], tiles[1], lat, nh, dn, dr, rank, cache.page_size,
-                self.window, self.scale):
-            out = torch.empty((T, nh, self.vdim), dtype=proj.dtype, device=proj.device)
+        lat = torch.empty((T, nh, rank), dtype=q.dtype, device=q.device)
+        if plan is not None and ops.latent_attention_prefill(
+                qa, q, gate, pages, cache.block_table, ctx, plan.arrays["tiles"], plan.values["n_tiles"], lat, nh, dn, dr, rank,
+                cache.page_size, self.window, self.scale):
             ops.gemm_batched(lat, self.w_uv, out)
-            return self.o_proj.forward(out.view(T, nh * self.vdim))
+            return
         # Steps of few tokens cut the visible keys over several blocks. The span is what the step's shape implies (the
         # window, else what the block table can hold), not the requests' lengths: a captured step replays it.
         span = self.window if self.window > 0 else cache.block_table.size(1) * cache.page_size
         splits, split_keys = ops.latent_attention_splits(
-            T, nh, span, ops.sm_count(proj.device),
-            mma=T <= ops.LATENT_FEW_TOKENS and ops.latent_decode_takes_mma(proj.dtype, rank, dr, cache.page_size))
+            T, nh, span, ops.sm_count(q.device),
+            mma=T <= ops.LATENT_FEW_TOKENS and ops.latent_decode_takes_mma(q.dtype, rank, dr, cache.page_size))
         ops.latent_attention(qa, q, gate, pages, cache.block_table, ctx, lat, nh, dn, dr, rank, cache.page_size,
                              self.window, self.scale, splits=splits, split_keys=split_keys)
-        out = torch.empty((T, nh, self.vdim), dtype=proj.dtype, device=proj.device)
         ops.gemm_batched(lat, self.w_uv, out)
-        return self.o_proj.forward(out.view(T, nh * self.vdim))
 
     @staticmethod
     def _pages(cache):
