@@ -11,7 +11,7 @@
 // Two kernels and a small third:
 //   prepare     a warp per (token, head), all tokens at once: decay, removal rate times unit key, unit key, and r, k, v
 //               widened, as six float32 rows [tokens, heads * d];
-//   (portions of eight tokens and more take `turns` and the walk in turns of four tokens instead of these two: state_walk.cuh;
+//   (portions of 48 tokens and more take `turns` and the walk in turns of four tokens instead of these two: state_walk.cuh;
 //   2,048 tokens of 32 heads of 64 x 64: 816 us walked one by one, 246 in turns; their rows 56 us where `prepare` takes 38)
 //   recurrence  one block per (request, head, slice of 16 value columns) walks the request's tokens of the step in
 //               order: a column of S depends on no other column, so the slices run side by side. Four adjacent lanes

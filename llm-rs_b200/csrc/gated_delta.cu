@@ -18,7 +18,7 @@
 //
 //   prepare      a block per token: convolutions + SiLU, unit q and k, g and beta, as float32 rows
 //   conv state   a block per request, after prepare: the request's last K - 1 convolution inputs
-//   recurrence   of portions of eight tokens and more: the coefficients of turns of four tokens, then the walk in turns
+//   recurrence   of portions of 48 tokens and more: the coefficients of turns of four tokens, then the walk in turns
 //                (state_walk.cuh). Of single tokens and shorter portions: a block per (request, head, slice of 16 value
 //                columns) walks the request's tokens one by one; four
 //                neighbouring lanes share a column, each with a quarter of the key channels in registers (lane p of the
@@ -94,7 +94,7 @@ constexpr int GD_COLS = 16;      // value columns of a block
 #ifndef LLMRS_GD_LANES
 #define LLMRS_GD_LANES 8
 #endif
-// (The kernel for single tokens and portions of fewer than eight.) With a decay per key channel a lane reads three rows a
+// (The kernel for single tokens and portions of fewer than 48.) With a decay per key channel a lane reads three rows a
 // token, not two: sixteen lanes a column shorten that where a step's blocks do not fill the device twice (walking 2,048 tokens
 // of 16 heads of 128 x 128: 813 against 896 us for the whole op), eight are ahead where they do.
 constexpr int GD_WIDE_MAX_BLOCKS = 296;

@@ -17,7 +17,7 @@
 //                a_t = exp(f_t + m_(t-1) - m_t), b_t = exp(i_t - m_t), floor_t = exp(-m_t); m is kept per slot;
 //   prepare      q, k, v of all tokens widened to float32 (optional SiLU, optional rotation of the first channels of every
 //                head of q and k by halves, q and k scaled, k multiplied by its gain);
-//   (portions of eight tokens and more: the coefficients of turns of four tokens, then the walk in turns, state_walk.cuh)
+//   (portions of 48 tokens and more: the coefficients of turns of four tokens, then the walk in turns, state_walk.cuh)
 //   recurrence   a block per (request, head, 16 value columns) walks the tokens in order; four or eight adjacent lanes
 //                share a column, each holding its part of the column's key channels in registers; rows arrive through two
 //                shared-memory buffers by 16-byte asynchronous copies. A step of one token and a prompt's portion

@@ -34,9 +34,11 @@
 enum { WALK_LINEAR = 0, WALK_GATED = 1, WALK_CHANNEL = 2, WALK_GENERAL = 3 };
 constexpr int WALK_TURN = 4, WALK_COLS = 16, WALK_LANES = 16, WALK_THREADS = WALK_COLS / 2 * WALK_LANES;
 constexpr int WALK_STAGE = 2 * WALK_TURN, WALK_STAGES = 4;      // tokens of a stage, stages
-// Portions at least this long may take the walk in turns; a step's host side knows tokens and requests, so a portion has
-// at most n_tokens - n_requests + 1. Single tokens are walked as they are, without the coefficients' kernel.
-constexpr int WALK_MIN_PORTION = 8;
+// Portions at least this long take the walk in turns (a step's host side knows tokens and requests, so a portion has at most
+// n_tokens - n_requests + 1); shorter ones and single tokens are walked one by one, without the coefficients' kernel. Measured,
+// one by one against in turns with its coefficients (us, one portion): 32 tokens gated 10.8 / 13.7, linear 11.5 / 12.8, general
+// 18.3 / 19.6; 48 tokens 14.6 / 15.9, 15.6 / 14.4, 24.2 / 21.4; 64 tokens 18.5 / 17.8, 19.6 / 16.0, 30.7 / 23.4.
+constexpr int WALK_MIN_PORTION = 48;
 
 // A turn's coefficients of one head, in floats. LINEAR, GATED, CHANNEL: P [4] (CHANNEL: ones), Z [4] (likewise), beta or gain
 // [4], K below the diagonal row by row [6] and two zeros, Q [4][4] (zero above the diagonal). GENERAL: A [6] + 2, B [6] + 2,

@@ -1,4 +1,4 @@
-"""Portions of eight tokens and more take the recurrences with a matrix state in turns of four tokens
+"""Portions of 48 tokens and more take the recurrences with a matrix state in turns of four tokens
 (csrc/state_walk.cuh), single tokens one by one: the same outputs and states from either, at the edges of turns, stages and
 copies, for many requests in one step. Both are float32 evaluations of one recurrence, each some 1e-6 from 64 bits in the
 2-norm at these sizes; single elements may lie sixteen times that apart."""
@@ -34,8 +34,8 @@ def _part(kind, d, dv):
 
 
 @pytest.mark.parametrize("kind", ["memory", "retention", "mamba", "gated", "channel", "general"])
-@pytest.mark.parametrize("d,dv,lens", [(64, 64, [8]), (128, 48, [9, 1, 13]), (30, 17, [12, 7]), (200, 20, [16, 33]),
-                                       (96, 130, [31]), (7, 3, [1, 2, 3, 4, 5, 11] * 7), (256, 16, [10, 0, 8])])
+@pytest.mark.parametrize("d,dv,lens", [(64, 64, [48]), (128, 48, [9, 1, 49]), (30, 17, [50, 7]), (200, 20, [16, 63]),
+                                       (96, 130, [51]), (7, 3, [1, 2, 3, 4, 5, 11] * 7), (256, 16, [40, 0, 18])])
 def test_portions_in_turns_match_single_tokens(kind, d, dv, lens):
     from llm_rs_b200.parts import Runtime
     g = torch.Generator().manual_seed(d + dv)
