@@ -24,7 +24,8 @@
 //   prefill   16 queries of one request per block against the keys they may see, online softmax (any type);
 //             bfloat16 with dk, dv multiples of 16 up to 128: 64 queries per block on the tensor cores (mma.sync);
 //   decode    one query per request: the visible keys are cut into runs that separate blocks take, and a second
-//             kernel merges the runs and adds the sink. Rows that can be read sixteen bytes a load: a block takes up
+//             kernel merges the runs and adds the sink. bfloat16 heads of 64 or 128 channels: tiles of 16 keys through rings
+//             in shared memory, products on the tensor cores. Other rows that can be read sixteen bytes a load: a block takes up
 //             to four query heads of one key head together, a lane per key for the scores, lanes over channels for
 //             the values. Any other size: a block per query head, a warp per key, lanes over channels.
 // With `gate` ([tokens, query heads], of q's type) the output is also multiplied by sigmoid(gate[token, head]).
@@ -32,7 +33,11 @@
 #include "common.cuh"
 #include "mma_util.cuh"
 
+using bf16 = __nv_bfloat16;
+
 enum { MASK_CAUSAL = 0, MASK_WINDOW = 1, MASK_CHUNK = 2 };
+
+static int g_scored_generic_only = 0;
 
 struct ScoreOpts {
   float scale, softcap;
@@ -463,7 +468,6 @@ scored_prefill_kernel(const T* __restrict__ q, long long q_stride, T* __restrict
 // ---------------------------------------------------------------------------------
 // prefill on the tensor cores: bfloat16, 64 queries per block (16 per warp), 64 keys per tile, two stages.
 // ---------------------------------------------------------------------------------
-using bf16 = __nv_bfloat16;
 constexpr int SM_BQ = 64, SM_BK = 64, SM_WARPS = 4, SM_THREADS = SM_WARPS * 32;
 
 template <int KCH, int VCH>
@@ -701,7 +705,6 @@ int llmrs_attn_prefill_tc_scored(const void* q, long long q_stride, int n_tokens
                                  float softcap, const float* sink, int chunk, float out_scale, int keep,
                                  const void* gate, long long gate_stride, int* error_flag, cudaStream_t stream);
 
-static int g_scored_generic_only = 0;
 // 1: bfloat16 also takes the kernel for any type (tests compare the two).
 LLMRS_API void llmrs_scored_generic_only(int on) { g_scored_generic_only = on; }
 
@@ -1087,30 +1090,259 @@ scored_decode_grouped_kernel(const T* __restrict__ q, long long q_stride, const 
   }
 }
 
+// The decode kernel for bfloat16 heads of 64 or 128 channels (keys and values alike): one block per (decode request, key head,
+// up to four of the query heads that share it, run of keys), four warps, each with a ring of three tiles of 16 keys that
+// asynchronous copies fill, a row's pieces by neighbouring lanes. The products run on the tensor cores (m16n8k16, the
+// bfloat16 products exact, the sums float32). Weights keep their 24 bits: a weight is the sum of three bfloat16 numbers, and
+// the rows of the tile that the heads leave free carry them, heads' first pieces in rows 0-3, second in 4-7, third in 8-11;
+// their three sums are added at the end. (Rows 4-7 of the queries repeat rows 0-3, so that the lanes that hold them have the
+// same scores.) Cap and exponential are tanhf and expf as in the other kernels.
+//
+// Against the kernel of a lane per key, whose neighbouring lanes read rows 512 bytes apart (both with the merge, us): 64 requests of
+// 2,041 keys, 16 heads over 4 of 128: 128 -> 73 (3.7 TB/s); 8 of 4,096: 50 -> 37; 1 of 4,000: 24 -> 18; 1 of 100: 13.4 -> 9.4;
+// 48 of 2,000 with heads of 64: 77 -> 34. Bound by the latency of three tiles in flight a warp.
+constexpr int SM_KEYS = 16, SM_STAGES = 3;
+template <int D> __host__ __device__ constexpr int sm_ring_bytes() { return SM_STAGES * 2 * SM_KEYS * (D + 8) * 2; }      // of a warp
+template <int D>
+__global__ void __launch_bounds__(SD_THREADS, 2)
+scored_decode_mma_kernel(const bf16* __restrict__ q, long long q_stride, const bf16* __restrict__ cache,
+                         const int* __restrict__ dec_reqs, const int* __restrict__ q_start, const int* __restrict__ cached_len,
+                         const int* __restrict__ block_table, int table_stride, float* __restrict__ part, int max_splits,
+                         int split_keys, int n_q_heads, int n_kv_heads, int page_size, ScoreOpts opt) {
+  constexpr int GH = 4, LD = D + 8, CH = D / 8;      // CH: 16-byte pieces of a row
+  extern __shared__ __align__(16) unsigned char sm_raw[];
+  __shared__ float s_m[SD_WARPS][GH], s_l[SD_WARPS][GH];
+  const int G = n_q_heads / n_kv_heads, hgroups = (G + GH - 1) / GH;
+  const int di = blockIdx.x, kvh = blockIdx.y / hgroups, g0 = (blockIdx.y % hgroups) * GH, split = blockIdx.z;
+  const int ng = min(GH, G - g0), head0 = kvh * G + g0;
+  const int req = dec_reqs[di], pos = cached_len[req];      // the new token's key is in the cache already
+  const Visible vis = visible_keys(opt, pos);
+  const int k_begin = split * split_keys, k_end = min(k_begin + split_keys, vis.n);
+  auto record = [&](int h) { return part + (((size_t)di * n_q_heads + head0 + h) * max_splits + split) * sd_part_stride(D); };
+  if (k_begin >= k_end) {
+    if (threadIdx.x < ng) {
+      float* pp = record(threadIdx.x);
+      pp[0] = -INFINITY;
+      pp[1] = 0.f;
+    }
+    return;
+  }
+  const int* table = block_table + (size_t)req * table_stride;
+  const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31, g = lane >> 2, t = lane & 3, h = g & 3;
+  bf16* ring = reinterpret_cast<bf16*>(sm_raw + warp * sm_ring_bytes<D>());
+  auto keys_of = [&](int stage) { return ring + stage * 2 * SM_KEYS * LD; };
+  uint32_t qa[D / 16][2];      // rows 0-7 of the queries' tile; rows 8-15 are zero
+  {
+    const uint32_t* qp = reinterpret_cast<const uint32_t*>(q + (size_t)q_start[req] * q_stride + (size_t)(head0 + min(h, ng - 1)) * D);
+#pragma unroll
+    for (int kk = 0; kk < D / 16; ++kk) {
+      qa[kk][0] = h < ng ? qp[kk * 8 + t] : 0u;
+      qa[kk][1] = h < ng ? qp[kk * 8 + 4 + t] : 0u;
+    }
+  }
+  // Places are counted in pieces of eight elements.
+  const size_t head_base = (size_t)kvh * page_size * 2 * CH, page_pieces = (size_t)n_kv_heads * page_size * 2 * CH;
+  const size_t v_apart = (size_t)page_size * D;
+  const int n_tiles = (k_end - k_begin + SM_KEYS - 1) / SM_KEYS, mine = (n_tiles - warp + SD_WARPS - 1) / SD_WARPS;
+  auto load = [&](int i) {      // this warp's i-th tile; keys past the run's end repeat its last one
+    const int key = vis.key(min(k_begin + (warp + i * SD_WARPS) * SM_KEYS + (lane & 15), k_end - 1));
+    const int page = LLMRS_CHECKED_PAGE(table[key / page_size], 3, key);
+    const size_t at = (size_t)page * page_pieces + head_base + (size_t)(key % page_size) * CH;
+    const uint32_t lo = (uint32_t)at, hi = (uint32_t)(at >> 32);
+    bf16* ks = keys_of(i % SM_STAGES);
+#pragma unroll
+    for (int c = 0; c < SM_KEYS * CH / 32; ++c) {
+      const int id = lane + 32 * c, row = id / CH, piece = id % CH;
+      const size_t from = ((size_t)__shfl_sync(0xffffffffu, hi, row) << 32 | __shfl_sync(0xffffffffu, lo, row)) + piece;
+      const bf16* src = cache + from * 8;
+      cp_async_16(ks + row * LD + piece * 8, src, 16);
+      cp_async_16(ks + (SM_KEYS + row) * LD + piece * 8, src + v_apart, 16);
+    }
+  };
+  float acc[D / 8][4], m = -INFINITY, l = 0.f;
+#pragma unroll
+  for (int n = 0; n < D / 8; ++n)
+#pragma unroll
+    for (int e = 0; e < 4; ++e) acc[n][e] = 0.f;
+#pragma unroll
+  for (int i = 0; i < SM_STAGES - 1; ++i) {
+    if (i < mine) load(i);
+    cp_async_commit();
+  }
+  const int lm = lane >> 3, lr = lane & 7;
+  for (int i = 0; i < mine; ++i) {
+    cp_async_wait<SM_STAGES - 2>();
+    __syncwarp();      // the tile is there for all lanes, and all are done with the stage that is filled next
+    if (i + SM_STAGES - 1 < mine) load(i + SM_STAGES - 1);
+    cp_async_commit();
+    const bf16* ks = keys_of(i % SM_STAGES);
+    float s[2][4] = {{0.f, 0.f, 0.f, 0.f}, {0.f, 0.f, 0.f, 0.f}};
+#pragma unroll
+    for (int kk = 0; kk < D / 16; ++kk) {
+      uint32_t b[4];      // keys 0-7 at channels 0-7 / 8-15, then keys 8-15
+      ldmatrix_x4(b, ks + ((lm >> 1) * 8 + lr) * LD + kk * 16 + (lm & 1) * 8);
+      const uint32_t a[4] = {qa[kk][0], 0u, qa[kk][1], 0u};
+      mma_bf16_16816(s[0], a, b[0], b[1]);
+      mma_bf16_16816(s[1], a, b[2], b[3]);
+    }
+    const int k0 = k_begin + (warp + i * SD_WARPS) * SM_KEYS;
+    float sc[2][2], mx = -INFINITY;
+#pragma unroll
+    for (int j = 0; j < 2; ++j)
+#pragma unroll
+      for (int e = 0; e < 2; ++e) {
+        const int at = k0 + 8 * j + 2 * t + e;
+        float v = -INFINITY;
+        if (at < k_end) {
+          v = capped(opt, s[j][e]);
+          if (opt.bias) v += dist_bias(opt, head0 + h, pos - vis.key(at));
+        }
+        sc[j][e] = v;
+        mx = fmaxf(mx, v);
+      }
+    mx = fmaxf(mx, __shfl_xor_sync(0xffffffffu, mx, 1));
+    mx = fmaxf(mx, __shfl_xor_sync(0xffffffffu, mx, 2));
+    const float m_new = fmaxf(m, mx), ref = m_new == -INFINITY ? 0.f : m_new;
+    const float corr = expf(m - ref);
+    m = m_new;
+    if (__any_sync(0xffffffffu, corr != 1.0f)) {
+      // Rows g and g + 8 of the sums belong to the same head.
+#pragma unroll
+      for (int n = 0; n < D / 8; ++n)
+#pragma unroll
+        for (int e = 0; e < 4; ++e) acc[n][e] *= corr;
+    }
+    l *= corr;
+    uint32_t a[4];
+#pragma unroll
+    for (int j = 0; j < 2; ++j) {
+      float first[2], second[2], third[2];
+#pragma unroll
+      for (int e = 0; e < 2; ++e) {
+        const float p = expf(sc[j][e] - ref);
+        l += p;
+        first[e] = __bfloat162float(__float2bfloat16_rn(p));
+        second[e] = __bfloat162float(__float2bfloat16_rn(p - first[e]));
+        third[e] = p - first[e] - second[e];
+      }
+      a[2 * j] = g < 4 ? pack_bf16(first[0], first[1]) : pack_bf16(second[0], second[1]);
+      a[2 * j + 1] = g < 4 ? pack_bf16(third[0], third[1]) : 0u;
+    }
+    const bf16* vs = ks + SM_KEYS * LD;
+#pragma unroll
+    for (int c = 0; c < D; c += 16) {
+      uint32_t b[4];      // channels c .. c + 7 of keys 0-7 / 8-15, then channels c + 8 ..
+      ldmatrix_x4_trans(b, vs + ((lm & 1) * 8 + lr) * LD + c + (lm >> 1) * 8);
+      mma_bf16_16816(acc[c / 8], a, b[0], b[1]);
+      mma_bf16_16816(acc[c / 8 + 1], a, b[2], b[3]);
+    }
+  }
+  cp_async_wait<0>();
+  __syncthreads();      // the rings become room for the warps' sums
+  float* s_o = reinterpret_cast<float*>(sm_raw);      // [SD_WARPS][GH][D]
+  l += __shfl_xor_sync(0xffffffffu, l, 1);
+  l += __shfl_xor_sync(0xffffffffu, l, 2);
+  if (g < GH && t == 0) {
+    s_m[warp][g] = m;
+    s_l[warp][g] = l;
+  }
+#pragma unroll
+  for (int n = 0; n < D / 8; ++n)
+#pragma unroll
+    for (int e = 0; e < 2; ++e) {
+      const float o = acc[n][e] + __shfl_xor_sync(0xffffffffu, acc[n][e], 16) + acc[n][e + 2];
+      if (g < GH) s_o[((size_t)warp * GH + g) * D + 8 * n + 2 * t + e] = o;
+    }
+  __syncthreads();
+  for (int i = threadIdx.x; i < ng * D; i += SD_THREADS) {
+    const int hh = i / D, c = i - hh * D;
+    float mm = -INFINITY, a = 0.f;
+#pragma unroll
+    for (int w = 0; w < SD_WARPS; ++w) mm = fmaxf(mm, s_m[w][hh]);
+#pragma unroll
+    for (int w = 0; w < SD_WARPS; ++w)
+      a += s_m[w][hh] == -INFINITY ? 0.f : s_o[((size_t)w * GH + hh) * D + c] * expf(s_m[w][hh] - mm);
+    float ls = 0.f;
+#pragma unroll
+    for (int w = 0; w < SD_WARPS; ++w) ls += s_l[w][hh];
+    if (a != a && ls == ls) {
+      // An infinite value times a weight's zero or negative piece is no number; times the weight it is infinite.
+      float most = -INFINITY, least = INFINITY;
+      bool none = false;
+      for (int at = k_begin; at < k_end; ++at) {
+        const int key = vis.key(at), page = LLMRS_CHECKED_PAGE(table[key / page_size], 3, key);
+        const float v = __bfloat162float(cache[((size_t)page * page_pieces + head_base + (size_t)(key % page_size) * CH) * 8 + v_apart + c]);
+        most = fmaxf(most, v);
+        least = fminf(least, v);
+        none |= v != v;
+      }
+      if (!none && (most == INFINITY) != (least == -INFINITY)) a = most == INFINITY ? INFINITY : -INFINITY;
+    }
+    record(hh)[2 + c] = a;
+  }
+  if (threadIdx.x < ng) {
+    const int hh = threadIdx.x;
+    float mm = -INFINITY, ll = 0.f;
+#pragma unroll
+    for (int w = 0; w < SD_WARPS; ++w) mm = fmaxf(mm, s_m[w][hh]);
+#pragma unroll
+    for (int w = 0; w < SD_WARPS; ++w) ll += s_m[w][hh] == -INFINITY ? 0.f : s_l[w][hh] * expf(s_m[w][hh] - mm);
+    float* pp = record(hh);
+    pp[0] = mm;
+    pp[1] = ll;
+  }
+}
+
+// The runs' sums of a head become its output: a block per (decode request, head), a quarter of it per every fourth run, several
+// runs' loads in flight (one request's 62 runs of 64 keys: 26 us by threads that walk all runs one after another, 11 so).
+constexpr int SD_MERGE_PARTS = 4, SD_MERGE_COLS = 64;
 template <typename T>
-__global__ void scored_decode_merge_kernel(const float* __restrict__ part, T* __restrict__ out, long long out_stride,
-                                           const int* __restrict__ dec_reqs, const int* __restrict__ q_start,
-                                           int max_splits, int n_q_heads, int dv, ScoreOpts opt) {
+__global__ void __launch_bounds__(SD_MERGE_PARTS * SD_MERGE_COLS)
+scored_decode_merge_kernel(const float* __restrict__ part, T* __restrict__ out, long long out_stride,
+                           const int* __restrict__ dec_reqs, const int* __restrict__ q_start, int max_splits, int n_q_heads,
+                           int dv, ScoreOpts opt) {
+  __shared__ float red[33], s_a[SD_MERGE_PARTS][SD_MERGE_COLS];
   const float* sink = opt.sink;
-  const int di = blockIdx.x, head = blockIdx.y;
-  const float* base = part + ((size_t)di * n_q_heads + head) * max_splits * sd_part_stride(dv);
-  float m = sink ? sink[head] : -INFINITY;
-  for (int s = 0; s < max_splits; ++s) m = fmaxf(m, base[(size_t)s * sd_part_stride(dv)]);
-  float l = sink ? expf(sink[head] - m) : 0.f;
-  for (int s = 0; s < max_splits; ++s) {
-    const float* pp = base + (size_t)s * sd_part_stride(dv);
+  const int di = blockIdx.x, head = blockIdx.y, lane = threadIdx.x & 31;
+  const size_t stride = sd_part_stride(dv);
+  const float* base = part + ((size_t)di * n_q_heads + head) * max_splits * stride;
+  float m = -INFINITY;
+  for (int s = threadIdx.x; s < max_splits; s += blockDim.x) m = fmaxf(m, base[s * stride]);
+#pragma unroll
+  for (int o = 16; o > 0; o >>= 1) m = fmaxf(m, __shfl_xor_sync(0xffffffffu, m, o));
+  if (lane == 0) red[threadIdx.x >> 5] = m;
+  __syncthreads();
+  m = sink ? sink[head] : -INFINITY;
+  for (int w = 0; w < (int)blockDim.x / 32; ++w) m = fmaxf(m, red[w]);
+  __syncthreads();
+  float l = sink && threadIdx.x == 0 ? expf(sink[head] - m) : 0.f;
+  for (int s = threadIdx.x; s < max_splits; s += blockDim.x) {
+    const float* pp = base + s * stride;
     if (pp[0] > -INFINITY) l += pp[1] * expf(pp[0] - m);
   }
-  const int tok = q_start[dec_reqs[di]];
+  l = block_sum(l, red);
+  const int tok = q_start[dec_reqs[di]], quarter = threadIdx.x / SD_MERGE_COLS, c_in = threadIdx.x % SD_MERGE_COLS;
   const float inv = l > 0.f ? head_factor<T>(opt, tok, head) / l : 0.f;
   T* o = out + (size_t)tok * out_stride + (size_t)head * dv;
-  for (int c = threadIdx.x; c < dv; c += blockDim.x) {
+  for (int c0 = 0; c0 < dv; c0 += SD_MERGE_COLS) {
+    const int c = c0 + c_in;
     float a = 0.f;
-    for (int s = 0; s < max_splits; ++s) {
-      const float* pp = base + (size_t)s * sd_part_stride(dv);
-      if (pp[0] > -INFINITY) a += pp[2 + c] * expf(pp[0] - m);
+    if (c < dv) {
+#pragma unroll 4
+      for (int s = quarter; s < max_splits; s += SD_MERGE_PARTS) {
+        const float* pp = base + s * stride;
+        const float ms = pp[0], x = pp[2 + c];      // (a run without keys leaves its sums unwritten)
+        if (ms > -INFINITY) a += x * expf(ms - m);
+      }
     }
-    o[c] = from_float<T>(a * inv);
+    s_a[quarter][c_in] = a;
+    __syncthreads();
+    if (quarter == 0 && c < dv) {
+#pragma unroll
+      for (int w = 1; w < SD_MERGE_PARTS; ++w) a += s_a[w][c_in];
+      o[c] = from_float<T>(a * inv);
+    }
+    __syncthreads();
   }
 }
 
@@ -1124,6 +1356,12 @@ LLMRS_API int llmrs_scored_decode_group(int n_q_heads, int n_kv_heads, int dk, i
     return 0;
   const int G = n_q_heads / n_kv_heads;
   return G >= 3 ? 4 : G;
+}
+
+// Whether the decode kernel on the tensor cores takes these heads (bfloat16, keys and values of 64 or 128 channels). It streams
+// tiles through rings: callers give it longer runs of keys.
+LLMRS_API int llmrs_scored_decode_on_tensor_cores(int dk, int dv, int dtype) {
+  return dtype == LLMRS_BF16 && dk == dv && (dk == 64 || dk == 128) && !g_scored_generic_only;
 }
 
 LLMRS_API long long llmrs_scored_decode_scratch_floats(int n_dec, int n_q_heads, int dv, int max_splits) {
@@ -1159,6 +1397,25 @@ LLMRS_API int llmrs_scored_decode(const void* q, long long q_stride, void* out, 
   const int gh = llmrs_scored_decode_group(n_q_heads, n_kv_heads, dk, dv, page_size, dtype);
   const bool grouped = gh > 0 && ((uintptr_t)cache & 15) == 0 && !g_scored_generic_only;
   const int G = n_q_heads / n_kv_heads;
+  if (llmrs_scored_decode_on_tensor_cores(dk, dv, dtype) && ((uintptr_t)cache & 15) == 0 && ((uintptr_t)q & 3) == 0 &&
+      q_stride % 2 == 0 && n_kv_heads * ((G + 3) / 4) <= 65535) {
+    const dim3 tgrid(n_dec, n_kv_heads * ((G + 3) / 4), max_splits);
+    auto go = [&](auto kernel, int ring) {
+      const int bytes = SD_WARPS * ring;
+      const cudaError_t e = cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, bytes);
+      if (e != cudaSuccess) return llmrs_fail("scored_decode: shared memory %d: %s", bytes, cudaGetErrorString(e));
+      kernel<<<tgrid, SD_THREADS, bytes, stream>>>((const bf16*)q, q_stride, (const bf16*)cache, dec_reqs, q_start, cached_len,
+                                                   block_table, table_stride, scratch, max_splits, split_keys, n_q_heads,
+                                                   n_kv_heads, page_size, opt);
+      return llmrs_launch_status("scored_decode (tensor cores)");
+    };
+    const int rc = dk == 128 ? go(scored_decode_mma_kernel<128>, sm_ring_bytes<128>())
+                             : go(scored_decode_mma_kernel<64>, sm_ring_bytes<64>());
+    if (rc) return rc;
+    scored_decode_merge_kernel<bf16><<<mgrid, SD_MERGE_PARTS * SD_MERGE_COLS, 0, stream>>>(
+        scratch, (bf16*)out, out_stride, dec_reqs, q_start, max_splits, n_q_heads, dv, opt);
+    return llmrs_launch_status("scored_decode (merge)");
+  }
   dim3 ggrid(n_dec, grouped ? n_kv_heads * ((G + gh - 1) / gh) : 1, max_splits);
   const size_t gsmem = grouped ? ((size_t)gh * dk + (size_t)SD_WARPS * gh * dv) * sizeof(float) : 0;
   LLMRS_REQUIRE(ggrid.y <= 65535, "scored_decode: too many head groups");
@@ -1191,13 +1448,13 @@ LLMRS_API int llmrs_scored_decode(const void* q, long long q_stride, void* out, 
     LLMRS_SD_LAUNCH(float);
     int rc = llmrs_launch_status("scored_decode");
     if (rc) return rc;
-    scored_decode_merge_kernel<float><<<mgrid, 64, 0, stream>>>(scratch, (float*)out, out_stride, dec_reqs, q_start,
+    scored_decode_merge_kernel<float><<<mgrid, SD_MERGE_PARTS * SD_MERGE_COLS, 0, stream>>>(scratch, (float*)out, out_stride, dec_reqs, q_start,
                                                                 max_splits, n_q_heads, dv, opt);
   } else if (dtype == LLMRS_BF16) {
     LLMRS_SD_LAUNCH(bf16);
     int rc = llmrs_launch_status("scored_decode");
     if (rc) return rc;
-    scored_decode_merge_kernel<bf16><<<mgrid, 64, 0, stream>>>(scratch, (bf16*)out, out_stride, dec_reqs, q_start,
+    scored_decode_merge_kernel<bf16><<<mgrid, SD_MERGE_PARTS * SD_MERGE_COLS, 0, stream>>>(scratch, (bf16*)out, out_stride, dec_reqs, q_start,
                                                                max_splits, n_q_heads, dv, opt);
   } else {
     return llmrs_fail("scored_decode: unknown dtype %d", dtype);

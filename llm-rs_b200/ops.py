@@ -1365,6 +1365,21 @@ def scored_decode_group(n_q_heads: int, n_kv_heads: int, dk: int, dv: int, page_
     return int(_lib().llmrs_scored_decode_group(n_q_heads, n_kv_heads, dk, dv, page_size, dtype_code(dtype)))
 
 
+DECODE_STREAM_BLOCKS = 1184     # blocks of the tensor-core decode kernel that a step's runs of keys are cut for (four waves)
+
+
+def scored_decode_runs(n_dec: int, n_q_heads: int, n_kv_heads: int, dk: int, dv: int, dtype: torch.dtype, span: int):
+    """(runs, keys per run) for the tensor-core decode kernel over at most ``span`` visible keys, or None where it does not take
+    these heads. A run of 64 keys is one tile for each of a block's four warps; longer runs keep their rings full, and the
+    merge reads fewer of them."""
+    if not _lib().llmrs_scored_decode_on_tensor_cores(dk, dv, dtype_code(dtype)):
+        return None
+    blocks = n_dec * n_kv_heads * -(-(n_q_heads // n_kv_heads) // 4)
+    runs = max(1, min(-(-DECODE_STREAM_BLOCKS // blocks), -(-span // 64)))
+    keys = -(-(-(-span // runs)) // 64) * 64
+    return -(-span // keys), keys
+
+
 def scored_decode(q, out, cache, dec_reqs, n_dec: int, ctx, table, max_splits: int, split_keys: int, n_q_heads: int,
                   n_kv_heads: int, dk: int, dv: int, page_size: int, scale: float, softcap: float, sink, mask: int,
                   mask_size: int, bias: Optional[torch.Tensor] = None, out_scale: float = 1.0, keep: int = 0,

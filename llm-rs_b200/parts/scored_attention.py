@@ -254,8 +254,10 @@ class ScoredAttention(Mixer):
                 n_decode * self.n_heads
             while blocks * -(-span // split_keys) > DECODE_MAX_BLOCKS and split_keys < 4096:
                 split_keys *= 2
-            ops.scored_decode(q, out, pages, plan.arrays["decode_reqs"], n_decode, ctx, table, -(-span // split_keys),
-                              split_keys, *args, bias=self.bias, out_scale=scale, keep=self.keep_first, gate=head_gate)
+            runs = ops.scored_decode_runs(n_decode, self.n_heads, self.n_kv_heads, self.dim, self.vdim, q.dtype, span)
+            n_runs, split_keys = runs if runs is not None else (-(-span // split_keys), split_keys)
+            ops.scored_decode(q, out, pages, plan.arrays["decode_reqs"], n_decode, ctx, table, n_runs, split_keys, *args,
+                              bias=self.bias, out_scale=scale, keep=self.keep_first, gate=head_gate)
         if gate is not None:
             ops.head_gate(out, gate, self.n_heads, self.vdim, out_scale)
         return out
