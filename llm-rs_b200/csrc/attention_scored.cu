@@ -263,6 +263,168 @@ __global__ void scored_prepare_kernel(T* __restrict__ q, long long q_stride, con
   write_values(page, slot);
 }
 
+// The same for bfloat16 rows that can be read sixteen bytes a load, without projection biases and without unit or mixed values.
+// A thread takes sixteen channels of a head, the two pieces of eight that turn together; a head's threads are neighbouring
+// lanes. An angle is made once by one thread (a sine and cosine in double are most of the kernel above, where the threads of
+// a token that has fewer angles than threads wait for them); TOK tokens a block give every thread about one.
+// Bound by memory. 2,048 tokens of 16 + 4 heads of 128, unit heads: 43 -> 14.4 us; 48 tokens: 7.0 -> 5.7.
+constexpr int SPW_THREADS = 256;
+template <int TOK>
+__global__ void __launch_bounds__(SPW_THREADS)
+scored_prepare_wide_kernel(bf16* __restrict__ q, long long q_stride, const bf16* __restrict__ k, long long k_stride,
+                           const bf16* __restrict__ v, long long v_stride, const float* __restrict__ q_norm_w,
+                           const float* __restrict__ k_norm_w, const double* __restrict__ inv_freq,
+                           const int* __restrict__ positions, const int* __restrict__ token_req,
+                           const int* __restrict__ block_table, int table_stride, bf16* __restrict__ cache, int n_tokens,
+                           int n_q_heads, int n_kv_heads, int dk, int dv, int rot_dims, int page_size, float eps, int head_norm,
+                           int pairs) {
+  constexpr int TPT = SPW_THREADS / TOK, WPT = TPT / 32;      // a token's threads and warps
+  struct alignas(16) Piece { bf16 x[8]; };
+  extern __shared__ float2 s_turn[];      // [TOK][half]: cosine, sine
+  __shared__ float red[2][SPW_THREADS / 32];
+  const int half = rot_dims / 2, lt = threadIdx.x % TPT, t = blockIdx.x * TOK + threadIdx.x / TPT;
+  for (int e = threadIdx.x; e < TOK * half; e += SPW_THREADS) {
+    const int tok = blockIdx.x * TOK + e / half;
+    if (tok < n_tokens) {
+      double s, c;
+      sincos((double)positions[tok] * inv_freq[e % half], &s, &c);
+      s_turn[e] = make_float2((float)c, (float)s);
+    }
+  }
+  const bool here = t < n_tokens;
+  bf16* q_row = q + (size_t)t * q_stride;
+  const bf16* k_row = k + (size_t)t * k_stride;
+  auto read = [](const bf16* from, float (&x)[8]) {
+    const Piece in = *reinterpret_cast<const Piece*>(from);
+#pragma unroll
+    for (int e = 0; e < 8; ++e) x[e] = __bfloat162float(in.x[e]);
+  };
+  float inv_q = 1.0f, inv_k = 1.0f;
+  if (!head_norm && (q_norm_w || k_norm_w)) {
+    float sq = 0.f, sk = 0.f, x[8];
+    if (here) {
+      for (int c = lt * 8; c < n_q_heads * dk; c += TPT * 8) {
+        read(q_row + c, x);
+#pragma unroll
+        for (int e = 0; e < 8; ++e) sq = fmaf(x[e], x[e], sq);
+      }
+      for (int c = lt * 8; k && c < n_kv_heads * dk; c += TPT * 8) {
+        read(k_row + c, x);
+#pragma unroll
+        for (int e = 0; e < 8; ++e) sk = fmaf(x[e], x[e], sk);
+      }
+    }
+    sq = warp_sum(sq);
+    sk = warp_sum(sk);
+    if ((threadIdx.x & 31) == 0) {
+      red[0][threadIdx.x >> 5] = sq;
+      red[1][threadIdx.x >> 5] = sk;
+    }
+    __syncthreads();
+    const int w0 = threadIdx.x / TPT * WPT;
+    sq = sk = 0.f;
+#pragma unroll
+    for (int w = 0; w < WPT; ++w) {
+      sq += red[0][w0 + w];
+      sk += red[1][w0 + w];
+    }
+    if (q_norm_w) inv_q = 1.0f / sqrtf(sq / (float)(n_q_heads * dk) + eps);
+    if (k_norm_w) inv_k = 1.0f / sqrtf(sk / (float)(n_kv_heads * dk) + eps);
+  }
+  __syncthreads();      // the angles are there, and the rows have been read for their sums
+  if (!here) return;
+  const float2* turn = s_turn + threadIdx.x / TPT * half;
+  const int units = dk / 16, n_heads = n_q_heads + (k ? n_kv_heads : 0);
+  int page = 0, slot = 0;
+  if (k) {
+    const int pos = positions[t];
+    page = LLMRS_CHECKED_PAGE(block_table[(size_t)token_req[t] * table_stride + pos / page_size], 2, t);
+    slot = pos % page_size;
+  }
+  for (int u = lt; u < n_heads * units; u += TPT) {
+    const int hh = u / units, j = u - hh * units;
+    const bool is_q = hh < n_q_heads, halves = !pairs && j < rot_dims / 16;
+    const int head = is_q ? hh : hh - n_q_heads;
+    const int c0 = halves ? 8 * j : 16 * j, c1 = halves ? c0 + half : c0 + 8;
+    const bf16* row = (is_q ? q_row : k_row) + (size_t)head * dk;
+    const float* w = is_q ? q_norm_w : k_norm_w;
+    if (head_norm == 1) w = nullptr;
+    if (w && !head_norm) w += (size_t)head * dk;
+    float a[8], b[8];
+    read(row + c0, a);
+    read(row + c1, b);
+    auto head_factor_of = [&]() {      // 1 / the head's root mean square of what the head's lanes hold
+      float ss = 0.f;
+#pragma unroll
+      for (int e = 0; e < 8; ++e) ss = fmaf(a[e], a[e], fmaf(b[e], b[e], ss));
+      const unsigned lanes = (units == 32 ? 0xffffffffu : (1u << units) - 1u) << (threadIdx.x & 31 & ~(units - 1));
+      for (int o = units / 2; o > 0; o >>= 1) ss += __shfl_xor_sync(lanes, ss, o);
+      return 1.0f / sqrtf(ss / (float)dk + eps);
+    };
+    const float inv = head_norm == 2 ? head_factor_of() : (head_norm ? 1.0f : (is_q ? inv_q : inv_k));
+#pragma unroll
+    for (int e = 0; e < 8; ++e) {
+      a[e] *= inv;
+      b[e] *= inv;
+    }
+    if (w) {
+#pragma unroll
+      for (int e = 0; e < 8; ++e) {
+        a[e] *= w[c0 + e];
+        b[e] *= w[c1 + e];
+      }
+    }
+    if (halves) {
+#pragma unroll
+      for (int e = 0; e < 8; ++e) {
+        const float2 r = turn[c0 + e];
+        const float x = a[e], y = b[e];
+        a[e] = x * r.x - y * r.y;
+        b[e] = y * r.x + x * r.y;
+      }
+    } else if (pairs) {
+      auto neighbours = [&](float (&x)[8], int c) {
+#pragma unroll
+        for (int e = 0; e < 8; e += 2)
+          if (c + e < rot_dims) {
+            const float2 r = turn[(c + e) >> 1];
+            const float lo = x[e], hi = x[e + 1];
+            x[e] = lo * r.x - hi * r.y;
+            x[e + 1] = hi * r.x + lo * r.y;
+          }
+      };
+      neighbours(a, c0);
+      neighbours(b, c1);
+    }
+    if (head_norm == 1) {
+      const float unit = head_factor_of();
+#pragma unroll
+      for (int e = 0; e < 8; ++e) {
+        a[e] *= unit;
+        b[e] *= unit;
+      }
+    }
+    bf16* to = is_q ? q_row + (size_t)head * dk
+                    : cache + page_head_offset(page, head, n_kv_heads, page_size, dk, dv) + (size_t)slot * dk;
+    Piece first, second;
+#pragma unroll
+    for (int e = 0; e < 8; ++e) {
+      first.x[e] = __float2bfloat16_rn(a[e]);
+      second.x[e] = __float2bfloat16_rn(b[e]);
+    }
+    *reinterpret_cast<Piece*>(to + c0) = first;
+    *reinterpret_cast<Piece*>(to + c1) = second;
+  }
+  if (k == nullptr) return;
+  const bf16* v_row = v + (size_t)t * v_stride;
+  const int v_units = dv / 8;
+  for (int u = lt; u < n_kv_heads * v_units; u += TPT) {
+    const int head = u / v_units, c = (u - head * v_units) * 8;
+    *reinterpret_cast<Piece*>(cache + page_head_offset(page, head, n_kv_heads, page_size, dk, dv) + (size_t)page_size * dk +
+                              (size_t)slot * dv + c) = *reinterpret_cast<const Piece*>(v_row + (size_t)head * dv + c);
+  }
+}
+
 // q: [tokens, n_q_heads * dk] rewritten in place; k, v: the new keys and values (null: the entry reads another
 // entry's pages and writes none); cache: one entry's pages. unit_values: every head's value is divided by its root mean
 // square before it is kept; v_first ([tokens, n_kv_heads * dv], rows v_first_stride apart) with v_mix (one float on the
@@ -285,6 +447,24 @@ LLMRS_API int llmrs_scored_prepare(void* q, long long q_stride, const void* k, l
   if (n_tokens == 0) return 0;
   const size_t smem = ((size_t)(n_q_heads + n_kv_heads) * dk + rot_dims) * sizeof(float);
   LLMRS_REQUIRE(smem <= 160 * 1024, "scored_prepare: rows of %zu bytes are too wide", smem);
+  // Sixteen bytes a load and store: every piece of eight channels on a boundary, pairs of pieces that turn together; heads
+  // with their own norm have a power of two of threads. Blocks of four tokens where that still gives the device four a
+  // multiprocessor.
+  auto wide_rows = [](const void* p, long long stride) { return ((uintptr_t)p & 15) == 0 && stride % 8 == 0; };
+  const int units = dk / 16;
+  if (dtype == LLMRS_BF16 && !proj_bias && !unit_values && !v_first && dk % 16 == 0 && dv % 8 == 0 &&
+      (pairs || rot_dims % 16 == 0) && (!head_norm || (units <= 32 && (units & (units - 1)) == 0)) && wide_rows(q, q_stride) &&
+      (k == nullptr || (wide_rows(k, k_stride) && wide_rows(v, v_stride) && wide_rows(cache, 8))) && !g_scored_generic_only) {
+#define LLMRS_SPW_LAUNCH(TOK)                                                                                              \
+  scored_prepare_wide_kernel<TOK><<<(n_tokens + TOK - 1) / TOK, SPW_THREADS, (size_t)TOK * rot_dims * sizeof(float), stream>>>( \
+      (bf16*)q, q_stride, (const bf16*)k, k_stride, (const bf16*)v, v_stride, q_norm_w, k_norm_w, inv_freq, positions,     \
+      token_req, block_table, table_stride, (bf16*)cache, n_tokens, n_q_heads, n_kv_heads, dk, dv, rot_dims, page_size, eps, \
+      head_norm, pairs)
+    if (n_tokens >= 4 * 148) LLMRS_SPW_LAUNCH(4);
+    else LLMRS_SPW_LAUNCH(1);
+#undef LLMRS_SPW_LAUNCH
+    return llmrs_launch_status("scored_prepare");
+  }
   const int threads = n_q_heads * dk >= 2048 ? 512 : 256;
 #define LLMRS_SP_LAUNCH(T)                                                                                          \
   do {                                                                                                              \

@@ -95,3 +95,40 @@ def test_decode_keeps_infinite_values(generic):
     rest = torch.ones_like(before, dtype=torch.bool)
     rest[0, :, 5], rest[0, :, 6], rest[1, :, 8] = False, False, False
     assert torch.equal(before[rest], after[rest])
+
+
+@pytest.mark.parametrize("dk,dv,rot,pairs", [(128, 128, 128, False), (64, 64, 32, False), (128, 64, 64, True), (96, 72, 96, False),
+                                             (64, 64, 12, True), (64, 64, 0, False), (16, 8, 16, False), (512, 64, 64, False)])
+@pytest.mark.parametrize("norm", ["none", "whole", "unit", "shared"])
+@pytest.mark.parametrize("n,kv", [(1, 2), (597, 1), (7, 0)])
+def test_prepare_by_pieces_is_the_general_kernel(dk, dv, rot, pairs, norm, n, kv):
+    """Both kernels compute in float32 and round once: they differ by one bfloat16 rounding at most."""
+    from llm_rs_b200 import ops
+    torch.manual_seed(dk + rot + n)
+    heads, page = 4, 16
+    kvh = max(kv, 1)
+    q0 = torch.randn(n, heads * dk + 8, device=DEV).bfloat16()
+    k = torch.randn(n, kvh * dk + 16, device=DEV).bfloat16()[:, : kvh * dk] if kv else None
+    v = torch.randn(n, kvh * dv, device=DEV).bfloat16() if kv else None
+    i32 = lambda x: torch.tensor(x, dtype=torch.int32, device=DEV)
+    n_pages = -(-(n + 5) // page)
+    table = torch.randperm(n_pages, device=DEV).to(torch.int32).view(1, n_pages)
+    ctx = SimpleNamespace(positions=i32(list(range(5, n + 5))), token_req=i32([0] * n))
+    inv_freq = 10000.0 ** (-torch.arange(rot // 2, dtype=torch.float64, device=DEV) / max(rot // 2, 1))
+    wq = wk = None
+    if norm in ("whole", "shared"):
+        wq = torch.rand(dk if norm == "shared" else heads * dk, device=DEV) + 0.5
+        wk = torch.rand(dk if norm == "shared" else kvh * dk, device=DEV) + 0.5
+    got = []
+    for generic in (True, False):
+        q = q0.clone()[:, : heads * dk]
+        cache = torch.zeros(n_pages, kvh, page * (dk + dv), device=DEV).bfloat16()
+        ops.scored_generic_only(generic)
+        try:
+            ops.scored_prepare(q, k, v, wq, wk, inv_freq, ctx, table, cache if kv else None, heads, kvh, dk, dv, rot, page, 1e-6,
+                               unit_heads=norm == "unit", shared_head_norm=norm == "shared", pairs=pairs)
+        finally:
+            ops.scored_generic_only(False)
+        got.append((q.float(), cache.float()))
+    for a, b in zip(*got):
+        assert bool(((a - b).abs() <= 2.0 ** -7 * a.abs() + 1e-5).all())
