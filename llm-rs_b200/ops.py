@@ -1178,7 +1178,7 @@ def gate_scan(gates: torch.Tensor, cap: float, m_state: torch.Tensor, ctx, n_hea
     decay, gain, floor = (torch.empty((n, n_heads), dtype=torch.float32, device=gates.device) for _ in range(3))
     _check(_lib().llmrs_gate_scan(_ptr(gates), _LL(_row_stride(gates, "gates")), ctypes.c_float(cap), _ptr(m_state),
                                   _ptr(ctx.q_start), _ptr(ctx.n_new), _ptr(ctx.slot_ids), _ptr(decay), _ptr(gain),
-                                  _ptr(floor), ctx.n_requests, n_heads, _stream()), "gate_scan")
+                                  _ptr(floor), n, ctx.n_requests, n_heads, _stream()), "gate_scan")
     return decay, gain, floor
 
 
