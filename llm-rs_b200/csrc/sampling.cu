@@ -11,7 +11,13 @@
 // and draws in vocabulary order with a Philox4x32-10 number keyed by (seed; request id,
 // index of the generated token), so a request's tokens do not depend on what else is
 // in the batch. The distribution drawn from is the reference's.
+//
+// Few rows are spread over the device, eight blocks a row (sample_spread_kernel); many rows run with a block each.
+#include <cooperative_groups.h>
+
 #include "common.cuh"
+
+namespace cg = cooperative_groups;
 
 constexpr int SM_THREADS = 1024;
 
@@ -193,6 +199,77 @@ __device__ uint32_t select_cut(const float* __restrict__ x, int vocab, uint32_t 
   return prefix > floor_bits ? prefix : floor_bits;
 }
 
+// The run among SM_THREADS consecutive runs of the vocabulary, `v` the kept mass of run threadIdx.x, in which a uniform number
+// times the total falls: the first run whose running sum (a fixed order of additions) exceeds it. d->run < 0: nothing is kept.
+struct Draw {
+  float target, before;      // before < 0: rounding left the target at or above the sum, the last run with kept mass owns it
+  int run;
+  float wsum[32];
+  int wfirst[32], wlast[32];
+};
+__device__ void draw_run(Draw* d, float v, int row, const unsigned long long* __restrict__ seeds,
+                         const unsigned long long* __restrict__ request_ids, const int* __restrict__ gen_index) {
+  const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
+  uint32_t r[4];
+  const unsigned long long seed = seeds ? seeds[row] : 0ull, rid = request_ids ? request_ids[row] : 0ull;
+  philox4x32_10((uint32_t)seed, (uint32_t)(seed >> 32), (uint32_t)rid, (uint32_t)(rid >> 32),
+                gen_index ? (uint32_t)gen_index[row] : 0u, 0u, r);
+  const float u = (float)(r[0] >> 8) * (1.0f / 16777216.0f);
+  if (tid == 0) d->run = -1;
+  float incl = v;
+#pragma unroll
+  for (int o = 1; o < 32; o <<= 1) {
+    const float up = __shfl_up_sync(0xffffffffu, incl, o);
+    if (lane >= o) incl += up;
+  }
+  if (lane == 31) d->wsum[warp] = incl;
+  __syncthreads();
+  float before_warp = 0.f, total = 0.f;
+  for (int w = 0; w < SM_THREADS / 32; ++w) {
+    if (w == warp) before_warp = total;
+    total += d->wsum[w];
+  }
+  incl += before_warp;
+  const float target = u * total;
+  const unsigned hit = __ballot_sync(0xffffffffu, incl > target);
+  const unsigned kept = __ballot_sync(0xffffffffu, v > 0.f);
+  if (lane == 0) {
+    d->wfirst[warp] = hit ? warp * 32 + __ffs(hit) - 1 : 0x7fffffff;
+    d->wlast[warp] = kept ? warp * 32 + 31 - __clz(kept) : -1;
+  }
+  __syncthreads();
+  int first = 0x7fffffff, last = -1;
+  for (int w = 0; w < SM_THREADS / 32; ++w) {
+    first = min(first, d->wfirst[w]);
+    last = max(last, d->wlast[w]);
+  }
+  if (first != 0x7fffffff) {
+    if (tid == first) { d->before = incl - v; d->target = target; d->run = first; }
+  } else if (tid == 0) {
+    d->before = -1.f;
+    d->target = target;
+    d->run = last;
+  }
+  __syncthreads();
+}
+// The token of a run of `n` values (indices from `lo` on) in which the target falls; one thread calls it.
+__device__ int walk_run(const Draw* d, const float* __restrict__ x, int n, int lo, float cut, int fallback) {
+  int pick = -1, last_kept = -1;
+  float run = d->before;
+  for (int i = 0; i < n; ++i) {
+    const float e = x[i];
+    if (e >= cut && e > 0.f) {
+      last_kept = lo + i;
+      if (d->before >= 0.f) {
+        run += e;
+        if (run > d->target) { pick = lo + i; break; }
+      }
+    }
+  }
+  // The walk reached the run's end without a pick: rounding; take the run's last kept token.
+  return pick >= 0 ? pick : (last_kept >= 0 ? last_kept : fallback);
+}
+
 // logits [n_rows, vocab] are changed in place (penalty, then exp(x - max)).
 __global__ void __launch_bounds__(SM_THREADS)
 sample_kernel(float* __restrict__ logits, int vocab, const float* __restrict__ temperature,
@@ -203,7 +280,7 @@ sample_kernel(float* __restrict__ logits, int vocab, const float* __restrict__ t
   __shared__ ArgMax ared[33];
   __shared__ SelectScratch sel;
   __shared__ float scan[SM_THREADS];
-  __shared__ int chosen;
+  __shared__ Draw draw;
   const int row = blockIdx.x, tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
   float* x = logits + (size_t)row * vocab;
 
@@ -304,81 +381,214 @@ sample_kernel(float* __restrict__ logits, int vocab, const float* __restrict__ t
       if (lane == 0) scan[c + q] = part[q];
     }
   }
-  if (tid == 0) chosen = -1;
   __syncthreads();
-  uint32_t r[4];
-  const unsigned long long seed = seeds ? seeds[row] : 0ull, rid = request_ids ? request_ids[row] : 0ull;
-  philox4x32_10((uint32_t)seed, (uint32_t)(seed >> 32), (uint32_t)rid, (uint32_t)(rid >> 32),
-                gen_index ? (uint32_t)gen_index[row] : 0u, 0u, r);
-  const float u = (float)(r[0] >> 8) * (1.0f / 16777216.0f);
-  __shared__ float s_target, s_before, wsum[32];
-  __shared__ int wfirst[32], wlast[32];
-  {
-    // Running sums of the 1024 runs by a block-wide scan (a fixed order of additions), then the first
-    // run whose running sum exceeds the target.
-    const float v = scan[tid];
-    float incl = v;
-#pragma unroll
-    for (int o = 1; o < 32; o <<= 1) {
-      const float up = __shfl_up_sync(0xffffffffu, incl, o);
-      if (lane >= o) incl += up;
-    }
-    if (lane == 31) wsum[warp] = incl;
-    __syncthreads();
-    float before_warp = 0.f, total = 0.f;
-    for (int w = 0; w < SM_THREADS / 32; ++w) {
-      if (w == warp) before_warp = total;
-      total += wsum[w];
-    }
-    incl += before_warp;
-    const float target = u * total;
-    const unsigned hit = __ballot_sync(0xffffffffu, incl > target);
-    const unsigned kept = __ballot_sync(0xffffffffu, v > 0.f);
-    if (lane == 0) {
-      wfirst[warp] = hit ? warp * 32 + __ffs(hit) - 1 : 0x7fffffff;
-      wlast[warp] = kept ? warp * 32 + 31 - __clz(kept) : -1;
-    }
-    __syncthreads();
-    int first = 0x7fffffff, last = -1;
-    for (int w = 0; w < SM_THREADS / 32; ++w) {
-      first = min(first, wfirst[w]);
-      last = max(last, wlast[w]);
-    }
-    if (first != 0x7fffffff) {
-      if (tid == first) { s_before = incl - v; s_target = target; chosen = first; }
-    } else if (tid == 0) {
-      // Rounding left the target at or above the sum: the last run with kept mass owns it.
-      s_before = -1.f;
-      s_target = target;
-      chosen = last;
-    }
-  }
-  __syncthreads();
-  const int owner = chosen;
+  draw_run(&draw, scan[tid], row, seeds, request_ids, gen_index);
   if (tid == 0) {
-    if (owner < 0) {
-      out_tokens[row] = best.i;
-    } else {
-      const float target = s_target, before = s_before;
-      const int lo = min(owner * chunk, vocab), hi = min(lo + chunk, vocab);
-      int pick = -1, last_kept = -1;
-      float run = before;
-      for (int i = lo; i < hi; ++i) {
-        const float e = x[i];
-        if (e >= cut && e > 0.f) {
-          last_kept = i;
-          if (before >= 0.f) {
-            run += e;
-            if (run > target) { pick = i; break; }
-          }
-        }
-      }
-      // The walk reached the run's end without a pick: rounding; take the run's last kept token.
-      if (pick < 0) pick = last_kept >= 0 ? last_kept : best.i;
-      out_tokens[row] = pick;
-    }
+    const int lo = min(max(draw.run, 0) * chunk, vocab), hi = min(lo + chunk, vocab);
+    out_tokens[row] = draw.run < 0 ? best.i : walk_run(&draw, x + lo, hi - lo, lo, cut, best.i);
   }
 }
+
+// The same choice with eight blocks (a cluster) a row: block b holds runs 128 b .. 128 b + 127 of the row's SM_THREADS runs in
+// shared memory, read once, where the kernel of a block per row reads the row from the L2 up to nine times. Histograms are
+// added up through distributed shared memory, an eighth of the bins by each block (whole numbers: no order), the runs' sums are made and
+// scanned in the same order, so the tokens are the same.
+constexpr int SS_BLOCKS = 8, SS_RUNS = SM_THREADS / SS_BLOCKS, SS_BINS = SEL_BINS / SS_BLOCKS;
+
+struct SpreadScratch {
+  SelectScratch sel;
+  unsigned long long part[SM_THREADS / SS_BINS][SS_BINS], totals[SS_BLOCKS];
+  ArgMax red[33], block_best[SS_BLOCKS];
+  unsigned long long block_mass;
+  float scan[SS_RUNS];
+  Draw draw;
+};
+
+// select_cut over the values of the cluster's blocks; every block finds the same cut.
+__device__ uint32_t select_cut_spread(cg::cluster_group& cluster, const float* x, int n, uint32_t floor_bits,
+                                      unsigned long long need, bool by_mass, SpreadScratch* sc) {
+  const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5, rank = (int)cluster.block_rank();
+  uint32_t prefix = 0, prefix_mask = 0;
+  const int shifts[3] = {19, 8, 0}, widths[3] = {11, 11, 8};
+  if (need == 0) need = 1;
+#pragma unroll 1
+  for (int level = 0; level < 3; ++level) {
+    for (int i = tid; i < SEL_BINS; i += SM_THREADS) sc->sel.lo[i] = sc->sel.hi[i] = 0u;
+    __syncthreads();
+    const int shift = shifts[level];
+    const uint32_t digit_mask = (1u << widths[level]) - 1u;
+    for (int i = tid; i < n; i += SM_THREADS) {
+      const float e = x[i];
+      const uint32_t bits = __float_as_uint(e);
+      if (bits >= floor_bits && (bits & prefix_mask) == prefix)
+        bin_add(&sc->sel, (bits >> shift) & digit_mask, by_mass ? to_fixed(e) : 1ull);
+    }
+    cluster.sync();      // every block's histogram is there
+    // Block b adds up the b-th eighth of the bins from the top; its sum goes to every block.
+    const int at = tid % SS_BINS, mine = SEL_BINS - 1 - rank * SS_BINS - at;
+    unsigned long long v = 0;
+    for (int r = tid / SS_BINS; r < SS_BLOCKS; r += SM_THREADS / SS_BINS) v += bin_value(cluster.map_shared_rank(&sc->sel, r), mine);
+    sc->part[tid / SS_BINS][at] = v;
+    __syncthreads();
+    unsigned long long incl = 0;
+    if (tid < SS_BINS) {
+      v = 0;
+#pragma unroll
+      for (int r = 0; r < SM_THREADS / SS_BINS; ++r) v += sc->part[r][at];
+      incl = v;
+#pragma unroll
+      for (int o = 1; o < 32; o <<= 1) {
+        const unsigned long long up = __shfl_up_sync(0xffffffffu, incl, o);
+        if (lane >= o) incl += up;
+      }
+      if (lane == 31) sc->sel.warp_tot[warp] = incl;
+    }
+    __syncthreads();
+    unsigned long long before = 0, total = 0;
+    for (int w = 0; w < SS_BINS / 32; ++w) {
+      if (w < warp) before += sc->sel.warp_tot[w];
+      total += sc->sel.warp_tot[w];
+    }
+    if (tid < SS_BLOCKS) cluster.map_shared_rank(sc, tid)->totals[rank] = total;
+    cluster.sync();      // the sums are there, and every block has read the histograms
+    unsigned long long all = 0;
+#pragma unroll
+    for (int r = 0; r < SS_BLOCKS; ++r) {
+      if (r < rank) before += sc->totals[r];
+      all += sc->totals[r];
+    }
+    if (all < need) return floor_bits;      // (in every block alike)
+    before += incl - v;
+    if (tid < SS_BINS && before < need && before + v >= need)      // one thread of the cluster
+      for (int r = 0; r < SS_BLOCKS; ++r) {
+        SpreadScratch* to = cluster.map_shared_rank(sc, r);
+        to->sel.found_bin = mine;
+        to->sel.found_above = before;
+      }
+    cluster.sync();
+    const int bin = sc->sel.found_bin;
+    need -= sc->sel.found_above;
+    prefix |= (uint32_t)bin << shift;
+    prefix_mask |= digit_mask << shift;
+  }
+  return prefix > floor_bits ? prefix : floor_bits;
+}
+
+__global__ void __cluster_dims__(SS_BLOCKS, 1, 1) __launch_bounds__(SM_THREADS, 2)
+sample_spread_kernel(const float* __restrict__ logits, int vocab, const float* __restrict__ temperature,
+                     const int* __restrict__ top_k, const float* __restrict__ top_p, const float* __restrict__ penalty,
+                     const int* __restrict__ hist_tokens, const int* __restrict__ hist_offsets,
+                     const unsigned long long* __restrict__ seeds, const unsigned long long* __restrict__ request_ids,
+                     const int* __restrict__ gen_index, int* __restrict__ out_tokens) {
+  extern __shared__ __align__(16) float x[];      // this block's values, then room for one run
+  __shared__ __align__(16) SpreadScratch sc;
+  cg::cluster_group cluster = cg::this_cluster();
+  const int row = blockIdx.x / SS_BLOCKS, rank = blockIdx.x % SS_BLOCKS, tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
+  const int chunk = (vocab + SM_THREADS - 1) / SM_THREADS;
+  const int lo = min(rank * SS_RUNS * chunk, vocab), n = min(SS_RUNS * chunk, vocab - lo);
+  const float* src = logits + (size_t)row * vocab + lo;
+  if ((vocab & 3) == 0 && (reinterpret_cast<uintptr_t>(src) & 15) == 0) {      // n is then a multiple of four too
+    const float4* s4 = reinterpret_cast<const float4*>(src);
+    for (int i = tid; i < n / 4; i += SM_THREADS) reinterpret_cast<float4*>(x)[i] = s4[i];
+  } else {
+    for (int i = tid; i < n; i += SM_THREADS) x[i] = src[i];
+  }
+  __syncthreads();
+  const float pen = penalty ? penalty[row] : 1.0f;
+  if (pen != 1.0f && hist_offsets) {
+    for (int j = hist_offsets[row] + tid; j < hist_offsets[row + 1]; j += SM_THREADS) {
+      const int idx = hist_tokens[j] - lo;      // distinct tokens: each index is touched once
+      if (idx >= 0 && idx < n) {
+        const float v = x[idx];
+        x[idx] = v > 0.f ? v / pen : v * pen;
+      }
+    }
+    __syncthreads();
+  }
+  const float T = temperature ? temperature[row] : 0.f;
+  ArgMax best{-INFINITY, 0x7fffffff};
+  for (int i = tid; i < n; i += SM_THREADS) best = better(best, ArgMax{x[i], lo + i});
+  best = block_argmax(best, sc.red);
+  cluster.sync();      // every block runs before its shared memory is written from outside
+  if (tid < SS_BLOCKS) *cluster.map_shared_rank(&sc.block_best[rank], tid) = best;
+  cluster.sync();
+  best = ArgMax{-INFINITY, 0x7fffffff};
+#pragma unroll
+  for (int r = 0; r < SS_BLOCKS; ++r) best = better(best, sc.block_best[r]);
+  if (best.i >= vocab) best.i = 0;      // a row of NaN has no maximum
+  if (T <= 1e-5f) {
+    if (rank == 0 && tid == 0) out_tokens[row] = best.i;
+    return;
+  }
+  const float mx = best.v / T;
+  for (int i = tid; i < n; i += SM_THREADS) {
+    const float e = expf(x[i] / T - mx);
+    x[i] = e >= 0.f ? e : 0.f;      // a NaN logit keeps no mass
+  }
+  __syncthreads();
+  uint32_t cut_bits = 0u;      // keep e_i >= cut
+  const int k = top_k ? top_k[row] : 0;
+  if (k > 0 && k < vocab) cut_bits = select_cut_spread(cluster, x, n, 0u, (unsigned long long)k, false, &sc);
+  const float p = top_p ? top_p[row] : 1.0f;
+  if (p < 1.0f) {
+    unsigned long long part = 0;      // the mass of what top_k kept
+    for (int i = tid; i < n; i += SM_THREADS)
+      if (__float_as_uint(x[i]) >= cut_bits) part += to_fixed(x[i]);
+#pragma unroll
+    for (int o = 16; o > 0; o >>= 1) part += __shfl_xor_sync(0xffffffffu, part, o);
+    __syncthreads();
+    if (lane == 0) sc.sel.warp_tot[warp] = part;
+    __syncthreads();
+    if (tid == 0) {
+      unsigned long long mass = 0;
+      for (int w = 0; w < SM_THREADS / 32; ++w) mass += sc.sel.warp_tot[w];
+      sc.block_mass = mass;
+    }
+    cluster.sync();
+    unsigned long long total_fx = 0;
+#pragma unroll
+    for (int r = 0; r < SS_BLOCKS; ++r) total_fx += *cluster.map_shared_rank(&sc.block_mass, r);
+    const unsigned long long need = (unsigned long long)((double)total_fx * (double)p);
+    cut_bits = select_cut_spread(cluster, x, n, cut_bits, need, true, &sc);
+  }
+  const float cut = __uint_as_float(cut_bits);
+  {      // this block's runs, four a warp
+    const int c = warp * 4;
+    float part[4] = {0.f, 0.f, 0.f, 0.f};
+    for (int off = lane; off < chunk; off += 32) {
+#pragma unroll
+      for (int q = 0; q < 4; ++q) {
+        const int lo_c = min((c + q) * chunk, n), hi_c = min(lo_c + chunk, n);
+        const float e = lo_c + off < hi_c ? x[lo_c + off] : 0.f;
+        part[q] += e >= cut ? e : 0.f;
+      }
+    }
+#pragma unroll
+    for (int q = 0; q < 4; ++q) {
+#pragma unroll
+      for (int o = 16; o > 0; o >>= 1) part[q] += __shfl_xor_sync(0xffffffffu, part[q], o);
+      if (lane == 0) sc.scan[c + q] = part[q];
+    }
+  }
+  cluster.sync();
+  if (rank == 0) {
+    const float v = cluster.map_shared_rank(sc.scan, tid / SS_RUNS)[tid % SS_RUNS];
+    draw_run(&sc.draw, v, row, seeds, request_ids, gen_index);
+    const int run = max(sc.draw.run, 0), at = run % SS_RUNS * chunk;
+    const int first = min(run * chunk, vocab), len = min(first + chunk, vocab) - first;
+    const float* other = cluster.map_shared_rank(x, run / SS_RUNS) + at;
+    float* mine = x + SS_RUNS * chunk;
+    for (int i = tid; i < len; i += SM_THREADS) mine[i] = other[i];
+    __syncthreads();
+    if (tid == 0) out_tokens[row] = sc.draw.run < 0 ? best.i : walk_run(&sc.draw, mine, len, first, cut, best.i);
+  }
+  cluster.sync();      // no block leaves while its values may be read
+}
+
+// Eight blocks a row while all rows' clusters run at once, two blocks a multiprocessor, and a row is long enough to pay for the
+// clusters' barriers; a row must fit the shared memory of its blocks. A block a row against eight, us: 32 rows of 151,936
+// 117 / 71, 8 rows 113 / 51, one 94 / 35; 64 rows 118 / 132; 32 rows of 32,000 39 / 46, 8 rows 39 / 36.
+constexpr int SS_MAX_ROWS = 32, SS_MIN_CHUNK = 64, SS_MAX_CHUNK = 340;
 
 LLMRS_API int llmrs_sample(float* logits, int n_rows, int vocab, const float* temperature, const int* top_k,
                            const float* top_p, const float* penalty, const int* hist_tokens,
@@ -387,6 +597,16 @@ LLMRS_API int llmrs_sample(float* logits, int n_rows, int vocab, const float* te
                            cudaStream_t stream) {
   LLMRS_REQUIRE(n_rows >= 0 && vocab > 0, "sample: bad sizes");
   if (n_rows == 0) return 0;
+  const int chunk = (vocab + SM_THREADS - 1) / SM_THREADS;
+  if (n_rows <= SS_MAX_ROWS && chunk >= SS_MIN_CHUNK && chunk <= SS_MAX_CHUNK) {
+    const size_t smem = (size_t)(SS_RUNS + 1) * chunk * sizeof(float);
+    const cudaError_t e = cudaFuncSetAttribute(sample_spread_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
+    if (e != cudaSuccess) return llmrs_fail("sample: shared memory %zu: %s", smem, cudaGetErrorString(e));
+    sample_spread_kernel<<<n_rows * SS_BLOCKS, SM_THREADS, smem, stream>>>(logits, vocab, temperature, top_k, top_p, penalty,
+                                                                           hist_tokens, hist_offsets, seeds, request_ids,
+                                                                           gen_index, out_tokens);
+    return llmrs_launch_status("sample");
+  }
   sample_kernel<<<n_rows, SM_THREADS, 0, stream>>>(logits, vocab, temperature, top_k, top_p, penalty, hist_tokens,
                                                    hist_offsets, seeds, request_ids, gen_index, out_tokens);
   return llmrs_launch_status("sample");

@@ -927,3 +927,26 @@ def test_attention_tcgen05_wait_runs_out_and_the_kernel_returns(skip, nq):
         got = out.double().cpu()
         assert torch.isfinite(got).all() and float((got - want).abs().max()) < 2.5e-2
     ops.check_attention_error()
+
+
+@pytest.mark.parametrize("vocab", [151936, 65536, 64513, 100003, 348160])
+def test_sampler_spread_over_blocks_chooses_the_same(vocab):
+    """Few rows run with eight blocks a row, many with one: every row's token is the same either way, with cut-offs by
+    number, by mass and by both, penalties, ties at a cut-off, rows of one value, of NaN and of infinities."""
+    from llm_rs_b200.sampling import SamplingParams
+    from llm_rs_b200.sampling.sampler import Sampler
+    g = torch.Generator(device=DEV).manual_seed(vocab)
+    logits = torch.randn(120, vocab, generator=g, device=DEV) * 3
+    logits[7] = 1.5
+    logits[8] = float("nan")
+    logits[9, 5:] = float("-inf")
+    logits[10] = torch.round(logits[10])
+    logits[11, 3] = float("inf")
+    logits[12, ::2] = float("nan")
+    rows = [(SamplingParams(temperature=[0.7, 1.0, 1.3, 0.0][r % 4], top_k=[0, 40, 7, 0, 1][r % 5], top_p=[1.0, 0.9, 0.5][r % 3],
+                            repetition_penalty=[1.0, 1.2][r % 2], seed=r), r * 11, r, list(range(r, r + 50)))
+            for r in range(120)]
+    s = Sampler(DEV)
+    together = s.sample(logits.clone(), rows).cpu().tolist()
+    for a, b in ((0, 32), (32, 50), (90, 120), (7, 8), (8, 13)):
+        assert s.sample(logits[a:b].clone(), rows[a:b]).cpu().tolist() == together[a:b], (a, b)
