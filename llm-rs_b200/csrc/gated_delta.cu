@@ -18,8 +18,9 @@
 //
 //   prepare      a block per token: convolutions + SiLU, unit q and k, g and beta, as float32 rows
 //   conv state   a block per request, after prepare: the request's last K - 1 convolution inputs
-//   recurrence   of portions of 48 tokens and more: the coefficients of turns of four tokens, then the walk in turns
-//                (state_walk.cuh). Of single tokens and shorter portions: a block per (request, head, slice of 16 value
+//   (steps with a portion of 48 tokens and more: the rows and coefficients of turns of four tokens by one kernel in place of
+//   `prepare`, then the walk in turns, state_walk.cuh)
+//   recurrence   of single tokens and shorter portions: a block per (request, head, slice of 16 value
 //                columns) walks the request's tokens one by one; four
 //                neighbouring lanes share a column, each with a quarter of the key channels in registers (lane p of the
 //                four holds channels 4 (p + 4 j) .. 4 (p + 4 j) + 3, so that the four read neighbouring 16-byte pieces
@@ -233,90 +234,210 @@ gdr_recurrence_kernel(const float* __restrict__ pq, const float* __restrict__ pk
 
 
 // ---- the walk in turns of four tokens (state_walk.cuh) ---------------------------------------------------------------
-// What it reads with a decay per key channel: a warp per (turn, value head) leaves the rows with their decays (qf, kf from the
-// turn's start up to and with the token, kb from the token to the turn's end), the whole turn's decay and the coefficients
-// between the turn's tokens. Products of decays, no quotients: nothing overflows.
-template <int CPL>
+// What it reads, made from the projections' rows in one kernel: a warp per (turn, key head) or (turn, 32 CPL value channels).
+// A key head's warp convolves its q and k for the turn's four tokens (the seven rows they need and four taps a channel in
+// registers), makes them unit vectors and, for every value head that shares them, the coefficients between the tokens. With a
+// decay per key channel it leaves the rows with their decays instead (qf, kf from the turn's start up to and with the token,
+// kb from the token to the turn's end) and the whole turn's decay. Products of decays, no quotients: nothing overflows.
+// Bound by memory. 2,048 tokens of 16 heads over 8 of 128 x 128: 58 us, where preparing the rows (a block a token, the
+// convolution a channel at a time) and their coefficients by two kernels took 68 + 13.
+template <int CPL, typename TA>
+__device__ __forceinline__ void gdr_convolve(const TA* __restrict__ x, long long stride, size_t t_req, int first, int have,
+                                             const float* __restrict__ taps, int K, bool taps4, const float* __restrict__ tail,
+                                             int C, int lane, int width, bool vec, float (&out)[4][CPL]) {
+  constexpr int V = CPL < 4 ? CPL : 4;
+  float in[7][CPL], w[4][CPL];      // the rows of tokens first - 3 .. first + 3; the taps of lags 0 .. 3
+#pragma unroll
+  for (int i = 0; i < 7; ++i) {
+    const int o = first - 3 + i;
+    if (o >= 0) walk_load<CPL>(x + (t_req + o) * stride, lane, width, o < first + have, vec, in[i]);
+    else walk_load<CPL>(tail + (long long)(K - 1 + o) * C, lane, width, K - 1 + o >= 0, vec, in[i]);
+  }
+#pragma unroll
+  for (int m = 0; m < CPL; ++m) {
+    const int c = V * lane + 32 * (m / V * V) + m % V;
+    float4 f = make_float4(0.f, 0.f, 0.f, 0.f);      // lags 3, 2, 1, 0
+    if (c < width) {
+      const float* at = taps + (size_t)c * K;
+      if (taps4) {
+        f = *reinterpret_cast<const float4*>(at);
+      } else {
+        f.w = at[K - 1];
+        if (K > 1) f.z = at[K - 2];
+        if (K > 2) f.y = at[K - 3];
+        if (K > 3) f.x = at[K - 4];
+      }
+    }
+    w[0][m] = f.w; w[1][m] = f.z; w[2][m] = f.y; w[3][m] = f.x;
+  }
+#pragma unroll
+  for (int t = 0; t < 4; ++t) {
+    float acc[CPL];
+#pragma unroll
+    for (int m = 0; m < CPL; ++m) acc[m] = 0.f;
+#pragma unroll
+    for (int lag = 0; lag < 4; ++lag)
+      if (lag < K)
+#pragma unroll
+        for (int m = 0; m < CPL; ++m) acc[m] = fmaf(w[lag][m], in[3 + t - lag][m], acc[m]);
+    for (int lag = 4; lag < K; ++lag) {      // (longer filters: the row and the tap from memory)
+      const int o = first + t - lag;
+      float row[CPL];
+      if (o >= 0) walk_load<CPL>(x + (t_req + o) * stride, lane, width, t < have, vec, row);
+      else walk_load<CPL>(tail + (long long)(K - 1 + o) * C, lane, width, t < have, vec, row);
+#pragma unroll
+      for (int m = 0; m < CPL; ++m) {
+        const int c = V * lane + 32 * (m / V * V) + m % V;
+        if (c < width) acc[m] = fmaf(taps[(size_t)c * K + K - 1 - lag], row[m], acc[m]);
+      }
+    }
+#pragma unroll
+    for (int m = 0; m < CPL; ++m) out[t][m] = t < have ? rec_silu(acc[m]) : 0.f;
+  }
+}
+
+template <typename TA, int CPL, bool CHANNEL>
 __global__ void __launch_bounds__(128)
-gdr_channel_turns_kernel(const float* __restrict__ pq, const float* __restrict__ pk, const float* __restrict__ pg,
-                         const float* __restrict__ pbeta, const int* __restrict__ q_start, const int* __restrict__ n_new,
-                         float* __restrict__ qf, float* __restrict__ kf, float* __restrict__ kb, float* __restrict__ w,
-                         float* __restrict__ tables, int n_requests, int G, int H, int d) {
-  const int place = blockIdx.x, head = blockIdx.y * 4 + (threadIdx.x >> 5), lane = threadIdx.x & 31;
-  if (head >= H) return;
+gdr_turns_kernel(const TA* __restrict__ x, long long stride, const float* __restrict__ taps, const float* __restrict__ ba,
+                 const TA* __restrict__ b, long long b_stride, const float* __restrict__ araw, const float* __restrict__ a_log,
+                 const float* __restrict__ dt_bias, const float* __restrict__ conv_state, const int* __restrict__ q_start,
+                 const int* __restrict__ n_new, const int* __restrict__ slot_ids, float* __restrict__ pq,
+                 float* __restrict__ pk, float* __restrict__ kb, float* __restrict__ pv, float* __restrict__ w,
+                 float* __restrict__ tables, int n_requests, int G, int H, int d, int dv, int K, float key_eps, float q_scale,
+                 bool vec, bool taps4) {
+  const int place = blockIdx.x, unit = blockIdx.y * 4 + (threadIdx.x >> 5), lane = threadIdx.x & 31;
+  const int wq = G * d, wv = H * dv, C = 2 * wq + wv;
+  if (unit >= G + (wv + 32 * CPL - 1) / (32 * CPL)) return;
   const int req = walk_request(q_start, n_requests, place), t_req = q_start[req];
   const int first = (place - walk_place(t_req, req)) * WALK_TURN, have = min(WALK_TURN, n_new[req] - first);
   if (first < 0 || have <= 0) return;
   const size_t t0 = (size_t)(t_req + first);
-  const int kh = head / (H / G);
-  const bool vec = d % 4 == 0;
-  float q[4][CPL], k[4][CPL], g[4][CPL], sums[16];
+  const float* tail = conv_state + (size_t)slot_ids[req] * (K - 1) * C;
+  auto convolve = [&](int c0, int width, float (&out)[4][CPL]) {
+    gdr_convolve<CPL>(x + c0, stride, (size_t)t_req, first, have, taps + (size_t)c0 * K, K, taps4, tail + c0, C, lane, width, vec, out);
+  };
+  if (unit >= G) {
+    const int c0 = (unit - G) * 32 * CPL, width = min(32 * CPL, wv - c0);
+    float v[4][CPL];
+    convolve(2 * wq + c0, width, v);
+#pragma unroll
+    for (int t = 0; t < 4; ++t)
+      if (t < have) walk_store<CPL>(pv + (t0 + t) * wv + c0, lane, width, vec, v[t]);
+    return;
+  }
+  float q[4][CPL], k[4][CPL];
+  convolve(unit * d, d, q);
+  convolve(wq + unit * d, d, k);
 #pragma unroll
   for (int t = 0; t < 4; ++t) {
-    walk_load<CPL>(pq + ((t0 + t) * G + kh) * d, lane, d, t < have, vec, q[t]);
-    walk_load<CPL>(pk + ((t0 + t) * G + kh) * d, lane, d, t < have, vec, k[t]);
-    walk_load<CPL>(pg + ((t0 + t) * H + head) * d, lane, d, t < have, vec, g[t]);
-    if (t >= have)
+    float sq = 0.f, sk = 0.f;
 #pragma unroll
-      for (int m = 0; m < CPL; ++m) g[t][m] = 1.f;
+    for (int m = 0; m < CPL; ++m) {
+      sq = fmaf(q[t][m], q[t][m], sq);
+      sk = fmaf(k[t][m], k[t][m], sk);
+    }
+    const float iq = 1.0f / sqrtf(warp_sum(sq) + key_eps) * q_scale, ik = 1.0f / sqrtf(warp_sum(sk) + key_eps);
+#pragma unroll
+    for (int m = 0; m < CPL; ++m) {      // (a token that is not there stays zero also where key_eps is)
+      q[t][m] = t < have ? q[t][m] * iq : 0.f;
+      k[t][m] = t < have ? k[t][m] * ik : 0.f;
+    }
+    if (!CHANNEL && t < have) {
+      walk_store<CPL>(pq + (t0 + t) * wq + (size_t)unit * d, lane, d, vec, q[t]);
+      walk_store<CPL>(pk + (t0 + t) * wq + (size_t)unit * d, lane, d, vec, k[t]);
+    }
   }
-  // q_i . k_j (j <= i) at i (i + 1) / 2 + j, k_i . k_j (j < i) at 10 + i (i - 1) / 2 + j, the decays after j up to and
-  // with i between them.
+  const int shared = H / G;
+  if constexpr (!CHANNEL) {
+    // q_i . k_j (j <= i) at i (i + 1) / 2 + j, k_i . k_j (j < i) at 10 + i (i - 1) / 2 + j.
+    float sums[16];
 #pragma unroll
-  for (int e = 0; e < 16; ++e) sums[e] = 0.f;
+    for (int e = 0; e < 16; ++e) sums[e] = 0.f;
 #pragma unroll
-  for (int m = 0; m < CPL; ++m)
+    for (int m = 0; m < CPL; ++m)
 #pragma unroll
-    for (int j = 0; j < 4; ++j) {
-      float kj = k[j][m];
-      sums[j * (j + 1) / 2 + j] = fmaf(q[j][m], kj, sums[j * (j + 1) / 2 + j]);
+      for (int i = 0; i < 4; ++i)
 #pragma unroll
-      for (int i = j + 1; i < 4; ++i) {
-        kj *= g[i][m];
-        sums[i * (i + 1) / 2 + j] = fmaf(q[i][m], kj, sums[i * (i + 1) / 2 + j]);
-        sums[10 + i * (i - 1) / 2 + j] = fmaf(k[i][m], kj, sums[10 + i * (i - 1) / 2 + j]);
+        for (int j = 0; j <= i; ++j) {
+          sums[i * (i + 1) / 2 + j] = fmaf(q[i][m], k[j][m], sums[i * (i + 1) / 2 + j]);
+          if (j < i) sums[10 + i * (i - 1) / 2 + j] = fmaf(k[i][m], k[j][m], sums[10 + i * (i - 1) / 2 + j]);
+        }
+    const float sum = walk_sum_all<16>(sums, lane);
+    for (int h = unit * shared; h < (unit + 1) * shared; ++h) {
+      float be = 0.f, decay = 1.f;      // of token lane & 3
+      if ((lane & 3) < have) {
+        const float* at = ba + (t0 + (lane & 3)) * 2 * H + h;
+        be = rec_sigmoid(at[0]);
+        decay = expf(-expf(a_log[h]) * rec_softplus(at[H] + dt_bias[h]));
       }
+      float g[4], bt[4];
+#pragma unroll
+      for (int t = 0; t < 4; ++t) {
+        g[t] = __shfl_sync(0xffffffffu, decay, t);
+        bt[t] = __shfl_sync(0xffffffffu, be, t);
+      }
+      walk_write_table<WALK_GATED>(tables + ((size_t)place * H + h) * 36, sum, g, bt, lane);
     }
-  float up[CPL], down[CPL], row[CPL];
+  } else {
+    for (int h = unit * shared; h < (unit + 1) * shared; ++h) {
+      const float rate = -expf(a_log[h]);
+      float g[4][CPL], bias[CPL], sums[16];
+      walk_load<CPL>(dt_bias + (size_t)h * d, lane, d, true, false, bias);
 #pragma unroll
-  for (int m = 0; m < CPL; ++m) up[m] = down[m] = 1.f;
+      for (int t = 0; t < 4; ++t) {
+        walk_load<CPL>(araw + (t0 + t) * H * d + (size_t)h * d, lane, d, t < have, vec, g[t]);
 #pragma unroll
-  for (int t = 0; t < 4; ++t) {
-    const int e = 3 - t;
+        for (int m = 0; m < CPL; ++m) g[t][m] = t < have ? expf(rate * rec_softplus(g[t][m] + bias[m])) : 1.f;
+      }
+      // The same products with the decays after j up to and with i between them.
 #pragma unroll
-    for (int m = 0; m < CPL; ++m) up[m] *= g[t][m];
-    if (t < have) {
-      const size_t at = ((t0 + t) * H + head) * d;
+      for (int e = 0; e < 16; ++e) sums[e] = 0.f;
 #pragma unroll
-      for (int m = 0; m < CPL; ++m) row[m] = q[t][m] * up[m];
-      walk_store<CPL>(qf + at, lane, d, vec, row);
+      for (int m = 0; m < CPL; ++m)
 #pragma unroll
-      for (int m = 0; m < CPL; ++m) row[m] = k[t][m] * up[m];
-      walk_store<CPL>(kf + at, lane, d, vec, row);
+        for (int j = 0; j < 4; ++j) {
+          float kj = k[j][m];
+          sums[j * (j + 1) / 2 + j] = fmaf(q[j][m], kj, sums[j * (j + 1) / 2 + j]);
+#pragma unroll
+          for (int i = j + 1; i < 4; ++i) {
+            kj *= g[i][m];
+            sums[i * (i + 1) / 2 + j] = fmaf(q[i][m], kj, sums[i * (i + 1) / 2 + j]);
+            sums[10 + i * (i - 1) / 2 + j] = fmaf(k[i][m], kj, sums[10 + i * (i - 1) / 2 + j]);
+          }
+        }
+      float up[CPL], down[CPL], row[CPL];
+#pragma unroll
+      for (int m = 0; m < CPL; ++m) up[m] = down[m] = 1.f;
+#pragma unroll
+      for (int t = 0; t < 4; ++t) {
+        const int e = 3 - t;
+#pragma unroll
+        for (int m = 0; m < CPL; ++m) up[m] *= g[t][m];
+        if (t < have) {
+          const size_t at = ((t0 + t) * H + h) * d;
+#pragma unroll
+          for (int m = 0; m < CPL; ++m) row[m] = q[t][m] * up[m];
+          walk_store<CPL>(pq + at, lane, d, vec, row);
+#pragma unroll
+          for (int m = 0; m < CPL; ++m) row[m] = k[t][m] * up[m];
+          walk_store<CPL>(pk + at, lane, d, vec, row);
+        }
+        if (e < have) {
+#pragma unroll
+          for (int m = 0; m < CPL; ++m) row[m] = k[e][m] * down[m];
+          walk_store<CPL>(kb + ((t0 + e) * H + h) * d, lane, d, vec, row);
+        }
+#pragma unroll
+        for (int m = 0; m < CPL; ++m) down[m] *= g[e][m];
+      }
+      walk_store<CPL>(w + ((size_t)place * H + h) * d, lane, d, vec, up);
+      const float sum = walk_sum_all<16>(sums, lane);
+      const float ones[4] = {1.f, 1.f, 1.f, 1.f};
+      float bt[4];
+#pragma unroll
+      for (int t = 0; t < 4; ++t) bt[t] = t < have ? rec_sigmoid(to_float(b[(t0 + t) * b_stride + h])) : 0.f;
+      walk_write_table<WALK_CHANNEL>(tables + ((size_t)place * H + h) * 36, sum, ones, bt, lane);
     }
-    if (e < have) {
-#pragma unroll
-      for (int m = 0; m < CPL; ++m) row[m] = k[e][m] * down[m];
-      walk_store<CPL>(kb + ((t0 + e) * H + head) * d, lane, d, vec, row);
-    }
-#pragma unroll
-    for (int m = 0; m < CPL; ++m) down[m] *= g[e][m];
-  }
-  walk_store<CPL>(w + ((size_t)place * H + head) * d, lane, d, vec, up);
-  float* to = tables + ((size_t)place * H + head) * 36;
-  const float sum = walk_sum_all<16>(sums, lane);
-  if (lane < 10) {      // row i of the lower triangle begins at 0, 1, 3, 6
-    const int i = lane < 1 ? 0 : (lane < 3 ? 1 : (lane < 6 ? 2 : 3));
-    to[WALK_Q + 4 * i + lane - i * (i + 1) / 2] = sum;
-  } else if (lane < 16) {
-    to[WALK_K + lane - 10] = sum;
-  } else if (lane < 18) {
-    *reinterpret_cast<float4*>(to + (lane == 16 ? WALK_P : WALK_Z)) = make_float4(1.f, 1.f, 1.f, 1.f);
-  } else if (lane < 22) {
-    to[WALK_BETA + lane - 18] = lane - 18 < have ? pbeta[(t0 + lane - 18) * H + head] : 0.f;
-  } else if (lane < 28) {
-    const int e = lane - 22;
-    to[WALK_Q + (e < 3 ? 1 + e : (e < 5 ? 3 + e : 11))] = 0.f;
   }
 }
 
@@ -597,36 +718,43 @@ static int launch_chunked(const float* pq, const float* pk, const float* pv, con
   return llmrs_launch_status("gated_delta (chunked recurrence)");
 }
 
-static int launch_turns(bool channel, const float* pq, const float* pk, const float* pv, const float* pbeta, const float* pg,
-                        float* qf, float* kf, float* kb, float* w, float* tables, float* state, const int* q_start,
-                        const int* n_new, const int* slot_ids, float* o_raw, int n_tokens, int n_requests, int G, int H, int d,
-                        int dv, cudaStream_t stream) {
+struct TurnRows {      // what gdr_turns_kernel leaves in the workspace
+  float *pq, *pk, *kb, *pv, *w, *tables;
+};
+template <typename TA>
+static int launch_turns(const TA* x, long long x_stride, const float* taps, const float* ba, const TA* b, long long b_stride,
+                        const float* araw, const float* a_log, const float* dt_bias, const float* conv_state, const TurnRows& r,
+                        const int* q_start, const int* n_new, const int* slot_ids, int n_tokens, int n_requests, int G, int H,
+                        int d, int dv, int K, float key_eps, float q_scale, cudaStream_t stream) {
+  auto rows_of_four = [](const void* p, size_t size, long long stride) { return ((uintptr_t)p & (4 * size - 1)) == 0 && stride % 4 == 0; };
+  const bool vec = d % 4 == 0 && H * dv % 4 == 0 && rows_of_four(x, sizeof(TA), x_stride) && rows_of_four(conv_state, 4, 4) &&
+                   rows_of_four(araw, 4, 4);
+  const bool taps4 = K == 4 && ((uintptr_t)taps & 15) == 0;
+  const int cpl = d <= 128 ? 4 : 8, units = G + (H * dv + 32 * cpl - 1) / (32 * cpl);
+  LLMRS_REQUIRE((units + 3) / 4 <= 65535, "gated_delta: too many heads");
+  const dim3 grid((unsigned)walk_places(n_tokens, n_requests), (units + 3) / 4);
+#define LLMRS_GD_TURNS(CPL, CH)                                                                                               \
+  gdr_turns_kernel<TA, CPL, CH><<<grid, 128, 0, stream>>>(x, x_stride, taps, ba, b, b_stride, araw, a_log, dt_bias, conv_state, \
+                                                          q_start, n_new, slot_ids, r.pq, r.pk, r.kb, r.pv, r.w, r.tables,    \
+                                                          n_requests, G, H, d, dv, K, key_eps, q_scale, vec, taps4)
+  if (araw && cpl == 4) LLMRS_GD_TURNS(4, true);
+  else if (araw) LLMRS_GD_TURNS(8, true);
+  else if (cpl == 4) LLMRS_GD_TURNS(4, false);
+  else LLMRS_GD_TURNS(8, false);
+#undef LLMRS_GD_TURNS
+  return llmrs_launch_status("gated_delta (turns)");
+}
+
+static int launch_turn_walk(bool channel, const TurnRows& r, float* state, const int* q_start, const int* n_new,
+                            const int* slot_ids, float* o_raw, int n_requests, int G, int H, int d, int dv, cudaStream_t stream) {
   WalkArgs a = {};
-  a.v = pv; a.tables = tables; a.state = state; a.o_raw = o_raw;
+  a.q = r.pq; a.k = r.pk; a.kb = r.kb; a.w = r.w;
+  a.v = r.pv; a.tables = r.tables; a.state = state; a.o_raw = o_raw;
   a.q_start = q_start; a.n_new = n_new; a.slot_ids = slot_ids;
   a.n_heads = H; a.d = d; a.dv = dv;
-  if (channel) {
-    const dim3 grid((unsigned)walk_places(n_tokens, n_requests), (H + 3) / 4);
-    if (d <= 128)
-      gdr_channel_turns_kernel<4><<<grid, 128, 0, stream>>>(pq, pk, pg, pbeta, q_start, n_new, qf, kf, kb, w, tables,
-                                                            n_requests, G, H, d);
-    else
-      gdr_channel_turns_kernel<8><<<grid, 128, 0, stream>>>(pq, pk, pg, pbeta, q_start, n_new, qf, kf, kb, w, tables,
-                                                            n_requests, G, H, d);
-    int rc = llmrs_launch_status("gated_delta (turns)");
-    if (rc != 0) return rc;
-    a.q = qf; a.k = kf; a.kb = kb; a.w = w;
-    a.q_stride = a.k_stride = a.b_stride = (long long)H * d;
-    a.n_groups = H;
-    return launch_state_walk<WALK_CHANNEL>(a, n_requests, dv, stream);
-  }
-  int rc = launch_walk_tables<WALK_GATED>(pq, pk, (long long)G * d, pg, nullptr, pbeta, q_start, n_new, tables, n_tokens,
-                                          n_requests, H, G, d, stream);
-  if (rc != 0) return rc;
-  a.q = pq; a.k = pk;
-  a.q_stride = a.k_stride = (long long)G * d;
-  a.n_groups = G;
-  return launch_state_walk<WALK_GATED>(a, n_requests, dv, stream);
+  a.n_groups = channel ? H : G;
+  a.q_stride = a.k_stride = a.b_stride = (long long)a.n_groups * d;
+  return channel ? launch_state_walk<WALK_CHANNEL>(a, n_requests, dv, stream) : launch_state_walk<WALK_GATED>(a, n_requests, dv, stream);
 }
 
 // Float32 workspace of the kernels, in floats: prepared q, k, v, beta, g and the raw read-outs.
@@ -712,11 +840,19 @@ LLMRS_API int llmrs_gated_delta(const void* x, long long x_stride, const void* g
         (const T*)x, x_stride, taps, ba, (const T*)b, b_stride, araw, a_log, dt_bias, conv_state, token_req, q_start,  \
         slot_ids, pq, pk, pv, pbeta, pg, plg, G, H, d, dv, K, key_eps, q_scale);                                       \
   } while (0)
+  const TurnRows turn_rows = {channel ? qf : pq, channel ? kf : pk, kb, pv, turn_w, tables};
 #define LLMRS_GD_LAUNCH(T)                                                                                             \
   do {                                                                                                                 \
-    if (channel) LLMRS_GD_PREPARE(T, true);                                                                            \
-    else LLMRS_GD_PREPARE(T, false);                                                                                   \
-    int rc = llmrs_launch_status("gated_delta (prepare)");                                                             \
+    int rc = 0;                                                                                                        \
+    if (turns) {                                                                                                       \
+      rc = launch_turns<T>((const T*)x, x_stride, taps, ba, (const T*)b, b_stride, araw, a_log, dt_bias, conv_state,   \
+                           turn_rows, q_start, n_new, slot_ids, n_tokens, n_requests, G, H, d, dv, K, key_eps,         \
+                           q_scale, stream);                                                                           \
+    } else {                                                                                                           \
+      if (channel) LLMRS_GD_PREPARE(T, true);                                                                          \
+      else LLMRS_GD_PREPARE(T, false);                                                                                 \
+      rc = llmrs_launch_status("gated_delta (prepare)");                                                               \
+    }                                                                                                                  \
     if (rc != 0) return rc;                                                                                            \
     rc = launch_short_conv_state((const T*)x, x_stride, conv_state, q_start, n_new, slot_ids, n_requests, C, K, stream); \
     if (rc != 0) return rc;                                                                                            \
@@ -725,8 +861,8 @@ LLMRS_API int llmrs_gated_delta(const void* x, long long x_stride, const void* g
                           max_chunks, G, H, d, dv, stream);                                                            \
       if (rc != 0) return rc;                                                                                          \
     } else if (turns) {                                                                                                \
-      rc = launch_turns(channel, pq, pk, pv, pbeta, pg, qf, kf, kb, turn_w, tables, state, q_start, n_new, slot_ids,   \
-                        o_raw, n_tokens, n_requests, G, H, d, dv, stream);                                             \
+      rc = launch_turn_walk(channel, turn_rows, state, q_start, n_new, slot_ids, o_raw, n_requests, G, H, d, dv,       \
+                            stream);                                                                                   \
       if (rc != 0) return rc;                                                                                          \
     } else if (channel && (long long)grid.x * grid.y * grid.z <= GD_WIDE_MAX_BLOCKS) LLMRS_GD_REC_ALL(true, 16);       \
     else if (channel) LLMRS_GD_REC_ALL(true, 8);                                                                       \

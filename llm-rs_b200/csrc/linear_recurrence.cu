@@ -367,7 +367,7 @@ LLMRS_API int llmrs_linear_recurrence_planes(const float* Q, const float* K, con
     LLMRS_REQUIRE(((uintptr_t)tables & 15) == 0 && tables != nullptr, "linear_recurrence: no workspace for a portion");
     LLMRS_REQUIRE(((uintptr_t)V & 15) == 0, "linear_recurrence: planes must be 16-byte aligned");
     const long long stride = (long long)n_groups * dk;
-    int rc = launch_walk_tables<WALK_LINEAR>(Q, K, stride, decay, head_decay, v_gain, q_start, n_new, tables, n_tokens,
+    int rc = launch_walk_tables(Q, K, stride, decay, head_decay, v_gain, q_start, n_new, tables, n_tokens,
                                              n_requests, n_heads, n_groups, dk, stream);
     if (rc != 0) return rc;
     WalkArgs a = {};

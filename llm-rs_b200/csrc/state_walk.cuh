@@ -470,9 +470,36 @@ __global__ void __launch_bounds__(WALK_THREADS, 2) state_walk_kernel(WalkArgs p,
     }
 }
 
-// The coefficients of WALK_LINEAR and WALK_GATED (a decay per token and head): a warp per (turn, head). decay [tokens, heads]
-// or null (then head_decay [heads], or 1); beta [tokens, heads] or null (1): write strengths, or gains on the values.
-template <int MODE, int CPL>
+// A turn's coefficients from the products of its rows, summed over the warp: lane l < 16 has sum l (q_i . k_j, j <= i, at
+// i (i + 1) / 2 + j; k_i . k_j, j < i, at 10 + i (i - 1) / 2 + j). g: the tokens' decays, be: their write strengths or gains.
+// With a decay per key channel the sums hold the decays already (and g is ones).
+template <int MODE>
+__device__ __forceinline__ void walk_write_table(float* __restrict__ to, float sum, const float (&g)[4], const float (&be)[4],
+                                                 int lane) {
+  // Lane l < 16 holds sum l: its factor is the decays after j up to and with i.
+#pragma unroll
+  for (int i = 0; i < 4; ++i) {
+    float between = 1.f;
+#pragma unroll
+    for (int j = i; j >= 0; --j) {
+      if (lane == i * (i + 1) / 2 + j) to[WALK_Q + 4 * i + j] = sum * between;
+      if (MODE != WALK_LINEAR && j < i && lane == 10 + i * (i - 1) / 2 + j) to[WALK_K + i * (i - 1) / 2 + j] = sum * between;
+      between *= g[j];
+    }
+  }
+  const float p1 = g[0] * g[1], p2 = p1 * g[2], z1 = g[3] * g[2], z0 = z1 * g[1];
+  if (lane == 16) *reinterpret_cast<float4*>(to + WALK_P) = make_float4(g[0], p1, p2, p2 * g[3]);
+  if (lane == 17) *reinterpret_cast<float4*>(to + WALK_Z) = make_float4(z0, z1, g[3], 1.f);
+  if (lane == 18) *reinterpret_cast<float4*>(to + WALK_BETA) = make_float4(be[0], be[1], be[2], be[3]);
+  if (lane >= 19 && lane < 25) {      // above the diagonal
+    const int e = lane - 19, at = e < 3 ? 1 + e : (e < 5 ? 3 + e : 11);      // (0,1) (0,2) (0,3) (1,2) (1,3) (2,3)
+    to[WALK_Q + at] = 0.f;
+  }
+}
+
+// The coefficients of WALK_LINEAR (a decay per token and head): a warp per (turn, head). decay [tokens, heads]
+// or null (then head_decay [heads], or 1); beta [tokens, heads] or null (1): gains on the values.
+template <int CPL>
 __global__ void __launch_bounds__(128)
 walk_tables_kernel(const float* __restrict__ q, const float* __restrict__ k, long long stride, const float* __restrict__ decay,
                    const float* __restrict__ head_decay, const float* __restrict__ beta, const int* __restrict__ q_start,
@@ -485,7 +512,7 @@ walk_tables_kernel(const float* __restrict__ q, const float* __restrict__ k, lon
   const size_t t0 = (size_t)(t_req + first);
   const float* qr = q + t0 * stride + (size_t)(head / (n_heads / n_groups)) * d;
   const float* kr = k + t0 * stride + (size_t)(head / (n_heads / n_groups)) * d;
-  float sums[16];      // q_i . k_j (j <= i) at i (i + 1) / 2 + j, k_i . k_j (j < i) at 10 + i (i - 1) / 2 + j
+  float sums[16];      // q_i . k_j (j <= i) at i (i + 1) / 2 + j
 #pragma unroll
   for (int e = 0; e < 16; ++e) sums[e] = 0.f;
   float qv[4][CPL], kv[4][CPL];
@@ -505,44 +532,20 @@ walk_tables_kernel(const float* __restrict__ q, const float* __restrict__ k, lon
 #pragma unroll
     for (int i = 0; i < 4; ++i)
 #pragma unroll
-      for (int j = 0; j <= i; ++j) {
-        sums[i * (i + 1) / 2 + j] = fmaf(qv[i][m], kv[j][m], sums[i * (i + 1) / 2 + j]);
-        if (MODE == WALK_GATED && j < i) sums[10 + i * (i - 1) / 2 + j] = fmaf(kv[i][m], kv[j][m], sums[10 + i * (i - 1) / 2 + j]);
-      }
-  float* to = tables + ((size_t)place * n_heads + head) * 36;
-  float sum = walk_sum_all<16>(sums, lane);
-  // Lane l < 16 holds sum l: its factor is the decays after j up to and with i.
-#pragma unroll
-  for (int i = 0; i < 4; ++i) {
-    float between = 1.f;
-#pragma unroll
-    for (int j = i; j >= 0; --j) {
-      if (lane == i * (i + 1) / 2 + j) to[WALK_Q + 4 * i + j] = sum * between;
-      if (j < i && lane == 10 + i * (i - 1) / 2 + j) to[WALK_K + i * (i - 1) / 2 + j] = sum * between;
-      between *= g[j];
-    }
-  }
-  const float p1 = g[0] * g[1], p2 = p1 * g[2], z1 = g[3] * g[2], z0 = z1 * g[1];
-  if (lane == 16) *reinterpret_cast<float4*>(to + WALK_P) = make_float4(g[0], p1, p2, p2 * g[3]);
-  if (lane == 17) *reinterpret_cast<float4*>(to + WALK_Z) = make_float4(z0, z1, g[3], 1.f);
-  if (lane == 18) *reinterpret_cast<float4*>(to + WALK_BETA) = make_float4(be[0], be[1], be[2], be[3]);
-  if (lane >= 19 && lane < 25) {      // above the diagonal
-    const int e = lane - 19, at = e < 3 ? 1 + e : (e < 5 ? 3 + e : 11);      // (0,1) (0,2) (0,3) (1,2) (1,3) (2,3)
-    to[WALK_Q + at] = 0.f;
-  }
+      for (int j = 0; j <= i; ++j) sums[i * (i + 1) / 2 + j] = fmaf(qv[i][m], kv[j][m], sums[i * (i + 1) / 2 + j]);
+  walk_write_table<WALK_LINEAR>(tables + ((size_t)place * n_heads + head) * 36, walk_sum_all<16>(sums, lane), g, be, lane);
 }
 
-template <int MODE>
 static int launch_walk_tables(const float* q, const float* k, long long stride, const float* decay, const float* head_decay,
                               const float* beta, const int* q_start, const int* n_new, float* tables, int n_tokens,
                               int n_requests, int n_heads, int n_groups, int d, cudaStream_t stream) {
   const dim3 grid((unsigned)walk_places(n_tokens, n_requests), (n_heads + 3) / 4);
   if (d <= 128)
-    walk_tables_kernel<MODE, 4><<<grid, 128, 0, stream>>>(q, k, stride, decay, head_decay, beta, q_start, n_new, tables,
-                                                          n_requests, n_heads, n_groups, d);
+    walk_tables_kernel<4><<<grid, 128, 0, stream>>>(q, k, stride, decay, head_decay, beta, q_start, n_new, tables,
+                                                    n_requests, n_heads, n_groups, d);
   else
-    walk_tables_kernel<MODE, 8><<<grid, 128, 0, stream>>>(q, k, stride, decay, head_decay, beta, q_start, n_new, tables,
-                                                          n_requests, n_heads, n_groups, d);
+    walk_tables_kernel<8><<<grid, 128, 0, stream>>>(q, k, stride, decay, head_decay, beta, q_start, n_new, tables,
+                                                    n_requests, n_heads, n_groups, d);
   return llmrs_launch_status("state walk (tables)");
 }
 

@@ -20,7 +20,7 @@ def _ctx(n_new, cached):
         positions=i32([c + i for c, n in zip(cached, n_new) for i in range(n)]))
 
 
-def _part(kind, d, dv):
+def _part(kind, d, dv, taps=3):
     from llm_rs_b200.parts.delta_rule import ChannelDelta, GatedDelta, GeneralDelta
     from llm_rs_b200.parts.recurrent import MatrixMemory, Retention
     from llm_rs_b200.parts.ssd import Mamba2
@@ -28,8 +28,8 @@ def _part(kind, d, dv):
     return D, {"memory": lambda: MatrixMemory(D, 3, d, dv, gate_cap=9.0, prefix="m."),
                "retention": lambda: Retention(D, 3, d, dv, [0.9, 0.0, 1.0], prefix="m."),
                "mamba": lambda: Mamba2(D, 4, dv, d, 2, 3, norm_parts=1, prefix="m."),
-               "gated": lambda: GatedDelta(D, 4, 2, d, dv, 3, prefix="m."),
-               "channel": lambda: ChannelDelta(D, 4, 2, d, dv, 3, 8, 8, prefix="m."),
+               "gated": lambda: GatedDelta(D, 4, 2, d, dv, taps, prefix="m."),
+               "channel": lambda: ChannelDelta(D, 4, 2, d, dv, taps, 8, 8, prefix="m."),
                "general": lambda: GeneralDelta(D, 3, d, 8, prefix="m.")}[kind]()
 
 
@@ -37,9 +37,21 @@ def _part(kind, d, dv):
 @pytest.mark.parametrize("d,dv,lens", [(64, 64, [48]), (128, 48, [9, 1, 49]), (30, 17, [50, 7]), (200, 20, [16, 63]),
                                        (96, 130, [51]), (7, 3, [1, 2, 3, 4, 5, 11] * 7), (256, 16, [40, 0, 18])])
 def test_portions_in_turns_match_single_tokens(kind, d, dv, lens):
+    _compare(kind, d, dv, lens, 3)
+
+
+@pytest.mark.parametrize("kind", ["gated", "channel"])
+@pytest.mark.parametrize("taps", [2, 4, 6])
+@pytest.mark.parametrize("d,dv,lens", [(64, 48, [9, 1, 49, 2]), (30, 17, [50, 7]), (136, 8, [48, 5])])
+def test_convolutions_of_turns(kind, taps, d, dv, lens):
+    """Rows and coefficients of turns are made with the convolution: filters up to four taps from registers, longer ones beside."""
+    _compare(kind, d, dv, lens, taps)
+
+
+def _compare(kind, d, dv, lens, taps):
     from llm_rs_b200.parts import Runtime
     g = torch.Generator().manual_seed(d + dv)
-    D, part = _part(kind, d, dv)
+    D, part = _part(kind, d, dv, taps)
     w = {s.name: (torch.randn(s.shape, generator=g) * (0.5 if len(s.shape) == 1 else s.shape[-1] ** -0.5)).to(DEV)
          for s in part.weight_specs()}
     part.bind(w, Runtime(torch.device(DEV), torch.float32, 4096))
