@@ -22,6 +22,7 @@
 //               end: a step of one token (decoding) and a prompt's portion are the same kernel;
 //   output      a warp per (token, head): divides by the head's root mean square, applies the weight and the gate.
 #include "common.cuh"
+#include "head_out.cuh"
 #include "mma_util.cuh"
 #include "state_walk.cuh"
 
@@ -294,6 +295,20 @@ __global__ void delta_out_kernel(const float* __restrict__ o_raw, const TA* __re
 }
 
 template <typename TA>
+static int launch_delta_out(const float* o_raw, const void* gate, long long gate_stride, const float* norm_w, void* out,
+                            int n_tokens, int n_heads, int d, float eps, cudaStream_t stream) {
+  HeadOutArgs a = {};
+  a.o = o_raw; a.gate = gate; a.gate_stride = gate_stride; a.w = norm_w; a.out = out; a.out_stride = (long long)n_heads * d;
+  a.n_tokens = n_tokens; a.n_heads = n_heads; a.dv = d; a.eps = eps; a.out_scale = 1.0f;
+  const int rows = n_tokens * n_heads;
+  if (head_out_takes<TA>(a)) launch_head_out<TA>(a, stream);
+  else
+    delta_out_kernel<TA><<<(rows + 3) / 4, 128, 0, stream>>>(o_raw, (const TA*)gate, gate_stride, norm_w, (TA*)out, rows,
+                                                             n_heads, d, eps);
+  return llmrs_launch_status("delta_rule (norm and gate)");
+}
+
+template <typename TA>
 static int launch_delta(int dmax, dim3 grid, cudaStream_t stream, const void* r, const void* k, const void* v,
                         const void* gate, const void* a_raw, long long in_stride, const float* decay_raw,
                         const float* decay_bias, const float* a_bias, const float* norm_w, float* state,
@@ -332,9 +347,7 @@ static int launch_delta(int dmax, dim3 grid, cudaStream_t stream, const void* r,
     a.n_heads = a.n_groups = n_heads; a.d = a.dv = d;
     rc = launch_state_walk<WALK_GENERAL>(a, n_requests, d, stream);
     if (rc != 0) return rc;
-    delta_out_kernel<TA><<<(rows + 3) / 4, 128, 0, stream>>>(o_raw, (const TA*)gate, in_stride, norm_w, (TA*)out, rows,
-                                                             n_heads, d, norm_eps);
-    return llmrs_launch_status("delta_rule (norm and gate)");
+    return launch_delta_out<TA>(o_raw, gate, in_stride, norm_w, out, n_tokens, n_heads, d, norm_eps, stream);
   }
   delta_prepare_kernel<TA><<<(rows + 3) / 4, 128, 0, stream>>>((const TA*)r, (const TA*)k, (const TA*)v,
                                                                (const TA*)a_raw, in_stride, decay_raw, decay_bias,
@@ -347,9 +360,7 @@ static int launch_delta(int dmax, dim3 grid, cudaStream_t stream, const void* r,
   else delta_rule_kernel<256><<<grid, DR_THREADS, 0, stream>>>(prep, state, q_start, n_new, slot_ids, o_raw, n_tokens, n_heads, d);
   rc = llmrs_launch_status("delta_rule");
   if (rc != 0) return rc;
-  delta_out_kernel<TA><<<(rows + 3) / 4, 128, 0, stream>>>(o_raw, (const TA*)gate, in_stride, norm_w, (TA*)out, rows,
-                                                           n_heads, d, norm_eps);
-  return llmrs_launch_status("delta_rule (norm and gate)");
+  return launch_delta_out<TA>(o_raw, gate, in_stride, norm_w, out, n_tokens, n_heads, d, norm_eps, stream);
 }
 
 // Float32 workspace the three kernels share, in floats.

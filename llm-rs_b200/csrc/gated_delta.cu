@@ -43,6 +43,7 @@
 // The chunked form is OFF by default (llmrs_gated_delta_chunked): its products read every operand from shared memory
 // and are bound by that (2,048 tokens of 16 heads of 128 x 128: some 500 us, the walk in turns 265).
 #include "common.cuh"
+#include "head_out.cuh"
 #include "mma_util.cuh"
 #include "short_conv.cuh"
 #include "state_walk.cuh"
@@ -817,6 +818,10 @@ LLMRS_API int llmrs_gated_delta(const void* x, long long x_stride, const void* g
   const int dmax = d <= 32 ? 32 : (d <= 64 ? 64 : (d <= 128 ? 128 : 256));
   dim3 grid(n_requests, H, (dv + GD_COLS - 1) / GD_COLS);
   const int rows = n_tokens * H;
+  HeadOutArgs head = {};
+  head.o = o_raw; head.gate = gate; head.gate_stride = gate_stride; head.w = norm_w; head.w_shared = 1;
+  head.out = out; head.out_stride = out_stride; head.n_tokens = n_tokens; head.n_heads = H; head.dv = dv;
+  head.eps = norm_eps; head.out_scale = out_scale; head.silu = !gate_sigmoid;
 #define LLMRS_GD_REC(DMAX, LANES, CH)                                                                             \
   gdr_recurrence_kernel<DMAX, LANES, CH><<<grid, GD_COLS * LANES, 0, stream>>>(pq, pk, pv, pbeta, pg, state, q_start, \
                                                                                n_new, slot_ids, o_raw, G, H, d, dv)
@@ -869,8 +874,10 @@ LLMRS_API int llmrs_gated_delta(const void* x, long long x_stride, const void* g
     else LLMRS_GD_REC_ALL(false, LLMRS_GD_LANES);                                                                      \
     rc = llmrs_launch_status("gated_delta (recurrence)");                                                              \
     if (rc != 0) return rc;                                                                                            \
-    gdr_out_kernel<T><<<(rows + 3) / 4, 128, 0, stream>>>(o_raw, (const T*)gate, gate_stride, norm_w, (T*)out,         \
-                                                          out_stride, rows, H, dv, norm_eps, out_scale, gate_sigmoid); \
+    if (head_out_takes<T>(head)) launch_head_out<T>(head, stream);                                                     \
+    else                                                                                                               \
+      gdr_out_kernel<T><<<(rows + 3) / 4, 128, 0, stream>>>(o_raw, (const T*)gate, gate_stride, norm_w, (T*)out,       \
+                                                            out_stride, rows, H, dv, norm_eps, out_scale, gate_sigmoid); \
   } while (0)
   if (dtype == LLMRS_F32) LLMRS_GD_LAUNCH(float);
   else if (dtype == LLMRS_BF16) LLMRS_GD_LAUNCH(__nv_bfloat16);

@@ -25,6 +25,7 @@
 //   output       divides by the normaliser, norms each head (or all heads together) by its root mean square,
 //                multiplies by a weight (or none) and by sigmoid(gate) or SiLU(gate), rounds to the activation type.
 #include "common.cuh"
+#include "head_out.cuh"
 #include "mma_util.cuh"
 #include "short_conv.cuh"
 #include "state_walk.cuh"
@@ -494,6 +495,18 @@ LLMRS_API int llmrs_recurrence_output(const float* o_raw, const float* nq, const
   LLMRS_REQUIRE(n_tokens >= 0 && n_heads > 0 && dv > 0 && n_heads <= 4096, "recurrence_output: bad sizes");
   LLMRS_REQUIRE((nq == nullptr) == (floor_ == nullptr), "recurrence_output: nq and floor come together");
   if (n_tokens == 0) return 0;
+  HeadOutArgs a = {};
+  a.o = o_raw; a.nq = nq; a.floor_ = floor_; a.den_eps = den_eps; a.gate = gate; a.gate_stride = gate_stride; a.w = norm_w;
+  a.out = out; a.out_stride = (long long)n_heads * dv; a.n_tokens = n_tokens; a.n_heads = n_heads; a.dv = dv;
+  a.eps = eps; a.out_scale = 1.0f; a.silu = gate_silu;
+  if (per_head && dtype == LLMRS_F32 && head_out_takes<float>(a)) {
+    launch_head_out<float>(a, stream);
+    return llmrs_launch_status("recurrence_output");
+  }
+  if (per_head && dtype == LLMRS_BF16 && head_out_takes<__nv_bfloat16>(a)) {
+    launch_head_out<__nv_bfloat16>(a, stream);
+    return llmrs_launch_status("recurrence_output");
+  }
   const int threads = n_heads * dv >= 2048 ? 256 : 128;
   const size_t smem = 2 * (size_t)n_heads * sizeof(float);
   if (dtype == LLMRS_F32)
