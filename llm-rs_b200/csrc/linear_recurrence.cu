@@ -216,6 +216,36 @@ __global__ void lr_prepare_kernel(const TA* __restrict__ q, const TA* __restrict
   for (int c = threadIdx.x; c < wv; c += blockDim.x) V[(size_t)t * wv + c] = at(v + (size_t)t * v_stride, c);
 }
 
+// The same without a rotation, for rows whose pieces of eight channels (four of float32) can be loaded sixteen bytes at a time.
+// Bound by memory: 1,793 tokens of 16 heads of 128, a channel a load -> this: 23.4 -> 12.7 us.
+template <typename TA>
+__global__ void __launch_bounds__(256)
+lr_prepare_wide_kernel(const TA* __restrict__ q, const TA* __restrict__ k, const TA* __restrict__ v, long long q_stride,
+                       long long k_stride, long long v_stride, const float* __restrict__ gain, float* __restrict__ Q,
+                       float* __restrict__ K, float* __restrict__ V, int n_tokens, int n_heads, int dk, int dv, int act,
+                       float q_scale, float k_scale) {
+  constexpr int N = 16 / sizeof(TA);
+  struct alignas(16) Piece { TA x[N]; };
+  const int wk = n_heads * dk, wv = n_heads * dv, pk = wk / N, pieces = 2 * pk + wv / N;
+  const long long id = (long long)blockIdx.x * 256 + threadIdx.x;
+  if (id >= (long long)n_tokens * pieces) return;
+  const int t = (int)(id / pieces), p = (int)(id - (long long)t * pieces);
+  const int which = p < pk ? 0 : (p < 2 * pk ? 1 : 2), c = (p - which * pk) * N;
+  const TA* from = which == 0 ? q + (size_t)t * q_stride : (which == 1 ? k + (size_t)t * k_stride : v + (size_t)t * v_stride);
+  float* to = which == 0 ? Q + (size_t)t * wk : (which == 1 ? K + (size_t)t * wk : V + (size_t)t * wv);
+  const Piece in = *reinterpret_cast<const Piece*>(from + c);
+  float scale = which == 0 ? q_scale : (which == 1 ? k_scale : 1.0f), own = 1.0f;
+  if (which == 1 && gain) own = gain[(size_t)t * n_heads + c / dk];
+  float y[N];
+#pragma unroll
+  for (int e = 0; e < N; ++e) {
+    const float x = to_float(in.x[e]);
+    y[e] = (act ? x * rec_sigmoid(x) : x) * scale * own;
+  }
+#pragma unroll
+  for (int e = 0; e < N; e += 4) *reinterpret_cast<float4*>(to + c + e) = make_float4(y[e], y[e + 1], y[e + 2], y[e + 3]);
+}
+
 // ---------------------------------------------------------------------------------
 // recurrence
 // ---------------------------------------------------------------------------------
@@ -428,10 +458,24 @@ LLMRS_API int llmrs_linear_recurrence(const void* q, const void* k, const void* 
   float* tables = V + ((size_t)n_tokens * n_heads * dv + 3) / 4 * 4;
   const int threads = n_heads * dk >= 1024 ? 256 : 128;
   const size_t smem = (size_t)rot_dims * sizeof(float);
-#define LLMRS_LR_PREPARE(T)                                                                                       \
-  lr_prepare_kernel<T><<<n_tokens, threads, smem, stream>>>((const T*)q, (const T*)k, (const T*)v, q_stride, k_stride, \
-                                                            v_stride, gain, inv_freq, positions, rot_dims, Q, K, V, \
-                                                            n_heads, dk, dv, act, q_scale, k_scale)
+  auto wide = [&](int size) {      // without a rotation, every piece of sixteen bytes within a head and on a boundary
+    const int piece = 16 / size;
+    auto starts = [&](const void* p, long long stride) { return ((uintptr_t)p & 15) == 0 && stride % piece == 0; };
+    return rot_dims == 0 && dk % piece == 0 && dv % piece == 0 && starts(q, q_stride) && starts(k, k_stride) && starts(v, v_stride);
+  };
+  const long long numbers = (long long)n_tokens * (2 * n_heads * dk + n_heads * dv);
+#define LLMRS_LR_PREPARE(T)                                                                                            \
+  do {                                                                                                                 \
+    if (wide(sizeof(T)))                                                                                               \
+      lr_prepare_wide_kernel<T><<<(unsigned)((numbers / (16 / (int)sizeof(T)) + 255) / 256), 256, 0, stream>>>(        \
+          (const T*)q, (const T*)k, (const T*)v, q_stride, k_stride, v_stride, gain, Q, K, V, n_tokens, n_heads, dk,   \
+          dv, act, q_scale, k_scale);                                                                                  \
+    else                                                                                                               \
+      lr_prepare_kernel<T><<<n_tokens, threads, smem, stream>>>((const T*)q, (const T*)k, (const T*)v, q_stride,       \
+                                                                k_stride, v_stride, gain, inv_freq, positions,         \
+                                                                rot_dims, Q, K, V, n_heads, dk, dv, act, q_scale,      \
+                                                                k_scale);                                              \
+  } while (0)
   if (dtype == LLMRS_F32) LLMRS_LR_PREPARE(float);
   else if (dtype == LLMRS_BF16) LLMRS_LR_PREPARE(__nv_bfloat16);
   else return llmrs_fail("linear_recurrence: unknown dtype %d", dtype);
