@@ -240,7 +240,8 @@ gdr_recurrence_kernel(const float* __restrict__ pq, const float* __restrict__ pk
 // registers), makes them unit vectors and, for every value head that shares them, the coefficients between the tokens. With a
 // decay per key channel it leaves the rows with their decays instead (qf, kf from the turn's start up to and with the token,
 // kb from the token to the turn's end) and the whole turn's decay. Products of decays, no quotients: nothing overflows.
-// Bound by memory. 2,048 tokens of 16 heads over 8 of 128 x 128: 58 us, where preparing the rows (a block a token, the
+// Bound by issue (some 1,700 instructions a warp, half of them SiLU's divisions and exponentials; six blocks an SM: 51 us, four:
+// 58). 2,048 tokens of 16 heads over 8 of 128 x 128: 51 us, where preparing the rows (a block a token, the
 // convolution a channel at a time) and their coefficients by two kernels took 68 + 13.
 template <int CPL, typename TA>
 __device__ __forceinline__ void gdr_convolve(const TA* __restrict__ x, long long stride, size_t t_req, int first, int have,
@@ -298,7 +299,7 @@ __device__ __forceinline__ void gdr_convolve(const TA* __restrict__ x, long long
 }
 
 template <typename TA, int CPL, bool CHANNEL>
-__global__ void __launch_bounds__(128)
+__global__ void __launch_bounds__(128, CPL == 4 ? 6 : 1)
 gdr_turns_kernel(const TA* __restrict__ x, long long stride, const float* __restrict__ taps, const float* __restrict__ ba,
                  const TA* __restrict__ b, long long b_stride, const float* __restrict__ araw, const float* __restrict__ a_log,
                  const float* __restrict__ dt_bias, const float* __restrict__ conv_state, const int* __restrict__ q_start,
