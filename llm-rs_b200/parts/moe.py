@@ -139,9 +139,10 @@ class MixtureOfExperts(FeedForward):
         if rows:
             self.router_w = torch.cat([r.to(torch.float32) for r in rows], dim=0).contiguous()
             self.router_b = torch.cat(bias, dim=0).contiguous()
-            # The same rows as the folder stores them (see ``ops.product_f32``).
+            # The same rows as the folder stores them, filled up to a multiple of eight (see ``ops.product_f32``).
             same = all(r.dtype == rows[0].dtype for r in rows)
-            self.router_w_stored = torch.cat(rows, dim=0).contiguous() if same else self.router_w
+            self.router_w_stored = (torch.nn.functional.pad(torch.cat(rows, dim=0), (0, 0, 0, -self.router_w.size(0) % 8))
+                                    if same else self.router_w)
         if self.shared_size:
             from .mlp import SwiGLU
             sp = self.prefix + self.names["shared"]
