@@ -147,26 +147,33 @@ __global__ void __launch_bounds__(GG_THREADS) gemm_grouped_kernel(const GroupedG
 
 // ---------------------------------------------------------------------------------
 // The same products on the tensor cores for bfloat16 operands (mma.sync m16n8k16, float32 accumulators): tiles of
-// 64 or 128 rows x 128 columns (64 of each product for the gated unit), k in steps of 32 through a ring of four stages of 16-byte asynchronous
-// copies, one block-wide barrier a step. Eight warps as
-// 2 x 4, each 32 or 64 rows x 32 (or 2 x 16) columns. Shared rows are 40 elements apart, which
-// spreads the fragments' 32-bit reads over all banks. A row's sums run over k in the same order whichever rows
-// share its tile. Needs K % 8 == 0 and 16-byte aligned rows of X and W.
+// 64 or 128 rows x 128 columns (64 of each product for the gated unit), or 32 rows x half of them; k in steps of 64 (32 with
+// 128 rows and for the gates) through a ring of stages of 16-byte asynchronous copies, one block-wide barrier a step. Warps as
+// 2 x 4 (2 x 2 with 32 rows). Shared rows are eight elements more than a step apart, which spreads the fragments' 32-bit reads
+// over all banks. A row's sums run over k in the same order whichever rows share its tile. Needs K % 8 == 0 and 16-byte aligned
+// rows of X and W.
+// Steps of 64 read whole 128-byte lines of the weights. 8 tokens, 4 of 32 experts of 2,048 x 1,024 each (some 250 MB of weights):
+// gated / down 58 / 31 us with steps of 32 and tiles of 64 rows; 55 / 27 with steps of 64 and 32 rows; 38 / 21 with half the columns too.
 // ---------------------------------------------------------------------------------
-constexpr int GM_BK = 32, GM_LD = GM_BK + 8, GM_THREADS = 256, GM_STAGES = 4;
+// Tiles of at most 32 rows (MT 1) are for a few rows an expert, where the weights' bytes are what counts: four warps, half the columns,
+// three stages, so that five blocks fit a multiprocessor and the tiles spread evenly.
+__host__ __device__ constexpr int gm_threads(int mt) { return mt == 1 ? 128 : 256; }
+__host__ __device__ constexpr int gm_stages(int mt) { return mt == 1 ? 3 : 4; }
 // Columns of a tile: 128, or 64 of each of the two products of the gated unit (the same shared memory either way).
-template <bool GLU> struct GmCols { static constexpr int value = GLU ? 64 : 128; };
+__host__ __device__ constexpr int gm_cols(bool glu, int mt) { return (glu ? 64 : 128) / (mt == 1 ? 2 : 1); }
 
 template <int EPI, int MT>
 __host__ __device__ constexpr int gm_stage_rows() {      // rows of a stage: the tile's of X, then those of W and of W2
-  return 32 * MT + GmCols<EPI != EPI_STORE>::value * (EPI != EPI_STORE ? 2 : 1);
+  return 32 * MT + gm_cols(EPI != EPI_STORE, MT) * (EPI != EPI_STORE ? 2 : 1);
 }
 
-template <typename TO, int EPI, int MT>      // MT: 16-row pieces per warp; the tile has 32 * MT rows
-__global__ void __launch_bounds__(GM_THREADS) gemm_grouped_mma_kernel(const GroupedGemmArgs a) {
+template <typename TO, int EPI, int MT, int GM_BK>      // MT: 16-row pieces per warp; the tile has 32 * MT rows
+__global__ void __launch_bounds__(gm_threads(MT)) gemm_grouped_mma_kernel(const GroupedGemmArgs a) {
   constexpr bool GLU = EPI != EPI_STORE;
-  constexpr int GM_BM = 32 * MT;
-  constexpr int GM_BN = GmCols<GLU>::value, NT = GM_BN / 32;      // NT: 8-column pieces per warp
+  constexpr int GM_THREADS = gm_threads(MT), GM_STAGES = gm_stages(MT), GM_BM = 32 * MT, GM_LD = GM_BK + 8;
+  constexpr int WARPS_N = GM_THREADS / 64;      // warps side by side; two lie below one another
+  constexpr int PIECES = GM_BK / 8, PASS = GM_THREADS / PIECES;      // 16-byte pieces of a row, rows that the block copies at once
+  constexpr int GM_BN = gm_cols(GLU, MT), NT = GM_BN / (8 * WARPS_N);      // NT: 8-column pieces per warp
   extern __shared__ __align__(16) unsigned char gm_smem[];      // GM_STAGES x (rows of X, rows of W, rows of W2)
   typedef __nv_bfloat16 Row[GM_LD];
   Row* const ring = reinterpret_cast<Row*>(gm_smem);
@@ -198,28 +205,28 @@ __global__ void __launch_bounds__(GM_THREADS) gemm_grouped_mma_kernel(const Grou
   const __nv_bfloat16* w2 = GLU ? (const __nv_bfloat16*)a.w2 + (size_t)group * a.w_batch : nullptr;
   const int n0 = blockIdx.x * GM_BN;
 
-  // Copies of one k step: rows x 4 pieces of 8 elements; a thread takes rows tid / 4, tid / 4 + 64, ...
-  const int a_row = tid >> 2, piece = (tid & 3) * 8;
-  long long a_off[GM_BM / 64];
+  // Copies of one k step: rows x PIECES pieces of 8 elements; a thread takes every PASS-th row.
+  const int a_row = tid / PIECES, piece = tid % PIECES * 8;
+  long long a_off[GM_BM / PASS];
 #pragma unroll
-  for (int h = 0; h < GM_BM / 64; ++h) a_off[h] = row_off[a_row + 64 * h];
+  for (int h = 0; h < GM_BM / PASS; ++h) a_off[h] = row_off[a_row + PASS * h];
   auto issue = [&](int stage, int k0) {
     const int k = k0 + piece;
     const int kb = k < a.K ? min(16, (a.K - k) * 2) : 0;      // bytes of this piece inside K (K % 8 == 0: 0 or 16)
 #pragma unroll
-    for (int h = 0; h < GM_BM / 64; ++h)
-      cp_async_16(&As(stage)[a_row + 64 * h][piece], x + (a_off[h] >= 0 ? a_off[h] : 0) + (kb ? k : 0),
+    for (int h = 0; h < GM_BM / PASS; ++h)
+      cp_async_16(&As(stage)[a_row + PASS * h][piece], x + (a_off[h] >= 0 ? a_off[h] : 0) + (kb ? k : 0),
                   a_off[h] >= 0 ? kb : 0);
 #pragma unroll
-    for (int h = 0; h < GM_BN / 64; ++h) {
-      const int r = a_row + 64 * h, n = n0 + r;
+    for (int h = 0; h < GM_BN / PASS; ++h) {
+      const int r = a_row + PASS * h, n = n0 + r;
       const bool in = n < a.N;
       cp_async_16(&Bs(stage)[r][piece], w + (in ? (size_t)n * a.K : 0) + (kb ? k : 0), in ? kb : 0);
       if (GLU) cp_async_16(&B2s(stage)[r][piece], w2 + (in ? (size_t)n * a.K : 0) + (kb ? k : 0), in ? kb : 0);
     }
   };
 
-  const int wm = (warp >> 2) * (16 * MT), wn = (warp & 3) * (8 * NT);
+  const int wm = warp / WARPS_N * (16 * MT), wn = warp % WARPS_N * (8 * NT);
   const int g = lane >> 2, t = lane & 3;
   float acc[MT][NT][4], acc2[GLU ? MT : 1][GLU ? NT : 1][4];
 #pragma unroll
@@ -307,23 +314,23 @@ __global__ void __launch_bounds__(GM_THREADS) gemm_grouped_mma_kernel(const Grou
     }
 }
 
-template <typename TO, int EPI, int MT>
+template <typename TO, int EPI, int MT, int BK>
 static int launch_mma(const GroupedGemmArgs& a, dim3 grid, cudaStream_t stream) {
-  constexpr int smem = GM_STAGES * gm_stage_rows<EPI, MT>() * GM_LD * (int)sizeof(__nv_bfloat16);
+  constexpr int smem = gm_stages(MT) * gm_stage_rows<EPI, MT>() * (BK + 8) * (int)sizeof(__nv_bfloat16);
   static bool configured = false;
   if (!configured) {
-    const cudaError_t e = cudaFuncSetAttribute(gemm_grouped_mma_kernel<TO, EPI, MT>,
+    const cudaError_t e = cudaFuncSetAttribute(gemm_grouped_mma_kernel<TO, EPI, MT, BK>,
                                                cudaFuncAttributeMaxDynamicSharedMemorySize, smem);
     if (e != cudaSuccess) return llmrs_fail("gemm_grouped: shared memory %d: %s", smem, cudaGetErrorString(e));
     configured = true;
   }
-  gemm_grouped_mma_kernel<TO, EPI, MT><<<grid, GM_THREADS, smem, stream>>>(a);
+  gemm_grouped_mma_kernel<TO, EPI, MT, BK><<<grid, gm_threads(MT), smem, stream>>>(a);
   return llmrs_launch_status("gemm_grouped (tensor cores)");
 }
 
-template <typename TO, int MT>
+template <typename TO, int MT, int BK>
 static int launch_grouped_mma(const GroupedGemmArgs& a, dim3 grid, cudaStream_t stream) {
-  return a.w2 != nullptr ? launch_mma<TO, EPI_UNIT, MT>(a, grid, stream) : launch_mma<TO, EPI_STORE, MT>(a, grid, stream);
+  return a.w2 != nullptr ? launch_mma<TO, EPI_UNIT, MT, BK>(a, grid, stream) : launch_mma<TO, EPI_STORE, MT, BK>(a, grid, stream);
 }
 
 // 0: the CUDA-core kernel for every product (set by tests that compare the two).
@@ -374,13 +381,15 @@ LLMRS_API int llmrs_gemm_grouped(const void* x, int x_dtype, long long x_stride,
     if (tile_rows == 128 && g_grouped_tc && src == nullptr && w_batch == (long long)N * K && x_stride > 0 &&
         (tiles || (K % 64 == 0 && x_batch > 0 && (long long)(batches - 1) * x_batch + K <= 0x7fffffffLL)))
       return launch_grouped_tc(a, out_dtype, x_rows, groups, batches, max_tiles, error_flag, stream);
-    const int cols = w2 ? GmCols<true>::value : GmCols<false>::value;
+    // Few rows: the weights' bytes are what counts. Tiles of at most 32 rows where the list cannot have longer ones.
+    const bool few = tiles && tile_rows == 64 && M <= 32, b16 = out_dtype == LLMRS_BF16;
+    const int cols = gm_cols(w2 != nullptr, few ? 1 : 2);
     dim3 mgrid((N + cols - 1) / cols, tiles ? max_tiles : (M + tile_rows - 1) / tile_rows, grid.z);
     if (tile_rows == 128)
-      return out_dtype == LLMRS_BF16 ? launch_grouped_mma<__nv_bfloat16, 4>(a, mgrid, stream)
-                                     : launch_grouped_mma<float, 4>(a, mgrid, stream);
-    return out_dtype == LLMRS_BF16 ? launch_grouped_mma<__nv_bfloat16, 2>(a, mgrid, stream)
-                                   : launch_grouped_mma<float, 2>(a, mgrid, stream);
+      return b16 ? launch_grouped_mma<__nv_bfloat16, 4, 32>(a, mgrid, stream) : launch_grouped_mma<float, 4, 32>(a, mgrid, stream);
+    if (few)
+      return b16 ? launch_grouped_mma<__nv_bfloat16, 1, 64>(a, mgrid, stream) : launch_grouped_mma<float, 1, 64>(a, mgrid, stream);
+    return b16 ? launch_grouped_mma<__nv_bfloat16, 2, 64>(a, mgrid, stream) : launch_grouped_mma<float, 2, 64>(a, mgrid, stream);
   }
   const int key = x_dtype * 4 + w_dtype * 2 + out_dtype;
   switch (key) {
@@ -411,7 +420,7 @@ LLMRS_API int llmrs_gemm_gates(const void* x, int x_dtype, long long x_stride, c
       ((uintptr_t)x & 15) == 0 && ((uintptr_t)w_r & 15) == 0 && ((uintptr_t)w_i & 15) == 0) {
     dim3 grid((n + 63) / 64, (M + tile_rows - 1) / tile_rows, blocks);
     LLMRS_REQUIRE(grid.y <= 65535, "gemm_gates: too many rows");
-    return launch_mma<float, EPI_GATES, 2>(a, grid, stream);
+    return launch_mma<float, EPI_GATES, 2, 32>(a, grid, stream);
   }
   dim3 grid((n + GG_BN - 1) / GG_BN, (M + GG_BM - 1) / GG_BM, blocks);
   LLMRS_REQUIRE(grid.y <= 65535, "gemm_gates: too many rows");

@@ -85,3 +85,66 @@ def test_a_wait_that_runs_out_is_reported():
     ops.gemm_batched(x.unflatten(1, (1, 256)), w, out)
     ops.check_tc_error(DEV)
     assert torch.allclose(out[:, 0].float(), x.float() @ w[0].float().t(), atol=0.5, rtol=2e-2)
+
+
+@pytest.mark.parametrize("out_dtype", [torch.float32, torch.bfloat16])
+@pytest.mark.parametrize("N,K,counts", [(64, 64, [1]), (200, 72, [3, 0, 29]), (33, 200, [16, 15]), (96, 8, [32]), (130, 136, [33, 1]),
+                                        (256, 512, [1] * 20), (65, 328, [64, 5])])
+def test_grouped_few_rows(N, K, counts, out_dtype):
+    """Tiles of 64 rows on mma.sync in steps of 64 of k, of 32 rows where the list has no more; beside the CUDA-core kernel."""
+    from llm_rs_b200 import ops
+    torch.manual_seed(N + K)
+    G, rows = len(counts), sum(counts)
+    w, w2 = (torch.randn(G, N, K, device=DEV).bfloat16() for _ in range(2))
+    x = torch.randn(9, K, device=DEV).bfloat16()
+    src = torch.randint(0, 9, (rows,), device=DEV, dtype=torch.int32)
+    starts = [sum(counts[:g]) for g in range(G)]
+    tiles = [(g, s + a, min(64, n - a)) for g, (s, n) in enumerate(zip(starts, counts)) for a in range(0, n, 64)]
+    n_tiles = torch.tensor([len(tiles)], dtype=torch.int32, device=DEV)
+    tiles = torch.tensor(tiles + [(0, 0, 0)] * 2, dtype=torch.int32, device=DEV)
+    out = torch.full((rows, N), 7.0, device=DEV, dtype=out_dtype)
+    ops.gemm_grouped(x, w, out, tiles, n_tiles, src, tile_rows=64)
+    for g, (s, n) in enumerate(zip(starts, counts)):
+        rows_x = x[src[s:s + n].long()]
+        want = rows_x.double() @ w[g].double().t()
+        assert bool(((out[s:s + n].double() - want).abs() <= _bound(rows_x, w[g], out_dtype, K)).all()), g
+    got, other = torch.empty(rows, N, device=DEV), torch.empty(rows, N, device=DEV)
+    for on, to in ((True, got), (False, other)):
+        ops.grouped_use_tensor_cores(on)
+        try:
+            ops.gemm_grouped(x, w, to, tiles, n_tiles, src, w2=w2, limit=7.0, alpha=1.702, shift=1.0, tile_rows=64)
+        finally:
+            ops.grouped_use_tensor_cores(True)
+    assert float((got - other).abs().max()) <= 1e-4 * max(1.0, float(other.abs().max()))
+
+
+@pytest.mark.parametrize("top,width,n", [(1, 4, 3), (4, 2048, 5), (5, 516, 2), (9, 1028, 1), (2, 30, 4)])
+@pytest.mark.parametrize("form", ["plain", "plain bf16", "shared", "shared gated bf16", "residual"])
+def test_combine(top, width, n, form):
+    """Sums of top + 2 products in float32 (an ulp each of the magnitudes) and one rounding of a bfloat16 output; a width of no
+    whole pieces takes the other kernel."""
+    from llm_rs_b200 import ops
+    torch.manual_seed(top + width)
+    rows = torch.randn(n * top, width, device=DEV)
+    row_of = torch.randperm(n * top, device=DEV).to(torch.int32)
+    weight = torch.rand(n * top, device=DEV)
+    parts = [(weight[t * top + k].double() * rows[row_of[t * top + k].long()].double()) for t in range(n) for k in range(top)]
+    parts = torch.stack(parts).view(n, top, width)
+    want, mag = parts.sum(1), parts.abs().sum(1)
+    rounding = 0.0
+    if form.startswith("plain"):
+        dtype = torch.bfloat16 if "bf16" in form else torch.float32
+        got = ops.moe_combine(rows, row_of, weight, top, dtype) if dtype == torch.bfloat16 else ops.moe_combine(rows, row_of, weight, top)
+        rounding = 2.0 ** -8 if dtype == torch.bfloat16 else 0.0
+    else:
+        shared = torch.randn(n, width, device=DEV).to(torch.bfloat16 if "bf16" in form else torch.float32)
+        gate = torch.randn(n, 3, device=DEV)[:, 1] if "gated" in form else None
+        own = shared.double() * (torch.sigmoid(gate.double())[:, None] if gate is not None else 1.0)
+        want, mag = want + own, mag + own.abs()
+        if form == "residual":
+            got = torch.randn(n, width, device=DEV)
+            want, mag = want + got.double(), mag + got.double().abs()
+            ops.moe_combine_shared(rows, row_of, weight, top, shared, gate, residual=got)
+        else:
+            got = ops.moe_combine_shared(rows, row_of, weight, top, shared, gate)
+    assert bool(((got.double() - want).abs() <= mag * (top + 4) * 2.0 ** -24 + rounding * want.abs() + 1e-30).all())
