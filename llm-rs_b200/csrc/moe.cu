@@ -129,6 +129,74 @@ LLMRS_API int llmrs_moe_sort(const int* expert_of, int* row_of, int* src_token, 
 }
 
 // ---------------------------------------------------------------------------------
+// The weighted sums below for widths of whole pieces of four on 16-byte boundaries, the same sums in the same order: a thread
+// takes a piece of a token, the token's rows four at a time with their loads in flight together, several blocks a token. A
+// block per token with a channel a load waited for every row's index and row in turn. 2,048 tokens of four rows of 2,048
+// beside a shared one (92 MB): 26.4 -> 18.3 us (5.0 TB/s); 8 tokens: 8.1 -> 2.4.
+// ---------------------------------------------------------------------------------
+constexpr int MC_THREADS = 128;
+template <typename TS, typename TO>
+__global__ void __launch_bounds__(MC_THREADS)
+moe_combine_wide_kernel(const float* __restrict__ rows, const int* __restrict__ row_of, const float* __restrict__ weight_of,
+                        const TS* __restrict__ shared, const float* __restrict__ gate, long long gate_stride, TO* __restrict__ out,
+                        int top, int width, int add) {
+  struct alignas(4 * sizeof(TS)) Piece { TS x[4]; };
+  struct alignas(4 * sizeof(TO)) Out { TO x[4]; };
+  const int t = blockIdx.x, c = (blockIdx.y * MC_THREADS + threadIdx.x) * 4;
+  if (c >= width) return;
+  const size_t at = (size_t)t * width + c;
+  Piece own;
+  Out before;
+  float raw_gate = 0.f;
+  if (shared) {
+    own = *reinterpret_cast<const Piece*>(shared + at);
+    if (gate) raw_gate = gate[(size_t)t * gate_stride];
+  }
+  if (add) before = *reinterpret_cast<const Out*>(out + at);
+  float s[4] = {0.f, 0.f, 0.f, 0.f};
+  for (int k0 = 0; k0 < top; k0 += 4) {
+    float4 x[4];
+    float w[4];
+#pragma unroll
+    for (int k = 0; k < 4; ++k)
+      if (k0 + k < top) {
+        w[k] = weight_of[t * top + k0 + k];
+        x[k] = *reinterpret_cast<const float4*>(rows + (size_t)row_of[t * top + k0 + k] * width + c);
+      }
+#pragma unroll
+    for (int k = 0; k < 4; ++k)
+      if (k0 + k < top) {
+        s[0] = fmaf(w[k], x[k].x, s[0]);
+        s[1] = fmaf(w[k], x[k].y, s[1]);
+        s[2] = fmaf(w[k], x[k].z, s[2]);
+        s[3] = fmaf(w[k], x[k].w, s[3]);
+      }
+  }
+  const float g = gate ? 1.0f / (1.0f + expf(-raw_gate)) : 1.0f;
+  Out y;
+#pragma unroll
+  for (int e = 0; e < 4; ++e) {
+    if (shared) s[e] = fmaf(g, to_float(own.x[e]), s[e]);
+    if (add) s[e] += to_float(before.x[e]);
+    y.x[e] = from_float<TO>(s[e]);
+  }
+  *reinterpret_cast<Out*>(out + at) = y;
+}
+
+// Launches it where the rows allow it.
+template <typename TS, typename TO>
+static bool combine_wide(const float* rows, const int* row_of, const float* weight_of, const TS* shared, const float* gate,
+                         long long gate_stride, TO* out, int n_tokens, int top, int width, int add, cudaStream_t stream) {
+  const int blocks = (width + 4 * MC_THREADS - 1) / (4 * MC_THREADS);
+  if (width % 4 != 0 || blocks > 65535 || ((uintptr_t)rows & 15) != 0 || ((uintptr_t)shared & (4 * sizeof(TS) - 1)) != 0 ||
+      ((uintptr_t)out & (4 * sizeof(TO) - 1)) != 0)
+    return false;
+  moe_combine_wide_kernel<TS, TO><<<dim3(n_tokens, blocks), MC_THREADS, 0, stream>>>(rows, row_of, weight_of, shared, gate,
+                                                                                    gate_stride, out, top, width, add);
+  return true;
+}
+
+// ---------------------------------------------------------------------------------
 // out[t, :] = sum_k weight_of[t * top + k] * rows[row_of[t * top + k], :], k in order, float32.
 // ---------------------------------------------------------------------------------
 template <typename TO>
@@ -147,6 +215,12 @@ LLMRS_API int llmrs_moe_combine(const float* rows, const int* row_of, const floa
                                 int out_dtype, int n_tokens, int top, int width, cudaStream_t stream) {
   LLMRS_REQUIRE(n_tokens >= 0 && top > 0 && width > 0, "moe_combine: bad sizes");
   if (n_tokens == 0) return 0;
+  const float* none = nullptr;
+  if ((out_dtype == LLMRS_F32 &&
+       combine_wide(rows, row_of, weight_of, none, none, 0, (float*)out, n_tokens, top, width, 0, stream)) ||
+      (out_dtype == LLMRS_BF16 &&
+       combine_wide(rows, row_of, weight_of, none, none, 0, (__nv_bfloat16*)out, n_tokens, top, width, 0, stream)))
+    return llmrs_launch_status("moe_combine");
   const int threads = width >= 1024 ? 256 : 128;
   if (out_dtype == LLMRS_F32)
     moe_combine_kernel<float><<<n_tokens, threads, 0, stream>>>(rows, row_of, weight_of, (float*)out, top, width);
@@ -245,8 +319,13 @@ LLMRS_API int llmrs_moe_combine_shared(const float* rows, const int* row_of, con
                                        float* out, int n_tokens, int top, int width, int add, cudaStream_t stream) {
   LLMRS_REQUIRE(n_tokens >= 0 && top > 0 && width > 0, "moe_combine_shared: bad sizes");
   if (n_tokens == 0) return 0;
+  const bool f32 = shared == nullptr || shared_dtype == LLMRS_F32;
+  if ((f32 && combine_wide(rows, row_of, weight_of, (const float*)shared, gate, gate_stride, out, n_tokens, top, width, add, stream)) ||
+      (!f32 && shared_dtype == LLMRS_BF16 &&
+       combine_wide(rows, row_of, weight_of, (const __nv_bfloat16*)shared, gate, gate_stride, out, n_tokens, top, width, add, stream)))
+    return llmrs_launch_status("moe_combine_shared");
   const int threads = width >= 1024 ? 256 : 128;
-  if (shared == nullptr || shared_dtype == LLMRS_F32)
+  if (f32)
     moe_combine_shared_kernel<float><<<n_tokens, threads, 0, stream>>>(rows, row_of, weight_of, (const float*)shared,
                                                                        gate, gate_stride, out, top, width, add);
   else if (shared_dtype == LLMRS_BF16)
