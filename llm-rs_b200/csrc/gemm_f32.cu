@@ -13,14 +13,19 @@
 // neighbouring rows' 16-byte reads fall into different banks; a thread reads four values of K of its TM rows and TN
 // features at a time and adds them in order of K. An output is ONE chain of fused multiply-adds whatever the tile, which
 // keeps its bits the same in every batch, and is why no tile splits K: a product of few rows is bound by that chain and by
-// the latency of its stages (K = 3,072 into 1,024 features, one row: 19 us, 236 before with one synchronous stage of 16
-// values), one of many features by the stream of its weights (1,024 into 32,000: 42 us, 3.1 TB/s; 185 before), one of many
+// the latency of its stages (K = 3,072 into 1,024 features, one row: 15.5 us, 236 before with one synchronous stage of 16
+// values), one of many features by the stream of its weights (1,024 into 32,000: 35 us, 3.7 TB/s; 185 before), one of many
 // rows by the FMA units (2,048 rows of 4,096 x 4,096: 1,867 us, 36.8 TFLOP/s; 2,711 before).
+// (A tile of few outputs has more threads than outputs: its copies are dealt out over four warps, so that the one that adds loses
+// less time to them.)
+__host__ __device__ constexpr int gf_threads(int bm, int bn, int tm, int tn) {
+  return (bm / tm) * (bn / tn) < 128 ? 128 : (bm / tm) * (bn / tn);
+}
 template <typename TX, int BM, int BN, int TM, int TN, int BK, int NS, int U, bool VEC>
-__global__ void __launch_bounds__((BM / TM) * (BN / TN))
+__global__ void __launch_bounds__(gf_threads(BM, BN, TM, TN))
 gemm_f32_kernel(const TX* __restrict__ x, const float* __restrict__ w, const float* __restrict__ bias,
                 float* __restrict__ out, int M, int N, int K, long long x_stride, long long out_stride) {
-  constexpr int THREADS = (BM / TM) * (BN / TN), CN = BN / TN, RM = BM / TM;
+  constexpr int THREADS = gf_threads(BM, BN, TM, TN), CN = BN / TN, RM = BM / TM;
   constexpr int XS = BK + 16 / (int)sizeof(TX), WS = BK + 4;      // elements a row of a stage takes
   extern __shared__ __align__(16) unsigned char gf_raw[];
   float* ws = reinterpret_cast<float*>(gf_raw);                   // [NS][BN][WS]
@@ -71,6 +76,7 @@ gemm_f32_kernel(const TX* __restrict__ x, const float* __restrict__ w, const flo
     __syncthreads();      // stage `it` is there for everyone, and everyone is done with the stage that is filled next
     if (it + NS - 1 < steps) load((it + NS - 1) % NS, (it + NS - 1) * BK);
     else cp_async_commit();
+    if (RM * CN < THREADS && tid >= RM * CN) continue;      // only copies
     const float* wr = ws + (it % NS) * BN * WS;
     const TX* xr = xs + (it % NS) * BM * XS;
     // The next U pieces are read while the present ones are added: a warp alone on its scheduler would otherwise wait
@@ -111,6 +117,7 @@ gemm_f32_kernel(const TX* __restrict__ x, const float* __restrict__ w, const flo
           }
     }
   }
+  if (RM * CN < THREADS && tid >= RM * CN) return;
 #pragma unroll
   for (int i = 0; i < TM; ++i) {
     const int m = m0 + ty + i * RM;
@@ -127,7 +134,7 @@ template <typename TX, int BM, int BN, int TM, int TN, int BK, int NS, int U>
 static int launch_gemm_f32(bool vec, const TX* x, long long x_stride, const float* w, const float* bias, float* out,
                            long long out_stride, int M, int N, int K, cudaStream_t stream) {
   constexpr size_t smem = (size_t)NS * (BN * (BK + 4) * sizeof(float) + BM * (BK * sizeof(TX) + 16));
-  constexpr int threads = (BM / TM) * (BN / TN);
+  constexpr int threads = gf_threads(BM, BN, TM, TN);
   const dim3 grid((N + BN - 1) / BN, (M + BM - 1) / BM);
   LLMRS_REQUIRE(grid.y <= 65535, "gemm_f32: M=%d is too large", M);
   auto go = [&](auto kernel) {
@@ -162,6 +169,13 @@ static int gemm_f32_any(const TX* x, long long x_stride, const float* w, const f
   if (M > 8 && blocks(16, 32) >= ENOUGH) LLMRS_GF(16, 32, 2, 2, 64, 4, 2);
   if (M > 4 && blocks(8, 32) >= ENOUGH) LLMRS_GF(8, 32, 2, 1, 64, 4, 4);
   if (M > 4) LLMRS_GF(8, 16, 1, 1, 64, 4, 4);
+  if (M == 1) {      // tiles of one row read the weights from shared memory once, where those of four rows read them for each: 1,024
+                     // into 32,000 features 35 us (46), into 6,144 9.8 (14), K = 3,072 into 1,024 15.5 (19)
+    if (N >= 64 * 2 * ENOUGH) LLMRS_GF(1, 64, 1, 1, 64, 3, 4);
+    if (N >= 32 * ENOUGH) LLMRS_GF(1, 32, 1, 1, 128, 4, 4);
+    if (N >= 16 * ENOUGH) LLMRS_GF(1, 16, 1, 1, 128, 6, 4);
+    LLMRS_GF(1, 8, 1, 1, 256, 6, 4);
+  }
   if (blocks(4, 32) >= 2 * ENOUGH) LLMRS_GF(4, 32, 1, 1, 64, 4, 4);
   LLMRS_GF(4, 8, 1, 1, 128, 4, 4);
 #undef LLMRS_GF

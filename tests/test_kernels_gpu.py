@@ -96,7 +96,7 @@ def test_gemm_f32_is_true_float32(M, N, K):
 
 @pytest.mark.parametrize("rows_dtype", [torch.float32, torch.bfloat16])
 @pytest.mark.parametrize("N,K,pad", [(300, 128, 0), (300, 132, 8), (1184, 68, 0), (1200, 100, 4), (4800, 36, 0), (301, 67, 1),
-                                     (2368, 260, 3)])
+                                     (2368, 260, 3), (19000, 44, 4)])
 def test_gemm_f32_tiles(N, K, pad, rows_dtype):
     """Every tile of the float32 product at its edges (rows, features and K that fill no tile, rows with a stride, rows
     that no sixteen-byte copy can take), against float64, and every row's bits the same in every batch. An output is one
