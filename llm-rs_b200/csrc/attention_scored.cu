@@ -1540,7 +1540,7 @@ LLMRS_API int llmrs_scored_decode_group(int n_q_heads, int n_kv_heads, int dk, i
 
 // Whether the decode kernel on the tensor cores takes these heads (bfloat16, keys and values of 64 or 128 channels). It streams
 // tiles through rings: callers give it longer runs of keys.
-LLMRS_API int llmrs_scored_decode_on_tensor_cores(int dk, int dv, int dtype) {
+static bool decode_on_tensor_cores(int dk, int dv, int dtype) {
   return dtype == LLMRS_BF16 && dk == dv && (dk == 64 || dk == 128) && !g_scored_generic_only;
 }
 
@@ -1577,7 +1577,7 @@ LLMRS_API int llmrs_scored_decode(const void* q, long long q_stride, void* out, 
   const int gh = llmrs_scored_decode_group(n_q_heads, n_kv_heads, dk, dv, page_size, dtype);
   const bool grouped = gh > 0 && ((uintptr_t)cache & 15) == 0 && !g_scored_generic_only;
   const int G = n_q_heads / n_kv_heads;
-  if (llmrs_scored_decode_on_tensor_cores(dk, dv, dtype) && ((uintptr_t)cache & 15) == 0 && ((uintptr_t)q & 3) == 0 &&
+  if (decode_on_tensor_cores(dk, dv, dtype) && ((uintptr_t)cache & 15) == 0 && ((uintptr_t)q & 3) == 0 &&
       q_stride % 2 == 0 && n_kv_heads * ((G + 3) / 4) <= 65535) {
     const dim3 tgrid(n_dec, n_kv_heads * ((G + 3) / 4), max_splits);
     auto go = [&](auto kernel, int ring) {

@@ -1375,7 +1375,7 @@ def scored_decode_runs(n_dec: int, n_q_heads: int, n_kv_heads: int, dk: int, dv:
     """(runs, keys per run) for the tensor-core decode kernel over at most ``span`` visible keys, or None where it does not take
     these heads. A run of 64 keys is one tile for each of a block's four warps; longer runs keep their rings full, and the
     merge reads fewer of them."""
-    if not _lib().llmrs_scored_decode_on_tensor_cores(dk, dv, dtype_code(dtype)):
+    if dtype != torch.bfloat16 or dk != dv or dk not in (64, 128):      # (csrc/attention_scored.cu decode_on_tensor_cores)
         return None
     blocks = n_dec * n_kv_heads * -(-(n_q_heads // n_kv_heads) // 4)
     runs = max(1, min(-(-DECODE_STREAM_BLOCKS // blocks), -(-span // 64)))
