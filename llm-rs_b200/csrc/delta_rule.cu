@@ -20,7 +20,8 @@
 //               (16-byte asynchronous copies), so the next chunk arrives while this one is walked, and are read as
 //               16-byte broadcasts. The state lives in float32 per request slot, read at the start and written at the
 //               end: a step of one token (decoding) and a prompt's portion are the same kernel;
-//   output      a warp per (token, head): divides by the head's root mean square, applies the weight and the gate.
+//   output      divides by the head's root mean square, applies the weight and the gate (head_out.cuh; heads that it does not
+//               take: a warp per token and head).
 #include "common.cuh"
 #include "head_out.cuh"
 #include "mma_util.cuh"

@@ -26,7 +26,7 @@
 //                four holds channels 4 (p + 4 j) .. 4 (p + 4 j) + 3, so that the four read neighbouring 16-byte pieces
 //                of a row in shared memory, not pieces a bank's stride apart); k^T S and q^T S are summed over the four
 //                by two shuffles. Rows come in chunks through two shared-memory buffers.
-//   output       a warp per (token, head): norm, weight, gate
+//   output       norm, weight, gate (head_out.cuh; heads that it does not take: a warp per token and head)
 //
 // Long portions may take the recurrence in CHUNKS of 32 tokens instead (the same numbers up to float32 rounding, all of it
 // float32 FMA). Within a chunk that starts from the state S_0, with L_t the sum of log g up to and including token t:
