@@ -1212,18 +1212,19 @@ def linear_recurrence(q, k, v, gate, norm_w, state, ctx, n_heads: int, dk: int, 
     if (normaliser is None) != (floor is None):
         raise KernelError("linear_recurrence: normaliser and floor come together")
     dev = q.device
-    work = torch.empty((int(_lib_ll("llmrs_linear_recurrence_work_floats")(n, ctx.n_requests, n_heads, dk, dv)),), dtype=torch.float32,
-                       device=dev)
-    o_raw = torch.empty((n, n_heads * dv), dtype=torch.float32, device=dev)
-    nq = torch.empty((n, n_heads), dtype=torch.float32, device=dev) if normaliser is not None else None
+    # One workspace: the kernels' rows, then the raw read-outs and the normaliser's products.
+    n_work = -(-int(_lib_ll("llmrs_linear_recurrence_work_floats")(n, ctx.n_requests, n_heads, dk, dv)) // 4) * 4
+    work = torch.empty((n_work + n * n_heads * (dv + 1),), dtype=torch.float32, device=dev)
+    o_raw = ctypes.c_void_p(work.data_ptr() + 4 * n_work)
+    nq = ctypes.c_void_p(work.data_ptr() + 4 * (n_work + n * n_heads * dv) if normaliser is not None else 0)
     _check(_lib().llmrs_linear_recurrence(
         _ptr(q), _ptr(k), _ptr(v), _LL(_row_stride(q, "q")), _LL(_row_stride(k, "k")), _LL(_row_stride(v, "v")),
         dtype_code(q.dtype), int(act_silu), ctypes.c_float(q_scale), ctypes.c_float(k_scale), _ptr(inv_freq),
         _ptr(ctx.positions) if rot_dims else None, rot_dims, _ptr(decay), _ptr(head_decay), _ptr(gain), _ptr(state), _ptr(normaliser), _ptr(ctx.q_start), _ptr(ctx.n_new), _ptr(ctx.slot_ids), _ptr(work),
-        _ptr(o_raw), _ptr(nq), n, ctx.n_requests, n_heads, dk, dv, _stream()), "linear_recurrence", 2)
+        o_raw, nq, n, ctx.n_requests, n_heads, dk, dv, _stream()), "linear_recurrence", 2)
     out = torch.empty((n, n_heads * dv), dtype=q.dtype, device=dev)
     _check(_lib().llmrs_recurrence_output(
-        _ptr(o_raw), _ptr(nq), _ptr(floor), ctypes.c_float(den_eps), _ptr(gate), _LL(_row_stride(gate, "gate")),
+        o_raw, nq, _ptr(floor), ctypes.c_float(den_eps), _ptr(gate), _LL(_row_stride(gate, "gate")),
         dtype_code(q.dtype), _ptr(norm_w), _ptr(out), n, n_heads, dv, int(per_head_norm), int(gate_silu),
         ctypes.c_float(norm_eps), _stream()), "recurrence_output")
     return out
