@@ -66,13 +66,16 @@ def portion_tiles(q_start, n_new, tile_tokens: int) -> np.ndarray:
 
 
 def expanded_rows(n_new, cached, window: int, row_bytes: int):
-    """Per request the position of the first key that is made for the step (a multiple of EXPAND_ALIGN), how many are, and
-    whether the request's portion is taken that way (``row_bytes`` a key; 0: none are; at most
-    ``ops.LATENT_EXPAND_BYTES`` together)."""
+    """Per request the position of the first key that is made for the step (a multiple of EXPAND_ALIGN), how many rows are made
+    for it, and whether the request's portion is taken that way (``row_bytes`` a row; 0: none are; at most
+    ``ops.LATENT_EXPAND_BYTES`` together). A request's rows are whole tiles of the attention kernel, zeros past its last key:
+    a tile that ran on into the next request's rows would multiply their values by weights of zero, which is no number where
+    they are infinite."""
     lo = np.maximum(0, cached - window + 1) if window > 0 else np.zeros_like(cached)
     first = lo // EXPAND_ALIGN * EXPAND_ALIGN
-    counts = cached + n_new - first
-    is_long = (n_new >= EXPAND_MIN_TOKENS) & (counts <= EXPAND_MAX_KEYS * n_new) & (row_bytes > 0)
+    keys = cached + n_new - first
+    counts = -(-keys // EXPAND_ALIGN) * EXPAND_ALIGN
+    is_long = (n_new >= EXPAND_MIN_TOKENS) & (keys <= EXPAND_MAX_KEYS * n_new) & (row_bytes > 0)
     is_long &= np.cumsum(np.where(is_long, counts, 0)) * row_bytes <= ops.LATENT_EXPAND_BYTES
     return first, np.where(is_long, counts, 0), is_long
 

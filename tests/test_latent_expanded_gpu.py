@@ -61,6 +61,41 @@ def _plain(part, w, x, dn, dr, rank, nh, window, cached, latents, parts):
     return out.reshape(n, -1) @ w["o"].t(), latents, parts
 
 
+def _small_part(window):
+    """A part of 4 heads of 64 + 32 over latents of 128, bound to random weights."""
+    from llm_rs_b200.parts import Runtime
+    from llm_rs_b200.parts import latent_attention as L
+    g = torch.Generator().manual_seed(5)
+    part = L.LatentAttention(96, 4, 64, 32, 128, 128, 96 ** -0.5, 900.0, window=window, prefix="m.")
+    part.bind({s.name: (torch.ones(s.shape) if len(s.shape) == 1 else torch.randn(s.shape, generator=g) * s.shape[1] ** -0.5)
+               .to(DEV, torch.float32 if len(s.shape) == 1 else torch.bfloat16) for s in part.weight_specs()},
+              Runtime(torch.device(DEV), torch.bfloat16, 4096))
+    return part
+
+
+def _small_cache(n_requests, n_pages):
+    pages = torch.zeros((n_requests * n_pages, 1, PAGE * (128 + 32)), dtype=torch.bfloat16, device=DEV)
+    planes = [pages[:, :, : PAGE * 128].unflatten(2, (PAGE, 128)), pages[:, :, PAGE * 128:].unflatten(2, (PAGE, 32))]
+    table = torch.arange(n_requests * n_pages, dtype=torch.int32, device=DEV).view(n_requests, n_pages)
+    return SimpleNamespace(planes=planes, block_table=table, page_size=PAGE, owns=True, state={})
+
+
+@pytest.mark.parametrize("bad", [float("inf"), float("-inf"), float("nan")])
+@pytest.mark.parametrize("lens", [(40, 50), (130, 64), (128, 33), (200, 255)])
+def test_a_neighbours_numbers_do_not_reach_a_request(lens, bad):
+    """Both requests' keys are made for the step: what the second one holds must not change a bit of the first one's output."""
+    part = _small_part(window=0)
+    x = torch.randn(sum(lens), 96, generator=torch.Generator().manual_seed(1)).to(DEV, torch.bfloat16)
+    ctx = _step(part, lens, (0, 0))
+    assert ctx.plans[part.plan_key()].values["n_long"] == sum(-(-n // 128) for n in lens)
+    want = part.forward(x, ctx, _small_cache(2, 16))
+    x = x.clone()
+    x[lens[0]:] = bad
+    got = part.forward(x, ctx, _small_cache(2, 16))
+    assert torch.equal(got[: lens[0]], want[: lens[0]])
+    assert torch.isnan(got[lens[0]:]).all()
+
+
 @pytest.mark.parametrize("dn,dr,rank,nh,window,gated,cuts", [
     (128, 64, 512, 8, 0, True, [(300, 64), (129, 1), (70, 200)]), (64, 32, 128, 8, 100, True, [(128, 90), (257, 64), (64, 13)]),
     (128, 16, 64, 5, 257, False, [(65, 700), (200, 127)]), (64, 64, 256, 16, 1024, True, [(1200, 1), (333, 1)]),
