@@ -1057,7 +1057,10 @@ LLMRS_API int llmrs_latent_attention_prefill(const void* qa, long long qa_token,
 // ---------------------------------------------------------------------------------
 // The cached rows that long prompt portions see, side by side: c [rows, rank] and kr [rows, dr]. row_of [requests][2]: the row
 // of a request's first key and that key's position; a warp per row. Keys before the request's first visible one (their pages
-// may be gone) are zeros, and so are rows of requests that have none.
+// may be gone) are zeros, and so are rows past its last one.
+// A latent that is infinite or no number goes into the key's SCORE: zeros in c, no numbers in kr. The queries that see the key
+// then get no number, as from the latent itself; the others of a tile, whose weight for it is zero, keep theirs, where zero
+// times its value would be no number.
 // ---------------------------------------------------------------------------------
 __global__ void __launch_bounds__(256)
 latent_gather_kernel(const __nv_bfloat16* __restrict__ cache, const int* __restrict__ table, int table_width,
@@ -1083,9 +1086,17 @@ latent_gather_kernel(const __nv_bfloat16* __restrict__ cache, const int* __restr
     src = reinterpret_cast<const uint4*>(base + (size_t)at * rank);
     src_r = reinterpret_cast<const uint4*>(base + (size_t)page_size * rank + (size_t)at * dr);
   }
-  const uint4 zero = make_uint4(0u, 0u, 0u, 0u);
-  for (int e = lane; e < rank / 8; e += 32) reinterpret_cast<uint4*>(c + (size_t)row * rank)[e] = seen ? src[e] : zero;
-  for (int e = lane; e < dr / 8; e += 32) reinterpret_cast<uint4*>(kr + (size_t)row * dr)[e] = seen ? src_r[e] : zero;
+  const uint4 zero = make_uint4(0u, 0u, 0u, 0u), no_number = make_uint4(0x7fc07fc0u, 0x7fc07fc0u, 0x7fc07fc0u, 0x7fc07fc0u);
+  auto not_finite = [](uint32_t pair) { return (pair & 0x7f80u) == 0x7f80u || (pair & 0x7f800000u) == 0x7f800000u; };
+  bool bad = false;
+  for (int e = lane; seen && e < rank / 8; e += 32) {
+    const uint4 x = src[e];
+    bad |= not_finite(x.x) || not_finite(x.y) || not_finite(x.z) || not_finite(x.w);
+  }
+  bad = __any_sync(0xffffffffu, bad);
+  for (int e = lane; e < rank / 8; e += 32) reinterpret_cast<uint4*>(c + (size_t)row * rank)[e] = seen && !bad ? src[e] : zero;
+  for (int e = lane; e < dr / 8; e += 32)
+    reinterpret_cast<uint4*>(kr + (size_t)row * dr)[e] = !seen ? zero : (bad ? no_number : src_r[e]);
 }
 
 LLMRS_API int llmrs_latent_gather(const void* cache, const int* table, int table_width, const int* row_of, const int* n_new,

@@ -1091,7 +1091,7 @@ def latent_gather(cache: torch.Tensor, table: torch.Tensor, ctx, row_of: torch.T
                   page_size: int, window: int):
     """The cached rows that a step's long portions see: (latents [n_rows, rank], rotated key parts [n_rows, dr]), bfloat16.
     ``row_of`` int32 [requests, 2]: the row of a request's first key and that key's position; keys no query of the step may
-    see are zeros."""
+    see are zeros. Of a key with a latent that is not finite the latent is zeros and the rotated part no numbers."""
     _need(cache, "cache", torch.bfloat16)
     _need(row_of, "row_of", torch.int32)
     c = torch.empty((n_rows, rank), dtype=torch.bfloat16, device=cache.device)

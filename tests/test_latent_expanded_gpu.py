@@ -96,6 +96,34 @@ def test_a_neighbours_numbers_do_not_reach_a_request(lens, bad):
     assert torch.isnan(got[lens[0]:]).all()
 
 
+@pytest.mark.parametrize("bad", [float("inf"), float("-inf"), float("nan")])
+@pytest.mark.parametrize("window,n,cached,at", [(0, 100, 0, 99), (0, 200, 60, 131), (0, 130, 0, 64), (20, 150, 40, 30),
+                                                (20, 100, 40, 38), (50, 260, 0, 128)])
+def test_a_key_that_is_not_finite_reaches_its_queries_only(window, n, cached, at, bad):
+    """The latent at position ``at`` (a cached one, or a new one) is ``bad`` in one channel: the queries before it, and those
+    whose window has passed it, keep every bit."""
+    part = _small_part(window)
+    x = torch.randn(n, 96, generator=torch.Generator().manual_seed(2)).to(DEV, torch.bfloat16)
+    ctx = _step(part, (n,), (cached,))
+    assert ctx.plans[part.plan_key()].values["n_long"] == -(-n // 128)
+
+    def run(poison):
+        cache = _small_cache(1, 20)
+        cache.planes[0].copy_(torch.randn(cache.planes[0].shape, generator=torch.Generator().manual_seed(3)))
+        if poison and at < cached:
+            cache.planes[0][at // PAGE, 0, at % PAGE, 77] = bad
+        rows = x.clone()
+        if poison and at >= cached:
+            rows[at - cached] = bad
+        return part.forward(rows, ctx, cache)
+    want, got = run(False), run(True)
+    pos = cached + torch.arange(n, device=DEV)
+    sees = (pos >= at) & ((pos < at + window) if window else True)
+    assert torch.isfinite(want).all() and sees.any() and not sees.all()
+    assert torch.equal(got[~sees], want[~sees])
+    assert torch.isnan(got[sees]).all()
+
+
 @pytest.mark.parametrize("dn,dr,rank,nh,window,gated,cuts", [
     (128, 64, 512, 8, 0, True, [(300, 64), (129, 1), (70, 200)]), (64, 32, 128, 8, 100, True, [(128, 90), (257, 64), (64, 13)]),
     (128, 16, 64, 5, 257, False, [(65, 700), (200, 127)]), (64, 64, 256, 16, 1024, True, [(1200, 1), (333, 1)]),
