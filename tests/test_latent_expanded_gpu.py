@@ -62,11 +62,11 @@ def _plain(part, w, x, dn, dr, rank, nh, window, cached, latents, parts):
 
 
 def _small_part(window):
-    """A part of 4 heads of 64 + 32 over latents of 128, bound to random weights."""
+    """A part of 8 heads of 64 + 32 over latents of 128, bound to random weights."""
     from llm_rs_b200.parts import Runtime
     from llm_rs_b200.parts import latent_attention as L
     g = torch.Generator().manual_seed(5)
-    part = L.LatentAttention(96, 4, 64, 32, 128, 128, 96 ** -0.5, 900.0, window=window, prefix="m.")
+    part = L.LatentAttention(96, 8, 64, 32, 128, 128, 96 ** -0.5, 900.0, window=window, prefix="m.")
     part.bind({s.name: (torch.ones(s.shape) if len(s.shape) == 1 else torch.randn(s.shape, generator=g) * s.shape[1] ** -0.5)
                .to(DEV, torch.float32 if len(s.shape) == 1 else torch.bfloat16) for s in part.weight_specs()},
               Runtime(torch.device(DEV), torch.bfloat16, 4096))
