@@ -21,7 +21,10 @@
 // than they save reads. Products run as packed pairs of float32 along the channels. The eight sums of a turn (four tokens,
 // two columns) are dealt out over the lanes as they are summed: eight shuffles instead of the 32 of eight full sums. Rows
 // arrive by 16-byte asynchronous copies through a ring of four stages of two turns, which are one stretch of code: a turn's
-// read-outs are summed under the next one's products.
+// read-outs are summed under the next one's products. What later tokens of the turn write is masked out of a token's read-out
+// bit by bit: a coefficient of zero would not do, zero times an infinite value is no number. (Gated 402 us without, 406 with it;
+// selects or branches in its place
+// broke the stretch up: 437 and 485.)
 //
 // Measured against the walk token by token (one by one -> in turns, the recurrence alone, bfloat16 models): gated, 2,048 tokens
 // of 16 heads of 128 x 128: 497 -> 265 us; general, 32 heads of 64 x 64: 816 -> 246 us; linear with a normaliser, portions of
@@ -84,6 +87,8 @@ __device__ __forceinline__ f2 f2_mul(f2 a, f2 b) {
   asm("mul.rn.f32x2 %0, %1, %2;" : "=l"(r) : "l"(a), "l"(b));
   return r;
 }
+
+__device__ __forceinline__ float walk_keep(float v, unsigned mask) { return __uint_as_float(__float_as_uint(v) & mask); }
 
 // Sums eight values over sixteen neighbouring lanes: lanes p and p + 8 end with the sum of value p & 7.
 __device__ __forceinline__ float walk_sum8(const float (&v)[8], int part) {
@@ -282,6 +287,7 @@ __global__ void __launch_bounds__(WALK_THREADS, 2) state_walk_kernel(WalkArgs p,
   }
   // The token of a turn and the column whose sum this lane ends with.
   const int mine = (part >> 1) & 3, my_c = part & 1;
+  const unsigned keep1 = mine < 1 ? 0u : ~0u, keep2 = mine < 2 ? 0u : ~0u, keep3 = mine < 3 ? 0u : ~0u;
   const bool my_norm = norm[my_c], writes = part < 8 && live[my_c];
   const float my_skip = p.skip ? p.skip[head] : 0.f;
   float* o_at = my_norm ? p.nq + (size_t)t0 * p.n_heads + head : p.o_raw + ((size_t)t0 * p.n_heads + head) * dv + col + my_c;
@@ -430,12 +436,12 @@ __global__ void __launch_bounds__(WALK_THREADS, 2) state_walk_kernel(WalkArgs p,
     float o = walk_sum8(qd, part);
     if (!CHANNEL) o *= tab[WALK_P + mine];
     const float4 Q = *reinterpret_cast<const float4*>(tab + (MODE == WALK_GENERAL ? WALK_GQ : WALK_Q) + 4 * mine);
-    o = fmaf(Q.w, my_c ? y[1][3] : y[0][3], fmaf(Q.z, my_c ? y[1][2] : y[0][2],
-        fmaf(Q.y, my_c ? y[1][1] : y[0][1], fmaf(Q.x, my_c ? y[1][0] : y[0][0], o))));
+    o = fmaf(Q.w, walk_keep(my_c ? y[1][3] : y[0][3], keep3), fmaf(Q.z, walk_keep(my_c ? y[1][2] : y[0][2], keep2),
+        fmaf(Q.y, walk_keep(my_c ? y[1][1] : y[0][1], keep1), fmaf(Q.x, my_c ? y[1][0] : y[0][0], o))));
     if constexpr (MODE == WALK_GENERAL) {
       const float4 R = *reinterpret_cast<const float4*>(tab + WALK_GR + 4 * mine);
-      o = fmaf(R.w, my_c ? v[1][3] : v[0][3], fmaf(R.z, my_c ? v[1][2] : v[0][2],
-          fmaf(R.y, my_c ? v[1][1] : v[0][1], fmaf(R.x, my_c ? v[1][0] : v[0][0], o))));
+      o = fmaf(R.w, walk_keep(my_c ? v[1][3] : v[0][3], keep3), fmaf(R.z, walk_keep(my_c ? v[1][2] : v[0][2], keep2),
+          fmaf(R.y, walk_keep(my_c ? v[1][1] : v[0][1], keep1), fmaf(R.x, my_c ? v[1][0] : v[0][0], o))));
     }
     if constexpr (MODE == WALK_LINEAR) {
       if (p.skip) o = fmaf(my_skip, base[AT_V + (g * WALK_TURN + mine) * WALK_COLS + c0 + my_c], o);

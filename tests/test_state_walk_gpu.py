@@ -72,3 +72,25 @@ def _compare(kind, d, dv, lens, taps):
     for name, a, b in [("output", got, want)] + [(k, whole[k], single[k]) for k in whole]:
         assert torch.isfinite(a).all(), name
         assert float((a - b).abs().max()) <= 3.2e-5 * max(1.0, float(b.abs().max())), name
+
+
+@pytest.mark.parametrize("kind", ["memory", "retention", "mamba", "gated", "channel", "general"])
+@pytest.mark.parametrize("at", [0, 1, 2, 3, 4, 53, 61])
+@pytest.mark.parametrize("bad", [float("inf"), float("nan")])
+def test_tokens_before_one_that_is_not_finite_keep_their_numbers(kind, at, bad):
+    """Wherever the token lies in its turn, earlier outputs keep every bit, and its own is no number."""
+    from llm_rs_b200.parts import Runtime
+    g = torch.Generator().manual_seed(3)
+    D, part = _part(kind, 64, 48)
+    w = {s.name: (torch.randn(s.shape, generator=g) * (0.5 if len(s.shape) == 1 else s.shape[-1] ** -0.5)).to(DEV)
+         for s in part.weight_specs()}
+    part.bind(w, Runtime(torch.device(DEV), torch.float32, 4096))
+    x = torch.randn(62, D, generator=g).to(DEV)
+    outs = []
+    for rows in (x, x.index_fill(0, torch.tensor([at], device=DEV), bad)):
+        state = {name: torch.zeros(1, *shape, device=DEV) for name, shape in part.state_need().tensors.items()}
+        outs.append(part.forward(rows, _ctx([62], [0]), SimpleNamespace(state=state)))
+    want, got = outs
+    assert torch.isfinite(want).all()
+    assert torch.equal(got[:at], want[:at])
+    assert not torch.isfinite(got[at]).any()
