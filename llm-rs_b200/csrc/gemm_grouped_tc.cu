@@ -253,13 +253,13 @@ int launch_grouped_tc(const GroupedGemmArgs& a, int out_dtype, int x_rows, int g
   const long long work = (long long)(a.tiles ? max_tiles : p.n_m * batches) * p.n_n;
   LLMRS_REQUIRE(work <= 0x7fffffffLL && (long long)groups * a.N <= 0x7fffffffLL, "gemm_grouped: too many tiles or weights");
   CUtensorMap mx, mw, mw2;
-  int rc;
+  int rc = 0;
   // All batches are one tensor of wide rows.
   p.x_batch = (int)a.x_batch;
   const cuuint64_t xdims[2] = {(cuuint64_t)(a.tiles ? a.K : (batches - 1) * a.x_batch + a.K), (cuuint64_t)x_rows};
   const cuuint64_t xstrides[1] = {(cuuint64_t)a.x_stride * 2};
   const cuuint32_t xbox[2] = {TC_BK, TC_BM};
-  rc = gt_map(&mx, a.x, xdims, xstrides, xbox);
+  if ((rc = gt_map(&mx, a.x, xdims, xstrides, xbox)) != 0) return rc;
   const cuuint64_t wdims[2] = {(cuuint64_t)a.K, (cuuint64_t)groups * a.N}, wstrides[1] = {(cuuint64_t)a.K * 2};
   const cuuint32_t wbox[2] = {TC_BK, GT_HALF};
   if ((rc = gt_map(&mw, a.w, wdims, wstrides, wbox)) != 0) return rc;
