@@ -376,10 +376,13 @@ LLMRS_API int llmrs_gemm_grouped(const void* x, int x_dtype, long long x_stride,
   if (g_grouped_mma && x_dtype == LLMRS_BF16 && w_dtype == LLMRS_BF16 && K % 8 == 0 && x_stride % 8 == 0 &&
       x_batch % 8 == 0 && ((uintptr_t)x & 15) == 0 && ((uintptr_t)w & 15) == 0 && (!w2 || ((uintptr_t)w2 & 15) == 0) &&
       (N * (long long)K) % 8 == 0) {
-    // Tiles of 128 rows go to tcgen05 where TMA can address the rows. Batches lie side by side in the rows of one tensor: a
-    // step of k past a batch's end would read the next one's numbers, so K must then be whole steps.
-    if (tile_rows == 128 && g_grouped_tc && src == nullptr && w_batch == (long long)N * K && x_stride > 0 &&
-        (tiles || (K % 64 == 0 && x_batch > 0 && (long long)(batches - 1) * x_batch + K <= 0x7fffffffLL)))
+    // Tiles of 128 rows go to tcgen05 where TMA can address the rows: as those of one matrix, which do not overlap and are less
+    // than 2^40 bytes apart. Batches lie side by side in its rows (batches whose rows lie between one another's, or one batch
+    // behind the other, stay on mma.sync); a step of k past a batch's end would read the next one's numbers, so K must then be
+    // whole steps.
+    const long long x_width = tiles ? K : (batches - 1) * x_batch + K;
+    if (tile_rows == 128 && g_grouped_tc && src == nullptr && w_batch == (long long)N * K && x_stride >= x_width &&
+        x_stride < 1LL << 39 && (tiles || (K % 64 == 0 && x_batch > 0 && x_width <= 0x7fffffffLL)))
       return launch_grouped_tc(a, out_dtype, x_rows, groups, batches, max_tiles, error_flag, stream);
     // Few rows: the weights' bytes are what counts. Tiles of at most 32 rows where the list cannot have longer ones.
     const bool few = tiles && tile_rows == 64 && M <= 32, b16 = out_dtype == LLMRS_BF16;

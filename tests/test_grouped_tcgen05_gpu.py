@@ -69,6 +69,40 @@ def test_batched(M, B, N, K, pad):
     assert bool((out[:, :, N:] == 3.0).all())
 
 
+@pytest.mark.parametrize("M,B,N,K,form", [(128, 3, 128, 64, "batch"), (300, 2, 40, 192, "batch"), (257, 4, 96, 128, "batch"),
+                                          (130, 3, 64, 64, "same rows"), (200, 5, 64, 128, "overlapping"), (129, 1, 64, 64, "batch")])
+def test_batched_in_other_orders(M, B, N, K, form):
+    """Batches one behind the other, the same rows for every batch, rows that overlap: any strides are taken."""
+    from llm_rs_b200 import ops
+    torch.manual_seed(M + N)
+    if form == "batch":
+        x = torch.randn(B, M, K, device=DEV).bfloat16().transpose(0, 1)
+    elif form == "same rows":
+        x = torch.randn(M, 1, K, device=DEV).bfloat16().expand(M, B, K)
+    else:
+        x = torch.randn(M * 64 + B * 64 + K, device=DEV).bfloat16().as_strided((M, B, K), (64, 64, 1))
+    w = torch.randn(B, N, K, device=DEV).bfloat16()
+    out = torch.empty((B, M, N), device=DEV, dtype=torch.bfloat16).transpose(0, 1)
+    ops.gemm_batched(x, w, out)
+    ops.check_tc_error(DEV)
+    for b in range(B):
+        want = x[:, b].double() @ w[b].double().t()
+        assert bool(((out[:, b].double() - want).abs() <= _bound(x[:, b], w[b], torch.bfloat16, K)).all()), b
+
+
+def test_one_row_of_any_stride():
+    from llm_rs_b200 import ops
+    x = torch.randn(1, 64, device=DEV).bfloat16()
+    w = torch.randn(2, 96, 64, device=DEV).bfloat16()
+    tiles, n_tiles = (torch.tensor(v, dtype=torch.int32, device=DEV) for v in ([[1, 0, 1]], [1]))
+    out = torch.empty(1, 96, device=DEV)
+    for stride in (8, 64, 1 << 40):
+        ops.gemm_grouped(x.as_strided((1, 64), (stride, 1)), w, out, tiles, n_tiles, None, tile_rows=128)
+        ops.check_tc_error(DEV)
+        want = x.double() @ w[1].double().t()
+        assert bool(((out.double() - want).abs() <= _bound(x, w[1], torch.float32, 64)).all())
+
+
 def test_a_wait_that_runs_out_is_reported():
     from llm_rs_b200 import ops
     x, w = torch.randn(256, 256, device=DEV).bfloat16(), torch.randn(1, 256, 256, device=DEV).bfloat16()
