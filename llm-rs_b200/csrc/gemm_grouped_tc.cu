@@ -274,23 +274,27 @@ int launch_grouped_tc(const GroupedGemmArgs& a, int out_dtype, int x_rows, int g
   return llmrs_launch_status("gemm_grouped (tcgen05)");
 }
 
-// out[r] = x[src[r]] for rows of `pieces` 16-byte pieces; a warp per row.
+// out[r] = x[src[r]] for rows of `pieces` 16-byte pieces; a warp per row. A row whose source is none of x's is left as it is: no
+// tile may name it, and a list of tiles need not cover all rows.
 __global__ void __launch_bounds__(256)
-gather_rows_kernel(const uint4* __restrict__ x, long long x_stride, const int* __restrict__ src, uint4* __restrict__ out, int rows,
-                   int pieces) {
+gather_rows_kernel(const uint4* __restrict__ x, long long x_stride, int x_rows, const int* __restrict__ src, uint4* __restrict__ out,
+                   int rows, int pieces) {
   const int r = blockIdx.x * 8 + (threadIdx.x >> 5), lane = threadIdx.x & 31;
   if (r >= rows) return;
-  const uint4* from = x + (size_t)src[r] * x_stride;
+  const int at = src[r];
+  if (at < 0 || at >= x_rows) return;
+  const uint4* from = x + (size_t)at * x_stride;
   uint4* to = out + (size_t)r * pieces;
 #pragma unroll 4
   for (int e = lane; e < pieces; e += 32) to[e] = from[e];
 }
 
-// x: bfloat16 rows of K values, x_stride apart; out [rows, K].
-LLMRS_API int llmrs_gather_rows(const void* x, long long x_stride, const int* src, void* out, int rows, int K, cudaStream_t stream) {
+// x: x_rows bfloat16 rows of K values, x_stride apart; out [rows, K].
+LLMRS_API int llmrs_gather_rows(const void* x, long long x_stride, int x_rows, const int* src, void* out, int rows, int K,
+                                cudaStream_t stream) {
   LLMRS_REQUIRE(rows >= 0 && K > 0 && K % 8 == 0 && x_stride % 8 == 0 && (((uintptr_t)x | (uintptr_t)out) & 15) == 0,
                 "gather_rows: rows of whole 16-byte pieces");
   if (rows == 0) return 0;
-  gather_rows_kernel<<<(rows + 7) / 8, 256, 0, stream>>>((const uint4*)x, x_stride / 8, src, (uint4*)out, rows, K / 8);
+  gather_rows_kernel<<<(rows + 7) / 8, 256, 0, stream>>>((const uint4*)x, x_stride / 8, x_rows, src, (uint4*)out, rows, K / 8);
   return llmrs_launch_status("gather_rows");
 }

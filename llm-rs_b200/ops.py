@@ -872,8 +872,8 @@ def gemm_grouped(x: torch.Tensor, w: torch.Tensor, out: torch.Tensor, tiles: tor
         if (tile_rows == 128 and x.dtype == w.dtype == torch.bfloat16 and K % 8 == 0 and _row_stride(x, "x") % 8 == 0
                 and x.data_ptr() % 16 == 0):      # the tcgen05 kernel reads rows as they lie
             rows = torch.empty((out.size(0), K), dtype=torch.bfloat16, device=x.device)
-            _check(_lib().llmrs_gather_rows(_ptr(x), _LL(_row_stride(x, "x")), _ptr(src), _ptr(rows), out.size(0), K, _stream()),
-                   "gather_rows")
+            _check(_lib().llmrs_gather_rows(_ptr(x), _LL(_row_stride(x, "x")), x.size(0), _ptr(src), _ptr(rows),
+                                            min(out.size(0), src.numel()), K, _stream()), "gather_rows")
             x, src = rows, None
     _check(_lib().llmrs_gemm_grouped(
         _ptr(x), dtype_code(x.dtype), _LL(_row_stride(x, "x")), _LL(0), _ptr(w), _ptr(w2), dtype_code(w.dtype),

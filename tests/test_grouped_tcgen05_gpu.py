@@ -90,6 +90,22 @@ def test_batched_in_other_orders(M, B, N, K, form):
         assert bool(((out[:, b].double() - want).abs() <= _bound(x[:, b], w[b], torch.bfloat16, K)).all()), b
 
 
+@pytest.mark.parametrize("tail", [[-1, 1 << 30], []])
+def test_rows_that_no_tile_names_need_no_source(tail):
+    """Rows are gathered ahead of the tcgen05 kernel: those past the tiles may name no row of X, or have no entry."""
+    from llm_rs_b200 import ops
+    torch.manual_seed(4)
+    x, w = torch.randn(20, 64, device=DEV).bfloat16(), torch.randn(1, 96, 64, device=DEV).bfloat16()
+    src = torch.tensor([19, 0, 7] + tail, dtype=torch.int32, device=DEV)
+    tiles, n_tiles = (torch.tensor(v, dtype=torch.int32, device=DEV) for v in ([[0, 0, 3]], [1]))
+    out = torch.full((5, 96), 7.0, device=DEV)
+    ops.gemm_grouped(x, w, out, tiles, n_tiles, src, tile_rows=128)
+    ops.check_tc_error(DEV)
+    rows = x[[19, 0, 7]]
+    assert bool(((out[:3].double() - rows.double() @ w[0].double().t()).abs() <= _bound(rows, w[0], torch.float32, 64)).all())
+    assert bool((out[3:] == 7.0).all())
+
+
 def test_one_row_of_any_stride():
     from llm_rs_b200 import ops
     x = torch.randn(1, 64, device=DEV).bfloat16()
