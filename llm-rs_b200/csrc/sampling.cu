@@ -589,6 +589,7 @@ sample_spread_kernel(const float* __restrict__ logits, int vocab, const float* _
 // clusters' barriers; a row must fit the shared memory of its blocks. A block a row against eight, us: 32 rows of 151,936
 // 117 / 71, 8 rows 113 / 51, one 94 / 35; 64 rows 118 / 132; 32 rows of 32,000 39 / 46, 8 rows 39 / 36.
 constexpr int SS_MAX_ROWS = 32, SS_MIN_CHUNK = 64, SS_MAX_CHUNK = 340;
+constexpr size_t ss_smem(int chunk) { return (size_t)(SS_RUNS + 1) * chunk * sizeof(float); }
 
 LLMRS_API int llmrs_sample(float* logits, int n_rows, int vocab, const float* temperature, const int* top_k,
                            const float* top_p, const float* penalty, const int* hist_tokens,
@@ -599,10 +600,11 @@ LLMRS_API int llmrs_sample(float* logits, int n_rows, int vocab, const float* te
   if (n_rows == 0) return 0;
   const int chunk = (vocab + SM_THREADS - 1) / SM_THREADS;
   if (n_rows <= SS_MAX_ROWS && chunk >= SS_MIN_CHUNK && chunk <= SS_MAX_CHUNK) {
-    const size_t smem = (size_t)(SS_RUNS + 1) * chunk * sizeof(float);
-    const cudaError_t e = cudaFuncSetAttribute(sample_spread_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
-    if (e != cudaSuccess) return llmrs_fail("sample: shared memory %zu: %s", smem, cudaGetErrorString(e));
-    sample_spread_kernel<<<n_rows * SS_BLOCKS, SM_THREADS, smem, stream>>>(logits, vocab, temperature, top_k, top_p, penalty,
+    // The limit is the largest row's, not this call's: another thread may set it between here and the launch.
+    const cudaError_t e =
+        cudaFuncSetAttribute(sample_spread_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)ss_smem(SS_MAX_CHUNK));
+    if (e != cudaSuccess) return llmrs_fail("sample: shared memory %zu: %s", ss_smem(SS_MAX_CHUNK), cudaGetErrorString(e));
+    sample_spread_kernel<<<n_rows * SS_BLOCKS, SM_THREADS, ss_smem(chunk), stream>>>(logits, vocab, temperature, top_k, top_p, penalty,
                                                                            hist_tokens, hist_offsets, seeds, request_ids,
                                                                            gen_index, out_tokens);
     return llmrs_launch_status("sample");

@@ -950,3 +950,28 @@ def test_sampler_spread_over_blocks_chooses_the_same(vocab):
     together = s.sample(logits.clone(), rows).cpu().tolist()
     for a, b in ((0, 32), (32, 50), (90, 120), (7, 8), (8, 13)):
         assert s.sample(logits[a:b].clone(), rows[a:b]).cpu().tolist() == together[a:b], (a, b)
+
+
+def test_sampler_of_two_threads_with_different_vocabularies():
+    """Each launch's shared memory follows its own vocabulary: neither thread may lower the other's limit."""
+    import threading
+    ops = _ops()
+    failed = []
+
+    def work(vocab):
+        try:
+            with torch.cuda.stream(torch.cuda.Stream()):
+                logits = torch.randn(1, vocab, device=DEV)
+                one = torch.ones(1, device=DEV)
+                whole, number = torch.ones(1, dtype=torch.int64, device=DEV), torch.zeros(1, dtype=torch.int32, device=DEV)
+                for _ in range(1500):
+                    ops.sample(logits, one, None, one, None, None, None, whole, whole, number)
+                torch.cuda.current_stream().synchronize()
+        except Exception as e:      # noqa: BLE001 - reported by the test's own thread
+            failed.append(repr(e))
+    threads = [threading.Thread(target=work, args=(v,)) for v in (66_000, 340_992, 66_000, 340_992)]
+    for t in threads:
+        t.start()
+    for t in threads:
+        t.join()
+    assert not failed, failed[:2]
