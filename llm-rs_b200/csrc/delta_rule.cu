@@ -11,7 +11,7 @@
 // Two kernels and a small third:
 //   prepare     a warp per (token, head), all tokens at once: decay, removal rate times unit key, unit key, and r, k, v
 //               widened, as six float32 rows [tokens, heads * d];
-//   (portions of 48 tokens and more take `turns` and the walk in turns of four tokens instead of these two: state_walk.cuh;
+//   (requests that are walked in turns take `turns` and the walk of state_walk.cuh instead of these two;
 //   2,048 tokens of 32 heads of 64 x 64: 816 us walked one by one, 246 in turns; their rows 56 us where `prepare` takes 38)
 //   recurrence  one block per (request, head, slice of 16 value columns) walks the request's tokens of the step in
 //               order: a column of S depends on no other column, so the slices run side by side. Four adjacent lanes
@@ -22,6 +22,8 @@
 //               end: a step of one token (decoding) and a prompt's portion are the same kernel;
 //   output      divides by the head's root mean square, applies the weight and the gate (head_out.cuh; heads that it does not
 //               take: a warp per token and head).
+#include <limits.h>
+
 #include "common.cuh"
 #include "head_out.cuh"
 #include "mma_util.cuh"
@@ -32,16 +34,18 @@ __device__ __forceinline__ float sigmoidf_(float x) { return 1.0f / (1.0f + expf
 constexpr int DR_COLS = 16, DR_LANES = 4, DR_THREADS = DR_COLS * DR_LANES;
 enum { DR_W = 0, DR_AU = 1, DR_U = 2, DR_K = 3, DR_R = 4, DR_V = 5, DR_ROWS = 6 };
 
-// prep: float32 [6][tokens][heads * d] in the order of the enum above.
+// prep: float32 [6][tokens][heads * d] in the order of the enum above; of requests of fewer than `below` tokens.
 template <typename TA>
 __global__ void delta_prepare_kernel(const TA* __restrict__ r, const TA* __restrict__ k, const TA* __restrict__ v,
                                      const TA* __restrict__ a_raw, long long in_stride,
                                      const float* __restrict__ decay_raw, const float* __restrict__ decay_bias,
-                                     const float* __restrict__ a_bias, float* __restrict__ prep, int n_tokens,
-                                     int n_heads, int d, float decay_scale, float key_eps) {
+                                     const float* __restrict__ a_bias, const int* __restrict__ q_start,
+                                     const int* __restrict__ n_new, float* __restrict__ prep, int n_tokens, int n_requests,
+                                     int n_heads, int d, float decay_scale, float key_eps, int below) {
   const int row = blockIdx.x * (blockDim.x / 32) + (threadIdx.x >> 5), lane = threadIdx.x & 31;
   if (row >= n_tokens * n_heads) return;
   const int t = row / n_heads, h = row % n_heads;
+  if (below < INT_MAX && n_new[walk_token_request(q_start, n_requests, t)] >= below) return;
   const size_t in0 = (size_t)t * in_stride + (size_t)h * d, out0 = (size_t)t * n_heads * d + (size_t)h * d;
   const size_t plane = (size_t)n_tokens * n_heads * d;
   float ss = 0.f;
@@ -72,12 +76,12 @@ delta_turns_kernel(const TA* __restrict__ r, const TA* __restrict__ k, const TA*
                    long long in_stride, const float* __restrict__ decay_raw, const float* __restrict__ decay_bias,
                    const float* __restrict__ a_bias, const int* __restrict__ q_start, const int* __restrict__ n_new,
                    float* __restrict__ rows, float* __restrict__ w, float* __restrict__ tables, int n_tokens, int n_requests,
-                   int n_heads, int d, float decay_scale, float key_eps, bool vec, bool vec_f) {
+                   int n_heads, int d, float decay_scale, float key_eps, bool vec, bool vec_f, int from) {
   const int place = blockIdx.x, h = blockIdx.y * 4 + (threadIdx.x >> 5), lane = threadIdx.x & 31;
   if (h >= n_heads) return;
   const int req = walk_request(q_start, n_requests, place), t_req = q_start[req];
   const int first = (place - walk_place(t_req, req)) * WALK_TURN, have = min(WALK_TURN, n_new[req] - first);
-  if (first < 0 || have <= 0) return;
+  if (first < 0 || have <= 0 || n_new[req] < from) return;
   const size_t t0 = (size_t)(t_req + first), width = (size_t)n_heads * d, plane = (size_t)n_tokens * width;
   float rv[4][CPL], kv[4][CPL], au[4][CPL], dec[4][CPL], bias_d[CPL], bias_a[CPL];
   walk_load<CPL>(decay_bias + (size_t)h * d, lane, d, true, false, bias_d);
@@ -175,11 +179,13 @@ delta_turns_kernel(const TA* __restrict__ r, const TA* __restrict__ k, const TA*
   }
 }
 
-template <int DMAX>
+// SOME: only requests of fewer than `below` tokens, the others are walked in turns. (A template: with the test in it the kernel
+// that takes all requests was compiled to 135 registers instead of 157 and took 115 us instead of 108.)
+template <int DMAX, bool SOME>
 __global__ void __launch_bounds__(DR_THREADS)
 delta_rule_kernel(const float* __restrict__ prep, float* __restrict__ state, const int* __restrict__ q_start,
                   const int* __restrict__ n_new, const int* __restrict__ slot_ids, float* __restrict__ o_raw,
-                  int n_tokens, int n_heads, int d) {
+                  int n_tokens, int n_heads, int d, int below) {
   constexpr int CHUNK = DMAX >= 256 ? 4 : (DMAX >= 128 ? 8 : 16);
   constexpr int IPL = DMAX / DR_LANES;             // key channels per lane
   __shared__ __align__(16) float s_in[2][5][CHUNK][DMAX];      // W, AU, U, K, R of a chunk's tokens; channels >= d stay 0
@@ -189,6 +195,7 @@ delta_rule_kernel(const float* __restrict__ prep, float* __restrict__ state, con
   const int col = col0 + tid / DR_LANES, part = tid % DR_LANES, i0 = part * IPL;
   const bool live = col < d;
   const int t0 = q_start[req], n = n_new[req];
+  if (SOME && n >= below) return;
   const int ch0 = head * d, width = n_heads * d;
   const size_t plane = (size_t)n_tokens * width;
   float* S_g = state + ((size_t)slot_ids[req] * n_heads + head) * d * d;
@@ -315,11 +322,11 @@ static int launch_delta(int dmax, dim3 grid, cudaStream_t stream, const void* r,
                         const float* decay_bias, const float* a_bias, const float* norm_w, float* state,
                         const int* q_start, const int* n_new, const int* slot_ids, float* work, void* out,
                         int n_tokens, int n_requests, int n_heads, int d, float decay_scale, float key_eps,
-                        float norm_eps) {
+                        float norm_eps, int walk_from) {
   const int rows = n_tokens * n_heads;
   float* prep = work;
   float* o_raw = work + (size_t)DR_ROWS * rows * d;
-  if (n_tokens - n_requests + 1 >= WALK_MIN_PORTION) {      // some request may bring a portion
+  if (walk_from > 0) {
     auto up4 = [](size_t v) { return (v + 3) & ~(size_t)3; };
     const size_t places = (size_t)walk_places(n_tokens, n_requests), plane = (size_t)rows * d;
     float* w = work + up4((size_t)(DR_ROWS + 1) * rows * d);
@@ -333,7 +340,8 @@ static int launch_delta(int dmax, dim3 grid, cudaStream_t stream, const void* r,
 #define LLMRS_DR_TURNS(CPL)                                                                                               \
   delta_turns_kernel<TA, CPL><<<grid_t, 128, 0, stream>>>((const TA*)r, (const TA*)k, (const TA*)v, (const TA*)a_raw, in_stride, \
                                                           decay_raw, decay_bias, a_bias, q_start, n_new, prep, w, tables, \
-                                                          n_tokens, n_requests, n_heads, d, decay_scale, key_eps, vec, vec_f)
+                                                          n_tokens, n_requests, n_heads, d, decay_scale, key_eps, vec, vec_f, \
+                                                          walk_from)
     if (d <= 64) LLMRS_DR_TURNS(2);
     else if (d <= 128) LLMRS_DR_TURNS(4);
     else LLMRS_DR_TURNS(8);
@@ -345,20 +353,32 @@ static int launch_delta(int dmax, dim3 grid, cudaStream_t stream, const void* r,
     a.q_stride = a.k_stride = a.b_stride = (long long)n_heads * d;
     a.tables = tables; a.state = state; a.o_raw = o_raw;
     a.q_start = q_start; a.n_new = n_new; a.slot_ids = slot_ids;
-    a.n_heads = a.n_groups = n_heads; a.d = a.dv = d;
+    a.n_heads = a.n_groups = n_heads; a.d = a.dv = d; a.from = walk_from;
     rc = launch_state_walk<WALK_GENERAL>(a, n_requests, d, stream);
     if (rc != 0) return rc;
-    return launch_delta_out<TA>(o_raw, gate, in_stride, norm_w, out, n_tokens, n_heads, d, norm_eps, stream);
+    if (walk_from == 1) return launch_delta_out<TA>(o_raw, gate, in_stride, norm_w, out, n_tokens, n_heads, d, norm_eps, stream);
   }
+  const int below = walk_from > 0 ? walk_from : INT_MAX;
   delta_prepare_kernel<TA><<<(rows + 3) / 4, 128, 0, stream>>>((const TA*)r, (const TA*)k, (const TA*)v,
                                                                (const TA*)a_raw, in_stride, decay_raw, decay_bias,
-                                                               a_bias, prep, n_tokens, n_heads, d, decay_scale, key_eps);
+                                                               a_bias, q_start, n_new, prep, n_tokens, n_requests, n_heads, d,
+                                                               decay_scale, key_eps, below);
   int rc = llmrs_launch_status("delta_rule (prepare)");
   if (rc != 0) return rc;
-  if (dmax == 32) delta_rule_kernel<32><<<grid, DR_THREADS, 0, stream>>>(prep, state, q_start, n_new, slot_ids, o_raw, n_tokens, n_heads, d);
-  else if (dmax == 64) delta_rule_kernel<64><<<grid, DR_THREADS, 0, stream>>>(prep, state, q_start, n_new, slot_ids, o_raw, n_tokens, n_heads, d);
-  else if (dmax == 128) delta_rule_kernel<128><<<grid, DR_THREADS, 0, stream>>>(prep, state, q_start, n_new, slot_ids, o_raw, n_tokens, n_heads, d);
-  else delta_rule_kernel<256><<<grid, DR_THREADS, 0, stream>>>(prep, state, q_start, n_new, slot_ids, o_raw, n_tokens, n_heads, d);
+#define LLMRS_DR_WALK(D)                                                                                                     \
+  do {                                                                                                                      \
+    if (walk_from > 0)                                                                                                      \
+      delta_rule_kernel<D, true><<<grid, DR_THREADS, 0, stream>>>(prep, state, q_start, n_new, slot_ids, o_raw, n_tokens,   \
+                                                                  n_heads, d, below);                                       \
+    else                                                                                                                    \
+      delta_rule_kernel<D, false><<<grid, DR_THREADS, 0, stream>>>(prep, state, q_start, n_new, slot_ids, o_raw, n_tokens,  \
+                                                                   n_heads, d, below);                                      \
+  } while (0)
+  if (dmax == 32) LLMRS_DR_WALK(32);
+  else if (dmax == 64) LLMRS_DR_WALK(64);
+  else if (dmax == 128) LLMRS_DR_WALK(128);
+  else LLMRS_DR_WALK(256);
+#undef LLMRS_DR_WALK
   rc = llmrs_launch_status("delta_rule");
   if (rc != 0) return rc;
   return launch_delta_out<TA>(o_raw, gate, in_stride, norm_w, out, n_tokens, n_heads, d, norm_eps, stream);
@@ -372,13 +392,14 @@ LLMRS_API long long llmrs_delta_rule_work_floats(int n_tokens, int n_requests, i
 
 // r, k, v, gate, a_raw: [tokens, ...] of the activation type, rows `in_stride` elements apart, each pointing at its
 // own first column (head h's channels at h * d); decay_raw: float32 [tokens, heads * d]; work: float32 workspace of
-// llmrs_delta_rule_work_floats, 16-byte aligned; out: [tokens, heads * d].
+// llmrs_delta_rule_work_floats, 16-byte aligned; out: [tokens, heads * d]. walk_from: requests of at least so many tokens are
+// walked in turns, the others token by token; 0: all of them are.
 LLMRS_API int llmrs_delta_rule(const void* r, const void* k, const void* v, const void* gate, const void* a_raw,
                                long long in_stride, int dtype, const float* decay_raw, const float* decay_bias,
                                const float* a_bias, const float* norm_w, float* state, const int* q_start,
                                const int* n_new, const int* slot_ids, float* work, void* out, int n_tokens,
                                int n_requests, int n_heads, int d, float decay_scale, float key_eps, float norm_eps,
-                               cudaStream_t stream) {
+                               int walk_from, cudaStream_t stream) {
   LLMRS_REQUIRE(n_requests >= 0 && n_tokens >= 0 && n_heads > 0 && d > 0, "delta_rule: bad sizes");
   LLMRS_REQUIRE(d <= 256, "delta_rule: heads of at most 256 channels, got %d", d);
   LLMRS_REQUIRE(n_heads <= 65535, "delta_rule: too many heads");
@@ -389,10 +410,10 @@ LLMRS_API int llmrs_delta_rule(const void* r, const void* k, const void* v, cons
   if (dtype == LLMRS_F32)
     return launch_delta<float>(dmax, grid, stream, r, k, v, gate, a_raw, in_stride, decay_raw, decay_bias, a_bias,
                                norm_w, state, q_start, n_new, slot_ids, work, out, n_tokens, n_requests, n_heads, d,
-                               decay_scale, key_eps, norm_eps);
+                               decay_scale, key_eps, norm_eps, walk_from);
   if (dtype == LLMRS_BF16)
     return launch_delta<__nv_bfloat16>(dmax, grid, stream, r, k, v, gate, a_raw, in_stride, decay_raw, decay_bias,
                                        a_bias, norm_w, state, q_start, n_new, slot_ids, work, out, n_tokens, n_requests,
-                                       n_heads, d, decay_scale, key_eps, norm_eps);
+                                       n_heads, d, decay_scale, key_eps, norm_eps, walk_from);
   return llmrs_fail("delta_rule: unknown dtype %d", dtype);
 }

@@ -18,10 +18,10 @@
 //
 //   prepare      a block per token: convolutions + SiLU, unit q and k, g and beta, as float32 rows
 //   conv state   a block per request, after prepare: the request's last K - 1 convolution inputs
-//   (steps with a portion of 48 tokens and more: the rows and coefficients of turns of four tokens by one kernel in place of
-//   `prepare`, then the walk in turns, state_walk.cuh)
-//   recurrence   of single tokens and shorter portions: a block per (request, head, slice of 16 value
-//                columns) walks the request's tokens one by one; four
+//   (requests that are walked in turns: the rows and coefficients of turns of four tokens by one kernel in place of
+//   `prepare`, then the walk, state_walk.cuh)
+//   recurrence   of the others, token by token: a block per (request, head, slice of 16 value
+//                columns) walks the request's tokens; four
 //                neighbouring lanes share a column, each with a quarter of the key channels in registers (lane p of the
 //                four holds channels 4 (p + 4 j) .. 4 (p + 4 j) + 3, so that the four read neighbouring 16-byte pieces
 //                of a row in shared memory, not pieces a bank's stride apart); k^T S and q^T S are summed over the four
@@ -42,6 +42,8 @@
 // one. A chunk's missing tokens (a portion's end) count as k = q = v = 0, beta = 0, g = 1 and change nothing.
 // The chunked form is OFF by default (llmrs_gated_delta_chunked): its products read every operand from shared memory
 // and are bound by that (2,048 tokens of 16 heads of 128 x 128: some 500 us, the walk in turns 265).
+#include <limits.h>
+
 #include "common.cuh"
 #include "head_out.cuh"
 #include "mma_util.cuh"
@@ -56,12 +58,13 @@ __global__ void gdr_prepare_kernel(const TA* __restrict__ x, long long stride, c
                                    const float* __restrict__ araw, const float* __restrict__ a_log,
                                    const float* __restrict__ dt_bias, const float* __restrict__ conv_state,
                                    const int* __restrict__ token_req, const int* __restrict__ q_start,
-                                   const int* __restrict__ slot_ids, float* __restrict__ pq, float* __restrict__ pk,
-                                   float* __restrict__ pv, float* __restrict__ pbeta, float* __restrict__ pg,
-                                   float* __restrict__ plg, int G, int H, int d, int dv, int K, float key_eps,
-                                   float q_scale) {
+                                   const int* __restrict__ n_new, const int* __restrict__ slot_ids,
+                                   float* __restrict__ pq, float* __restrict__ pk, float* __restrict__ pv,
+                                   float* __restrict__ pbeta, float* __restrict__ pg, float* __restrict__ plg, int G, int H,
+                                   int d, int dv, int K, float key_eps, float q_scale, int below) {
   extern __shared__ float row[];      // [C] after convolution and SiLU
   const int t = blockIdx.x, req = token_req[t], off = t - q_start[req];
+  if (below < INT_MAX && n_new[req] >= below) return;      // walked in turns
   const int wq = G * d, wv = H * dv, C = 2 * wq + wv;
   const float* tail = conv_state + (size_t)slot_ids[req] * (K - 1) * C;
   for (int c = threadIdx.x; c < C; c += blockDim.x)
@@ -96,7 +99,7 @@ constexpr int GD_COLS = 16;      // value columns of a block
 #ifndef LLMRS_GD_LANES
 #define LLMRS_GD_LANES 8
 #endif
-// (The kernel for single tokens and portions of fewer than 48.) With a decay per key channel a lane reads three rows a
+// (The kernel that walks token by token.) With a decay per key channel a lane reads three rows a
 // token, not two: sixteen lanes a column shorten that where a step's blocks do not fill the device twice (walking 2,048 tokens
 // of 16 heads of 128 x 128: 813 against 896 us for the whole op), eight are ahead where they do.
 constexpr int GD_WIDE_MAX_BLOCKS = 296;
@@ -108,7 +111,7 @@ __global__ void __launch_bounds__(GD_COLS * LANES)
 gdr_recurrence_kernel(const float* __restrict__ pq, const float* __restrict__ pk, const float* __restrict__ pv,
                       const float* __restrict__ pbeta, const float* __restrict__ pg, float* __restrict__ state,
                       const int* __restrict__ q_start, const int* __restrict__ n_new,
-                      const int* __restrict__ slot_ids, float* __restrict__ o_raw, int G, int H, int d, int dv) {
+                      const int* __restrict__ slot_ids, float* __restrict__ o_raw, int G, int H, int d, int dv, int below) {
   constexpr int CHUNK = CHANNEL ? (DMAX >= 256 ? 4 : (DMAX >= 128 ? 8 : 16)) : (DMAX >= 256 ? 8 : 16);
   constexpr int PLANES = CHANNEL ? 3 : 2;
   constexpr int GD_LANES = LANES, GD_THREADS = GD_COLS * LANES;
@@ -127,6 +130,7 @@ gdr_recurrence_kernel(const float* __restrict__ pq, const float* __restrict__ pk
   auto ch = [&](int i) { return ((i >> 2) * GD_LANES + part) * 4 + (i & 3); };
   const bool live = col < dv;
   const int t0 = q_start[req], n = n_new[req];
+  if (n >= below) return;      // walked in turns
   const int wq = G * d, wv = H * dv;
   float* S_g = state + ((size_t)slot_ids[req] * H + head) * d * dv;
   float S[IPL];
@@ -306,13 +310,13 @@ gdr_turns_kernel(const TA* __restrict__ x, long long stride, const float* __rest
                  const int* __restrict__ n_new, const int* __restrict__ slot_ids, float* __restrict__ pq,
                  float* __restrict__ pk, float* __restrict__ kb, float* __restrict__ pv, float* __restrict__ w,
                  float* __restrict__ tables, int n_requests, int G, int H, int d, int dv, int K, float key_eps, float q_scale,
-                 bool vec, bool taps4) {
+                 bool vec, bool taps4, int from) {
   const int place = blockIdx.x, unit = blockIdx.y * 4 + (threadIdx.x >> 5), lane = threadIdx.x & 31;
   const int wq = G * d, wv = H * dv, C = 2 * wq + wv;
   if (unit >= G + (wv + 32 * CPL - 1) / (32 * CPL)) return;
   const int req = walk_request(q_start, n_requests, place), t_req = q_start[req];
   const int first = (place - walk_place(t_req, req)) * WALK_TURN, have = min(WALK_TURN, n_new[req] - first);
-  if (first < 0 || have <= 0) return;
+  if (first < 0 || have <= 0 || n_new[req] < from) return;
   const size_t t0 = (size_t)(t_req + first);
   const float* tail = conv_state + (size_t)slot_ids[req] * (K - 1) * C;
   auto convolve = [&](int c0, int width, float (&out)[4][CPL]) {
@@ -727,7 +731,7 @@ template <typename TA>
 static int launch_turns(const TA* x, long long x_stride, const float* taps, const float* ba, const TA* b, long long b_stride,
                         const float* araw, const float* a_log, const float* dt_bias, const float* conv_state, const TurnRows& r,
                         const int* q_start, const int* n_new, const int* slot_ids, int n_tokens, int n_requests, int G, int H,
-                        int d, int dv, int K, float key_eps, float q_scale, cudaStream_t stream) {
+                        int d, int dv, int K, float key_eps, float q_scale, int from, cudaStream_t stream) {
   auto rows_of_four = [](const void* p, size_t size, long long stride) { return ((uintptr_t)p & (4 * size - 1)) == 0 && stride % 4 == 0; };
   const bool vec = d % 4 == 0 && H * dv % 4 == 0 && rows_of_four(x, sizeof(TA), x_stride) && rows_of_four(conv_state, 4, 4) &&
                    rows_of_four(araw, 4, 4);
@@ -738,7 +742,7 @@ static int launch_turns(const TA* x, long long x_stride, const float* taps, cons
 #define LLMRS_GD_TURNS(CPL, CH)                                                                                               \
   gdr_turns_kernel<TA, CPL, CH><<<grid, 128, 0, stream>>>(x, x_stride, taps, ba, b, b_stride, araw, a_log, dt_bias, conv_state, \
                                                           q_start, n_new, slot_ids, r.pq, r.pk, r.kb, r.pv, r.w, r.tables,    \
-                                                          n_requests, G, H, d, dv, K, key_eps, q_scale, vec, taps4)
+                                                          n_requests, G, H, d, dv, K, key_eps, q_scale, vec, taps4, from)
   if (araw && cpl == 4) LLMRS_GD_TURNS(4, true);
   else if (araw) LLMRS_GD_TURNS(8, true);
   else if (cpl == 4) LLMRS_GD_TURNS(4, false);
@@ -748,12 +752,13 @@ static int launch_turns(const TA* x, long long x_stride, const float* taps, cons
 }
 
 static int launch_turn_walk(bool channel, const TurnRows& r, float* state, const int* q_start, const int* n_new,
-                            const int* slot_ids, float* o_raw, int n_requests, int G, int H, int d, int dv, cudaStream_t stream) {
+                            const int* slot_ids, float* o_raw, int n_requests, int G, int H, int d, int dv, int from,
+                            cudaStream_t stream) {
   WalkArgs a = {};
   a.q = r.pq; a.k = r.pk; a.kb = r.kb; a.w = r.w;
   a.v = r.pv; a.tables = r.tables; a.state = state; a.o_raw = o_raw;
   a.q_start = q_start; a.n_new = n_new; a.slot_ids = slot_ids;
-  a.n_heads = H; a.d = d; a.dv = dv;
+  a.n_heads = H; a.d = d; a.dv = dv; a.from = from;
   a.n_groups = channel ? H : G;
   a.q_stride = a.k_stride = a.b_stride = (long long)a.n_groups * d;
   return channel ? launch_state_walk<WALK_CHANNEL>(a, n_requests, dv, stream) : launch_state_walk<WALK_GATED>(a, n_requests, dv, stream);
@@ -778,13 +783,14 @@ LLMRS_API void llmrs_gated_delta_chunked(int on) { g_gd_chunked = on; }
 // conv_state: float32 [slots, K - 1, 2 G d + H dv]; work: 16-byte aligned; out: [tokens, H dv] rows `out_stride` apart,
 // multiplied by `out_scale`. A decay per head: ba float32 [tokens, 2 H] (b, then a), dt_bias [H]. A decay per key channel
 // (araw not null; ba unused): b [tokens, H] of `dtype` rows `b_stride` apart, araw float32 [tokens, H d], dt_bias [H d].
+// walk_from: requests of at least so many tokens are walked in turns, the others token by token; 0: all of them are.
 LLMRS_API int llmrs_gated_delta(const void* x, long long x_stride, const void* gate, long long gate_stride, int dtype,
                                 const float* taps, const float* ba, const void* b, long long b_stride, const float* araw,
                                 const float* a_log, const float* dt_bias, const float* norm_w, float* state,
                                 float* conv_state, const int* token_req, const int* q_start, const int* n_new,
                                 const int* slot_ids, float* work, void* out, long long out_stride, int n_tokens,
                                 int n_requests, int G, int H, int d, int dv, int K, float key_eps, float q_scale,
-                                float norm_eps, float out_scale, int gate_sigmoid, cudaStream_t stream) {
+                                float norm_eps, float out_scale, int gate_sigmoid, int walk_from, cudaStream_t stream) {
   LLMRS_REQUIRE(n_requests >= 0 && n_tokens >= 0 && G > 0 && H > 0 && d > 0 && dv > 0 && K >= 1, "gated_delta: bad sizes");
   LLMRS_REQUIRE(H % G == 0, "gated_delta: %d value heads are no multiple of %d key heads", H, G);
   LLMRS_REQUIRE(d <= 256, "gated_delta: key heads of at most 256 channels, got %d", d);
@@ -810,7 +816,7 @@ LLMRS_API int llmrs_gated_delta(const void* x, long long x_stride, const void* g
   const bool chunked = g_gd_chunked && !channel && n_tokens - n_requests + 1 >= 2 * GC_C && d % 4 == 0 && dv % 4 == 0 &&
                        (size_t)gc_smem_floats(d) * sizeof(float) <= 200 * 1024;
   const int max_chunks = (n_tokens - n_requests + 1 + GC_C - 1) / GC_C;
-  const bool turns = !chunked && n_tokens - n_requests + 1 >= WALK_MIN_PORTION;      // some request may bring a portion
+  const int from = chunked ? 0 : walk_from, below = from > 0 ? from : INT_MAX;
   // The walk's rows with a decay per key channel follow o_raw; its tables lie where the chunked form's would.
   const size_t hd = up4((size_t)n_tokens * H * d);
   float *qf = tables, *kf = qf + hd, *kb = kf + hd, *turn_w = kb + hd;
@@ -825,7 +831,7 @@ LLMRS_API int llmrs_gated_delta(const void* x, long long x_stride, const void* g
   head.eps = norm_eps; head.out_scale = out_scale; head.silu = !gate_sigmoid;
 #define LLMRS_GD_REC(DMAX, LANES, CH)                                                                             \
   gdr_recurrence_kernel<DMAX, LANES, CH><<<grid, GD_COLS * LANES, 0, stream>>>(pq, pk, pv, pbeta, pg, state, q_start, \
-                                                                               n_new, slot_ids, o_raw, G, H, d, dv)
+                                                                               n_new, slot_ids, o_raw, G, H, d, dv, below)
 #define LLMRS_GD_REC_ALL(CH, LANES)                                                                              \
   do {                                                                                                           \
     if (dmax == 32) LLMRS_GD_REC(32, (LANES < 8 ? LANES : 8), CH);                                               \
@@ -844,17 +850,19 @@ LLMRS_API int llmrs_gated_delta(const void* x, long long x_stride, const void* g
     }                                                                                                                  \
     gdr_prepare_kernel<T, CH><<<n_tokens, 256, smem, stream>>>(                                                        \
         (const T*)x, x_stride, taps, ba, (const T*)b, b_stride, araw, a_log, dt_bias, conv_state, token_req, q_start,  \
-        slot_ids, pq, pk, pv, pbeta, pg, plg, G, H, d, dv, K, key_eps, q_scale);                                       \
+        n_new, slot_ids, pq, pk, pv, pbeta, pg, plg, G, H, d, dv, K, key_eps, q_scale, below);                         \
   } while (0)
   const TurnRows turn_rows = {channel ? qf : pq, channel ? kf : pk, kb, pv, turn_w, tables};
 #define LLMRS_GD_LAUNCH(T)                                                                                             \
   do {                                                                                                                 \
     int rc = 0;                                                                                                        \
-    if (turns) {                                                                                                       \
+    if (from > 0) {                                                                                                    \
       rc = launch_turns<T>((const T*)x, x_stride, taps, ba, (const T*)b, b_stride, araw, a_log, dt_bias, conv_state,   \
                            turn_rows, q_start, n_new, slot_ids, n_tokens, n_requests, G, H, d, dv, K, key_eps,         \
-                           q_scale, stream);                                                                           \
-    } else {                                                                                                           \
+                           q_scale, from, stream);                                                                     \
+      if (rc != 0) return rc;                                                                                          \
+    }                                                                                                                  \
+    if (from != 1) {                                                                                                   \
       if (channel) LLMRS_GD_PREPARE(T, true);                                                                          \
       else LLMRS_GD_PREPARE(T, false);                                                                                 \
       rc = llmrs_launch_status("gated_delta (prepare)");                                                               \
@@ -866,10 +874,12 @@ LLMRS_API int llmrs_gated_delta(const void* x, long long x_stride, const void* g
       rc = launch_chunked(pq, pk, pv, pbeta, plg, tables, state, q_start, n_new, slot_ids, o_raw, n_requests,          \
                           max_chunks, G, H, d, dv, stream);                                                            \
       if (rc != 0) return rc;                                                                                          \
-    } else if (turns) {                                                                                                \
-      rc = launch_turn_walk(channel, turn_rows, state, q_start, n_new, slot_ids, o_raw, n_requests, G, H, d, dv,       \
+    } else if (from > 0) {                                                                                             \
+      rc = launch_turn_walk(channel, turn_rows, state, q_start, n_new, slot_ids, o_raw, n_requests, G, H, d, dv, from, \
                             stream);                                                                                   \
       if (rc != 0) return rc;                                                                                          \
+    }                                                                                                                  \
+    if (chunked || from == 1) {                                                                                        \
     } else if (channel && (long long)grid.x * grid.y * grid.z <= GD_WIDE_MAX_BLOCKS) LLMRS_GD_REC_ALL(true, 16);       \
     else if (channel) LLMRS_GD_REC_ALL(true, 8);                                                                       \
     else LLMRS_GD_REC_ALL(false, LLMRS_GD_LANES);                                                                      \

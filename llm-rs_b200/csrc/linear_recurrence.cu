@@ -17,13 +17,15 @@
 //                a_t = exp(f_t + m_(t-1) - m_t), b_t = exp(i_t - m_t), floor_t = exp(-m_t); m is kept per slot;
 //   prepare      q, k, v of all tokens widened to float32 (optional SiLU, optional rotation of the first channels of every
 //                head of q and k by halves, q and k scaled, k multiplied by its gain);
-//   (portions of 48 tokens and more: the coefficients of turns of four tokens, then the walk in turns, state_walk.cuh)
-//   recurrence   a block per (request, head, 16 value columns) walks the tokens in order; four or eight adjacent lanes
+//   (requests that are walked in turns: the coefficients of turns of four tokens, then the walk, state_walk.cuh)
+//   recurrence   of the others: a block per (request, head, 16 value columns) walks the tokens in order; four or eight adjacent lanes
 //                share a column, each holding its part of the column's key channels in registers; rows arrive through two
 //                shared-memory buffers by 16-byte asynchronous copies. A step of one token and a prompt's portion
 //                are the same kernel;
 //   output       divides by the normaliser, norms each head (or all heads together) by its root mean square,
 //                multiplies by a weight (or none) and by sigmoid(gate) or SiLU(gate), rounds to the activation type.
+#include <limits.h>
+
 #include "common.cuh"
 #include "head_out.cuh"
 #include "mma_util.cuh"
@@ -259,7 +261,7 @@ linear_recurrence_kernel(const float* __restrict__ Q, const float* __restrict__ 
                          const float* __restrict__ decay, const float* __restrict__ head_decay,
                          const float* __restrict__ v_gain, const float* __restrict__ skip, float* __restrict__ S_all, float* __restrict__ N_all, const int* __restrict__ q_start,
                          const int* __restrict__ n_new, const int* __restrict__ slot_ids, float* __restrict__ o_raw,
-                         float* __restrict__ nq, int n_heads, int n_groups, int dk, int dv) {
+                         float* __restrict__ nq, int n_heads, int n_groups, int dk, int dv, int below) {
   constexpr int CHUNK = DMAX >= 256 ? 8 : 16;
   constexpr int LR_THREADS = LR_COLS * LR_LANES;
   constexpr int IPL = DMAX / LR_LANES;             // key channels per lane
@@ -277,6 +279,7 @@ linear_recurrence_kernel(const float* __restrict__ Q, const float* __restrict__ 
   const int n_cols = dv + (N_all != nullptr ? 1 : 0);      // the normaliser is one more column, whose value is 1
   const bool live = col < n_cols, is_norm = col == dv;
   const int t0 = q_start[req], n = n_new[req];
+  if (n >= below) return;      // walked in turns
   const int wk = n_groups * dk, wv = n_heads * dv, group = head / (n_heads / n_groups);
   const size_t slot = (size_t)slot_ids[req];
   float* S_g = S_all + (slot * n_heads + head) * (size_t)dk * dv;
@@ -378,12 +381,14 @@ linear_recurrence_kernel(const float* __restrict__ Q, const float* __restrict__ 
 // [tokens, heads] or null (then head_decay [heads], or 1 when that is null too); v_gain [tokens, heads] or null (1)
 // multiplies the value that enters the state; skip [heads] or null (0): o += skip * value (without its gain);
 // S [slots, heads, dk, dv]; N [slots, heads, dk] or null (no normaliser: nq is not written; with one, v_gain and skip must
-// be null); tables: workspace of llmrs_linear_recurrence_table_floats; o_raw float32 [tokens, heads * dv]; nq float32 [tokens, heads].
+// be null); tables: workspace of llmrs_linear_recurrence_table_floats; o_raw float32 [tokens, heads * dv]; nq float32 [tokens,
+// heads]. walk_from: requests of at least so many tokens are walked in turns, the others token by token; 0: all of them are.
 LLMRS_API int llmrs_linear_recurrence_planes(const float* Q, const float* K, const float* V, const float* decay,
                                              const float* head_decay, const float* v_gain, const float* skip, float* S,
                                              float* N, const int* q_start, const int* n_new, const int* slot_ids,
                                              float* tables, float* o_raw, float* nq, int n_tokens, int n_requests,
-                                             int n_heads, int n_groups, int dk, int dv, cudaStream_t stream) {
+                                             int n_heads, int n_groups, int dk, int dv, int walk_from,
+                                             cudaStream_t stream) {
   LLMRS_REQUIRE(n_requests >= 0 && n_tokens >= 0 && n_heads > 0 && dk > 0 && dv > 0, "linear_recurrence: bad sizes");
   LLMRS_REQUIRE(n_groups > 0 && n_heads % n_groups == 0, "linear_recurrence: %d heads are no multiple of %d groups",
                 n_heads, n_groups);
@@ -394,25 +399,27 @@ LLMRS_API int llmrs_linear_recurrence_planes(const float* Q, const float* K, con
   LLMRS_REQUIRE((((uintptr_t)Q | (uintptr_t)K) & 15) == 0, "linear_recurrence: planes must be 16-byte aligned");
   if (n_requests == 0 || n_tokens == 0) return 0;
   const int cols = dv + (N != nullptr ? 1 : 0);
-  if (n_tokens - n_requests + 1 >= WALK_MIN_PORTION) {      // some request may bring a portion
+  if (walk_from > 0) {
     LLMRS_REQUIRE(((uintptr_t)tables & 15) == 0 && tables != nullptr, "linear_recurrence: no workspace for a portion");
     LLMRS_REQUIRE(((uintptr_t)V & 15) == 0, "linear_recurrence: planes must be 16-byte aligned");
     const long long stride = (long long)n_groups * dk;
     int rc = launch_walk_tables(Q, K, stride, decay, head_decay, v_gain, q_start, n_new, tables, n_tokens,
-                                             n_requests, n_heads, n_groups, dk, stream);
+                                             n_requests, n_heads, n_groups, dk, walk_from, stream);
     if (rc != 0) return rc;
     WalkArgs a = {};
     a.q = Q; a.k = K; a.q_stride = a.k_stride = stride; a.v = V; a.tables = tables; a.skip = skip;
     a.state = S; a.norm_state = N; a.o_raw = o_raw; a.nq = nq;
     a.q_start = q_start; a.n_new = n_new; a.slot_ids = slot_ids;
-    a.n_heads = n_heads; a.n_groups = n_groups; a.d = dk; a.dv = dv;
-    return launch_state_walk<WALK_LINEAR>(a, n_requests, cols, stream);
+    a.n_heads = n_heads; a.n_groups = n_groups; a.d = dk; a.dv = dv; a.from = walk_from;
+    rc = launch_state_walk<WALK_LINEAR>(a, n_requests, cols, stream);
+    if (rc != 0 || walk_from == 1) return rc;
   }
+  const int below = walk_from > 0 ? walk_from : INT_MAX;
   dim3 grid(n_requests, n_heads, (cols + LR_COLS - 1) / LR_COLS);
 #define LLMRS_LR_LAUNCH(D, L)                                                                                     \
   linear_recurrence_kernel<D, L><<<grid, LR_COLS * L, 0, stream>>>(Q, K, V, decay, head_decay, v_gain, skip, S, N, \
                                                                    q_start, n_new, slot_ids, o_raw, nq, n_heads,  \
-                                                                   n_groups, dk, dv)
+                                                                   n_groups, dk, dv, below)
   if (dk <= 32) LLMRS_LR_LAUNCH(32, 4);
   else if (dk <= 64) LLMRS_LR_LAUNCH(64, 4);
   else if (dk <= 128) LLMRS_LR_LAUNCH(128, 8);
@@ -443,7 +450,7 @@ LLMRS_API int llmrs_linear_recurrence(const void* q, const void* k, const void* 
                                       const float* decay, const float* head_decay, const float* gain, float* S,
                                       float* N, const int* q_start, const int* n_new, const int* slot_ids,
                                       float* work, float* o_raw, float* nq, int n_tokens, int n_requests, int n_heads,
-                                      int dk, int dv, cudaStream_t stream) {
+                                      int dk, int dv, int walk_from, cudaStream_t stream) {
   LLMRS_REQUIRE(n_requests >= 0 && n_tokens >= 0 && n_heads > 0 && dk > 0 && dv > 0, "linear_recurrence: bad sizes");
   LLMRS_REQUIRE(rot_dims >= 0 && rot_dims % 2 == 0 && rot_dims <= dk, "linear_recurrence: rot_dims %d of %d", rot_dims, dk);
   LLMRS_REQUIRE(rot_dims == 0 || (inv_freq != nullptr && positions != nullptr),
@@ -483,7 +490,7 @@ LLMRS_API int llmrs_linear_recurrence(const void* q, const void* k, const void* 
   int rc = llmrs_launch_status("linear_recurrence (prepare)");
   if (rc != 0) return rc;
   return llmrs_linear_recurrence_planes(Q, K, V, decay, head_decay, nullptr, nullptr, S, N, q_start, n_new, slot_ids,
-                                        tables, o_raw, nq, n_tokens, n_requests, n_heads, n_heads, dk, dv, stream);
+                                        tables, o_raw, nq, n_tokens, n_requests, n_heads, n_heads, dk, dv, walk_from, stream);
 }
 
 // ---------------------------------------------------------------------------------

@@ -37,11 +37,10 @@
 enum { WALK_LINEAR = 0, WALK_GATED = 1, WALK_CHANNEL = 2, WALK_GENERAL = 3 };
 constexpr int WALK_TURN = 4, WALK_COLS = 16, WALK_LANES = 16, WALK_THREADS = WALK_COLS / 2 * WALK_LANES;
 constexpr int WALK_STAGE = 2 * WALK_TURN, WALK_STAGES = 4;      // tokens of a stage, stages
-// Portions at least this long take the walk in turns (a step's host side knows tokens and requests, so a portion has at most
-// n_tokens - n_requests + 1); shorter ones and single tokens are walked one by one, without the coefficients' kernel. Measured,
-// one by one against in turns with its coefficients (us, one portion): 32 tokens gated 10.8 / 13.7, linear 11.5 / 12.8, general
+// Which requests of a step are walked in turns is the caller's choice, by their tokens (`from`; see ops.walk_from): the kernels
+// here leave shorter requests alone, the ones that walk token by token leave the others. Measured, token by token against in
+// turns with its coefficients (us, one portion, the two kernels alone): 32 tokens gated 10.8 / 13.7, linear 11.5 / 12.8, general
 // 18.3 / 19.6; 48 tokens 14.6 / 15.9, 15.6 / 14.4, 24.2 / 21.4; 64 tokens 18.5 / 17.8, 19.6 / 16.0, 30.7 / 23.4.
-constexpr int WALK_MIN_PORTION = 48;
 
 // A turn's coefficients of one head, in floats. LINEAR, GATED, CHANNEL: P [4] (CHANNEL: ones), Z [4] (likewise), beta or gain
 // [4], K below the diagonal row by row [6] and two zeros, Q [4][4] (zero above the diagonal). GENERAL: A [6] + 2, B [6] + 2,
@@ -59,6 +58,18 @@ __device__ __forceinline__ int walk_request(const int* __restrict__ q_start, int
   for (int base = 0; base < n_requests; base += 32) {
     const int r = base + (threadIdx.x & 31);
     const unsigned hit = __ballot_sync(0xffffffffu, r < n_requests && walk_place(q_start[r], r) <= p);
+    if (hit == 0) break;
+    found = base + 31 - __clz(hit);
+  }
+  return found;
+}
+
+// The request that token t belongs to; all lanes of a warp call it.
+__device__ __forceinline__ int walk_token_request(const int* __restrict__ q_start, int n_requests, int t) {
+  int found = 0;
+  for (int base = 0; base < n_requests; base += 32) {
+    const int r = base + (threadIdx.x & 31);
+    const unsigned hit = __ballot_sync(0xffffffffu, r < n_requests && q_start[r] <= t);
     if (hit == 0) break;
     found = base + 31 - __clz(hit);
   }
@@ -170,6 +181,7 @@ struct WalkArgs {
   float *o_raw, *nq;           // [tokens, heads * dv], [tokens, heads]
   const int *q_start, *n_new, *slot_ids;
   int n_heads, n_groups, d, dv;
+  int from;                    // requests of fewer tokens are not walked here
 };
 
 // Rows a token brings in a stage.
@@ -192,7 +204,7 @@ __global__ void __launch_bounds__(WALK_THREADS, 2) state_walk_kernel(WalkArgs p,
   const int col0 = blockIdx.x % col_blocks * WALK_COLS, tid = threadIdx.x;
   const int part = tid % WALK_LANES, c0 = tid / WALK_LANES * 2, col = col0 + c0;      // this thread's columns: col, col + 1
   const int n = p.n_new[req], t0 = p.q_start[req], d = p.d, dv = p.dv, kh = head / (p.n_heads / p.n_groups);
-  if (n <= 0) return;
+  if (n < p.from) return;
   const size_t slot = (size_t)p.slot_ids[req];
   float* S_g = p.state + (slot * p.n_heads + head) * (size_t)d * dv;
   float* N_g = p.norm_state ? p.norm_state + (slot * p.n_heads + head) * (size_t)d : nullptr;
@@ -509,12 +521,13 @@ template <int CPL>
 __global__ void __launch_bounds__(128)
 walk_tables_kernel(const float* __restrict__ q, const float* __restrict__ k, long long stride, const float* __restrict__ decay,
                    const float* __restrict__ head_decay, const float* __restrict__ beta, const int* __restrict__ q_start,
-                   const int* __restrict__ n_new, float* __restrict__ tables, int n_requests, int n_heads, int n_groups, int d) {
+                   const int* __restrict__ n_new, float* __restrict__ tables, int n_requests, int n_heads, int n_groups, int d,
+                   int from) {
   const int place = blockIdx.x, head = blockIdx.y * 4 + (threadIdx.x >> 5), lane = threadIdx.x & 31;
   if (head >= n_heads) return;
   const int req = walk_request(q_start, n_requests, place), t_req = q_start[req];
   const int first = (place - walk_place(t_req, req)) * WALK_TURN, have = min(WALK_TURN, n_new[req] - first);
-  if (first < 0 || have <= 0) return;
+  if (first < 0 || have <= 0 || n_new[req] < from) return;
   const size_t t0 = (size_t)(t_req + first);
   const float* qr = q + t0 * stride + (size_t)(head / (n_heads / n_groups)) * d;
   const float* kr = k + t0 * stride + (size_t)(head / (n_heads / n_groups)) * d;
@@ -544,14 +557,14 @@ walk_tables_kernel(const float* __restrict__ q, const float* __restrict__ k, lon
 
 static int launch_walk_tables(const float* q, const float* k, long long stride, const float* decay, const float* head_decay,
                               const float* beta, const int* q_start, const int* n_new, float* tables, int n_tokens,
-                              int n_requests, int n_heads, int n_groups, int d, cudaStream_t stream) {
+                              int n_requests, int n_heads, int n_groups, int d, int from, cudaStream_t stream) {
   const dim3 grid((unsigned)walk_places(n_tokens, n_requests), (n_heads + 3) / 4);
   if (d <= 128)
     walk_tables_kernel<4><<<grid, 128, 0, stream>>>(q, k, stride, decay, head_decay, beta, q_start, n_new, tables,
-                                                    n_requests, n_heads, n_groups, d);
+                                                    n_requests, n_heads, n_groups, d, from);
   else
     walk_tables_kernel<8><<<grid, 128, 0, stream>>>(q, k, stride, decay, head_decay, beta, q_start, n_new, tables,
-                                                    n_requests, n_heads, n_groups, d);
+                                                    n_requests, n_heads, n_groups, d, from);
   return llmrs_launch_status("state walk (tables)");
 }
 

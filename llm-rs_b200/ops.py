@@ -927,6 +927,54 @@ def moe_combine(rows: torch.Tensor, row_of: torch.Tensor, weight_of: torch.Tenso
     return out
 
 
+# -- recurrences with a matrix state: which requests of a step are walked in turns ------------------------
+WALK_PORTION = 48       # requests of fewer tokens count as short
+
+
+def walk_from(ctx, n_tokens: int, blocks: int, least: int = WALK_PORTION, per: int = 64, few: int = 2048) -> int:
+    """From how many tokens on a request is walked in turns of four tokens (csrc/state_walk.cuh) in this step, the others token
+    by token; 0: none is, 1: all are. ``blocks``: blocks of the walk that a request takes.
+
+    A portion by itself is faster in turns from ``least`` tokens on. Short requests beside it are not: their blocks read and write
+    the state and little else, which the walk's large blocks do at half the pace (a single token of 16 heads of 128 x 128 2.4 us,
+    token by token 1.0). So ``few`` blocks of them ride along; more take the kernels token by token behind the walk, which costs
+    those kernels' launches and gives up that they run beside the portion: worth it where the portion has a token more for every
+    ``per`` blocks of short requests. Measured, token by token / all in turns / both (us, a whole mixer, 16 heads of 128 x 128,
+    the generalized rule 32 of 64 x 64), single tokens + a portion:
+      gated    15 + 256 165 / 142 / 150    63 + 64 137 / 223 / 175    63 + 256 217 / 264 / 215    63 + 512 333 / 318 / 268
+      linear   15 + 64 75 / 85 / 73        63 + 64 133 / 201 / 145    63 + 128 163 / 216 / 160    63 + 512 341 / 285 / 229
+      general  15 + 64 83 / 73 / 76        63 + 64 115 / 145 / 119    63 + 128 163 / 162 / 134    63 + 512 458 / 277 / 242
+    A request's numbers differ in their last float32 bits between the two ways."""
+    n = ctx.n_requests
+    if n_tokens < WALK_PORTION or n_tokens == n:
+        return 0
+    lens = getattr(ctx, "host_n_new", None)
+    if lens:
+        longest, short = max(lens), sum(k < WALK_PORTION for k in lens)
+    else:       # without the step's host lists: one portion, and single tokens beside it
+        longest, short = n_tokens - n + 1, n - 1
+    if longest < least + short * max(1, blocks // per):
+        return 0
+    return 1 if short * blocks <= few else WALK_PORTION
+
+
+def _walk_blocks(n_heads: int, cols: int) -> int:
+    return n_heads * -(-cols // 16)
+
+
+def _gated_walk_least(channels: int, d: int, channel: bool) -> int:
+    """Tokens from which on one portion of the gated delta rule is faster in turns: the kernel that makes a turn's rows takes some
+    18 us however few channels (30 with a decay per channel), the one that prepares single tokens 4.5 for 1,024 channels, and a
+    token saves 0.09 us of the walk with heads of 64 and 0.15 with heads of 128. Measured crossings (key heads of d, ``channels``
+    of the convolution): 64, 512: 220 tokens; 64, 2,048: 135; 96 and 128, 2,048: 85 to 112; 128, 4,096: below 48; with a decay per
+    channel 64, 512: 380; 64, 2,048: 300; 128, 1,536: 112; 128, 4,096: 90; 128, 8,192: below 48."""
+    if channel:
+        line = 400 - 50 * channels // 1024 if d <= 64 else 160 - 20 * channels // 1024
+    else:
+        line = 240 - 54 * channels // 1024 if d <= 64 else 140 - 25 * channels // 1024
+    return max(WALK_PORTION, line)
+
+
 # -- the generalized delta rule -------------------------------------------------------------------------
 def delta_rule(r, k, v, gate, a_raw, decay_raw, decay_bias, a_bias, norm_w, state, ctx, n_heads: int, d: int,
                decay_scale: float, key_eps: float, norm_eps: float) -> torch.Tensor:
@@ -943,11 +991,13 @@ def delta_rule(r, k, v, gate, a_raw, decay_raw, decay_bias, a_bias, norm_w, stat
     out = torch.empty((r.size(0), n_heads * d), dtype=r.dtype, device=r.device)
     work = torch.empty((int(_lib_ll("llmrs_delta_rule_work_floats")(r.size(0), ctx.n_requests, n_heads, d)),),
                        dtype=torch.float32, device=r.device)
+    # (heads of 32: one portion 128 tokens 47 / 47 us, heads of 64: 48 tokens 54 / 48)
+    turns = walk_from(ctx, r.size(0), _walk_blocks(n_heads, d), least=128 if d <= 32 else WALK_PORTION)
     _check(_lib().llmrs_delta_rule(
         _ptr(r), _ptr(k), _ptr(v), _ptr(gate), _ptr(a_raw), _LL(stride), dtype_code(r.dtype), _ptr(decay_raw),
         _ptr(decay_bias), _ptr(a_bias), _ptr(norm_w), _ptr(state), _ptr(ctx.q_start), _ptr(ctx.n_new),
         _ptr(ctx.slot_ids), _ptr(work), _ptr(out), r.size(0), ctx.n_requests, n_heads, d, ctypes.c_float(decay_scale),
-        ctypes.c_float(key_eps), ctypes.c_float(norm_eps), _stream()), "delta_rule", 3)
+        ctypes.c_float(key_eps), ctypes.c_float(norm_eps), turns, _stream()), "delta_rule", 5 if turns > 1 else 3)
     return out
 
 
@@ -1212,6 +1262,7 @@ def linear_recurrence(q, k, v, gate, norm_w, state, ctx, n_heads: int, dk: int, 
     if (normaliser is None) != (floor is None):
         raise KernelError("linear_recurrence: normaliser and floor come together")
     dev = q.device
+    turns = walk_from(ctx, n, _walk_blocks(n_heads, dv + (normaliser is not None)), few=1024)
     # One workspace: the kernels' rows, then the raw read-outs and the normaliser's products.
     n_work = -(-int(_lib_ll("llmrs_linear_recurrence_work_floats")(n, ctx.n_requests, n_heads, dk, dv)) // 4) * 4
     work = torch.empty((n_work + n * n_heads * (dv + 1),), dtype=torch.float32, device=dev)
@@ -1221,7 +1272,8 @@ def linear_recurrence(q, k, v, gate, norm_w, state, ctx, n_heads: int, dk: int, 
         _ptr(q), _ptr(k), _ptr(v), _LL(_row_stride(q, "q")), _LL(_row_stride(k, "k")), _LL(_row_stride(v, "v")),
         dtype_code(q.dtype), int(act_silu), ctypes.c_float(q_scale), ctypes.c_float(k_scale), _ptr(inv_freq),
         _ptr(ctx.positions) if rot_dims else None, rot_dims, _ptr(decay), _ptr(head_decay), _ptr(gain), _ptr(state), _ptr(normaliser), _ptr(ctx.q_start), _ptr(ctx.n_new), _ptr(ctx.slot_ids), _ptr(work),
-        o_raw, nq, n, ctx.n_requests, n_heads, dk, dv, _stream()), "linear_recurrence", 2)
+        o_raw, nq, n, ctx.n_requests, n_heads, dk, dv, turns, _stream()), "linear_recurrence",
+        4 if turns > 1 else (3 if turns else 2))
     out = torch.empty((n, n_heads * dv), dtype=q.dtype, device=dev)
     _check(_lib().llmrs_recurrence_output(
         o_raw, nq, _ptr(floor), ctypes.c_float(den_eps), _ptr(gate), _LL(_row_stride(gate, "gate")),
@@ -1257,7 +1309,8 @@ def ssd(xbc: torch.Tensor, z: torch.Tensor, dt_raw: torch.Tensor, taps: torch.Te
     _need(out, "out", xbc.dtype, contiguous=False)
     empty = lambda width: torch.empty((n, width), dtype=torch.float32, device=xbc.device)
     X, B, Cq, decay, step, y = empty(inner), empty(wk), empty(wk), empty(n_heads), empty(n_heads), empty(inner)
-    tables = torch.empty((int(_lib_ll("llmrs_linear_recurrence_table_floats")(n, ctx.n_requests, n_heads)),),
+    turns = walk_from(ctx, n, _walk_blocks(n_heads, vdim), few=1024)
+    tables = torch.empty((int(_lib_ll("llmrs_linear_recurrence_table_floats")(n, ctx.n_requests, n_heads)) if turns else 0,),
                          dtype=torch.float32, device=xbc.device)
     _check(_lib().llmrs_ssd_prepare(
         _ptr(xbc), _LL(_row_stride(xbc, "xbc")), _ptr(dt_raw), _LL(_row_stride(dt_raw, "dt_raw")), dtype_code(xbc.dtype),
@@ -1267,7 +1320,7 @@ def ssd(xbc: torch.Tensor, z: torch.Tensor, dt_raw: torch.Tensor, taps: torch.Te
     _check(_lib().llmrs_linear_recurrence_planes(
         _ptr(Cq), _ptr(B), _ptr(X), _ptr(decay), None, _ptr(step), _ptr(skip), _ptr(state), None, _ptr(ctx.q_start),
         _ptr(ctx.n_new), _ptr(ctx.slot_ids), _ptr(tables), _ptr(y), None, n, ctx.n_requests, n_heads, n_groups, n_state, vdim,
-        _stream()), "linear_recurrence_planes")
+        turns, _stream()), "linear_recurrence_planes", 3 if turns > 1 else (2 if turns else 1))
     _check(_lib().llmrs_ssd_output(
         _ptr(y), _ptr(z), _LL(_row_stride(z, "z")), dtype_code(xbc.dtype), _ptr(norm_w), _ptr(out),
         _LL(_row_stride(out, "out")), n, inner, norm_parts_, ctypes.c_float(norm_eps), ctypes.c_float(out_scale),
@@ -1683,13 +1736,15 @@ def gated_delta(x: torch.Tensor, gate: torch.Tensor, taps: torch.Tensor, ba: Opt
     work = torch.empty((int(_lib_ll("llmrs_gated_delta_work_floats")(n, ctx.n_requests, n_kv_heads, n_heads, dk, dv,
                                                                      int(channel))),),
                        dtype=torch.float32, device=x.device)
+    turns = walk_from(ctx, n, _walk_blocks(n_heads, dv), least=_gated_walk_least(C, dk, channel), per=32)
     _check(_lib().llmrs_gated_delta(
         _ptr(x), _LL(_row_stride(x, "x")), _ptr(gate), _LL(_row_stride(gate, "gate")), dtype_code(x.dtype), _ptr(taps),
         _ptr(None if channel else ba), _ptr(b), _LL(_row_stride(b, "b") if channel else 0), _ptr(channel_decay),
         _ptr(a_log), _ptr(dt_bias), _ptr(norm_w), _ptr(state), _ptr(conv_state), _ptr(ctx.token_req), _ptr(ctx.q_start),
         _ptr(ctx.n_new), _ptr(ctx.slot_ids), _ptr(work), _ptr(out), _LL(_row_stride(out, "out")), n, ctx.n_requests,
         n_kv_heads, n_heads, dk, dv, K, ctypes.c_float(key_eps), ctypes.c_float(q_scale), ctypes.c_float(norm_eps),
-        ctypes.c_float(out_scale), int(gate_sigmoid), _stream()), "gated_delta", 4 if K > 1 else 3)
+        ctypes.c_float(out_scale), int(gate_sigmoid), turns, _stream()), "gated_delta",
+        (4 if K > 1 else 3) + (2 if turns > 1 else 0))
     return out
 
 

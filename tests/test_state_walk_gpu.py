@@ -1,6 +1,6 @@
-"""Portions of 48 tokens and more take the recurrences with a matrix state in turns of four tokens
-(csrc/state_walk.cuh), single tokens one by one: the same outputs and states from either, at the edges of turns, stages and
-copies, for many requests in one step. Both are float32 evaluations of one recurrence, each some 1e-6 from 64 bits in the
+"""The recurrences with a matrix state walked in turns of four tokens (csrc/state_walk.cuh) and token by token: the same outputs
+and states from either, at the edges of turns, stages and copies, for many requests in one step, with all of a step's requests
+in turns or those from some length on. Both are float32 evaluations of one recurrence, each some 1e-6 from 64 bits in the
 2-norm at these sizes; single elements may lie sixteen times that apart."""
 from types import SimpleNamespace
 
@@ -40,6 +40,14 @@ def test_portions_in_turns_match_single_tokens(kind, d, dv, lens):
     _compare(kind, d, dv, lens, 3)
 
 
+@pytest.mark.parametrize("kind", ["memory", "retention", "mamba", "gated", "channel", "general"])
+@pytest.mark.parametrize("d,dv,lens,turns", [(64, 64, [1, 49, 1, 7, 48], 48), (30, 17, [5, 0, 9, 4, 8, 1] * 6, 5),
+                                             (128, 48, [1] * 40 + [50], 50), (96, 20, [3, 2, 1], 48)])
+def test_some_requests_in_turns(kind, d, dv, lens, turns):
+    """Both ways in one step: requests of at least ``turns`` tokens in turns, the others token by token."""
+    _compare(kind, d, dv, lens, 3, turns)
+
+
 @pytest.mark.parametrize("kind", ["gated", "channel"])
 @pytest.mark.parametrize("taps", [2, 4, 6])
 @pytest.mark.parametrize("d,dv,lens", [(64, 48, [9, 1, 49, 2]), (30, 17, [50, 7]), (136, 8, [48, 5])])
@@ -48,7 +56,22 @@ def test_convolutions_of_turns(kind, taps, d, dv, lens):
     _compare(kind, d, dv, lens, taps)
 
 
-def _compare(kind, d, dv, lens, taps):
+class _in_turns:
+    """The step's requests of at least ``turns`` tokens are walked in turns, whatever the rule says."""
+
+    def __init__(self, turns):
+        self.turns = turns
+
+    def __enter__(self):
+        from llm_rs_b200 import ops
+        self.rule, ops.walk_from = ops.walk_from, lambda *a, **k: self.turns
+
+    def __exit__(self, *a):
+        from llm_rs_b200 import ops
+        ops.walk_from = self.rule
+
+
+def _compare(kind, d, dv, lens, taps, turns=1):
     from llm_rs_b200.parts import Runtime
     g = torch.Generator().manual_seed(d + dv)
     D, part = _part(kind, d, dv, taps)
@@ -59,7 +82,8 @@ def _compare(kind, d, dv, lens, taps):
     start = {name: 0.3 * torch.randn(len(lens), *shape, generator=g).to(DEV)
              for name, shape in part.state_need().tensors.items()}
     whole = {k: t.clone() for k, t in start.items()}
-    got = part.forward(torch.cat(x), _ctx(lens, [0] * len(lens)), SimpleNamespace(state=whole))
+    with _in_turns(turns):
+        got = part.forward(torch.cat(x), _ctx(lens, [0] * len(lens)), SimpleNamespace(state=whole))
     single = {k: t.clone() for k, t in start.items()}
     rows = [[] for _ in lens]
     for i in range(max(lens)):
@@ -89,7 +113,8 @@ def test_tokens_before_one_that_is_not_finite_keep_their_numbers(kind, at, bad):
     outs = []
     for rows in (x, x.index_fill(0, torch.tensor([at], device=DEV), bad)):
         state = {name: torch.zeros(1, *shape, device=DEV) for name, shape in part.state_need().tensors.items()}
-        outs.append(part.forward(rows, _ctx([62], [0]), SimpleNamespace(state=state)))
+        with _in_turns(1):
+            outs.append(part.forward(rows, _ctx([62], [0]), SimpleNamespace(state=state)))
     want, got = outs
     assert torch.isfinite(want).all()
     assert torch.equal(got[:at], want[:at])
