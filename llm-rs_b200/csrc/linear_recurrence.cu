@@ -13,7 +13,7 @@
 // Kernels:
 //   gate_scan    exponential gates with a running maximum m (m_t = max(f_t + m_(t-1), i_t), log-space input gate i and
 //                forget gate f, both soft-capped): a warp per (request, head) scans the request's tokens of the step,
-//                32 at a time (portions of 128 tokens and more: a block, eight tokens a thread), with the associative form of the (max, +) recurrence, and leaves
+//                32 at a time (portions of 128 tokens and more: a block each, eight tokens a thread), with the associative form of the (max, +) recurrence, and leaves
 //                a_t = exp(f_t + m_(t-1) - m_t), b_t = exp(i_t - m_t), floor_t = exp(-m_t); m is kept per slot;
 //   prepare      q, k, v of all tokens widened to float32 (optional SiLU, optional rotation of the first channels of every
 //                head of q and k by halves, q and k scaled, k multiplied by its gain);
@@ -38,16 +38,11 @@ __device__ __forceinline__ float lr_logsigmoid(float x) { return fminf(x, 0.f) -
 // gate_scan
 // ---------------------------------------------------------------------------------
 // gates: float32 [tokens, 2 * heads] (row stride given): the input gate's pre-activations, then the forget gate's.
-__global__ void gate_scan_kernel(const float* __restrict__ gates, long long stride, float cap,
-                                 float* __restrict__ m_state, const int* __restrict__ q_start,
-                                 const int* __restrict__ n_new, const int* __restrict__ slot_ids,
-                                 float* __restrict__ decay, float* __restrict__ gain, float* __restrict__ floor_,
-                                 int n_heads) {
-  const int req = blockIdx.x, lane = threadIdx.x & 31;
-  const int head = blockIdx.y * (blockDim.x >> 5) + (threadIdx.x >> 5);
-  if (head >= n_heads) return;
-  const int t0 = q_start[req], n = n_new[req];
-  float* mp = m_state + (size_t)slot_ids[req] * n_heads + head;
+// One head of a request, tokens t0 .. t0 + n - 1, by a warp; *mp: its running maximum.
+__device__ __forceinline__ void gate_scan_warp(const float* __restrict__ gates, long long stride, float cap, float* __restrict__ mp,
+                                               int t0, int n, int head, float* __restrict__ decay, float* __restrict__ gain,
+                                               float* __restrict__ floor_, int n_heads) {
+  const int lane = threadIdx.x & 31;
   float m = *mp;
   for (int base = 0; base < n; base += 32) {
     const int t = base + lane;
@@ -83,11 +78,24 @@ __global__ void gate_scan_kernel(const float* __restrict__ gates, long long stri
   if (lane == 0) *mp = m;
 }
 
-// The same for portions: a block per (request, head), a run of GS_RUN tokens a thread. A run's steps compose to one step of the
-// recurrence (F, I); those are scanned over the block, and each thread then walks its run from the maximum that it starts with.
-// One warp, 32 tokens at a time, waits for a chain of shuffles and for memory in each of its turns: 1,311 tokens of 16 heads
-// 40 us, in runs 8.5.
-constexpr int GS_RUN = 8, GS_THREADS = 256;
+__global__ void gate_scan_kernel(const float* __restrict__ gates, long long stride, float cap,
+                                 float* __restrict__ m_state, const int* __restrict__ q_start,
+                                 const int* __restrict__ n_new, const int* __restrict__ slot_ids,
+                                 float* __restrict__ decay, float* __restrict__ gain, float* __restrict__ floor_,
+                                 int n_heads) {
+  const int req = blockIdx.x, head = blockIdx.y * (blockDim.x >> 5) + (threadIdx.x >> 5);
+  if (head >= n_heads) return;
+  gate_scan_warp(gates, stride, cap, m_state + (size_t)slot_ids[req] * n_heads + head, q_start[req], n_new[req], head, decay, gain,
+                 floor_, n_heads);
+}
+
+// The same for steps with a portion of GS_PORTION tokens or more: a block per (request, head), a run of GS_RUN tokens a thread.
+// A run's steps compose to one step of the recurrence (F, I); those are scanned over the block, and each thread then walks its
+// run from the maximum that it starts with. One warp, 32 tokens at a time, waits for a chain of shuffles and for memory in each
+// of its turns: 1,311 tokens of 16 heads 40 us, in runs 8.5. Shorter requests of the step take a warp a head here too, eight
+// heads a block, the other blocks of theirs leave at once (with a block a head 257 requests, one of 128 tokens: 22 us).
+// One portion by a warp / in runs, us: 96 tokens 4.3 / 4.9, 128 5.2 / 5.0, 192 6.9 / 5.1, 512 15.5 / 5.7.
+constexpr int GS_RUN = 8, GS_THREADS = 256, GS_PORTION = 128;
 __global__ void __launch_bounds__(GS_THREADS)
 gate_scan_runs_kernel(const float* __restrict__ gates, long long stride, float cap, float* __restrict__ m_state,
                       const int* __restrict__ q_start, const int* __restrict__ n_new, const int* __restrict__ slot_ids,
@@ -95,6 +103,12 @@ gate_scan_runs_kernel(const float* __restrict__ gates, long long stride, float c
   __shared__ float s_F[GS_THREADS / 32], s_I[GS_THREADS / 32];
   const int req = blockIdx.x, head = blockIdx.y, warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
   const int t0 = q_start[req], n = n_new[req];
+  if (n < GS_PORTION) {
+    const int own = head + warp;
+    if (head % (GS_THREADS / 32) == 0 && own < n_heads)
+      gate_scan_warp(gates, stride, cap, m_state + (size_t)slot_ids[req] * n_heads + own, t0, n, own, decay, gain, floor_, n_heads);
+    return;
+  }
   float* mp = m_state + (size_t)slot_ids[req] * n_heads + head;
   float m = *mp;
   __syncthreads();      // every thread has the old maximum before one thread writes the new one
@@ -153,13 +167,13 @@ gate_scan_runs_kernel(const float* __restrict__ gates, long long stride, float c
   }
 }
 
+// longest: no request of the step brings more tokens (it chooses the kernel, not the numbers).
 LLMRS_API int llmrs_gate_scan(const float* gates, long long stride, float cap, float* m_state, const int* q_start,
                               const int* n_new, const int* slot_ids, float* decay, float* gain, float* floor_,
-                              int n_tokens, int n_requests, int n_heads, cudaStream_t stream) {
+                              int longest, int n_requests, int n_heads, cudaStream_t stream) {
   LLMRS_REQUIRE(n_requests >= 0 && n_heads > 0 && cap > 0.f, "gate_scan: bad arguments");
   if (n_requests == 0) return 0;
-  // Some request may bring a portion of four turns of a warp: 63 tokens take 3.1 us by a warp, 64 to 128 take 4.9 in runs.
-  if (n_tokens - n_requests + 1 >= 128 && n_heads <= 65535) {
+  if (longest >= GS_PORTION && n_heads <= 65535) {
     gate_scan_runs_kernel<<<dim3(n_requests, n_heads), GS_THREADS, 0, stream>>>(gates, stride, cap, m_state, q_start, n_new,
                                                                                 slot_ids, decay, gain, floor_, n_heads);
     return llmrs_launch_status("gate_scan");

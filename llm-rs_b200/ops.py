@@ -928,6 +928,12 @@ def moe_combine(rows: torch.Tensor, row_of: torch.Tensor, weight_of: torch.Tenso
 
 
 # -- recurrences with a matrix state: which requests of a step are walked in turns ------------------------
+def longest_portion(ctx, n_tokens: int) -> int:
+    """Tokens of the step's longest request; without the step's host lists the most that it can be."""
+    lens = getattr(ctx, "host_n_new", None)
+    return max(lens) if lens else n_tokens - ctx.n_requests + 1
+
+
 WALK_PORTION = 48       # requests of fewer tokens count as short
 
 
@@ -948,11 +954,9 @@ def walk_from(ctx, n_tokens: int, blocks: int, least: int = WALK_PORTION, per: i
     n = ctx.n_requests
     if n_tokens < WALK_PORTION or n_tokens == n:
         return 0
-    lens = getattr(ctx, "host_n_new", None)
-    if lens:
-        longest, short = max(lens), sum(k < WALK_PORTION for k in lens)
-    else:       # without the step's host lists: one portion, and single tokens beside it
-        longest, short = n_tokens - n + 1, n - 1
+    longest = longest_portion(ctx, n_tokens)
+    lens = getattr(ctx, "host_n_new", None)      # without it: one portion, and single tokens beside it
+    short = sum(k < WALK_PORTION for k in lens) if lens else n - 1
     if longest < least + short * max(1, blocks // per):
         return 0
     return 1 if short * blocks <= few else WALK_PORTION
@@ -1231,7 +1235,7 @@ def gate_scan(gates: torch.Tensor, cap: float, m_state: torch.Tensor, ctx, n_hea
     decay, gain, floor = (torch.empty((n, n_heads), dtype=torch.float32, device=gates.device) for _ in range(3))
     _check(_lib().llmrs_gate_scan(_ptr(gates), _LL(_row_stride(gates, "gates")), ctypes.c_float(cap), _ptr(m_state),
                                   _ptr(ctx.q_start), _ptr(ctx.n_new), _ptr(ctx.slot_ids), _ptr(decay), _ptr(gain),
-                                  _ptr(floor), n, ctx.n_requests, n_heads, _stream()), "gate_scan")
+                                  _ptr(floor), longest_portion(ctx, n), ctx.n_requests, n_heads, _stream()), "gate_scan")
     return decay, gain, floor
 
 
