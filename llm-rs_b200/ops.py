@@ -1375,8 +1375,13 @@ def scored_prepare(q: torch.Tensor, k: Optional[torch.Tensor], v: Optional[torch
         _stream()), "scored_prepare")
 
 
+_scored_generic_only = False
+
+
 def scored_generic_only(on: bool) -> None:
     """True: bfloat16 prompt portions take the kernel for any type too (tests compare it with the tensor-core one)."""
+    global _scored_generic_only
+    _scored_generic_only = bool(on)
     fn = _lib().llmrs_scored_generic_only
     fn.restype, fn.argtypes = None, [ctypes.c_int]
     fn(1 if on else 0)
@@ -1429,11 +1434,13 @@ def scored_decode_group(n_q_heads: int, n_kv_heads: int, dk: int, dv: int, page_
 DECODE_STREAM_BLOCKS = 1184     # blocks of the tensor-core decode kernel that a step's runs of keys are cut for (four waves)
 
 
-def scored_decode_runs(n_dec: int, n_q_heads: int, n_kv_heads: int, dk: int, dv: int, dtype: torch.dtype, span: int):
+def scored_decode_runs(n_dec: int, n_q_heads: int, n_kv_heads: int, q: torch.Tensor, cache: torch.Tensor, dk: int, dv: int,
+                       span: int):
     """(runs, keys per run) for the tensor-core decode kernel over at most ``span`` visible keys, or None where it does not take
-    these heads. A run of 64 keys is one tile for each of a block's four warps; longer runs keep their rings full, and the
+    these heads or rows. A run of 64 keys is one tile for each of a block's four warps; longer runs keep their rings full, and the
     merge reads fewer of them."""
-    if dtype != torch.bfloat16 or dk != dv or dk not in (64, 128):      # (csrc/attention_scored.cu decode_on_tensor_cores)
+    if (q.dtype != torch.bfloat16 or dk != dv or dk not in (64, 128) or _scored_generic_only or cache.data_ptr() % 16
+            or q.data_ptr() % 4 or q.stride(0) % 2):      # (what csrc/attention_scored.cu llmrs_scored_decode asks for)
         return None
     blocks = n_dec * n_kv_heads * -(-(n_q_heads // n_kv_heads) // 4)
     runs = max(1, min(-(-DECODE_STREAM_BLOCKS // blocks), -(-span // 64)))

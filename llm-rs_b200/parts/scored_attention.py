@@ -248,19 +248,23 @@ class ScoredAttention(Mixer):
                                out_scale=scale, keep=self.keep_first, gate=head_gate)
         if n_decode:
             span = max(1, min(max_kv, self.mask_size + self.keep_first) if self.mask_size else max_kv)   # keys a query can see at most
-            group = ops.scored_decode_group(self.n_heads, self.n_kv_heads, self.dim, self.vdim, cache.page_size, q.dtype)
-            split_keys = DECODE_SPLIT_KEYS[group > 0]
-            blocks = n_decode * self.n_kv_heads * -(-(self.n_heads // self.n_kv_heads) // group) if group else \
-                n_decode * self.n_heads
-            while blocks * -(-span // split_keys) > DECODE_MAX_BLOCKS and split_keys < 4096:
-                split_keys *= 2
-            runs = ops.scored_decode_runs(n_decode, self.n_heads, self.n_kv_heads, self.dim, self.vdim, q.dtype, span)
-            n_runs, split_keys = runs if runs is not None else (-(-span // split_keys), split_keys)
+            n_runs, split_keys = (ops.scored_decode_runs(n_decode, self.n_heads, self.n_kv_heads, q, pages, self.dim, self.vdim, span)
+                                  or self._decode_splits(n_decode, span, cache.page_size, q.dtype))
             ops.scored_decode(q, out, pages, plan.arrays["decode_reqs"], n_decode, ctx, table, n_runs, split_keys, *args,
                               bias=self.bias, out_scale=scale, keep=self.keep_first, gate=head_gate)
         if gate is not None:
             ops.head_gate(out, gate, self.n_heads, self.vdim, out_scale)
         return out
+
+    def _decode_splits(self, n_decode: int, span: int, page_size: int, dtype):
+        """(runs, keys per run) for the decode kernels on the CUDA cores."""
+        group = ops.scored_decode_group(self.n_heads, self.n_kv_heads, self.dim, self.vdim, page_size, dtype)
+        split_keys = DECODE_SPLIT_KEYS[group > 0]
+        blocks = n_decode * self.n_kv_heads * -(-(self.n_heads // self.n_kv_heads) // group) if group else \
+            n_decode * self.n_heads
+        while blocks * -(-span // split_keys) > DECODE_MAX_BLOCKS and split_keys < 4096:
+            split_keys *= 2
+        return -(-span // split_keys), split_keys
 
     def chain(self):
         return [self.qkv_proj, self.o_proj]
