@@ -1432,19 +1432,24 @@ def scored_decode_group(n_q_heads: int, n_kv_heads: int, dk: int, dv: int, page_
 
 
 DECODE_STREAM_BLOCKS = 1184     # blocks of the tensor-core decode kernel that a step's runs of keys are cut for (four waves)
+# Keys of a run at most. Measured (no limit / 2,048 / 1,024 / 512, us, a whole mixer of 16 heads, 4 key heads of 128 and 8 of 64):
+# 47 requests of 500 keys and one of 30,000 150 / 110 / 95 / 105 and 241 / 116 / 97 / 103; 63 of 200 and one of 8,000 86 / 85 / 70 /
+# 68 and 112 / 99 / 76 / 67; 24 of 30,000 325 / 314 / 332 / 366 and 430 / 373 / 383 / 402; even batches of less do not reach it.
+DECODE_RUN_KEYS = 1024
 
 
 def scored_decode_runs(n_dec: int, n_q_heads: int, n_kv_heads: int, q: torch.Tensor, cache: torch.Tensor, dk: int, dv: int,
                        span: int):
     """(runs, keys per run) for the tensor-core decode kernel over at most ``span`` visible keys, or None where it does not take
     these heads or rows. A run of 64 keys is one tile for each of a block's four warps; longer runs keep their rings full, and the
-    merge reads fewer of them."""
+    merge reads fewer of them. Requests are cut alike, so that one which is much longer than the others has only its own runs at
+    work in the end: they are kept short."""
     if (q.dtype != torch.bfloat16 or dk != dv or dk not in (64, 128) or _scored_generic_only or cache.data_ptr() % 16
             or q.data_ptr() % 4 or q.stride(0) % 2):      # (what csrc/attention_scored.cu llmrs_scored_decode asks for)
         return None
     blocks = n_dec * n_kv_heads * -(-(n_q_heads // n_kv_heads) // 4)
     runs = max(1, min(-(-DECODE_STREAM_BLOCKS // blocks), -(-span // 64)))
-    keys = -(-(-(-span // runs)) // 64) * 64
+    keys = min(-(-(-(-span // runs)) // 64) * 64, DECODE_RUN_KEYS)
     return -(-span // keys), keys
 
 

@@ -24,3 +24,11 @@ def test_rows_and_heads_that_the_tensor_cores_do_not_take_are_cut_for_the_other_
 def test_runs_cover_the_span(span, n_dec, heads, kv):
     n, keys = _runs(span, n_dec, heads, kv)
     assert keys % 64 == 0 and n * keys >= span > (n - 1) * keys
+
+
+@pytest.mark.parametrize("n_dec", [1, 48, 64, 256])
+@pytest.mark.parametrize("span", [3000, 30000, 131072])
+def test_runs_stay_short_however_long_the_longest_request(n_dec, span):
+    """The span is the longest request's; the runs of all requests are cut from it."""
+    from llm_rs_b200 import ops
+    assert _runs(span, n_dec)[1] <= ops.DECODE_RUN_KEYS == 1024
