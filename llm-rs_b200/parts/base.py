@@ -10,7 +10,7 @@ Life of a part:  construct -> ``weight_specs()`` tells the loader which tensors 
 from __future__ import annotations
 
 from dataclasses import dataclass
-from typing import TYPE_CHECKING, Dict, List, Optional
+from typing import TYPE_CHECKING, Any, Dict, List, Optional
 
 if TYPE_CHECKING:
     import numpy as np
@@ -54,7 +54,7 @@ class Plan:
 
     ``arrays``  int32 numpy arrays; they travel to the device in the same copy as the step's other index
                 arrays and reach ``forward`` as device tensors (``ctx.plan(key).arrays[name]``).
-    ``values``  host integers that size launches (``ctx.plan(key).values[name]``).
+    ``values``  host integers, or tuples of them, that size launches (``ctx.plan(key).values[name]``).
 
     A step of single tokens may be captured in a CUDA graph and replayed for later steps. The graph is chosen by
     the batch's shape AND by every plan's array sizes and values, so a replayed launch always sees the sizes
@@ -62,7 +62,7 @@ class Plan:
     therefore round its values up to what the batch's shape implies (say, a table's width instead of the longest
     request), or every step captures a graph of its own."""
     arrays: Dict[str, "np.ndarray"]
-    values: Dict[str, int]
+    values: Dict[str, Any]
 
     def signature(self):
         return (tuple(sorted((k, int(v.size)) for k, v in self.arrays.items())), tuple(sorted(self.values.items())))

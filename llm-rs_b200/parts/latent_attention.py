@@ -28,6 +28,9 @@ PREFILL_MIN_TOKENS = 32
 # measured and stay folded.
 EXPAND_MIN_TOKENS, EXPAND_MAX_KEYS = 32, 128
 EXPAND_ALIGN = 128      # keys per tile of that kernel
+# Tokens of long portions between two runs of other tokens that the folded form's products take along: fewer cost less than
+# another launch of each of the two products.
+FOLD_GAP = 256
 
 
 def rescaled_frequencies(dims: int, base: float, scaling: Optional[Mapping] = None):
@@ -65,6 +68,20 @@ def portion_tiles(q_start, n_new, tile_tokens: int) -> np.ndarray:
     return np.stack([np.concatenate(firsts), np.concatenate(counts)], axis=1).astype(np.int32)
 
 
+def other_ranges(q_start, n_new, is_long, n_tokens: int):
+    """The step's tokens that are of no long portion, as ranges (first, end); ranges less than FOLD_GAP apart are one."""
+    ranges, at = [], 0
+    for r in np.nonzero(is_long)[0].tolist() + [None]:
+        end = n_tokens if r is None else int(q_start[r])
+        if end > at:
+            if ranges and at - ranges[-1][1] <= FOLD_GAP:
+                ranges[-1] = (ranges[-1][0], end)
+            else:
+                ranges.append((at, end))
+        at = end if r is None else end + int(n_new[r])
+    return tuple(ranges)
+
+
 def expanded_rows(n_new, cached, window: int, row_bytes: int):
     """Per request the position of the first key that is made for the step (a multiple of EXPAND_ALIGN), how many rows are made
     for it, and whether the request's portion is taken that way (``row_bytes`` a row; 0: none are; at most
@@ -78,6 +95,15 @@ def expanded_rows(n_new, cached, window: int, row_bytes: int):
     is_long = (n_new >= EXPAND_MIN_TOKENS) & (keys <= EXPAND_MAX_KEYS * n_new) & (row_bytes > 0)
     is_long &= np.cumsum(np.where(is_long, counts, 0)) * row_bytes <= ops.LATENT_EXPAND_BYTES
     return first, np.where(is_long, counts, 0), is_long
+
+
+class _TokenRange:
+    """Tokens a .. b - 1 of a step, as the attention of few tokens reads them."""
+
+    def __init__(self, ctx, a: int, b: int):
+        self.positions, self.token_req = ctx.positions[a:b], ctx.token_req[a:b]
+        if hasattr(ctx, "scratch"):
+            self.scratch = ctx.scratch
 
 
 @register("mixer", "latent_attention")
@@ -216,14 +242,16 @@ class LatentAttention(Mixer):
         its first key), the others into the tiles of the kernel that reads the pages."""
         none = np.zeros((0, 2), np.int32)
         if step.for_graph or step.n_tokens < PREFILL_MIN_TOKENS or int(np.max(step.n_new, initial=0)) <= 1:
-            return Plan(arrays={"tiles": none, "long": none, "rows": none}, values={"n_tiles": 0, "n_long": 0, "n_rows": 0})
+            return Plan(arrays={"tiles": none, "long": none, "rows": none},
+                        values={"n_tiles": 0, "n_long": 0, "n_rows": 0, "others": ((0, step.n_tokens),)})
         n_new, cached = np.asarray(step.n_new, np.int64), np.asarray(step.cached_len, np.int64)
         first, counts, is_long = expanded_rows(n_new, cached, self.window, self._expand_row_bytes())
         tiles = portion_tiles(step.q_start, np.where(is_long, 0, n_new), self._tile_tokens())
         long_tiles = [(r, a) for r in np.nonzero(is_long)[0].tolist() for a in range(0, int(n_new[r]), EXPAND_ALIGN)]
         rows = np.stack([np.cumsum(counts) - counts, first], axis=1).astype(np.int32)
         return Plan(arrays={"tiles": tiles, "long": np.asarray(long_tiles, np.int32).reshape(-1, 2), "rows": rows},
-                    values={"n_tiles": int(tiles.shape[0]), "n_long": len(long_tiles), "n_rows": int(counts.sum())})
+                    values={"n_tiles": int(tiles.shape[0]), "n_long": len(long_tiles), "n_rows": int(counts.sum()),
+                            "others": other_ranges(step.q_start, n_new, is_long, step.n_tokens)})
 
     def _plan_of(self, ctx):
         """The step's plan; outside the step function (a part alone) it is made here, from the device's arrays."""
@@ -263,7 +291,7 @@ class LatentAttention(Mixer):
         out = torch.empty((T, nh, self.vdim), dtype=proj.dtype, device=proj.device)
         if n_long == 0 or n_tiles:
             self._folded(q, gate, pages, cache, ctx, plan if n_tiles else None, out)
-        if n_long:      # rows of their own: what the folded form left there is overwritten
+        if n_long:      # (what the folded form left in rows of theirs between its ranges is overwritten)
             c, kr = ops.latent_gather(pages, cache.block_table, ctx, plan.arrays["rows"], plan.values["n_rows"], rank, dr,
                                       cache.page_size, self.window)
             kv = ops.gemm_bf16(c, self.w_expand)
@@ -272,27 +300,30 @@ class LatentAttention(Mixer):
         return self.o_proj.forward(out.view(T, nh * self.vdim))
 
     def _folded(self, q, gate, pages, cache, ctx, plan, out) -> None:
-        """The attention-weighted latents through the value up-projection into ``out`` [tokens, heads, vdim]."""
+        """The attention-weighted latents through the value up-projection into ``out`` [tokens, heads, vdim], for the tokens
+        that are of no long portion (``plan``; all of them without one)."""
         nh, dn, dr, rank = self.n_heads, self.dim, self.rot_dim, self.rank
         T = ctx.n_tokens
+        ranges = plan.values["others"] if plan is not None else ((0, T),)
         q3 = q.unflatten(1, (nh, dn + dr))
         qa = torch.empty((T, nh, rank), dtype=q.dtype, device=q.device)
-        ops.gemm_batched(q3[:, :, :dn], self.w_uk_t, qa)
         lat = torch.empty((T, nh, rank), dtype=q.dtype, device=q.device)
-        if plan is not None and ops.latent_attention_prefill(
+        for a, b in ranges:
+            ops.gemm_batched(q3[a:b, :, :dn], self.w_uk_t, qa[a:b])
+        if plan is None or not ops.latent_attention_prefill(
                 qa, q, gate, pages, cache.block_table, ctx, plan.arrays["tiles"], plan.values["n_tiles"], lat, nh, dn, dr, rank,
                 cache.page_size, self.window, self.scale):
-            ops.gemm_batched(lat, self.w_uv, out)
-            return
-        # Steps of few tokens cut the visible keys over several blocks. The span is what the step's shape implies (the
-        # window, else what the block table can hold), not the requests' lengths: a captured step replays it.
-        span = self.window if self.window > 0 else cache.block_table.size(1) * cache.page_size
-        splits, split_keys = ops.latent_attention_splits(
-            T, nh, span, ops.sm_count(q.device),
-            mma=T <= ops.LATENT_FEW_TOKENS and ops.latent_decode_takes_mma(q.dtype, rank, dr, cache.page_size))
-        ops.latent_attention(qa, q, gate, pages, cache.block_table, ctx, lat, nh, dn, dr, rank, cache.page_size,
-                             self.window, self.scale, splits=splits, split_keys=split_keys)
-        ops.gemm_batched(lat, self.w_uv, out)
+            # Steps of few tokens cut the visible keys over several blocks. The span is what the step's shape implies (the
+            # window, else what the block table can hold), not the requests' lengths: a captured step replays it.
+            span = self.window if self.window > 0 else cache.block_table.size(1) * cache.page_size
+            for a, b in ranges:
+                splits, split_keys = ops.latent_attention_splits(
+                    b - a, nh, span, ops.sm_count(q.device),
+                    mma=b - a <= ops.LATENT_FEW_TOKENS and ops.latent_decode_takes_mma(q.dtype, rank, dr, cache.page_size))
+                ops.latent_attention(qa[a:b], q[a:b], gate[a:b], pages, cache.block_table, _TokenRange(ctx, a, b), lat[a:b], nh, dn,
+                                     dr, rank, cache.page_size, self.window, self.scale, splits=splits, split_keys=split_keys)
+        for a, b in ranges:
+            ops.gemm_batched(lat[a:b], self.w_uv, out[a:b])
 
     @staticmethod
     def _pages(cache):

@@ -4,6 +4,7 @@ channels, shared parts of 16 to 64, windows that end inside a tile and none, por
 and single tokens in the same step, with and without the gate. Both forms round queries, keys, values or latents to bfloat16
 once each: an element may be off by some 2^-7 of the largest output."""
 import math
+import sys
 from types import SimpleNamespace
 
 import numpy as np
@@ -174,3 +175,29 @@ def test_long_portions_with_keys_made_for_the_step(dn, dr, rank, nh, window, gat
                     if int(table[r, pg]) >= 0:
                         pages[int(table[r, pg])] = float("nan")
                         table[r, pg] = -1
+
+
+@pytest.mark.parametrize("page", [16, 8])
+def test_single_tokens_between_long_portions(page, monkeypatch):
+    """The folded form takes the tokens between long portions alone (pages of 8 keys: by the kernel of few tokens); the same
+    numbers as from the folded form for all."""
+    from llm_rs_b200.parts import latent_attention as L
+    monkeypatch.setattr(sys.modules[__name__], "PAGE", page)
+    monkeypatch.setattr(L, "FOLD_GAP", 50)
+    part = _small_part(window=0)
+    n_new, cached = (1, 3, 140, 1, 40, 2, 200, 1), (30, 0, 5, 100, 9, 64, 0, 7)
+    x = torch.randn(sum(n_new), 96, generator=torch.Generator().manual_seed(6)).to(DEV, torch.bfloat16)
+    fill = torch.randn((8 * 256 // page, 1, page * 160), generator=torch.Generator().manual_seed(7)).to(DEV, torch.bfloat16)
+
+    def run():
+        ctx = _step(part, n_new, cached)
+        cache = _small_cache(8, 256 // page)
+        for plane, width, at in ((cache.planes[0], 128, 0), (cache.planes[1], 32, page * 128)):
+            plane.copy_(fill[:, :, at: at + page * width].unflatten(2, (page, width)))
+        return ctx.plans[part.plan_key()].values, part.forward(x, ctx, cache).float()
+    values, got = run()
+    assert values["n_long"] == 2 + 1 + 2 and values["others"] == ((0, 4), (144, 187), (387, 388))
+    monkeypatch.setattr(L, "EXPAND_MIN_TOKENS", 1 << 30)
+    values, want = run()
+    assert values["n_long"] == 0
+    assert float((got - want).abs().max()) <= 0.03 * float(want.abs().max())

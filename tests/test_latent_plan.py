@@ -1,0 +1,20 @@
+"""Which tokens of a step latent attention takes which way (parts/latent_attention.py): plans, made on the host."""
+import numpy as np
+import pytest
+
+
+def _ranges(lens, longs):
+    from llm_rs_b200.parts.latent_attention import other_ranges
+    n_new = np.asarray(lens, np.int64)
+    q_start = np.concatenate([[0], np.cumsum(n_new)[:-1]])
+    return other_ranges(q_start, n_new, np.asarray(longs, bool), int(n_new.sum()))
+
+
+@pytest.mark.parametrize("lens,longs,want", [
+    ([5], [0], ((0, 5),)), ([300], [1], ()), ([1] * 8 + [1700], [0] * 8 + [1], ((0, 8),)), ([1700] + [1] * 8, [1] + [0] * 8, ((1700, 1708),)),
+    ([3, 1000, 4, 2000, 5], [0, 1, 0, 1, 0], ((0, 3), (1003, 1007), (3007, 3012))),
+    ([3, 100, 4, 2000, 5], [0, 1, 0, 1, 0], ((0, 107), (2107, 2112))),      # a short gap is taken along
+    ([400, 500, 0, 7], [1, 1, 0, 0], ((900, 907),)), ([400, 0, 500], [1, 0, 1], ())])
+def test_tokens_of_no_long_portion(lens, longs, want):
+    """The folded form's products run over these tokens only: not over a long portion's, which has its own."""
+    assert _ranges(lens, longs) == want
