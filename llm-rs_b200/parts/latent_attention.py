@@ -93,7 +93,11 @@ def expanded_rows(n_new, cached, window: int, row_bytes: int):
     keys = cached + n_new - first
     counts = -(-keys // EXPAND_ALIGN) * EXPAND_ALIGN
     is_long = (n_new >= EXPAND_MIN_TOKENS) & (keys <= EXPAND_MAX_KEYS * n_new) & (row_bytes > 0)
-    is_long &= np.cumsum(np.where(is_long, counts, 0)) * row_bytes <= ops.LATENT_EXPAND_BYTES
+    room = ops.LATENT_EXPAND_BYTES
+    for r in np.nonzero(is_long)[0].tolist():      # one that does not fit leaves the room to those behind it
+        need = int(counts[r]) * row_bytes
+        is_long[r] = need <= room
+        room -= need if need <= room else 0
     return first, np.where(is_long, counts, 0), is_long
 
 

@@ -18,3 +18,15 @@ def _ranges(lens, longs):
 def test_tokens_of_no_long_portion(lens, longs, want):
     """The folded form's products run over these tokens only: not over a long portion's, which has its own."""
     assert _ranges(lens, longs) == want
+
+
+def test_a_portion_that_does_not_fit_leaves_the_room_to_others(monkeypatch):
+    from llm_rs_b200 import ops
+    from llm_rs_b200.parts.latent_attention import expanded_rows
+    monkeypatch.setattr(ops, "LATENT_EXPAND_BYTES", 1024 * 100)
+    n_new, cached = np.array([500, 2000, 128, 300], np.int64), np.zeros(4, np.int64)
+    first, counts, is_long = expanded_rows(n_new, cached, 0, 100)
+    assert is_long.tolist() == [True, False, True, True]
+    assert counts.tolist() == [512, 0, 128, 384] and first.tolist() == [0, 0, 0, 0]
+    monkeypatch.setattr(ops, "LATENT_EXPAND_BYTES", 1024 * 100 - 1)
+    assert expanded_rows(n_new, cached, 0, 100)[2].tolist() == [True, False, True, False]
