@@ -26,7 +26,11 @@ PREFILL_MIN_TOKENS = 32
 # 16 heads, a whole mixer, folded against made (us): 2,000 tokens through a window of 1,024 799 / 133; 64 tokens after 4,096
 # 793 / 119, after 8,000 1,486 / 187; 32 after 2,048 418 / 77, after 256 98 / 55. Fewer tokens over more keys were not
 # measured and stay folded.
-EXPAND_MIN_TOKENS, EXPAND_MAX_KEYS = 32, 128
+# A step with other tokens runs the folded kernel all the same, which takes a few tokens more along for little: there the long
+# portions need EXPAND_BESIDE tokens together. Single tokens after 900 keys + a portion after 800, folded together / the portion
+# apart (us): 1 + 64 197 / 216, 63 + 64 240 / 282, 1 + 128 205 / 225, 1 + 256 228 / 238, 8 + 256 276 / 242, 1 + 512 284 / 253,
+# 63 + 512 502 / 312.
+EXPAND_MIN_TOKENS, EXPAND_MAX_KEYS, EXPAND_BESIDE = 32, 128, 320
 EXPAND_ALIGN = 128      # keys per tile of that kernel
 # Tokens of long portions between two runs of other tokens that the folded form's products take along: fewer cost less than
 # another launch of each of the two products.
@@ -98,6 +102,8 @@ def expanded_rows(n_new, cached, window: int, row_bytes: int):
         need = int(counts[r]) * row_bytes
         is_long[r] = need <= room
         room -= need if need <= room else 0
+    if ((n_new > 0) & ~is_long).any() and int(n_new[is_long].sum()) < EXPAND_BESIDE:
+        is_long[:] = False
     return first, np.where(is_long, counts, 0), is_long
 
 

@@ -129,9 +129,10 @@ def test_a_key_that_is_not_finite_reaches_its_queries_only(window, n, cached, at
     (128, 64, 512, 8, 0, True, [(300, 64), (129, 1), (70, 200)]), (64, 32, 128, 8, 100, True, [(128, 90), (257, 64), (64, 13)]),
     (128, 16, 64, 5, 257, False, [(65, 700), (200, 127)]), (64, 64, 256, 16, 1024, True, [(1200, 1), (333, 1)]),
     (128, 48, 192, 8, 1, True, [(130, 66), (64, 64)]), (128, 64, 512, 16, 128, True, [(255, 256, 1, 40, 64)])])
-def test_long_portions_with_keys_made_for_the_step(dn, dr, rank, nh, window, gated, cuts):
+def test_long_portions_with_keys_made_for_the_step(dn, dr, rank, nh, window, gated, cuts, monkeypatch):
     from llm_rs_b200.parts import Runtime
     from llm_rs_b200.parts import latent_attention as L
+    monkeypatch.setattr(L, "EXPAND_BESIDE", 0)      # also beside other tokens
     g = torch.Generator().manual_seed(dn + dr + nh)
     D = 96
     part = L.LatentAttention(D, nh, dn, dr, 128, rank, (dn + dr) ** -0.5, 900.0, window=window, gated=gated, prefix="m.")

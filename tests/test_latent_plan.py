@@ -30,3 +30,11 @@ def test_a_portion_that_does_not_fit_leaves_the_room_to_others(monkeypatch):
     assert counts.tolist() == [512, 0, 128, 384] and first.tolist() == [0, 0, 0, 0]
     monkeypatch.setattr(ops, "LATENT_EXPAND_BYTES", 1024 * 100 - 1)
     assert expanded_rows(n_new, cached, 0, 100)[2].tolist() == [True, False, True, False]
+
+
+@pytest.mark.parametrize("n_new,want", [([64], [1]), ([64, 64], [1, 1]), ([1] * 63 + [64], [0] * 64), ([1, 319], [0, 0]), ([1, 320], [0, 1]),
+                                        ([200, 1, 120], [1, 0, 1]), ([200, 1, 119], [0, 0, 0]), ([64, 0], [1, 0]), ([20, 64], [0, 0])])
+def test_portions_beside_other_tokens_need_more_of_them(n_new, want):
+    from llm_rs_b200.parts.latent_attention import expanded_rows
+    n_new = np.asarray(n_new, np.int64)
+    assert expanded_rows(n_new, np.zeros_like(n_new), 0, 100)[2].tolist() == [bool(w) for w in want]
