@@ -204,7 +204,7 @@ __global__ void __launch_bounds__(WALK_THREADS, 2) state_walk_kernel(WalkArgs p,
   const int col0 = blockIdx.x % col_blocks * WALK_COLS, tid = threadIdx.x;
   const int part = tid % WALK_LANES, c0 = tid / WALK_LANES * 2, col = col0 + c0;      // this thread's columns: col, col + 1
   const int n = p.n_new[req], t0 = p.q_start[req], d = p.d, dv = p.dv, kh = head / (p.n_heads / p.n_groups);
-  if (n < p.from) return;
+  if (n <= 0 || n < p.from) return;
   const size_t slot = (size_t)p.slot_ids[req];
   float* S_g = p.state + (slot * p.n_heads + head) * (size_t)d * dv;
   float* N_g = p.norm_state ? p.norm_state + (slot * p.n_heads + head) * (size_t)d : nullptr;
