@@ -468,7 +468,7 @@ LLMRS_API int llmrs_scored_prepare(void* q, long long q_stride, const void* k, l
   const int threads = n_q_heads * dk >= 2048 ? 512 : 256;
 #define LLMRS_SP_LAUNCH(T)                                                                                          \
   do {                                                                                                              \
-    static size_t configured = 48 * 1024;                                                                           \
+    static size_t configured = 40 * 1024;                                                                           \
     if (smem > configured) {                                                                                        \
       cudaError_t e = cudaFuncSetAttribute(scored_prepare_kernel<T>, cudaFuncAttributeMaxDynamicSharedMemorySize,   \
                                            (int)smem);                                                              \

@@ -276,12 +276,13 @@ LLMRS_API int llmrs_gemm_f32_skinny(const void* x, int x_dtype, long long x_stri
   if (M == 0) return 0;
   const size_t smem = (size_t)SK_TOKENS * K * (x_dtype == LLMRS_F32 ? 4 : 2);
   LLMRS_REQUIRE(smem <= 200 * 1024, "gemm_f32_skinny: rows of %d values are too long", K);
+  // (48 KB need no asking, but the kernel's own `parts` counts too: eight rows of 1,536 floats are 48 KB by themselves.)
   const bool split = M <= 4 * SK_TOKENS;       // few rows: a block per feature
   dim3 grid((M + SK_TOKENS - 1) / SK_TOKENS, split ? N : (N + SK_WARPS - 1) / SK_WARPS);
   LLMRS_REQUIRE(grid.y <= 65535, "gemm_f32_skinny: N=%d is too large", N);
 #define LLMRS_SK_LAUNCH(T, S)                                                                                         \
   do {                                                                                                                \
-    static size_t configured = 48 * 1024;                                                                             \
+    static size_t configured = 40 * 1024;                                                                             \
     if (smem > configured) {                                                                                          \
       cudaError_t e = cudaFuncSetAttribute(gemm_f32_skinny_kernel<T, S>, cudaFuncAttributeMaxDynamicSharedMemorySize, \
                                            (int)smem);                                                                \

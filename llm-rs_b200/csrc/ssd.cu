@@ -107,7 +107,7 @@ LLMRS_API int llmrs_ssd_output(const float* y, const void* z, long long z_stride
   const int threads = inner >= 2048 ? 512 : (inner >= 512 ? 256 : 128);
 #define LLMRS_SSD_OUTPUT(T)                                                                                            \
   do {                                                                                                                 \
-    static size_t configured = 48 * 1024;                                                                              \
+    static size_t configured = 40 * 1024;                                                                              \
     if (smem > configured) {                                                                                           \
       cudaError_t e = cudaFuncSetAttribute(ssd_output_kernel<T>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem); \
       if (e != cudaSuccess) return llmrs_fail("ssd_output: shared memory %zu: %s", smem, cudaGetErrorString(e));       \

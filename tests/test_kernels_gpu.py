@@ -975,3 +975,15 @@ def test_sampler_of_two_threads_with_different_vocabularies():
     for t in threads:
         t.join()
     assert not failed, failed[:2]
+
+
+@pytest.mark.parametrize("dtype,K", [(torch.float32, 1536), (torch.bfloat16, 3072), (torch.float32, 1532), (torch.float32, 1540)])
+@pytest.mark.parametrize("M", [1, 40])
+def test_gemm_f32_few_features_at_48_kilobytes_of_rows(M, K, dtype):
+    """Eight rows of 1,536 floats fill what a kernel may have without asking, and the kernel has some of its own."""
+    ops = _ops()
+    torch.manual_seed(K)
+    x, w = torch.randn(M, K, device=DEV).to(dtype), torch.randn(65, K, device=DEV)
+    want = x.double() @ w.double().t()
+    bound = x.double().abs() @ w.double().abs().t() * K * 2.0 ** -24
+    assert bool(((ops.gemm_f32(x, w).double() - want).abs() <= bound).all())

@@ -132,3 +132,17 @@ def test_prepare_by_pieces_is_the_general_kernel(dk, dv, rot, pairs, norm, n, kv
         got.append((q.float(), cache.float()))
     for a, b in zip(*got):
         assert bool(((a - b).abs() <= 2.0 ** -7 * a.abs() + 1e-5).all())
+
+
+def test_prepare_of_rows_of_48_kilobytes():
+    """The general kernel's rows fill what a kernel may have without asking, beside a reduction of its own."""
+    from llm_rs_b200 import ops
+    heads, kv, d, page = 88, 8, 128, 16
+    q, k, v = (torch.randn(3, h * d, device=DEV) for h in (heads, kv, kv))
+    i32 = lambda x: torch.tensor(x, dtype=torch.int32, device=DEV)
+    ctx = SimpleNamespace(positions=i32([0, 1, 2]), token_req=i32([0] * 3))
+    cache = torch.zeros(1, kv, page * 2 * d, device=DEV)
+    q0 = q.clone()
+    ops.scored_prepare(q, k, v, None, None, torch.zeros(0, dtype=torch.float64, device=DEV), ctx, i32([[0]]), cache, heads, kv, d, d, 0,
+                       page, 1e-6)
+    assert torch.equal(q, q0) and torch.equal(cache[0, :, : 3 * d], k.view(3, kv, d).transpose(0, 1).flatten(1))
