@@ -49,13 +49,29 @@ gemm_f32_kernel(const TX* __restrict__ x, const float* __restrict__ w, const flo
         else cp_async_8(xd + r * XS + c, src, in ? 8 : 0);
       }
     } else {
-      for (int e = tid; e < BN * BK; e += THREADS) {
-        const int r = e / BK, c = e % BK;
-        wd[r * WS + c] = (n0 + r < N && k0 + c < K) ? w[(size_t)(n0 + r) * K + k0 + c] : 0.f;
-      }
-      for (int e = tid; e < BM * BK; e += THREADS) {
-        const int r = e / BK, c = e % BK;
-        xd[r * XS + c] = (m0 + r < M && k0 + c < K) ? x[(size_t)(m0 + r) * x_stride + k0 + c] : TX(0.f);
+      // Value by value: a thread keeps to a column (to every THREADS-th of a wide step) and goes down the rows, so that an address
+      // is one addition (1,000 rows of 1,023 into 1,024 features 72 us; 141 with an address and plain loads a value, 94 by the
+      // kernel before; 2,050 into 2,048 276, 523 and 367).
+      constexpr int COLS = BK < THREADS ? BK : THREADS, PASS = THREADS / COLS;
+#pragma unroll
+      for (int c0 = 0; c0 < BK; c0 += COLS) {
+        const int c = c0 + tid % COLS, r0 = tid / COLS;
+        const bool k_in = k0 + c < K;
+        const float* wp = w + (size_t)(n0 + r0) * K + k0 + c;
+#pragma unroll
+        for (int r = 0; r < BN; r += PASS, wp += (size_t)PASS * K) {
+          const bool in = k_in && n0 + r0 + r < N;
+          if (BN % PASS == 0 || r0 + r < BN) cp_async_4(wd + (r0 + r) * WS + c, in ? wp : w, in ? 4 : 0);
+        }
+        const TX* xp = x + (size_t)(m0 + r0) * x_stride + k0 + c;
+#pragma unroll
+        for (int r = 0; r < BM; r += PASS, xp += PASS * x_stride) {
+          const bool in = k_in && m0 + r0 + r < M;
+          if (BM % PASS == 0 || r0 + r < BM) {
+            if constexpr (sizeof(TX) == 4) cp_async_4(xd + (r0 + r) * XS + c, in ? xp : x, in ? 4 : 0);
+            else xd[(r0 + r) * XS + c] = in ? *xp : TX(0.f);      // (no asynchronous copy has two bytes)
+          }
+        }
       }
     }
     cp_async_commit();
