@@ -800,14 +800,26 @@ def tanh_slice(x: torch.Tensor, out_dtype: torch.dtype) -> torch.Tensor:
 
 
 # -- many small products in one launch ----------------------------------------------------------------
-GROUPED_TILE_ROWS = 64      # rows of a tile of the grouped product; 128 where groups have a few rows (``grouped_tile_rows``)
+GROUPED_TILE_ROWS = 64      # rows of a tile of the grouped product; 128 where groups have many rows (``grouped_tile_rows``)
+# (millions of weights in a product's groups, rows a group from which on tiles of 128 rows are ahead)
+_GROUPED_LINES = ((64, 4), (48, 16), (16, 56), (8, 160), (0, 512))
 
 
-def grouped_tile_rows(n_rows: int, n_groups: int) -> int:
-    """Rows per tile for ``moe_sort`` and ``gemm_grouped``: 128 (the tcgen05 kernel for bfloat16) from two rows a group on, else
-    64 (mma.sync). 32 experts of 1,024 at width 2,048, both products, 64 against 128 rows a tile (us): half a row a group 65 / 72,
-    one 90 / 103, two 122 / 107, eight 123 / 107, 64 164 / 112, 256 482 / 196."""
-    return 128 if n_rows >= 2 * n_groups else GROUPED_TILE_ROWS
+def grouped_tile_rows(n_rows: int, n_groups: int, weights: Optional[int] = None) -> int:
+    """Rows per tile for ``moe_sort`` and ``gemm_grouped``: 128 (the tcgen05 kernel for bfloat16) or 64 (mma.sync). ``weights``:
+    numbers in one product's weights, all groups together. The tcgen05 kernel's tiles of 128 x 256 take some 40 us for both of an
+    expert's products however small they are, and leave multiprocessors idle where the weights make few of them; tiles of 64 rows
+    read the weights again from the second tile of a group on. Both products, 64 against 128 rows a tile (us), by rows a group:
+      67 M weights (32 of 1,024 x 2,048)  2 87 / 102   4 107 / 105   16 110 / 98   64 172 / 106   256 451 / 170
+      50 M (32 of 1,024 x 1,536)          4 84 / 96   16 87 / 86   64 127 / 94
+      33 M (16 of 1,024 x 2,048)          16 59 / 70   48 65 / 73   64 96 / 73   128 147 / 93
+      9 M (8 of 768 x 1,536)              32 31 / 47   96 51 / 52   128 52 / 55   256 83 / 60
+      4 M (8 of 512 x 1,024)              64 25 / 43   256 39 / 46
+    The two kernels add the same products in float32, in orders of their own: a row's last bits change where the step's rows cross
+    the line."""
+    millions = 64 if weights is None else weights / 1e6
+    line = next(rows for least, rows in _GROUPED_LINES if millions >= least)
+    return 128 if n_rows >= line * n_groups else GROUPED_TILE_ROWS
 
 
 def _strides3(t: torch.Tensor, name: str):

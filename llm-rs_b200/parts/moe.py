@@ -172,7 +172,7 @@ class MixtureOfExperts(FeedForward):
             expert_of, weight_of = ops.moe_route_biased(logits, self.correction, self.n_experts + self.n_identity,
                                                         self.n_experts, self.top)
         n_rows = expert_of.numel()
-        tile_rows = ops.grouped_tile_rows(n_rows, self.n_experts)
+        tile_rows = ops.grouped_tile_rows(n_rows, self.n_experts, self.w_gate.numel())
         if self.n_identity:
             # Assignments to identity experts are sorted into one more group that runs no product; the weighted sum
             # takes the token's own row for them.
