@@ -30,7 +30,9 @@ PREFILL_MIN_TOKENS = 32
 # portions need EXPAND_BESIDE tokens together. Single tokens after 900 keys + a portion after 800, folded together / the portion
 # apart (us): 1 + 64 197 / 216, 63 + 64 240 / 282, 1 + 128 205 / 225, 1 + 256 228 / 238, 8 + 256 276 / 242, 1 + 512 284 / 253,
 # 63 + 512 502 / 312.
-EXPAND_MIN_TOKENS, EXPAND_MAX_KEYS, EXPAND_BESIDE = 32, 128, 320
+# A portion over fewer than EXPAND_MIN_KEYS keys is folded at no more cost: heads of 64 + 32, a latent of 256, 40 tokens after none
+# 45 / 49, 64 after none 50 / 50, 32 after 256 82 / 51; heads of 128 + 64, a latent of 512, 32 after none 50 / 50.
+EXPAND_MIN_TOKENS, EXPAND_MIN_KEYS, EXPAND_MAX_KEYS, EXPAND_BESIDE = 32, 64, 128, 320
 EXPAND_ALIGN = 128      # keys per tile of that kernel
 # Tokens of long portions between two runs of other tokens that the folded form's products take along: fewer cost less than
 # another launch of each of the two products.
@@ -96,7 +98,7 @@ def expanded_rows(n_new, cached, window: int, row_bytes: int):
     first = lo // EXPAND_ALIGN * EXPAND_ALIGN
     keys = cached + n_new - first
     counts = -(-keys // EXPAND_ALIGN) * EXPAND_ALIGN
-    is_long = (n_new >= EXPAND_MIN_TOKENS) & (keys <= EXPAND_MAX_KEYS * n_new) & (row_bytes > 0)
+    is_long = (n_new >= EXPAND_MIN_TOKENS) & (keys >= EXPAND_MIN_KEYS) & (keys <= EXPAND_MAX_KEYS * n_new) & (row_bytes > 0)
     room = ops.LATENT_EXPAND_BYTES
     for r in np.nonzero(is_long)[0].tolist():      # one that does not fit leaves the room to those behind it
         need = int(counts[r]) * row_bytes

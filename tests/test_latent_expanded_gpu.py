@@ -82,7 +82,7 @@ def _small_cache(n_requests, n_pages):
 
 
 @pytest.mark.parametrize("bad", [float("inf"), float("-inf"), float("nan")])
-@pytest.mark.parametrize("lens", [(40, 50), (130, 64), (128, 33), (200, 255)])
+@pytest.mark.parametrize("lens", [(64, 70), (130, 64), (128, 81), (200, 255)])
 def test_a_neighbours_numbers_do_not_reach_a_request(lens, bad):
     """Both requests' keys are made for the step: what the second one holds must not change a bit of the first one's output."""
     part = _small_part(window=0)
@@ -132,7 +132,8 @@ def test_a_key_that_is_not_finite_reaches_its_queries_only(window, n, cached, at
 def test_long_portions_with_keys_made_for_the_step(dn, dr, rank, nh, window, gated, cuts, monkeypatch):
     from llm_rs_b200.parts import Runtime
     from llm_rs_b200.parts import latent_attention as L
-    monkeypatch.setattr(L, "EXPAND_BESIDE", 0)      # also beside other tokens
+    monkeypatch.setattr(L, "EXPAND_BESIDE", 0)      # also beside other tokens, and over few keys
+    monkeypatch.setattr(L, "EXPAND_MIN_KEYS", 0)
     g = torch.Generator().manual_seed(dn + dr + nh)
     D = 96
     part = L.LatentAttention(D, nh, dn, dr, 128, rank, (dn + dr) ** -0.5, 900.0, window=window, gated=gated, prefix="m.")
@@ -186,7 +187,7 @@ def test_single_tokens_between_long_portions(page, monkeypatch):
     monkeypatch.setattr(sys.modules[__name__], "PAGE", page)
     monkeypatch.setattr(L, "FOLD_GAP", 50)
     part = _small_part(window=0)
-    n_new, cached = (1, 3, 140, 1, 40, 2, 200, 1), (30, 0, 5, 100, 9, 64, 0, 7)
+    n_new, cached = (1, 3, 140, 1, 40, 2, 200, 1), (30, 0, 5, 100, 30, 64, 0, 7)
     x = torch.randn(sum(n_new), 96, generator=torch.Generator().manual_seed(6)).to(DEV, torch.bfloat16)
     fill = torch.randn((8 * 256 // page, 1, page * 160), generator=torch.Generator().manual_seed(7)).to(DEV, torch.bfloat16)
 

@@ -38,3 +38,10 @@ def test_portions_beside_other_tokens_need_more_of_them(n_new, want):
     from llm_rs_b200.parts.latent_attention import expanded_rows
     n_new = np.asarray(n_new, np.int64)
     assert expanded_rows(n_new, np.zeros_like(n_new), 0, 100)[2].tolist() == [bool(w) for w in want]
+
+
+@pytest.mark.parametrize("n_new,cached,window,want", [(63, 0, 0, False), (64, 0, 0, True), (32, 32, 0, True), (32, 31, 0, False),
+                                                      (40, 1000, 8, True), (31, 500, 0, False)])
+def test_portions_over_few_keys_stay_folded(n_new, cached, window, want):
+    from llm_rs_b200.parts.latent_attention import expanded_rows
+    assert expanded_rows(np.array([n_new]), np.array([cached]), window, 100)[2].tolist() == [want]
