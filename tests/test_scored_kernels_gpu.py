@@ -97,12 +97,28 @@ def test_decode_keeps_infinite_values(generic):
     assert torch.equal(before[rest], after[rest])
 
 
+def _prepared(x, heads, dk, norm, weight, inv_freq, positions, rot, pairs):
+    """Heads normed and rotated in float64 by the definition."""
+    x = x.double().view(-1, heads, dk)
+    if norm == "whole":
+        x = x / torch.sqrt((x ** 2).mean((1, 2), keepdim=True) + 1e-6) * weight.double().view(heads, dk)
+    elif norm in ("unit", "shared"):
+        x = x / torch.sqrt((x ** 2).mean(2, keepdim=True) + 1e-6) * (weight.double() if norm == "shared" else 1.0)
+    angle = (positions.double()[:, None] * inv_freq)[:, None]
+    turned = x[..., :rot].unflatten(2, (rot // 2, 2)).transpose(2, 3) if pairs else x[..., :rot].unflatten(2, (2, rot // 2))
+    a, b = turned[:, :, 0], turned[:, :, 1]
+    turned = torch.stack([a * angle.cos() - b * angle.sin(), b * angle.cos() + a * angle.sin()], 2)
+    turned = (turned.transpose(2, 3) if pairs else turned).flatten(2)
+    return torch.cat([turned, x[..., rot:]], 2)
+
+
 @pytest.mark.parametrize("dk,dv,rot,pairs", [(128, 128, 128, False), (64, 64, 32, False), (128, 64, 64, True), (96, 72, 96, False),
                                              (64, 64, 12, True), (64, 64, 0, False), (16, 8, 16, False), (512, 64, 64, False)])
 @pytest.mark.parametrize("norm", ["none", "whole", "unit", "shared"])
 @pytest.mark.parametrize("n,kv", [(1, 2), (597, 1), (7, 0)])
 def test_prepare_by_pieces_is_the_general_kernel(dk, dv, rot, pairs, norm, n, kv):
-    """Both kernels compute in float32 and round once: they differ by one bfloat16 rounding at most."""
+    """Both kernels compute in float32 and round once: each is within one bfloat16 rounding (2^-9 of the number, and float32's
+    error beside it) of the definition in float64, they differ by two at most, and values are copied."""
     from llm_rs_b200 import ops
     torch.manual_seed(dk + rot + n)
     heads, page = 4, 16
@@ -132,6 +148,16 @@ def test_prepare_by_pieces_is_the_general_kernel(dk, dv, rot, pairs, norm, n, kv
         got.append((q.float(), cache.float()))
     for a, b in zip(*got):
         assert bool(((a - b).abs() <= 2.0 ** -7 * a.abs() + 1e-5).all())
+    want = lambda x, h, w: _prepared(x, h, dk, norm, w, inv_freq, ctx.positions, rot, pairs)
+    close = lambda a, b: bool(((a.double() - b).abs() <= 2.0 ** -8 * b.abs() + 1e-5).all())
+    want_q = want(q0[:, : heads * dk], heads, wq).flatten(1)
+    page_of, slot = table[0, ctx.positions.long() // page].long(), ctx.positions.long() % page
+    for q, cache in got:
+        assert close(q, want_q)
+        if kv:
+            keys = cache[:, :, : page * dk].unflatten(2, (page, dk))[page_of, :, slot]
+            values = cache[:, :, page * dk:].unflatten(2, (page, dv))[page_of, :, slot]
+            assert close(keys, want(k, kvh, wk)) and torch.equal(values.flatten(1), v.float())
 
 
 def test_prepare_of_rows_of_48_kilobytes():
