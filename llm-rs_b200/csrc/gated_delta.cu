@@ -244,8 +244,7 @@ gdr_recurrence_kernel(const float* __restrict__ pq, const float* __restrict__ pk
 // registers), makes them unit vectors and, for every value head that shares them, the coefficients between the tokens. With a
 // decay per key channel it leaves the rows with their decays instead (qf, kf from the turn's start up to and with the token,
 // kb from the token to the turn's end) and the whole turn's decay. Products of decays, no quotients: nothing overflows.
-// Bound by issue (some 1,700 instructions a warp, half of them SiLU's divisions and exponentials; six blocks an SM: 51 us, four:
-// 58). 2,048 tokens of 16 heads over 8 of 128 x 128: 51 us, where preparing the rows (a block a token, the
+// Six blocks an SM take 51 us, four 58. 2,048 tokens of 16 heads over 8 of 128 x 128: 51 us, where preparing the rows (a block a token, the
 // convolution a channel at a time) and their coefficients by two kernels took 68 + 13.
 template <int CPL, typename TA>
 __device__ __forceinline__ void gdr_convolve(const TA* __restrict__ x, long long stride, size_t t_req, int first, int have,

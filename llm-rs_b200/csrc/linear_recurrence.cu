@@ -93,7 +93,8 @@ __global__ void gate_scan_kernel(const float* __restrict__ gates, long long stri
 // A run's steps compose to one step of the recurrence (F, I); those are scanned over the block, and each thread then walks its
 // run from the maximum that it starts with. One warp, 32 tokens at a time, waits for a chain of shuffles and for memory in each
 // of its turns: 1,311 tokens of 16 heads 40 us, in runs 8.5. Shorter requests of the step take a warp a head here too, eight
-// heads a block, the other blocks of theirs leave at once (with a block a head 257 requests, one of 128 tokens: 22 us).
+// heads a block, the other blocks of theirs leave at once (257 requests, one of 128 tokens: 9.5 us, 22 with a block a head, 5.6
+// by warps alone; 64 requests, one of 512: 6.5, 15.7 by warps alone).
 // One portion by a warp / in runs, us: 96 tokens 4.3 / 4.9, 128 5.2 / 5.0, 192 6.9 / 5.1, 512 15.5 / 5.7.
 constexpr int GS_RUN = 8, GS_THREADS = 256, GS_PORTION = 128;
 __global__ void __launch_bounds__(GS_THREADS)

@@ -585,9 +585,12 @@ sample_spread_kernel(const float* __restrict__ logits, int vocab, const float* _
   cluster.sync();      // no block leaves while its values may be read
 }
 
-// Eight blocks a row while all rows' clusters run at once, two blocks a multiprocessor, and a row is long enough to pay for the
-// clusters' barriers; a row must fit the shared memory of its blocks. A block a row against eight, us: 32 rows of 151,936
-// 117 / 71, 8 rows 113 / 51, one 94 / 35; 64 rows 118 / 132; 32 rows of 32,000 39 / 46, 8 rows 39 / 36.
+// Eight blocks a row where that is faster, and a row is long enough to pay for the clusters' barriers; a row must fit the shared
+// memory of its blocks. A block a row against eight, us: 32 rows of 151,936 117 / 71, 8 rows 113 / 51, one 94 / 35; 64 rows
+// 118 / 132; 32 rows of 32,000 39 / 46, 8 rows 39 / 36. Up to some 170,000 numbers a row two blocks fit a multiprocessor and the
+// clusters of 32 rows run at once; longer rows leave room for one, and those of more than 18 rows run in two waves, still ahead
+// (whole calls of the sampler): 32 rows of 200,064 157 / 136, of 256,000 195 / 150, of 340,992 245 / 188; 24 rows of 200,064
+// 156 / 101.
 constexpr int SS_MAX_ROWS = 32, SS_MIN_CHUNK = 64, SS_MAX_CHUNK = 340;
 constexpr size_t ss_smem(int chunk) { return (size_t)(SS_RUNS + 1) * chunk * sizeof(float); }
 
