@@ -26,6 +26,8 @@
 //                multiplies by a weight (or none) and by sigmoid(gate) or SiLU(gate), rounds to the activation type.
 #include <limits.h>
 
+#include <type_traits>
+
 #include "common.cuh"
 #include "head_out.cuh"
 #include "mma_util.cuh"
@@ -270,7 +272,9 @@ constexpr int LR_COLS = 16;
 
 // LR_LANES adjacent lanes share a column: 4 for heads of up to 64 key channels, 8 above (16 and 32 channels per lane
 // instead of 32 and 64: shorter chains of dependent sums per token, and twice the warps on an SM that holds few blocks).
-template <int DMAX, int LR_LANES>
+// SOME: only requests of fewer than `below` tokens, the others are walked in turns. (A template: with the test in it a decode step
+// of 48 requests of Mamba-2 took 84 us instead of 79.)
+template <int DMAX, int LR_LANES, bool SOME>
 __global__ void __launch_bounds__(LR_COLS * LR_LANES)
 linear_recurrence_kernel(const float* __restrict__ Q, const float* __restrict__ K, const float* __restrict__ V,
                          const float* __restrict__ decay, const float* __restrict__ head_decay,
@@ -294,7 +298,7 @@ linear_recurrence_kernel(const float* __restrict__ Q, const float* __restrict__ 
   const int n_cols = dv + (N_all != nullptr ? 1 : 0);      // the normaliser is one more column, whose value is 1
   const bool live = col < n_cols, is_norm = col == dv;
   const int t0 = q_start[req], n = n_new[req];
-  if (n >= below) return;      // walked in turns
+  if (SOME && n >= below) return;
   const int wk = n_groups * dk, wv = n_heads * dv, group = head / (n_heads / n_groups);
   const size_t slot = (size_t)slot_ids[req];
   float* S_g = S_all + (slot * n_heads + head) * (size_t)dk * dv;
@@ -432,13 +436,18 @@ LLMRS_API int llmrs_linear_recurrence_planes(const float* Q, const float* K, con
   const int below = walk_from > 0 ? walk_from : INT_MAX;
   dim3 grid(n_requests, n_heads, (cols + LR_COLS - 1) / LR_COLS);
 #define LLMRS_LR_LAUNCH(D, L)                                                                                     \
-  linear_recurrence_kernel<D, L><<<grid, LR_COLS * L, 0, stream>>>(Q, K, V, decay, head_decay, v_gain, skip, S, N, \
-                                                                   q_start, n_new, slot_ids, o_raw, nq, n_heads,  \
-                                                                   n_groups, dk, dv, below)
-  if (dk <= 32) LLMRS_LR_LAUNCH(32, 4);
-  else if (dk <= 64) LLMRS_LR_LAUNCH(64, 4);
-  else if (dk <= 128) LLMRS_LR_LAUNCH(128, 8);
-  else LLMRS_LR_LAUNCH(256, 8);
+  linear_recurrence_kernel<D, L, SOME><<<grid, LR_COLS * L, 0, stream>>>(Q, K, V, decay, head_decay, v_gain, skip, S, N, \
+                                                                         q_start, n_new, slot_ids, o_raw, nq, n_heads,  \
+                                                                         n_groups, dk, dv, below)
+  auto launch = [&](auto some) {
+    constexpr bool SOME = decltype(some)::value;
+    if (dk <= 32) LLMRS_LR_LAUNCH(32, 4);
+    else if (dk <= 64) LLMRS_LR_LAUNCH(64, 4);
+    else if (dk <= 128) LLMRS_LR_LAUNCH(128, 8);
+    else LLMRS_LR_LAUNCH(256, 8);
+  };
+  if (walk_from > 0) launch(std::true_type());
+  else launch(std::false_type());
 #undef LLMRS_LR_LAUNCH
   return llmrs_launch_status("linear_recurrence");
 }
