@@ -106,7 +106,9 @@ constexpr int GD_WIDE_MAX_BLOCKS = 296;
 
 // LANES: neighbouring lanes that share a column (4, 8 or 16; at most DMAX / 4, so that a lane holds whole pieces of
 // four channels). CHANNEL: pg holds a decay per key channel, [tokens, H d], which travels like q and k.
-template <int DMAX, int LANES, bool CHANNEL>
+// SOME: only requests of fewer than `below` tokens, the others are walked in turns (a template: the test alone cost decode steps
+// of 200 requests 2 %).
+template <int DMAX, int LANES, bool CHANNEL, bool SOME>
 __global__ void __launch_bounds__(GD_COLS * LANES)
 gdr_recurrence_kernel(const float* __restrict__ pq, const float* __restrict__ pk, const float* __restrict__ pv,
                       const float* __restrict__ pbeta, const float* __restrict__ pg, float* __restrict__ state,
@@ -130,7 +132,7 @@ gdr_recurrence_kernel(const float* __restrict__ pq, const float* __restrict__ pk
   auto ch = [&](int i) { return ((i >> 2) * GD_LANES + part) * 4 + (i & 3); };
   const bool live = col < dv;
   const int t0 = q_start[req], n = n_new[req];
-  if (n >= below) return;      // walked in turns
+  if (SOME && n >= below) return;
   const int wq = G * d, wv = H * dv;
   float* S_g = state + ((size_t)slot_ids[req] * H + head) * d * dv;
   float S[IPL];
@@ -829,8 +831,14 @@ LLMRS_API int llmrs_gated_delta(const void* x, long long x_stride, const void* g
   head.out = out; head.out_stride = out_stride; head.n_tokens = n_tokens; head.n_heads = H; head.dv = dv;
   head.eps = norm_eps; head.out_scale = out_scale; head.silu = !gate_sigmoid;
 #define LLMRS_GD_REC(DMAX, LANES, CH)                                                                             \
-  gdr_recurrence_kernel<DMAX, LANES, CH><<<grid, GD_COLS * LANES, 0, stream>>>(pq, pk, pv, pbeta, pg, state, q_start, \
-                                                                               n_new, slot_ids, o_raw, G, H, d, dv, below)
+  do {                                                                                                           \
+    if (from > 0)                                                                                                \
+      gdr_recurrence_kernel<DMAX, LANES, CH, true><<<grid, GD_COLS * LANES, 0, stream>>>(                        \
+          pq, pk, pv, pbeta, pg, state, q_start, n_new, slot_ids, o_raw, G, H, d, dv, below);                    \
+    else                                                                                                         \
+      gdr_recurrence_kernel<DMAX, LANES, CH, false><<<grid, GD_COLS * LANES, 0, stream>>>(                       \
+          pq, pk, pv, pbeta, pg, state, q_start, n_new, slot_ids, o_raw, G, H, d, dv, below);                    \
+  } while (0)
 #define LLMRS_GD_REC_ALL(CH, LANES)                                                                              \
   do {                                                                                                           \
     if (dmax == 32) LLMRS_GD_REC(32, (LANES < 8 ? LANES : 8), CH);                                               \
