@@ -8,28 +8,70 @@
 #include "common.cuh"
 #include "mma_util.cuh"
 
-// A block owns a tile of BM rows x BN features and walks K in steps of BK through NS stages of shared memory, filled by
-// asynchronous copies NS - 1 steps ahead. Both operands stay in rows along K as they come, a row padded by 16 bytes so that
-// neighbouring rows' 16-byte reads fall into different banks; a thread reads four values of K of its TM rows and TN
-// features at a time and adds them in order of K. An output is ONE chain of fused multiply-adds whatever the tile, which
-// keeps its bits the same in every batch, and is why no tile splits K: a product of few rows is bound by that chain and by
-// the latency of its stages (K = 3,072 into 1,024 features, one row: 15.5 us, 236 before with one synchronous stage of 16
-// values), one of many features by the stream of its weights (1,024 into 32,000: 35 us, 3.7 TB/s; 185 before), one of many
-// rows by the FMA units (2,048 rows of 4,096 x 4,096: 1,867 us, 36.8 TFLOP/s; 2,711 before).
-// (A tile of few outputs has more threads than outputs: its copies are dealt out over four warps, so that the one that adds loses
-// less time to them.)
-__host__ __device__ constexpr int gf_threads(int bm, int bn, int tm, int tn) {
-  return (bm / tm) * (bn / tn) < 128 ? 128 : (bm / tm) * (bn / tn);
+#include <algorithm>
+#include <type_traits>
+
+// The order of an output's sum: K falls into segments of GF_SEG values; a segment is one chain of fused multiply-adds in order
+// of k, starting at zero, and the segments' sums are added in order, starting at zero. Every kernel below keeps to that order,
+// whatever its tile, so an output has the same bits in every batch; and a product of few rows may walk its segments side by
+// side, which a single chain over K could not.
+constexpr int GF_SEG = 256;
+
+// Four values of a row as floats.
+__device__ __forceinline__ float4 gf_four(const float* p) { return *reinterpret_cast<const float4*>(p); }
+__device__ __forceinline__ float4 gf_four(const __nv_bfloat16* p) {
+  const float2 lo = __bfloat1622float2(*reinterpret_cast<const __nv_bfloat162*>(p));
+  const float2 hi = __bfloat1622float2(*reinterpret_cast<const __nv_bfloat162*>(p + 2));
+  return make_float4(lo.x, lo.y, hi.x, hi.y);
 }
-template <typename TX, int BM, int BN, int TM, int TN, int BK, int NS, int U, bool VEC>
-__global__ void __launch_bounds__(gf_threads(BM, BN, TM, TN))
+
+template <int TM, int TN>
+__device__ __forceinline__ void gf_add(float (&acc)[TM][TN], const float4 (&a)[TM], const float4 (&b)[TN]) {
+#pragma unroll
+  for (int i = 0; i < TM; ++i)
+#pragma unroll
+    for (int j = 0; j < TN; ++j)
+      acc[i][j] = fmaf(a[i].w, b[j].w, fmaf(a[i].z, b[j].z, fmaf(a[i].y, b[j].y, fmaf(a[i].x, b[j].x, acc[i][j]))));
+}
+
+// The barrier between a round's sums and their readers: of the cluster, or of the block that is alone.
+__device__ __forceinline__ void gf_round_arrive(int n_blocks) {
+  if (n_blocks > 1) asm volatile("barrier.cluster.arrive.release;" ::: "memory");
+}
+__device__ __forceinline__ void gf_round_wait(int n_blocks) {
+  if (n_blocks > 1) asm volatile("barrier.cluster.wait.acquire;" ::: "memory");
+  else __syncthreads();
+}
+// *p in the shared memory of the cluster's block `rank`.
+__device__ __forceinline__ float gf_peer(const float* p, int rank, int n_blocks) {
+  if (n_blocks == 1) return *p;
+  uint32_t remote;
+  float v;
+  asm volatile("mapa.shared::cluster.u32 %0, %1, %2;" : "=r"(remote) : "r"(smem_addr(p)), "r"(rank));
+  asm volatile("ld.shared::cluster.f32 %0, [%1];" : "=f"(v) : "r"(remote));      // (volatile: stays behind the barrier)
+  return v;
+}
+
+// ---------------------------------------------------------------------------------
+// Many rows: a block owns a tile of BM rows x BN features and walks K in steps of BK through NS stages of shared memory, filled
+// by asynchronous copies NS - 1 steps ahead. Both operands stay in rows along K as they come, a row padded by 16 bytes so that
+// neighbouring rows' 16-byte reads fall into different banks; a thread reads four values of K of its TM rows and TN
+// features at a time and adds them in order of K. The sums of the segments before lie in registers, or, IN_REGS false, in shared
+// memory (each thread its own, touched once in 256 values of K), where a thread's registers are full of operands read ahead.
+// Bound by the path from shared memory to registers, 16 reads for 64 multiply-adds, beside the FMA units: 2,048 rows of
+// 1,024 into 6,144 features 688 us (37.5 TFLOP/s; 705 as one chain over K, 2,048 x 4,096 x 12,288 5,437 and 5,550).
+// ---------------------------------------------------------------------------------
+template <typename TX, int BM, int BN, int TM, int TN, int BK, int NS, bool VEC, bool IN_REGS>
+__global__ void __launch_bounds__((BM / TM) * (BN / TN))
 gemm_f32_kernel(const TX* __restrict__ x, const float* __restrict__ w, const float* __restrict__ bias,
                 float* __restrict__ out, int M, int N, int K, long long x_stride, long long out_stride) {
-  constexpr int THREADS = gf_threads(BM, BN, TM, TN), CN = BN / TN, RM = BM / TM;
+  constexpr int THREADS = (BM / TM) * (BN / TN), CN = BN / TN, RM = BM / TM;
   constexpr int XS = BK + 16 / (int)sizeof(TX), WS = BK + 4;      // elements a row of a stage takes
+  static_assert(GF_SEG % BK == 0, "a step lies in one segment");
   extern __shared__ __align__(16) unsigned char gf_raw[];
-  float* ws = reinterpret_cast<float*>(gf_raw);                   // [NS][BN][WS]
-  TX* xs = reinterpret_cast<TX*>(gf_raw + sizeof(float) * NS * BN * WS);      // [NS][BM][XS]
+  float* tot = reinterpret_cast<float*>(gf_raw);                  // [TM * TN][THREADS]
+  float* ws = tot + (IN_REGS ? 0 : TM * TN * THREADS);                 // [NS][BN][WS]
+  TX* xs = reinterpret_cast<TX*>(ws + NS * BN * WS);              // [NS][BM][XS]
   const int tid = threadIdx.x, tx = tid % CN, ty = tid / CN;
   const int m0 = blockIdx.y * BM, n0 = blockIdx.x * BN;
   auto load = [&](int stage, int k0) {
@@ -49,38 +91,39 @@ gemm_f32_kernel(const TX* __restrict__ x, const float* __restrict__ w, const flo
         else cp_async_8(xd + r * XS + c, src, in ? 8 : 0);
       }
     } else {
-      // Value by value: a thread keeps to a column (to every THREADS-th of a wide step) and goes down the rows, so that an address
-      // is one addition (1,000 rows of 1,023 into 1,024 features 72 us; 141 with an address and plain loads a value, 94 by the
-      // kernel before; 2,050 into 2,048 276, 523 and 367).
-      constexpr int COLS = BK < THREADS ? BK : THREADS, PASS = THREADS / COLS;
+      // Value by value: a thread keeps to a column and goes down the rows, so that an address is one addition (1,000 rows of
+      // 1,023 into 1,024 features 72 us; 141 with an address and plain loads a value; 2,050 into 2,048 276 and 523).
+      static_assert(THREADS % BK == 0, "whole rows a pass");
+      constexpr int PASS = THREADS / BK;
+      const int c = tid % BK, r0 = tid / BK;
+      const bool k_in = k0 + c < K;
+      const float* wp = w + (size_t)(n0 + r0) * K + k0 + c;
 #pragma unroll
-      for (int c0 = 0; c0 < BK; c0 += COLS) {
-        const int c = c0 + tid % COLS, r0 = tid / COLS;
-        const bool k_in = k0 + c < K;
-        const float* wp = w + (size_t)(n0 + r0) * K + k0 + c;
+      for (int r = 0; r < BN; r += PASS, wp += (size_t)PASS * K) {
+        const bool in = k_in && n0 + r0 + r < N;
+        if (BN % PASS == 0 || r0 + r < BN) cp_async_4(wd + (r0 + r) * WS + c, in ? wp : w, in ? 4 : 0);
+      }
+      const TX* xp = x + (size_t)(m0 + r0) * x_stride + k0 + c;
 #pragma unroll
-        for (int r = 0; r < BN; r += PASS, wp += (size_t)PASS * K) {
-          const bool in = k_in && n0 + r0 + r < N;
-          if (BN % PASS == 0 || r0 + r < BN) cp_async_4(wd + (r0 + r) * WS + c, in ? wp : w, in ? 4 : 0);
-        }
-        const TX* xp = x + (size_t)(m0 + r0) * x_stride + k0 + c;
-#pragma unroll
-        for (int r = 0; r < BM; r += PASS, xp += PASS * x_stride) {
-          const bool in = k_in && m0 + r0 + r < M;
-          if (BM % PASS == 0 || r0 + r < BM) {
-            if constexpr (sizeof(TX) == 4) cp_async_4(xd + (r0 + r) * XS + c, in ? xp : x, in ? 4 : 0);
-            else xd[(r0 + r) * XS + c] = in ? *xp : TX(0.f);      // (no asynchronous copy has two bytes)
-          }
+      for (int r = 0; r < BM; r += PASS, xp += PASS * x_stride) {
+        const bool in = k_in && m0 + r0 + r < M;
+        if (BM % PASS == 0 || r0 + r < BM) {
+          if constexpr (sizeof(TX) == 4) cp_async_4(xd + (r0 + r) * XS + c, in ? xp : x, in ? 4 : 0);
+          else xd[(r0 + r) * XS + c] = in ? *xp : TX(0.f);      // (no asynchronous copy has two bytes)
         }
       }
     }
     cp_async_commit();
   };
-  float acc[TM][TN];
+  float acc[TM][TN], held[IN_REGS ? TM : 1][IN_REGS ? TN : 1];
+  auto before = [&](int i, int j) -> float& {      // the segments before, of this thread's output (i, j)
+    if constexpr (IN_REGS) return held[i][j];
+    else return tot[(i * TN + j) * THREADS + tid];
+  };
 #pragma unroll
   for (int i = 0; i < TM; ++i)
 #pragma unroll
-    for (int j = 0; j < TN; ++j) acc[i][j] = 0.f;
+    for (int j = 0; j < TN; ++j) acc[i][j] = before(i, j) = 0.f;
   const int steps = (K + BK - 1) / BK;
 #pragma unroll
   for (int s = 0; s < NS - 1; ++s) {
@@ -92,48 +135,44 @@ gemm_f32_kernel(const TX* __restrict__ x, const float* __restrict__ w, const flo
     __syncthreads();      // stage `it` is there for everyone, and everyone is done with the stage that is filled next
     if (it + NS - 1 < steps) load((it + NS - 1) % NS, (it + NS - 1) * BK);
     else cp_async_commit();
-    if (RM * CN < THREADS && tid >= RM * CN) continue;      // only copies
+    if (it % (GF_SEG / BK) == 0 && it) {
+#pragma unroll
+      for (int i = 0; i < TM; ++i)
+#pragma unroll
+        for (int j = 0; j < TN; ++j) {
+          before(i, j) += acc[i][j];
+          acc[i][j] = 0.f;
+        }
+    }
     const float* wr = ws + (it % NS) * BN * WS;
     const TX* xr = xs + (it % NS) * BM * XS;
-    // The next U pieces are read while the present ones are added: a warp alone on its scheduler would otherwise wait
-    // for shared memory in every step of its chains.
-    float4 av[2][U][TM], bv[2][U][TN];
-    auto fetch = [&](int buf, int k0) {
+    if constexpr (IN_REGS && TM * TN > 32) {      // no registers left to read ahead
+      float4 av[TM], bv[TN];
 #pragma unroll
-      for (int u = 0; u < U; ++u) {
+      for (int k = 0; k < BK; k += 4) {
 #pragma unroll
-        for (int i = 0; i < TM; ++i) {
-          const TX* p = xr + (ty + i * RM) * XS + k0 + 4 * u;
-          if constexpr (sizeof(TX) == 4) {
-            av[buf][u][i] = *reinterpret_cast<const float4*>(p);
-          } else {
-            const float2 lo = __bfloat1622float2(*reinterpret_cast<const __nv_bfloat162*>(p));
-            const float2 hi = __bfloat1622float2(*reinterpret_cast<const __nv_bfloat162*>(p + 2));
-            av[buf][u][i] = make_float4(lo.x, lo.y, hi.x, hi.y);
-          }
-        }
+        for (int i = 0; i < TM; ++i) av[i] = gf_four(xr + (ty + i * RM) * XS + k);
 #pragma unroll
-        for (int j = 0; j < TN; ++j)
-          bv[buf][u][j] = *reinterpret_cast<const float4*>(wr + (tx + j * CN) * WS + k0 + 4 * u);
+        for (int j = 0; j < TN; ++j) bv[j] = gf_four(wr + (tx + j * CN) * WS + k);
+        gf_add<TM, TN>(acc, av, bv);
       }
-    };
-    fetch(0, 0);
+    } else {      // the next piece is read while the present one is added
+      float4 av[2][TM], bv[2][TN];
+      auto fetch = [&](int buf, int k0) {
 #pragma unroll
-    for (int k = 0; k < BK; k += 4 * U) {
-      const int cur = (k / (4 * U)) & 1;
-      if (k + 4 * U < BK) fetch(cur ^ 1, k + 4 * U);
+        for (int i = 0; i < TM; ++i) av[buf][i] = gf_four(xr + (ty + i * RM) * XS + k0);
 #pragma unroll
-      for (int u = 0; u < U; ++u)
+        for (int j = 0; j < TN; ++j) bv[buf][j] = gf_four(wr + (tx + j * CN) * WS + k0);
+      };
+      fetch(0, 0);
 #pragma unroll
-        for (int i = 0; i < TM; ++i)
-#pragma unroll
-          for (int j = 0; j < TN; ++j) {
-            const float4 a = av[cur][u][i], b = bv[cur][u][j];
-            acc[i][j] = fmaf(a.w, b.w, fmaf(a.z, b.z, fmaf(a.y, b.y, fmaf(a.x, b.x, acc[i][j]))));
-          }
+      for (int k = 0; k < BK; k += 4) {
+        const int cur = (k / 4) & 1;
+        if (k + 4 < BK) fetch(cur ^ 1, k + 4);
+        gf_add<TM, TN>(acc, av[cur], bv[cur]);
+      }
     }
   }
-  if (RM * CN < THREADS && tid >= RM * CN) return;
 #pragma unroll
   for (int i = 0; i < TM; ++i) {
     const int m = m0 + ty + i * RM;
@@ -141,33 +180,229 @@ gemm_f32_kernel(const TX* __restrict__ x, const float* __restrict__ w, const flo
 #pragma unroll
     for (int j = 0; j < TN; ++j) {
       const int n = n0 + tx + j * CN;
-      if (n < N) out[(size_t)m * out_stride + n] = acc[i][j] + (bias ? bias[n] : 0.f);
+      if (n < N) out[(size_t)m * out_stride + n] = before(i, j) + acc[i][j] + (bias ? bias[n] : 0.f);
     }
   }
 }
 
-template <typename TX, int BM, int BN, int TM, int TN, int BK, int NS, int U>
-static int launch_gemm_f32(bool vec, const TX* x, long long x_stride, const float* w, const float* bias, float* out,
-                           long long out_stride, int M, int N, int K, cudaStream_t stream) {
-  constexpr size_t smem = (size_t)NS * (BN * (BK + 4) * sizeof(float) + BM * (BK * sizeof(TX) + 16));
-  constexpr int threads = gf_threads(BM, BN, TM, TN);
-  const dim3 grid((N + BN - 1) / BN, (M + BM - 1) / BM);
-  LLMRS_REQUIRE(grid.y <= 65535, "gemm_f32: M=%d is too large", M);
-  auto go = [&](auto kernel) {
-    if (smem > 48 * 1024) {
-      cudaError_t e = cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
-      if (e != cudaSuccess) return llmrs_fail("gemm_f32: shared memory %zu: %s", smem, cudaGetErrorString(e));
+// ---------------------------------------------------------------------------------
+// Few rows, or few tiles: KG groups of RM x CN threads walk KG segments of the block's tile side by side, a thread TM rows x TN
+// features of one segment, and the blocks of a cluster take KG segments each. After such a round every sum of a segment lies
+// in its block's shared memory, and each block adds its share of the tile over all of them in order. What bounds it: one row
+// is the stream of the weights (every one read from shared memory once) and the latency of a launch, a segment's chain being
+// 0.6 us; rows that fill TM the path from shared memory to registers, (TM + TN) reads for TM x TN multiply-adds.
+// One row: 1,024 into 1,024 features 4.6 us (5.8 as one chain over K), K = 3,072 6.2 (14.9), 12,288 into 4,096 51 (81), 1,024 into
+// 32,000 27 (4.9 TB/s). Eight rows, K = 3,072 into 1,024: 13.8 (24.8); 37 rows: 28 (46), 1,024 into 6,144 25 (47). KG = 1 (64 threads
+// a block, several blocks an SM) for more than eight rows: with four segments in a block each SM's shared memory feeds four times
+// the threads and fewer SMs have a block (37 rows, K = 1,024 into 1,024: 13 us, 23 before the blocks were made this small).
+// ---------------------------------------------------------------------------------
+template <typename TX, int RM, int TM, int CN, int TN, int KG, int BK, int NS, bool VEC>
+__global__ void __launch_bounds__(RM * CN * KG)
+gemm_f32_seg_kernel(const TX* __restrict__ x, const float* __restrict__ w, const float* __restrict__ bias,
+                    float* __restrict__ out, int M, int N, int K, long long x_stride, long long out_stride, int n_blocks) {
+  constexpr int BM = RM * TM, BN = CN * TN, GT = RM * CN, THREADS = GT * KG, TILE = BM * BN;
+  constexpr int XS = BK + 16 / (int)sizeof(TX), WS = BK + 4, STEPS = GF_SEG / BK;
+  extern __shared__ __align__(16) unsigned char gf_raw[];
+  float* part = reinterpret_cast<float*>(gf_raw);                 // [KG][TILE]
+  float* total = part + KG * TILE;                                // [TILE]: of the rounds before, each element one thread's
+  float* ws = total + TILE;                                       // [NS][KG][BN][WS]
+  TX* xs = reinterpret_cast<TX*>(ws + NS * KG * BN * WS);         // [NS][KG][BM][XS]
+  const int tid = threadIdx.x, g = tid / GT, tx = tid % GT % CN, ty = tid % GT / CN;
+  const int n0 = blockIdx.x * BN, m0 = blockIdx.y * BM, rank = blockIdx.z;      // n_blocks = the cluster's size = gridDim.z
+  const int segments = (K + GF_SEG - 1) / GF_SEG, rounds = (segments + KG * n_blocks - 1) / (KG * n_blocks);
+  const int steps = rounds * STEPS;
+  pdl_launch_dependents();
+  // Step `it` of round `it / STEPS`: BK values of each of the block's KG segments. A step that starts beyond K is neither filled nor read.
+  auto k_of = [&](int it, int group) { return ((it / STEPS * n_blocks + rank) * KG + group) * GF_SEG + it % STEPS * BK; };
+  // `rows` of each of the KG segments. Pieces of four values: those beyond the matrix are filled with zeros. Value by value a
+  // thread's copies are many, so steps that start beyond K (which nothing reads) are left out.
+  auto load = [&](auto* dst, const auto* src, long long src_stride, auto rows, int row0, int n_rows, int it) {
+    using T = std::remove_reference_t<decltype(*dst)>;
+    constexpr int ROWS = decltype(rows)::value, STRIDE = BK + 16 / (int)sizeof(T);
+    dst += it % NS * (KG * ROWS * STRIDE);
+    if constexpr (VEC) {
+#pragma unroll
+      for (int e = tid; e < KG * ROWS * (BK / 4); e += THREADS) {
+        const int r = e / (BK / 4), c = e % (BK / 4) * 4, k = k_of(it, r / ROWS) + c, row = row0 + r % ROWS;
+        const bool in = row < n_rows && k < K;
+        const auto* from = in ? src + row * src_stride + k : src;
+        if constexpr (sizeof(T) == 4) cp_async_16(dst + r * STRIDE + c, from, in ? 16 : 0);
+        else cp_async_8(dst + r * STRIDE + c, from, in ? 8 : 0);
+      }
+    } else {
+      constexpr int PASS = THREADS / BK;
+      static_assert(THREADS % BK == 0, "whole rows a pass");
+      const int c = tid % BK, k0 = k_of(it, 0);
+      const int live = KG == 1 ? ROWS : min(KG, (K - k0 + GF_SEG - 1) / GF_SEG) * ROWS;
+#pragma unroll
+      for (int r0 = 0; r0 < KG * ROWS; r0 += PASS) {
+        const int r = r0 + tid / BK;
+        if (r >= live) break;
+        const int k = k0 + r / ROWS * GF_SEG + c, row = row0 + r % ROWS;
+        const bool in = row < n_rows && k < K;
+        const auto* from = in ? src + row * src_stride + k : src;
+        if constexpr (sizeof(T) == 4) cp_async_4(dst + r * STRIDE + c, from, in ? 4 : 0);
+        else dst[r * STRIDE + c] = in ? *from : T(0.f);      // (no asynchronous copy has two bytes)
+      }
     }
-    kernel<<<grid, threads, smem, stream>>>(x, w, bias, out, M, N, K, x_stride, out_stride);
-    return llmrs_launch_status("gemm_f32");
   };
-  return vec ? go(gemm_f32_kernel<TX, BM, BN, TM, TN, BK, NS, U, true>) : go(gemm_f32_kernel<TX, BM, BN, TM, TN, BK, NS, U, false>);
+  auto load_w = [&](int it) { load(ws, w, (long long)K, std::integral_constant<int, BN>{}, n0, N, it); };
+  auto load_x = [&](int it) { load(xs, x, x_stride, std::integral_constant<int, BM>{}, m0, M, it); };
+  // The weights of the first steps are on their way before the kernel that makes the rows has ended (steps >= NS - 1:
+  // a round has GF_SEG / BK steps).
+  static_assert(STEPS >= NS - 1, "the first stages lie in the first round");
+#pragma unroll
+  for (int s = 0; s < NS - 1; ++s) load_w(s);
+  pdl_wait();
+#pragma unroll
+  for (int s = 0; s < NS - 1; ++s) {
+    load_x(s);
+    cp_async_commit();      // (the first group holds the weights of all of them)
+  }
+  float acc[TM][TN];
+#pragma unroll
+  for (int i = 0; i < TM; ++i)
+#pragma unroll
+    for (int j = 0; j < TN; ++j) acc[i][j] = 0.f;
+  const int share = (TILE + n_blocks - 1) / n_blocks, own_lo = rank * share, own_hi = min(TILE, own_lo + share);
+  for (int it = 0; it < steps; ++it) {
+    cp_async_wait<NS - 2>();
+    __syncthreads();      // stage `it` is there for everyone, and everyone is done with the stage that is filled next
+    if (it + NS - 1 < steps) {
+      load_w(it + NS - 1);
+      load_x(it + NS - 1);
+    }
+    cp_async_commit();
+    const float* wr = ws + (it % NS * KG + g) * (BN * WS);
+    const TX* xr = xs + (it % NS * KG + g) * (BM * XS);
+    if (k_of(it, g) < K) {
+      float4 av[2][TM], bv[2][TN];
+      auto fetch = [&](int buf, int k0) {
+#pragma unroll
+        for (int i = 0; i < TM; ++i) av[buf][i] = gf_four(xr + (ty + i * RM) * XS + k0);
+#pragma unroll
+        for (int j = 0; j < TN; ++j) bv[buf][j] = gf_four(wr + (tx + j * CN) * WS + k0);
+      };
+      fetch(0, 0);
+#pragma unroll
+      for (int k = 0; k < BK; k += 4) {
+        const int cur = (k / 4) & 1;
+        if (k + 4 < BK) fetch(cur ^ 1, k + 4);
+        gf_add<TM, TN>(acc, av[cur], bv[cur]);
+      }
+    }
+    if (it % STEPS != STEPS - 1) continue;
+    // The end of a round. (Segments beyond K leave zeros, which are not added.)
+    if (it >= STEPS) gf_round_wait(n_blocks);      // everyone has read the sums of the round before
+#pragma unroll
+    for (int i = 0; i < TM; ++i)
+#pragma unroll
+      for (int j = 0; j < TN; ++j) {
+        part[g * TILE + (ty + i * RM) * BN + tx + j * CN] = acc[i][j];
+        acc[i][j] = 0.f;
+      }
+    gf_round_arrive(n_blocks);
+    gf_round_wait(n_blocks);
+    const int first = it / STEPS * n_blocks * KG, here = min(segments - first, n_blocks * KG);
+    constexpr int AT_ONCE = 4;      // elements of a thread whose reads from a peer are in flight together
+    for (int e0 = own_lo + tid; e0 < own_hi; e0 += AT_ONCE * THREADS) {
+      float sum[AT_ONCE];
+#pragma unroll
+      for (int i = 0; i < AT_ONCE; ++i) sum[i] = it < STEPS || e0 + i * THREADS >= own_hi ? 0.f : total[e0 + i * THREADS];
+      for (int s = 0; s < here; ++s) {
+        const float* from = part + s % KG * TILE + e0;
+        float v[AT_ONCE];
+#pragma unroll
+        for (int i = 0; i < AT_ONCE; ++i) v[i] = gf_peer(from + (e0 + i * THREADS < own_hi ? i * THREADS : 0), s / KG, n_blocks);
+#pragma unroll
+        for (int i = 0; i < AT_ONCE; ++i) sum[i] += v[i];
+      }
+#pragma unroll
+      for (int i = 0; i < AT_ONCE; ++i) {
+        const int e = e0 + i * THREADS, m = m0 + e / BN, n = n0 + e % BN;
+        if (e >= own_hi) continue;
+        if (it + 1 < steps) total[e] = sum[i];
+        else if (m < M && n < N) out[(size_t)m * out_stride + n] = sum[i] + (bias ? bias[n] : 0.f);
+      }
+    }
+    gf_round_arrive(n_blocks);
+  }
+  gf_round_wait(n_blocks);      // no block leaves while its sums may be read
 }
 
-// The largest tile of which there are enough blocks for the SMs: larger tiles read the operands less often, smaller ones
-// spread a short product over the device, and no tile has more rows than the product would half fill. Both sides of the
-// line, measured: 16 rows of 2,048 into 6,144 features 43 us in tiles of 16 x 32, 72 in tiles of 32 x 32 whose second half
-// is empty; 37 rows of 1,024 into 6,144 features 48 us in 384 tiles of 32 x 32, 80 in 96 tiles of 64 x 64 (as before).
+
+template <typename F, typename... Args>
+static int gf_launch(F kernel, dim3 grid, int threads, size_t smem, bool pdl, cudaStream_t stream, Args... args) {
+  if (smem > 48 * 1024) {
+    cudaError_t e = cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
+    if (e != cudaSuccess) return llmrs_fail("gemm_f32: shared memory %zu: %s", smem, cudaGetErrorString(e));
+  }
+  cudaLaunchConfig_t cfg = {};
+  cfg.gridDim = grid;
+  cfg.blockDim = dim3(threads);
+  cfg.dynamicSmemBytes = smem;
+  cfg.stream = stream;
+  cudaLaunchAttribute attr[2];
+  if (grid.z > 1) {
+    attr[cfg.numAttrs].id = cudaLaunchAttributeClusterDimension;
+    attr[cfg.numAttrs].val.clusterDim.x = attr[cfg.numAttrs].val.clusterDim.y = 1;
+    attr[cfg.numAttrs++].val.clusterDim.z = grid.z;
+  }
+  if (pdl && g_llmrs_pdl) {
+    attr[cfg.numAttrs].id = cudaLaunchAttributeProgrammaticStreamSerialization;
+    attr[cfg.numAttrs++].val.programmaticStreamSerializationAllowed = 1;
+  }
+  cfg.attrs = attr;
+  cudaLaunchKernelEx(&cfg, kernel, args...);
+  return llmrs_launch_status("gemm_f32");
+}
+
+template <typename TX>
+struct GfArgs {
+  const TX* x;
+  long long x_stride;
+  const float *w, *bias;
+  float* out;
+  long long out_stride;
+  int M, N, K;
+  bool vec;
+  cudaStream_t stream;
+};
+
+template <int BM, int BN, int TM, int TN, int BK, int NS, bool IN_REGS, typename TX>
+static int gf_tiles(const GfArgs<TX>& a) {
+  constexpr int threads = (BM / TM) * (BN / TN);
+  constexpr size_t smem = (IN_REGS ? 0 : (size_t)TM * TN * threads * 4) + (size_t)NS * (BN * (BK + 4) * 4 + BM * (BK * sizeof(TX) + 16));
+  const dim3 grid((a.N + BN - 1) / BN, (a.M + BM - 1) / BM);
+  LLMRS_REQUIRE(grid.y <= 65535, "gemm_f32: M=%d is too large", a.M);
+  return gf_launch(a.vec ? gemm_f32_kernel<TX, BM, BN, TM, TN, BK, NS, true, IN_REGS> : gemm_f32_kernel<TX, BM, BN, TM, TN, BK, NS, false, IN_REGS>,
+                   grid, threads, smem, false, a.stream, a.x, a.w, a.bias, a.out, a.M, a.N, a.K, a.x_stride, a.out_stride);
+}
+
+// Blocks a cluster: as many as the device holds at a time, at most one for every KG segments, at most eight, and no more than
+// leave the last round's blocks with segments (6,144 features of 16 rows, K = 1,024: four blocks 14.3 us, three, the last of which
+// walk a second round alone, 25).
+template <int RM, int TM, int CN, int TN, int KG, int BK, int NS, typename TX>
+static int gf_segments(const GfArgs<TX>& a) {
+  constexpr int BM = RM * TM, BN = CN * TN, threads = RM * CN * KG, BLOCKS = 148 * (KG > 1 ? 2 : 6);
+  constexpr size_t smem = (size_t)(KG + 1) * BM * BN * 4 + (size_t)NS * KG * (BN * (BK + 4) * 4 + BM * (BK * sizeof(TX) + 16));
+  static_assert(smem <= 227 * 1024, "the block's shared memory");
+  const long long tiles_n = (a.N + BN - 1) / BN, tiles_m = (a.M + BM - 1) / BM;
+  LLMRS_REQUIRE(tiles_m <= 65535, "gemm_f32: M=%d is too large", a.M);
+  const long long turns = ((a.K + GF_SEG - 1) / GF_SEG + KG - 1) / KG;
+  const long long most = std::min(8ll, std::max(1ll, BLOCKS / (tiles_n * tiles_m))), rounds = (turns + most - 1) / most;
+  const long long cluster = (turns + rounds - 1) / rounds;
+  const dim3 grid((unsigned)tiles_n, (unsigned)tiles_m, (unsigned)cluster);
+  return gf_launch(a.vec ? gemm_f32_seg_kernel<TX, RM, TM, CN, TN, KG, BK, NS, true>
+                         : gemm_f32_seg_kernel<TX, RM, TM, CN, TN, KG, BK, NS, false>,
+                   grid, threads, smem, true, a.stream, a.x, a.w, a.bias, a.out, a.M, a.N, a.K, a.x_stride, a.out_stride,
+                   (int)cluster);
+}
+
+// Many rows: the largest tile of which there are enough blocks for the SMs, since larger tiles read the operands less often.
+// Otherwise segments side by side. Both sides of the lines, measured: 48 rows of 1,024 into 6,144 features 31 us by segments,
+// 47 in tiles of 64 x 64; 90 rows 59 in tiles of 48 rows by segments, 76 in 192 tiles of 64 x 64, but 300 rows 144 so and 148;
+// 16 rows of tiles of eight features (K = 1,024 into 2,048) 12.1 us, 2,048 features of one row 5.0 in tiles of eight, 7.0 in tiles of 32.
 template <typename TX>
 static int gemm_f32_any(const TX* x, long long x_stride, const float* w, const float* bias, float* out,
                         long long out_stride, int M, int N, int K, cudaStream_t stream) {
@@ -175,26 +410,31 @@ static int gemm_f32_any(const TX* x, long long x_stride, const float* w, const f
   if (M == 0) return 0;
   // Pieces of four values by one asynchronous copy each: every row of both operands must start on such a piece.
   const bool vec = K % 4 == 0 && x_stride % 4 == 0 && ((uintptr_t)w & 15) == 0 && ((uintptr_t)x & (4 * sizeof(TX) - 1)) == 0;
+  const GfArgs<TX> a{x, x_stride, w, bias, out, out_stride, M, N, K, vec, stream};
   auto blocks = [&](int bm, int bn) { return (long long)((M + bm - 1) / bm) * ((N + bn - 1) / bn); };
   constexpr int ENOUGH = 148;
-#define LLMRS_GF(BM, BN, TM, TN, BK, NS, U) \
-  return launch_gemm_f32<TX, BM, BN, TM, TN, BK, NS, U>(vec, x, x_stride, w, bias, out, out_stride, M, N, K, stream)
-  if (M > 64 && blocks(128, 128) >= ENOUGH) LLMRS_GF(128, 128, 8, 8, 16, 4, 1);
-  if (M > 32 && blocks(64, 64) >= ENOUGH) LLMRS_GF(64, 64, 4, 8, 32, 4, 1);
-  if (M > 16 && blocks(32, 32) >= ENOUGH) LLMRS_GF(32, 32, 2, 4, 32, 4, 1);
-  if (M > 8 && blocks(16, 32) >= ENOUGH) LLMRS_GF(16, 32, 2, 2, 64, 4, 2);
-  if (M > 4 && blocks(8, 32) >= ENOUGH) LLMRS_GF(8, 32, 2, 1, 64, 4, 4);
-  if (M > 4) LLMRS_GF(8, 16, 1, 1, 64, 4, 4);
-  if (M == 1) {      // tiles of one row read the weights from shared memory once, where those of four rows read them for each: 1,024
-                     // into 32,000 features 35 us (46), into 6,144 9.8 (14), K = 3,072 into 1,024 15.5 (19)
-    if (N >= 64 * 2 * ENOUGH) LLMRS_GF(1, 64, 1, 1, 64, 3, 4);
-    if (N >= 32 * ENOUGH) LLMRS_GF(1, 32, 1, 1, 128, 4, 4);
-    if (N >= 16 * ENOUGH) LLMRS_GF(1, 16, 1, 1, 128, 6, 4);
-    LLMRS_GF(1, 8, 1, 1, 256, 6, 4);
+  if (M > 64 && blocks(128, 128) >= ENOUGH) {
+    if (!vec) return gf_tiles<128, 128, 8, 8, 32, 4, true>(a);
+    return gf_tiles<128, 128, 8, 8, 32, sizeof(TX) == 4 ? 3 : 4, false>(a);
   }
-  if (blocks(4, 32) >= 2 * ENOUGH) LLMRS_GF(4, 32, 1, 1, 64, 4, 4);
-  LLMRS_GF(4, 8, 1, 1, 128, 4, 4);
-#undef LLMRS_GF
+  if (M > 48 && blocks(64, 64) >= ENOUGH) return gf_tiles<64, 64, 4, 8, 32, 4, true>(a);
+  const bool narrow = N <= 16 * ENOUGH;      // tiles of eight features: twice as many as SMs at most
+  if (M == 1) return narrow ? gf_segments<1, 1, 8, 1, 16, 32, 4>(a) : gf_segments<1, 1, 32, 1, 4, 32, 4>(a);
+  if (M <= 4) return narrow ? gf_segments<1, 4, 8, 1, 16, 32, 3>(a) : gf_segments<1, 4, 32, 1, 4, 32, 4>(a);
+  if (M <= 8) return narrow ? gf_segments<1, 8, 8, 1, 16, 32, 3>(a) : gf_segments<1, 8, 32, 1, 4, 32, 4>(a);
+  if (M <= 16) return gf_segments<4, 4, 8, 4, 1, 32, 3>(a);
+  // (Value by value a block of 128 threads gets its copies out sooner: 300 rows of 1,023 into 1,500 features 54 us, 75 by segments.)
+  if (!vec && M > 64) return gf_tiles<32, 32, 2, 4, 32, 4, true>(a);
+  int rows = 0;      // of a tile: those that leave the fewest empty, of equals the most
+  for (int r : {64, 48, 40, 32, 24})
+    if (rows == 0 || blocks(r, N) * r < blocks(rows, N) * rows) rows = r;
+  switch (rows) {
+    case 24: return gf_segments<8, 3, 8, 4, 1, 32, 3>(a);
+    case 32: return gf_segments<8, 4, 8, 4, 1, 32, 3>(a);
+    case 40: return gf_segments<8, 5, 8, 4, 1, 32, 3>(a);
+    case 48: return gf_segments<8, 6, 8, 4, 1, 32, 3>(a);
+    default: return gf_segments<8, 8, 8, 4, 1, 32, 3>(a);
+  }
 }
 
 LLMRS_API int llmrs_gemm_f32(const float* x, long long x_stride, const float* w, const float* bias, float* out,

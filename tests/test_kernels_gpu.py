@@ -112,6 +112,24 @@ def test_gemm_f32_tiles(N, K, pad, rows_dtype):
         assert torch.equal(ops.gemm_f32(x[:M], w, b), whole[:M]), M
 
 
+@pytest.mark.parametrize("rows_dtype", [torch.float32, torch.bfloat16])
+@pytest.mark.parametrize("N,K,pad", [(300, 256, 0), (300, 1028, 0), (301, 1279, 3), (2400, 516, 4), (289, 4100, 0), (5000, 260, 1),
+                                     (300, 12288, 0)])
+def test_gemm_f32_segments(N, K, pad, rows_dtype):
+    """K in one segment of 256, just beyond, in many (several rounds of a cluster), at every number of rows a tile takes. A segment is
+    a chain of at most 256 fused multiply-adds and the segments' sums are added one after the other: the error is at most
+    256 + ceil(K / 256) + 1 half ulps of the sum of the products' magnitudes."""
+    ops = _ops()
+    torch.manual_seed(N + K)
+    x = torch.randn(300, K + pad, device=DEV).to(rows_dtype)[:, :K]
+    w, b = torch.randn(N, K, device=DEV), torch.randn(N, device=DEV)
+    whole = ops.gemm_f32(x, w, b)
+    bound = (x.double().abs() @ w.double().abs().t() + b.double().abs()) * (256 + -(-K // 256) + 1) * 2.0 ** -24
+    assert bool(((whole.double() - (x.double() @ w.double().t() + b.double())).abs() <= bound).all())
+    for M in (1, 2, 4, 7, 12, 17, 25, 33, 41, 47, 49, 63, 65, 90, 150):
+        assert torch.equal(ops.gemm_f32(x[:M], w, b), whole[:M]), M
+
+
 # -- norm + rotation + cache write ---------------------------------------------------------
 def _paged_setup(lens, new, n_kv, d, page, dtype, seed=0):
     """Random cache with scattered pages; returns tensors for kernels and dense copies for the reference."""
