@@ -11,8 +11,9 @@
 // Two kernels and a small third:
 //   prepare     a warp per (token, head), all tokens at once: decay, removal rate times unit key, unit key, and r, k, v
 //               widened, as six float32 rows [tokens, heads * d];
-//   (requests that are walked in turns take `turns` and the walk of state_walk.cuh instead of these two;
-//   2,048 tokens of 32 heads of 64 x 64: 816 us walked one by one, 246 in turns; their rows 56 us where `prepare` takes 38)
+//   (requests that are walked take their rows and the walk of state_chunks.cuh instead of these two, heads of more than 64 channels
+//   `turns` and the walk of state_walk.cuh; 2,048 tokens of 32 heads of 64 x 64: 816 us walked one by one, 246 in turns, 92 in
+//   chunks; their rows 136 us, those of turns 56, where `prepare` takes 38)
 //   recurrence  one block per (request, head, slice of 16 value columns) walks the request's tokens of the step in
 //               order: a column of S depends on no other column, so the slices run side by side. Four adjacent lanes
 //               share a column, each keeping a quarter of its key channels in registers; u^T S and S^T r are summed
@@ -27,7 +28,7 @@
 #include "common.cuh"
 #include "head_out.cuh"
 #include "mma_util.cuh"
-#include "state_walk.cuh"
+#include "state_chunks.cuh"
 
 __device__ __forceinline__ float sigmoidf_(float x) { return 1.0f / (1.0f + expf(-x)); }
 
@@ -176,6 +177,181 @@ delta_turns_kernel(const TA* __restrict__ r, const TA* __restrict__ k, const TA*
   if (lane < 12) {      // above the diagonals
     const int e = lane % 6;
     to[(lane < 6 ? WALK_GR : WALK_GQ) + (e < 3 ? 1 + e : (e < 5 ? 3 + e : 11))] = 0.f;
+  }
+}
+
+// The same for chunks of sixteen tokens (state_chunks.cuh), heads of at most 64 channels: a block per (place, head). Half a warp
+// walks a token j through the tokens after it, the decays multiplied on as they go, and then token 15 - j, so that every one has
+// seventeen steps; then a warp makes the rows of sixteen channels, which are sixteen value columns too.
+template <typename TA>
+__global__ void __launch_bounds__(128, 4)
+delta_rows_kernel(const TA* __restrict__ r, const TA* __restrict__ k, const TA* __restrict__ v, const TA* __restrict__ a_raw,
+                  long long in_stride, const float* __restrict__ decay_raw, const float* __restrict__ decay_bias,
+                  const float* __restrict__ a_bias, const int* __restrict__ q_start, const int* __restrict__ n_new,
+                  float* __restrict__ tiles, float* __restrict__ u_out, float* __restrict__ g_out, float* __restrict__ v_out,
+                  int n_requests, int n_heads, int d, float decay_scale, float key_eps, int from) {
+  constexpr int GS = CK + 1, DMAX = 64, RS = DMAX + 4, ROW = DMAX + 8;
+  extern __shared__ __align__(128) float dr_raw[];
+  float* tile = dr_raw;
+  auto ks = reinterpret_cast<float (*)[RS]>(tile + ck_tile(CK_GENERAL, DMAX));
+  auto rs = ks + CK, us = rs + CK, as = us + CK, ws = as + CK;
+  __shared__ __align__(16) __nv_bfloat16 E[CK_MATRIX], R[CK_MATRIX], Q[CK_MATRIX], T[CK_MATRIX];
+  __shared__ float sums[4][CK][GS];      // u_i . k_j, u_i . a_j, r_i . k_j, r_i . a_j
+  const int h = blockIdx.y, tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
+  const int place = blockIdx.x;
+  int t_req, n_req;
+  const int req = ck_request(q_start, n_new, n_requests, place, t_req, n_req);
+  const int first = (place - ck_place(t_req, req)) * CK, have = min(CK, n_req - first);
+  if (first < 0 || have <= 0 || n_req < from) return;
+  const size_t t0 = (size_t)(t_req + first), width = (size_t)n_heads * d;
+  {
+    float kv[CK / 4][2], rv[CK / 4][2], av[CK / 4][2], dec[CK / 4][2], bias_a[2], bias_d[2];      // a warp a token, all on their way together
+#pragma unroll
+    for (int m = 0; m < 2; ++m) {
+      const int c = lane + 32 * m;
+      const size_t ch = (size_t)h * d + c;
+      bias_a[m] = c < d ? a_bias[ch] : 0.f;
+      bias_d[m] = c < d ? decay_bias[ch] : 0.f;
+#pragma unroll
+      for (int x = 0; x < CK / 4; ++x) {
+        const int t = 4 * x + warp;
+        const size_t at = (t0 + t) * in_stride + ch;
+        kv[x][m] = rv[x][m] = av[x][m] = dec[x][m] = 0.f;
+        if (t < have && c < d) {
+          kv[x][m] = to_float(k[at]);
+          rv[x][m] = to_float(r[at]);
+          av[x][m] = to_float(a_raw[at]);
+          dec[x][m] = decay_raw[(t0 + t) * width + ch];
+        }
+      }
+    }
+#pragma unroll
+    for (int x = 0; x < CK / 4; ++x) {
+      const int t = 4 * x + warp;
+      const float inv = 1.0f / sqrtf(warp_sum(fmaf(kv[x][0], kv[x][0], kv[x][1] * kv[x][1])) + key_eps);
+#pragma unroll
+      for (int m = 0; m < 2; ++m) {
+        const int c = lane + 32 * m;
+        const bool there = t < have && c < d;
+        const float u = there ? kv[x][m] * inv : 0.f;
+        ks[t][c] = kv[x][m];
+        us[t][c] = u;
+        rs[t][c] = rv[x][m];
+        as[t][c] = there ? -sigmoidf_(av[x][m] + bias_a[m]) * u : 0.f;
+        ws[t][c] = there ? expf(-decay_scale * sigmoidf_(dec[x][m] + bias_d[m])) : 1.f;
+      }
+    }
+  }
+  // The values that this warp needs below are on their way.
+  const int c0 = 16 * warp;
+  float value[8];
+#pragma unroll
+  for (int e = 0; e < 8; ++e) {
+    const int t = ck_token(lane, e), c = c0 + ck_channel(lane, e);
+    value[e] = t < have && c < d ? to_float(v[(t0 + t) * in_stride + (size_t)h * d + c]) : 0.f;
+  }
+  __syncthreads();
+  {
+    const int pair = tid >> 4, at = (tid & 15) * 4;
+    auto four = [](const float* p) { return *reinterpret_cast<const float4*>(p); };
+    auto dot = [](const float4& x, const float4& y) { return fmaf(x.x, y.x, fmaf(x.y, y.y, fmaf(x.z, y.z, x.w * y.w))); };
+    auto times = [](float4& x, const float4& w) { x.x *= w.x; x.y *= w.y; x.z *= w.z; x.w *= w.w; };
+    float4 kj = four(&ks[pair][at]), aj = four(&as[pair][at]);
+    for (int step = 0; step <= CK; ++step) {      // token `pair` through the tokens from it on, then token 15 - pair
+      const bool second = step >= CK - pair;
+      const int j = second ? CK - 1 - pair : pair, i = second ? step - 1 : pair + step;
+      if (step == CK - pair) {
+        kj = four(&ks[j][at]);
+        aj = four(&as[j][at]);
+      }
+      const float4 u = four(&us[i][at]), x = four(&rs[i][at]), w = four(&ws[i][at]);
+      const float uk = dot(u, kj), ua = dot(u, aj);      // with the decays up to the token before i
+      if (i > j) {
+        times(kj, w);
+        times(aj, w);
+      }
+      const float rk = dot(x, kj), ra = dot(x, aj);      // with i's own too
+      // Four sums over sixteen lanes: lane bits 3 and 2 say whose.
+      const bool b3 = tid & 8, b2 = tid & 4;
+      const float x0 = (b3 ? rk : uk) + __shfl_xor_sync(0xffffffffu, b3 ? uk : rk, 8);
+      const float x1 = (b3 ? ra : ua) + __shfl_xor_sync(0xffffffffu, b3 ? ua : ra, 8);
+      float s = (b2 ? x1 : x0) + __shfl_xor_sync(0xffffffffu, b2 ? x0 : x1, 4);
+      s += __shfl_xor_sync(0xffffffffu, s, 2);
+      s += __shfl_xor_sync(0xffffffffu, s, 1);
+      if ((tid & 3) == 0) sums[tid >> 2 & 3][i][j] = s;
+    }
+  }
+  __syncthreads();
+  // The rows with their decays: u and r from the chunk's start, k and a to its end. Beside that the system.
+  if (tid < DMAX) {
+    float up = 1.f, down = 1.f;
+#pragma unroll
+    for (int t = CK - 1; t >= 0; --t) {
+      ks[t][tid] *= down;
+      as[t][tid] *= down;
+      down *= ws[t][tid];
+    }
+#pragma unroll
+    for (int t = 0; t < CK; ++t) {
+      us[t][tid] *= up;
+      up *= ws[t][tid];
+      rs[t][tid] *= up;
+    }
+    tile[ck_rows(CK_GENERAL, DMAX) + tid] = up;
+  } else if (warp == 3) {
+    if (lane < CK) ck_solve(&sums[1][0][0], GS, -1.f, lane, 1.f, T);
+  } else {
+    for (int e = lane; e < CK * CK; e += 32) {
+      const int i = e / CK, j = e % CK;
+      ck_set(E, i, j, j < i ? sums[0][i][j] : 0.f);
+      ck_set(R, i, j, j <= i ? sums[2][i][j] : 0.f);
+      ck_set(Q, i, j, j <= i ? sums[3][i][j] : 0.f);
+    }
+  }
+  __syncthreads();
+  {
+    uint32_t a[3][4];
+    float x[8], f[8];
+    auto rows_of = [&](const float (*m)[RS], float (&y)[8]) {
+#pragma unroll
+      for (int e = 0; e < 8; ++e) y[e] = m[ck_token(lane, e)][c0 + ck_channel(lane, e)];
+    };
+    rows_of(us, x);
+    rows_of(rs, f);
+    ck_system_rows(tile, ROW, c0, lane, T, Q, x, f);
+    ck_operand(f, a);
+    ck_put(tile, CK_F, ROW, c0, lane, a);
+    rows_of(as, x);
+    ck_operand(x, a);
+    ck_put(tile, CK_B, ROW, c0, lane, a);
+    rows_of(ks, x);
+    ck_operand(x, a);
+    ck_put(tile, CK_C, ROW, c0, lane, a);
+  }
+  {
+    float e_v[8], y[8], o[8];
+#pragma unroll
+    for (int e = 0; e < 8; ++e) e_v[e] = y[e] = o[e] = 0.f;
+    ck_apply(R, value, lane, o);
+    ck_apply(E, value, lane, e_v);
+    ck_apply(T, e_v, lane, y);
+    ck_apply(Q, y, lane, o);
+#pragma unroll
+    for (int e = 0; e < 8; ++e) {
+      const int t = ck_token(lane, e), c = c0 + ck_channel(lane, e);
+      if (t < have && c < d) {
+        const size_t to = (t0 + t) * width + (size_t)h * d + c;
+        v_out[to] = value[e];
+        u_out[to] = y[e];
+        g_out[to] = o[e];
+      }
+    }
+  }
+  ck_tile_written();
+  __syncthreads();
+  if (tid == 0) {
+    ck_tile_leaves(tiles + ((size_t)place * n_heads + h) * ck_tile(CK_GENERAL, DMAX), tile, ck_tile(CK_GENERAL, DMAX));
+    ck_tile_left();
   }
 }
 
@@ -328,33 +504,52 @@ static int launch_delta(int dmax, dim3 grid, cudaStream_t stream, const void* r,
   float* o_raw = work + (size_t)DR_ROWS * rows * d;
   if (walk_from > 0) {
     auto up4 = [](size_t v) { return (v + 3) & ~(size_t)3; };
-    const size_t places = (size_t)walk_places(n_tokens, n_requests), plane = (size_t)rows * d;
-    float* w = work + up4((size_t)(DR_ROWS + 1) * rows * d);
-    float* tables = w + up4(places * n_heads * d);
-    const dim3 grid_t((unsigned)places, (n_heads + 3) / 4);
-    const int piece = d <= 64 ? 2 : 4;
-    auto starts = [&](const void* p, size_t size) { return ((uintptr_t)p & (piece * size - 1)) == 0; };
-    const bool vec_f = d % piece == 0 && starts(decay_raw, 4);
-    const bool vec = d % piece == 0 && in_stride % piece == 0 && starts(r, sizeof(TA)) && starts(k, sizeof(TA)) &&
-                     starts(v, sizeof(TA)) && starts(a_raw, sizeof(TA));
+    int rc;
+    if (ck_takes(CK_GENERAL, d, d)) {
+      const size_t plane = (size_t)rows * d;
+      float *u = work + up4((size_t)(DR_ROWS + 1) * rows * d), *g = u + plane, *v_rows = g + plane, *tiles = v_rows + plane;
+      constexpr size_t smem_rows = 4 * (ck_tile(CK_GENERAL, 64) + 5 * CK * 68);
+      cudaError_t e = cudaFuncSetAttribute(delta_rows_kernel<TA>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem_rows);
+      if (e != cudaSuccess) return llmrs_fail("delta_rule: shared memory %zu: %s", smem_rows, cudaGetErrorString(e));
+      delta_rows_kernel<TA><<<dim3((unsigned)ck_places(n_tokens, n_requests), n_heads), 128, smem_rows, stream>>>(
+          (const TA*)r, (const TA*)k, (const TA*)v, (const TA*)a_raw, in_stride, decay_raw, decay_bias, a_bias, q_start, n_new, tiles,
+          u, g, v_rows, n_requests, n_heads, d, decay_scale, key_eps, walk_from);
+      rc = llmrs_launch_status("delta_rule (chunks)");
+      if (rc != 0) return rc;
+      ChunkArgs a = {};
+      a.tiles = tiles; a.u = u; a.g = g; a.v = v_rows; a.state = state; a.o_raw = o_raw;
+      a.q_start = q_start; a.n_new = n_new; a.slot_ids = slot_ids;
+      a.n_heads = n_heads; a.d = a.dv = a.columns = d; a.from = walk_from;
+      rc = launch_state_chunks<CK_GENERAL>(a, n_requests, stream);
+    } else {
+      const size_t places = (size_t)walk_places(n_tokens, n_requests), plane = (size_t)rows * d;
+      float* w = work + up4((size_t)(DR_ROWS + 1) * rows * d);
+      float* tables = w + up4(places * n_heads * d);
+      const dim3 grid_t((unsigned)places, (n_heads + 3) / 4);
+      const int piece = d <= 64 ? 2 : 4;
+      auto starts = [&](const void* p, size_t size) { return ((uintptr_t)p & (piece * size - 1)) == 0; };
+      const bool vec_f = d % piece == 0 && starts(decay_raw, 4);
+      const bool vec = d % piece == 0 && in_stride % piece == 0 && starts(r, sizeof(TA)) && starts(k, sizeof(TA)) &&
+                       starts(v, sizeof(TA)) && starts(a_raw, sizeof(TA));
 #define LLMRS_DR_TURNS(CPL)                                                                                               \
-  delta_turns_kernel<TA, CPL><<<grid_t, 128, 0, stream>>>((const TA*)r, (const TA*)k, (const TA*)v, (const TA*)a_raw, in_stride, \
-                                                          decay_raw, decay_bias, a_bias, q_start, n_new, prep, w, tables, \
-                                                          n_tokens, n_requests, n_heads, d, decay_scale, key_eps, vec, vec_f, \
-                                                          walk_from)
-    if (d <= 64) LLMRS_DR_TURNS(2);
-    else if (d <= 128) LLMRS_DR_TURNS(4);
-    else LLMRS_DR_TURNS(8);
+    delta_turns_kernel<TA, CPL><<<grid_t, 128, 0, stream>>>((const TA*)r, (const TA*)k, (const TA*)v, (const TA*)a_raw, in_stride, \
+                                                            decay_raw, decay_bias, a_bias, q_start, n_new, prep, w, tables, \
+                                                            n_tokens, n_requests, n_heads, d, decay_scale, key_eps, vec, vec_f, \
+                                                            walk_from)
+      if (d <= 64) LLMRS_DR_TURNS(2);
+      else if (d <= 128) LLMRS_DR_TURNS(4);
+      else LLMRS_DR_TURNS(8);
 #undef LLMRS_DR_TURNS
-    int rc = llmrs_launch_status("delta_rule (turns)");
-    if (rc != 0) return rc;
-    WalkArgs a = {};
-    a.q = prep; a.k = prep + plane; a.kb = prep + 2 * plane; a.ab = prep + 3 * plane; a.v = prep + 4 * plane; a.w = w;
-    a.q_stride = a.k_stride = a.b_stride = (long long)n_heads * d;
-    a.tables = tables; a.state = state; a.o_raw = o_raw;
-    a.q_start = q_start; a.n_new = n_new; a.slot_ids = slot_ids;
-    a.n_heads = a.n_groups = n_heads; a.d = a.dv = d; a.from = walk_from;
-    rc = launch_state_walk<WALK_GENERAL>(a, n_requests, d, stream);
+      rc = llmrs_launch_status("delta_rule (turns)");
+      if (rc != 0) return rc;
+      WalkArgs a = {};
+      a.q = prep; a.k = prep + plane; a.kb = prep + 2 * plane; a.ab = prep + 3 * plane; a.v = prep + 4 * plane; a.w = w;
+      a.q_stride = a.k_stride = a.b_stride = (long long)n_heads * d;
+      a.tables = tables; a.state = state; a.o_raw = o_raw;
+      a.q_start = q_start; a.n_new = n_new; a.slot_ids = slot_ids;
+      a.n_heads = a.n_groups = n_heads; a.d = a.dv = d; a.from = walk_from;
+      rc = launch_state_walk<WALK_GENERAL>(a, n_requests, d, stream);
+    }
     if (rc != 0) return rc;
     if (walk_from == 1) return launch_delta_out<TA>(o_raw, gate, in_stride, norm_w, out, n_tokens, n_heads, d, norm_eps, stream);
   }
@@ -387,7 +582,9 @@ static int launch_delta(int dmax, dim3 grid, cudaStream_t stream, const void* r,
 // Float32 workspace the three kernels share, in floats.
 LLMRS_API long long llmrs_delta_rule_work_floats(int n_tokens, int n_requests, int n_heads, int d) {
   return (long long)(DR_ROWS + 1) * n_tokens * n_heads * d + 16 +
-         walk_places(n_tokens, n_requests) * n_heads * (d + walk_table(WALK_GENERAL));
+         std::max(walk_places(n_tokens, n_requests) * n_heads * (d + walk_table(WALK_GENERAL)),
+                  ck_takes(CK_GENERAL, d, d) ? ck_work_floats(CK_GENERAL, n_tokens, n_requests, n_heads, d, d) + (long long)n_tokens * n_heads * d
+                                             : 0);
 }
 
 // r, k, v, gate, a_raw: [tokens, ...] of the activation type, rows `in_stride` elements apart, each pointing at its

@@ -18,8 +18,8 @@
 //
 //   prepare      a block per token: convolutions + SiLU, unit q and k, g and beta, as float32 rows
 //   conv state   a block per request, after prepare: the request's last K - 1 convolution inputs
-//   (requests that are walked in turns: the rows and coefficients of turns of four tokens by one kernel in place of
-//   `prepare`, then the walk, state_walk.cuh)
+//   (requests that are walked: rows by one kernel in place of `prepare`, then, heads of up to 128 channels, the chunks' rows and
+//   the walk of state_chunks.cuh; others the coefficients of turns of four tokens with the rows and the walk of state_walk.cuh)
 //   recurrence   of the others, token by token: a block per (request, head, slice of 16 value
 //                columns) walks the request's tokens; four
 //                neighbouring lanes share a column, each with a quarter of the key channels in registers (lane p of the
@@ -41,14 +41,14 @@
 // products per chunk over rows that arrive through two shared-memory buffers, 32 tokens per sequential step instead of
 // one. A chunk's missing tokens (a portion's end) count as k = q = v = 0, beta = 0, g = 1 and change nothing.
 // The chunked form is OFF by default (llmrs_gated_delta_chunked): its products read every operand from shared memory
-// and are bound by that (2,048 tokens of 16 heads of 128 x 128: some 500 us, the walk in turns 265).
+// and are bound by that (2,048 tokens of 16 heads of 128 x 128: some 500 us, the walk in turns 265, in chunks on the tensor cores 116).
 #include <limits.h>
 
 #include "common.cuh"
 #include "head_out.cuh"
 #include "mma_util.cuh"
 #include "short_conv.cuh"
-#include "state_walk.cuh"
+#include "state_chunks.cuh"
 
 // CHANNEL: a decay per key channel; ba is then unused, b (activation type) and araw (float32 [tokens, H d]) take its place
 // and pg is [tokens, H d].
@@ -303,14 +303,14 @@ __device__ __forceinline__ void gdr_convolve(const TA* __restrict__ x, long long
   }
 }
 
-template <typename TA, int CPL, bool CHANNEL>
+template <typename TA, int CPL, bool CHANNEL, bool CHUNKS>
 __global__ void __launch_bounds__(128, CPL == 4 ? 6 : 1)
 gdr_turns_kernel(const TA* __restrict__ x, long long stride, const float* __restrict__ taps, const float* __restrict__ ba,
                  const TA* __restrict__ b, long long b_stride, const float* __restrict__ araw, const float* __restrict__ a_log,
                  const float* __restrict__ dt_bias, const float* __restrict__ conv_state, const int* __restrict__ q_start,
                  const int* __restrict__ n_new, const int* __restrict__ slot_ids, float* __restrict__ pq,
                  float* __restrict__ pk, float* __restrict__ kb, float* __restrict__ pv, float* __restrict__ w,
-                 float* __restrict__ tables, int n_requests, int G, int H, int d, int dv, int K, float key_eps, float q_scale,
+                 float* __restrict__ tables, float* __restrict__ pbeta, float* __restrict__ pg, int n_requests, int G, int H, int d, int dv, int K, float key_eps, float q_scale,
                  bool vec, bool taps4, int from) {
   const int place = blockIdx.x, unit = blockIdx.y * 4 + (threadIdx.x >> 5), lane = threadIdx.x & 31;
   const int wq = G * d, wv = H * dv, C = 2 * wq + wv;
@@ -349,13 +349,24 @@ gdr_turns_kernel(const TA* __restrict__ x, long long stride, const float* __rest
       q[t][m] = t < have ? q[t][m] * iq : 0.f;
       k[t][m] = t < have ? k[t][m] * ik : 0.f;
     }
-    if (!CHANNEL && t < have) {
+    if ((CHUNKS || !CHANNEL) && t < have) {
       walk_store<CPL>(pq + (t0 + t) * wq + (size_t)unit * d, lane, d, vec, q[t]);
       walk_store<CPL>(pk + (t0 + t) * wq + (size_t)unit * d, lane, d, vec, k[t]);
     }
   }
   const int shared = H / G;
-  if constexpr (!CHANNEL) {
+  if constexpr (CHUNKS) {      // the rows as they are, each token's write strengths and, one a head, decays
+    for (int e = lane; e < have * shared; e += 32) {
+      const int h = unit * shared + e % shared;
+      const size_t at = t0 + e / shared;
+      if (CHANNEL) {
+        pbeta[at * H + h] = rec_sigmoid(to_float(b[at * b_stride + h]));
+      } else {
+        pbeta[at * H + h] = rec_sigmoid(ba[at * 2 * H + h]);
+        pg[at * H + h] = expf(-expf(a_log[h]) * rec_softplus(ba[at * 2 * H + H + h] + dt_bias[h]));
+      }
+    }
+  } else if constexpr (!CHANNEL) {
     // q_i . k_j (j <= i) at i (i + 1) / 2 + j, k_i . k_j (j < i) at 10 + i (i - 1) / 2 + j.
     float sums[16];
 #pragma unroll
@@ -446,6 +457,175 @@ gdr_turns_kernel(const TA* __restrict__ x, long long stride, const float* __rest
       walk_write_table<WALK_CHANNEL>(tables + ((size_t)place * H + h) * 36, sum, ones, bt, lane);
     }
   }
+}
+
+// ---- the walk in chunks of sixteen tokens (state_chunks.cuh) with a decay per key channel ---------------------------------
+// A block per (place, head). The coefficients between the tokens are products over the channels with the decays between them: a warp
+// walks a token j through the tokens after it, the decays multiplied on as they go (no quotients: nothing overflows), and then token
+// 15 - j, so that every warp has seventeen steps. Then sixteen channels and sixteen columns a warp at a time.
+constexpr int GCR_THREADS = 256;
+__host__ __device__ constexpr int gcr_smem(int dmax) { return 4 * (ck_tile(CK_SYSTEM, dmax) + 3 * CK * (dmax + 4)); }
+template <int DMAX>
+__global__ void __launch_bounds__(GCR_THREADS)
+gdr_channel_rows_kernel(const float* __restrict__ pq, const float* __restrict__ pk, const float* __restrict__ pv,
+                        const float* __restrict__ pbeta, const float* __restrict__ araw, const float* __restrict__ a_log,
+                        const float* __restrict__ dt_bias, const int* __restrict__ q_start, const int* __restrict__ n_new,
+                        float* __restrict__ tiles, float* __restrict__ u, float* __restrict__ g_out, int n_requests, int G, int H,
+                        int d, int dv, int from) {
+  constexpr int GS = CK + 1, RS = DMAX + 4, ROW = DMAX + 8, PER = DMAX / 32;
+  constexpr int EACH = (CK * (DMAX / 4) + GCR_THREADS - 1) / GCR_THREADS;
+  extern __shared__ __align__(128) float gcr_raw[];
+  float* tile = gcr_raw;
+  auto q = reinterpret_cast<float (*)[RS]>(tile + ck_tile(CK_SYSTEM, DMAX));
+  auto k = q + CK, g = k + CK;
+  __shared__ __align__(16) __nv_bfloat16 Q[CK_MATRIX], T[CK_MATRIX];
+  __shared__ float sums[2][CK][GS], strength[CK];
+  const int place = blockIdx.x, h = blockIdx.y, tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
+  int t_req, n_req;
+  const int req = ck_request(q_start, n_new, n_requests, place, t_req, n_req);
+  const int first = (place - ck_place(t_req, req)) * CK, have = min(CK, n_req - first);
+  if (first < 0 || have <= 0 || n_req < from) return;
+  const size_t t0 = (size_t)(t_req + first);
+  const int kh = h / (H / G);
+  {
+    float4 in[EACH][3], bias[EACH];
+    const float strong = tid < have ? pbeta[(t0 + tid) * H + h] : 0.f, rate = -expf(a_log[h]);
+#pragma unroll
+    for (int x = 0; x < EACH; ++x) {
+      const int e = tid + x * GCR_THREADS, t = e / (DMAX / 4), c = e % (DMAX / 4) * 4;
+      in[x][0] = in[x][1] = in[x][2] = bias[x] = make_float4(0.f, 0.f, 0.f, 0.f);
+      if (t < have && c < d) {
+        const size_t at = ((t0 + t) * G + kh) * d + c;
+        in[x][0] = __ldg(reinterpret_cast<const float4*>(pq + at));
+        in[x][1] = __ldg(reinterpret_cast<const float4*>(pk + at));
+        const float *a = araw + ((t0 + t) * H + h) * d + c, *b = dt_bias + (size_t)h * d + c;      // (any alignment)
+        in[x][2] = make_float4(__ldg(a), __ldg(a + 1), __ldg(a + 2), __ldg(a + 3));
+        bias[x] = make_float4(__ldg(b), __ldg(b + 1), __ldg(b + 2), __ldg(b + 3));
+      }
+    }
+    if (tid < CK) strength[tid] = strong;
+    auto decay = [&](float a, float b) { return expf(rate * rec_softplus(a + b)); };
+#pragma unroll
+    for (int x = 0; x < EACH; ++x) {
+      const int e = tid + x * GCR_THREADS, t = e / (DMAX / 4), c = e % (DMAX / 4) * 4;
+      if (t >= CK) continue;
+      float4 w = make_float4(1.f, 1.f, 1.f, 1.f);
+      if (t < have && c < d)
+        w = make_float4(decay(in[x][2].x, bias[x].x), decay(in[x][2].y, bias[x].y), decay(in[x][2].z, bias[x].z), decay(in[x][2].w, bias[x].w));
+      *reinterpret_cast<float4*>(&q[t][c]) = in[x][0];
+      *reinterpret_cast<float4*>(&k[t][c]) = in[x][1];
+      *reinterpret_cast<float4*>(&g[t][c]) = w;
+    }
+  }
+  __syncthreads();
+  {
+    struct alignas(4 * PER) Piece { float x[PER]; };
+    auto piece = [&](const float* row) { return *reinterpret_cast<const Piece*>(row + PER * lane); };
+    Piece kj = piece(k[warp]);
+    for (int step = 0; step <= CK; ++step) {      // token `warp` through the tokens from it on, then token 15 - warp
+      const bool second = step >= CK - warp;
+      const int j = second ? CK - 1 - warp : warp, i = second ? step - 1 : warp + step;
+      if (step == CK - warp) kj = piece(k[j]);
+      const Piece qi = piece(q[i]), ki = piece(k[i]), w = piece(g[i]);
+      float a = 0.f, b = 0.f;                     // q_i . k_j, k_i . k_j
+#pragma unroll
+      for (int m = 0; m < PER; ++m) {
+        if (i > j) kj.x[m] *= w.x[m];
+        a = fmaf(qi.x[m], kj.x[m], a);
+        b = fmaf(ki.x[m], kj.x[m], b);
+      }
+      const bool high = lane & 16;
+      float s = (high ? b : a) + __shfl_xor_sync(0xffffffffu, high ? a : b, 16);
+#pragma unroll
+      for (int x = 8; x > 0; x >>= 1) s += __shfl_xor_sync(0xffffffffu, s, x);
+      if ((lane & 15) == 0) sums[high][i][j] = s;
+    }
+  }
+  // The values that this warp needs below are on their way.
+  float v[8];
+  auto fetch = [&](int group) {
+#pragma unroll
+    for (int e = 0; e < 8; ++e) {
+      const int t = ck_token(lane, e), col = 16 * group + ck_channel(lane, e);
+      v[e] = t < have && col < dv ? __ldg(pv + ((t0 + t) * H + h) * dv + col) : 0.f;
+    }
+  };
+  if (16 * warp < dv) fetch(warp);
+  __syncthreads();
+  // The rows with their decays: q and -k from the chunk's start, k to its end (in g's place). Beside that the system.
+  if (tid < DMAX) {
+    float up = 1.f, down = 1.f, to_end[CK];
+#pragma unroll
+    for (int t = CK - 1; t >= 0; --t) {
+      to_end[t] = k[t][tid] * down;
+      down *= g[t][tid];
+    }
+#pragma unroll
+    for (int t = 0; t < CK; ++t) {
+      up *= g[t][tid];
+      q[t][tid] *= up;
+      k[t][tid] *= -up;
+      g[t][tid] = to_end[t];
+    }
+    tile[ck_rows(CK_SYSTEM, DMAX) + tid] = up;
+  } else if (warp == 4 && lane < CK) {
+#pragma unroll
+    for (int i = 0; i < CK; ++i) sums[1][i][lane] *= strength[i];      // (each lane its own column)
+    __syncwarp(0xffffu);
+    ck_solve(&sums[1][0][0], GS, 1.f, lane, strength[lane], T);
+  } else if (warp > 4) {
+    for (int e = tid - 160; e < CK * CK; e += GCR_THREADS - 160) ck_set(Q, e / CK, e % CK, e % CK <= e / CK ? sums[0][e / CK][e % CK] : 0.f);
+  }
+  __syncthreads();
+  for (int c0 = 16 * warp; c0 < DMAX; c0 += 16 * (GCR_THREADS / 32)) {
+    uint32_t a[3][4];
+    float x[8], f[8], b[8];
+#pragma unroll
+    for (int e = 0; e < 8; ++e) {
+      const int t = ck_token(lane, e), c = c0 + ck_channel(lane, e);
+      x[e] = k[t][c];
+      f[e] = q[t][c];
+      b[e] = g[t][c];
+    }
+    ck_system_rows(tile, ROW, c0, lane, T, Q, x, f);
+    ck_operand(f, a);
+    ck_put(tile, CK_F, ROW, c0, lane, a);
+    ck_operand(b, a);
+    ck_put(tile, CK_B, ROW, c0, lane, a);
+  }
+  ck_tile_written();
+  for (int group = warp; 16 * group < dv; group += GCR_THREADS / 32) {
+    if (group != warp) fetch(group);
+    float y[8], o[8];
+#pragma unroll
+    for (int e = 0; e < 8; ++e) y[e] = o[e] = 0.f;
+    ck_apply(T, v, lane, y);
+    ck_apply(Q, y, lane, o);
+#pragma unroll
+    for (int e = 0; e < 8; ++e) {
+      const int t = ck_token(lane, e), col = 16 * group + ck_channel(lane, e);
+      if (t < have && col < dv) {
+        u[((t0 + t) * H + h) * dv + col] = y[e];
+        g_out[((t0 + t) * H + h) * dv + col] = o[e];
+      }
+    }
+  }
+  __syncthreads();
+  if (tid == 0) {
+    ck_tile_leaves(tiles + ((size_t)place * H + h) * ck_tile(CK_SYSTEM, DMAX), tile, ck_tile(CK_SYSTEM, DMAX));
+    ck_tile_left();
+  }
+}
+template <int DMAX>
+static int launch_channel_rows(dim3 grid, cudaStream_t stream, const float* pq, const float* pk, const float* pv, const float* pbeta,
+                               const float* araw, const float* a_log, const float* dt_bias, const int* q_start, const int* n_new,
+                               float* tiles, float* u, float* g, int n_requests, int G, int H, int d, int dv, int from) {
+  constexpr size_t smem = gcr_smem(DMAX);
+  cudaError_t e = cudaFuncSetAttribute(gdr_channel_rows_kernel<DMAX>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
+  if (e != cudaSuccess) return llmrs_fail("gated_delta: shared memory %zu: %s", smem, cudaGetErrorString(e));
+  gdr_channel_rows_kernel<DMAX><<<grid, GCR_THREADS, smem, stream>>>(pq, pk, pv, pbeta, araw, a_log, dt_bias, q_start, n_new, tiles, u,
+                                                                     g, n_requests, G, H, d, dv, from);
+  return llmrs_launch_status("gated_delta (chunks)");
 }
 
 // ---- the recurrence in chunks ------------------------------------------------------------------------------------
@@ -726,13 +906,13 @@ static int launch_chunked(const float* pq, const float* pk, const float* pv, con
 }
 
 struct TurnRows {      // what gdr_turns_kernel leaves in the workspace
-  float *pq, *pk, *kb, *pv, *w, *tables;
+  float *pq, *pk, *kb, *pv, *w, *tables, *pbeta, *pg;
 };
 template <typename TA>
 static int launch_turns(const TA* x, long long x_stride, const float* taps, const float* ba, const TA* b, long long b_stride,
                         const float* araw, const float* a_log, const float* dt_bias, const float* conv_state, const TurnRows& r,
                         const int* q_start, const int* n_new, const int* slot_ids, int n_tokens, int n_requests, int G, int H,
-                        int d, int dv, int K, float key_eps, float q_scale, int from, cudaStream_t stream) {
+                        int d, int dv, int K, float key_eps, float q_scale, int from, bool chunks, cudaStream_t stream) {
   auto rows_of_four = [](const void* p, size_t size, long long stride) { return ((uintptr_t)p & (4 * size - 1)) == 0 && stride % 4 == 0; };
   const bool vec = d % 4 == 0 && H * dv % 4 == 0 && rows_of_four(x, sizeof(TA), x_stride) && rows_of_four(conv_state, 4, 4) &&
                    rows_of_four(araw, 4, 4);
@@ -740,14 +920,16 @@ static int launch_turns(const TA* x, long long x_stride, const float* taps, cons
   const int cpl = d <= 128 ? 4 : 8, units = G + (H * dv + 32 * cpl - 1) / (32 * cpl);
   LLMRS_REQUIRE((units + 3) / 4 <= 65535, "gated_delta: too many heads");
   const dim3 grid((unsigned)walk_places(n_tokens, n_requests), (units + 3) / 4);
-#define LLMRS_GD_TURNS(CPL, CH)                                                                                               \
-  gdr_turns_kernel<TA, CPL, CH><<<grid, 128, 0, stream>>>(x, x_stride, taps, ba, b, b_stride, araw, a_log, dt_bias, conv_state, \
-                                                          q_start, n_new, slot_ids, r.pq, r.pk, r.kb, r.pv, r.w, r.tables,    \
+#define LLMRS_GD_TURNS(CPL, CH, CHUNKS)                                                                                       \
+  gdr_turns_kernel<TA, CPL, CH, CHUNKS><<<grid, 128, 0, stream>>>(x, x_stride, taps, ba, b, b_stride, araw, a_log, dt_bias, conv_state, \
+                                                          q_start, n_new, slot_ids, r.pq, r.pk, r.kb, r.pv, r.w, r.tables, r.pbeta, r.pg, \
                                                           n_requests, G, H, d, dv, K, key_eps, q_scale, vec, taps4, from)
-  if (araw && cpl == 4) LLMRS_GD_TURNS(4, true);
-  else if (araw) LLMRS_GD_TURNS(8, true);
-  else if (cpl == 4) LLMRS_GD_TURNS(4, false);
-  else LLMRS_GD_TURNS(8, false);
+  if (araw && chunks) LLMRS_GD_TURNS(4, true, true);
+  else if (chunks) LLMRS_GD_TURNS(4, false, true);
+  else if (araw && cpl == 4) LLMRS_GD_TURNS(4, true, false);
+  else if (araw) LLMRS_GD_TURNS(8, true, false);
+  else if (cpl == 4) LLMRS_GD_TURNS(4, false, false);
+  else LLMRS_GD_TURNS(8, false, false);
 #undef LLMRS_GD_TURNS
   return llmrs_launch_status("gated_delta (turns)");
 }
@@ -765,13 +947,43 @@ static int launch_turn_walk(bool channel, const TurnRows& r, float* state, const
   return channel ? launch_state_walk<WALK_CHANNEL>(a, n_requests, dv, stream) : launch_state_walk<WALK_GATED>(a, n_requests, dv, stream);
 }
 
+// The chunks' counterpart: pq, pk, pv, pbeta (and pg) hold the rows as gdr_turns_kernel<CHUNKS> left them.
+static int launch_chunk_walk(bool channel, const TurnRows& r, float* work, const float* araw, const float* a_log,
+                             const float* dt_bias, float* state, const int* q_start, const int* n_new, const int* slot_ids,
+                             float* o_raw, int n_tokens, int n_requests, int G, int H, int d, int dv, int from,
+                             cudaStream_t stream) {
+  float *u = work, *g = u + (size_t)n_tokens * H * dv, *tiles = g + (size_t)n_tokens * H * dv;
+  int rc;
+  if (channel) {
+    LLMRS_REQUIRE(H <= 65535, "gated_delta: too many heads");
+    const dim3 grid((unsigned)ck_places(n_tokens, n_requests), H);
+    rc = (d <= 64 ? launch_channel_rows<64> : launch_channel_rows<128>)(grid, stream, r.pq, r.pk, r.pv, r.pbeta, araw, a_log, dt_bias,
+                                                                        q_start, n_new, tiles, u, g, n_requests, G, H, d, dv, from);
+  } else {
+    ChunkRowsArgs a = {};
+    a.q = r.pq; a.k = r.pk; a.stride = (long long)G * d; a.v = r.pv; a.decay = r.pg; a.beta = r.pbeta;
+    a.q_start = q_start; a.n_new = n_new; a.tiles = tiles; a.u = u; a.g = g;
+    a.n_requests = n_requests; a.n_heads = H; a.n_groups = G; a.d = d; a.dv = a.columns = dv; a.from = from;
+    rc = launch_ck_rows<CK_SYSTEM>(a, n_tokens, stream);
+  }
+  if (rc != 0) return rc;
+  ChunkArgs a = {};
+  a.tiles = tiles; a.u = u; a.g = g; a.state = state; a.o_raw = o_raw;
+  a.q_start = q_start; a.n_new = n_new; a.slot_ids = slot_ids;
+  a.n_heads = H; a.d = d; a.dv = a.columns = dv; a.from = from;
+  return launch_state_chunks<CK_SYSTEM>(a, n_requests, stream);
+}
+
 // Float32 workspace of the kernels, in floats: prepared q, k, v, beta, g and the raw read-outs.
 LLMRS_API long long llmrs_gated_delta_work_floats(int n_tokens, int n_requests, int G, int H, int d, int dv, int channel) {
-  const long long turns = walk_places(n_tokens, n_requests) * H;      // the walk in turns: coefficients, decays
+  // The walk in turns: coefficients, decays; in chunks: their rows.
+  const long long turns = walk_places(n_tokens, n_requests) * H;
+  const long long sixteens = ck_takes(CK_SYSTEM, d, dv) ? ck_work_floats(CK_SYSTEM, n_tokens, n_requests, H, d, dv) : 0;
   if (channel)
-    return (long long)n_tokens * (2LL * G * d + 2LL * H * dv + 4LL * H * d + H) + 48 + turns * (d + walk_table(WALK_CHANNEL));
+    return (long long)n_tokens * (2LL * G * d + 2LL * H * dv + 1LL * H * d + H) + 48 +
+           std::max(3LL * n_tokens * H * d + turns * (d + walk_table(WALK_CHANNEL)), sixteens);
   const long long chunk_places = n_tokens / GC_C + n_requests + 1;
-  const long long chunks = chunk_places * H * GC_TABLE, tables = turns * walk_table(WALK_GATED);
+  const long long chunks = chunk_places * H * GC_TABLE, tables = std::max(turns * walk_table(WALK_GATED), sixteens);
   return (long long)n_tokens * (2LL * G * d + 2LL * H * dv + 3LL * H) + 24 + (chunks > tables ? chunks : tables);
 }
 
@@ -821,6 +1033,8 @@ LLMRS_API int llmrs_gated_delta(const void* x, long long x_stride, const void* g
   // The walk's rows with a decay per key channel follow o_raw; its tables lie where the chunked form's would.
   const size_t hd = up4((size_t)n_tokens * H * d);
   float *qf = tables, *kf = qf + hd, *kb = kf + hd, *turn_w = kb + hd;
+  const bool sixteens = from > 0 && ck_takes(CK_SYSTEM, d, dv);
+  float* chunk_work = tables;
   if (channel) tables = turn_w + up4((size_t)walk_places(n_tokens, n_requests) * H * d);
   const size_t smem = (size_t)C * sizeof(float);
   const int dmax = d <= 32 ? 32 : (d <= 64 ? 64 : (d <= 128 ? 128 : 256));
@@ -859,14 +1073,15 @@ LLMRS_API int llmrs_gated_delta(const void* x, long long x_stride, const void* g
         (const T*)x, x_stride, taps, ba, (const T*)b, b_stride, araw, a_log, dt_bias, conv_state, token_req, q_start,  \
         n_new, slot_ids, pq, pk, pv, pbeta, pg, plg, G, H, d, dv, K, key_eps, q_scale, below);                         \
   } while (0)
-  const TurnRows turn_rows = {channel ? qf : pq, channel ? kf : pk, kb, pv, turn_w, tables};
+  const bool decayed = channel && !sixteens;
+  const TurnRows turn_rows = {decayed ? qf : pq, decayed ? kf : pk, kb, pv, turn_w, tables, pbeta, pg};
 #define LLMRS_GD_LAUNCH(T)                                                                                             \
   do {                                                                                                                 \
     int rc = 0;                                                                                                        \
     if (from > 0) {                                                                                                    \
       rc = launch_turns<T>((const T*)x, x_stride, taps, ba, (const T*)b, b_stride, araw, a_log, dt_bias, conv_state,   \
                            turn_rows, q_start, n_new, slot_ids, n_tokens, n_requests, G, H, d, dv, K, key_eps,         \
-                           q_scale, from, stream);                                                                     \
+                           q_scale, from, sixteens, stream);                                                           \
       if (rc != 0) return rc;                                                                                          \
     }                                                                                                                  \
     if (from != 1) {                                                                                                   \
@@ -880,6 +1095,10 @@ LLMRS_API int llmrs_gated_delta(const void* x, long long x_stride, const void* g
     if (chunked) {                                                                                                     \
       rc = launch_chunked(pq, pk, pv, pbeta, plg, tables, state, q_start, n_new, slot_ids, o_raw, n_requests,          \
                           max_chunks, G, H, d, dv, stream);                                                            \
+      if (rc != 0) return rc;                                                                                          \
+    } else if (sixteens) {                                                                                             \
+      rc = launch_chunk_walk(channel, turn_rows, chunk_work, araw, a_log, dt_bias, state, q_start, n_new, slot_ids, o_raw, \
+                             n_tokens, n_requests, G, H, d, dv, from, stream);                                         \
       if (rc != 0) return rc;                                                                                          \
     } else if (from > 0) {                                                                                             \
       rc = launch_turn_walk(channel, turn_rows, state, q_start, n_new, slot_ids, o_raw, n_requests, G, H, d, dv, from, \

@@ -17,7 +17,8 @@
 //                a_t = exp(f_t + m_(t-1) - m_t), b_t = exp(i_t - m_t), floor_t = exp(-m_t); m is kept per slot;
 //   prepare      q, k, v of all tokens widened to float32 (optional SiLU, optional rotation of the first channels of every
 //                head of q and k by halves, q and k scaled, k multiplied by its gain);
-//   (requests that are walked in turns: the coefficients of turns of four tokens, then the walk, state_walk.cuh)
+//   (requests that are walked: the rows of chunks of sixteen tokens, then the walk, state_chunks.cuh; heads that it does not take: the
+//   coefficients of turns of four tokens, then the walk, state_walk.cuh)
 //   recurrence   of the others: a block per (request, head, 16 value columns) walks the tokens in order; four or eight adjacent lanes
 //                share a column, each holding its part of the column's key channels in registers; rows arrive through two
 //                shared-memory buffers by 16-byte asynchronous copies. A step of one token and a prompt's portion
@@ -32,7 +33,7 @@
 #include "head_out.cuh"
 #include "mma_util.cuh"
 #include "short_conv.cuh"
-#include "state_walk.cuh"
+#include "state_chunks.cuh"
 
 __device__ __forceinline__ float lr_logsigmoid(float x) { return fminf(x, 0.f) - log1pf(expf(-fabsf(x))); }
 
@@ -422,15 +423,32 @@ LLMRS_API int llmrs_linear_recurrence_planes(const float* Q, const float* K, con
     LLMRS_REQUIRE(((uintptr_t)tables & 15) == 0 && tables != nullptr, "linear_recurrence: no workspace for a portion");
     LLMRS_REQUIRE(((uintptr_t)V & 15) == 0, "linear_recurrence: planes must be 16-byte aligned");
     const long long stride = (long long)n_groups * dk;
-    int rc = launch_walk_tables(Q, K, stride, decay, head_decay, v_gain, q_start, n_new, tables, n_tokens,
-                                             n_requests, n_heads, n_groups, dk, walk_from, stream);
-    if (rc != 0) return rc;
-    WalkArgs a = {};
-    a.q = Q; a.k = K; a.q_stride = a.k_stride = stride; a.v = V; a.tables = tables; a.skip = skip;
-    a.state = S; a.norm_state = N; a.o_raw = o_raw; a.nq = nq;
-    a.q_start = q_start; a.n_new = n_new; a.slot_ids = slot_ids;
-    a.n_heads = n_heads; a.n_groups = n_groups; a.d = dk; a.dv = dv; a.from = walk_from;
-    rc = launch_state_walk<WALK_LINEAR>(a, n_requests, cols, stream);
+    int rc;
+    if (ck_takes(CK_LINEAR, dk, dv)) {
+      const int columns = ck_columns(dv, N != nullptr);
+      ChunkRowsArgs r = {};
+      r.q = Q; r.k = K; r.stride = stride; r.v = V; r.decay = decay; r.head_decay = head_decay; r.beta = v_gain; r.skip = skip;
+      r.q_start = q_start; r.n_new = n_new; r.n_requests = n_requests; r.n_heads = n_heads; r.n_groups = n_groups;
+      r.d = dk; r.dv = dv; r.columns = columns; r.from = walk_from; r.norm = N != nullptr;
+      r.u = tables; r.g = r.u + (size_t)n_tokens * n_heads * columns; r.tiles = r.g + (size_t)n_tokens * n_heads * columns;
+      rc = launch_ck_rows<CK_LINEAR>(r, n_tokens, stream);
+      if (rc != 0) return rc;
+      ChunkArgs a = {};
+      a.tiles = r.tiles; a.u = r.u; a.g = r.g; a.state = S; a.norm_state = N; a.o_raw = o_raw; a.nq = nq;
+      a.q_start = q_start; a.n_new = n_new; a.slot_ids = slot_ids;
+      a.n_heads = n_heads; a.d = dk; a.dv = dv; a.columns = columns; a.from = walk_from;
+      rc = launch_state_chunks<CK_LINEAR>(a, n_requests, stream);
+    } else {
+      rc = launch_walk_tables(Q, K, stride, decay, head_decay, v_gain, q_start, n_new, tables, n_tokens,
+                                               n_requests, n_heads, n_groups, dk, walk_from, stream);
+      if (rc != 0) return rc;
+      WalkArgs a = {};
+      a.q = Q; a.k = K; a.q_stride = a.k_stride = stride; a.v = V; a.tables = tables; a.skip = skip;
+      a.state = S; a.norm_state = N; a.o_raw = o_raw; a.nq = nq;
+      a.q_start = q_start; a.n_new = n_new; a.slot_ids = slot_ids;
+      a.n_heads = n_heads; a.n_groups = n_groups; a.d = dk; a.dv = dv; a.from = walk_from;
+      rc = launch_state_walk<WALK_LINEAR>(a, n_requests, cols, stream);
+    }
     if (rc != 0 || walk_from == 1) return rc;
   }
   const int below = walk_from > 0 ? walk_from : INT_MAX;
@@ -452,15 +470,16 @@ LLMRS_API int llmrs_linear_recurrence_planes(const float* Q, const float* K, con
   return llmrs_launch_status("linear_recurrence");
 }
 
-// Floats of the workspace `tables` of llmrs_linear_recurrence_planes: the coefficients of a portion's turns.
-LLMRS_API long long llmrs_linear_recurrence_table_floats(int n_tokens, int n_requests, int n_heads) {
+// Floats of the workspace `tables` of llmrs_linear_recurrence_planes: the coefficients of a portion's turns, or the rows of its chunks.
+LLMRS_API long long llmrs_linear_recurrence_table_floats(int n_tokens, int n_requests, int n_heads, int dk, int dv) {
+  if (ck_takes(CK_LINEAR, dk, dv)) return ck_work_floats(CK_LINEAR, n_tokens, n_requests, n_heads, dk, ck_columns(dv, true));
   return walk_places(n_tokens, n_requests) * n_heads * walk_table(WALK_LINEAR);
 }
 
 // Floats of workspace for llmrs_linear_recurrence: the three prepared planes and the tables.
 LLMRS_API long long llmrs_linear_recurrence_work_floats(int n_tokens, int n_requests, int n_heads, int dk, int dv) {
   return (long long)n_tokens * n_heads * (2LL * dk + dv) + 12 +
-         llmrs_linear_recurrence_table_floats(n_tokens, n_requests, n_heads);
+         llmrs_linear_recurrence_table_floats(n_tokens, n_requests, n_heads, dk, dv);
 }
 
 // q, k, v: [tokens, ...] of the activation type with their row strides, head h's channels at h * dk (h * dv);

@@ -978,6 +978,23 @@ def _walk_blocks(n_heads: int, cols: int) -> int:
     return n_heads * -(-cols // 16)
 
 
+def _in_chunks(d: int, dv: int, most: int = 128) -> bool:
+    """Walked requests go sixteen tokens a time on the tensor cores (csrc/state_chunks.cuh ``ck_takes``), others four a turn."""
+    return d % 4 == 0 and dv % 4 == 0 and d <= most
+
+
+def _chunk_rule(least: int, few: int, per: int) -> dict:
+    """``walk_from``'s lines where walked requests go in chunks: their blocks weigh three times a turn's, so fewer short requests ride
+    along. Measured, token by token / all in chunks / both (us, a whole mixer, as in ``walk_from``):
+      gated    3 + 64 78 / 67 / 81    15 + 64 84 / 107 / 98    15 + 256 165 / 134 / 127    63 + 128 161 / 302 / 185    63 + 256 211 / 319 / 196
+      linear   3 + 64 66 / 55 / 52    15 + 64 73 / 100 / 70    15 + 256 160 / 123 / 90     63 + 64 130 / 286 / 147     63 + 128 156 / 292 / 154
+      general  3 + 64 89 / 52 / 54    15 + 64 82 / 89 / 66     15 + 256 220 / 117 / 91     63 + 64 108 / 249 / 115     63 + 128 155 / 262 / 124"""
+    return dict(least=least, few=few, per=per)
+
+
+LINEAR_CHUNKS = _chunk_rule(WALK_PORTION, 400, 128)
+
+
 def _gated_walk_least(channels: int, d: int, channel: bool) -> int:
     """Tokens from which on one portion of the gated delta rule is faster in turns: the kernel that makes a turn's rows takes some
     18 us however few channels (30 with a decay per channel), the one that prepares single tokens 4.5 for 1,024 channels, and a
@@ -989,6 +1006,12 @@ def _gated_walk_least(channels: int, d: int, channel: bool) -> int:
     else:
         line = 240 - 54 * channels // 1024 if d <= 64 else 140 - 25 * channels // 1024
     return max(WALK_PORTION, line)
+
+
+def _gated_chunk_least(channels: int, channel: bool) -> int:
+    """The same line for chunks. Measured crossings (one portion, token by token against in chunks): 1,024 channels 132 tokens, 4,096 45;
+    with a decay per channel 2,048 92, 4,096 below 16."""
+    return max(WALK_PORTION, (140 - 24 * channels // 1024) if channel else (160 - 28 * channels // 1024))
 
 
 # -- the generalized delta rule -------------------------------------------------------------------------
@@ -1007,8 +1030,9 @@ def delta_rule(r, k, v, gate, a_raw, decay_raw, decay_bias, a_bias, norm_w, stat
     out = torch.empty((r.size(0), n_heads * d), dtype=r.dtype, device=r.device)
     work = torch.empty((int(_lib_ll("llmrs_delta_rule_work_floats")(r.size(0), ctx.n_requests, n_heads, d)),),
                        dtype=torch.float32, device=r.device)
-    # (heads of 32: one portion 128 tokens 47 / 47 us, heads of 64: 48 tokens 54 / 48)
-    turns = walk_from(ctx, r.size(0), _walk_blocks(n_heads, d), least=128 if d <= 32 else WALK_PORTION)
+    # (in chunks heads of 32: one portion of 48 tokens 40 / 41 us, 64 tokens 45 / 43; heads of 64: 32 tokens 48 / 46)
+    rule = _chunk_rule(64 if d <= 32 else WALK_PORTION, 640, 128) if _in_chunks(d, d, 64) else dict(least=128 if d <= 32 else WALK_PORTION)
+    turns = walk_from(ctx, r.size(0), _walk_blocks(n_heads, d), **rule)
     _check(_lib().llmrs_delta_rule(
         _ptr(r), _ptr(k), _ptr(v), _ptr(gate), _ptr(a_raw), _LL(stride), dtype_code(r.dtype), _ptr(decay_raw),
         _ptr(decay_bias), _ptr(a_bias), _ptr(norm_w), _ptr(state), _ptr(ctx.q_start), _ptr(ctx.n_new),
@@ -1278,7 +1302,8 @@ def linear_recurrence(q, k, v, gate, norm_w, state, ctx, n_heads: int, dk: int, 
     if (normaliser is None) != (floor is None):
         raise KernelError("linear_recurrence: normaliser and floor come together")
     dev = q.device
-    turns = walk_from(ctx, n, _walk_blocks(n_heads, dv + (normaliser is not None)), few=1024)
+    turns = walk_from(ctx, n, _walk_blocks(n_heads, dv + (normaliser is not None)),
+                      **(LINEAR_CHUNKS if _in_chunks(dk, dv) else dict(few=1024)))
     # One workspace: the kernels' rows, then the raw read-outs and the normaliser's products.
     n_work = -(-int(_lib_ll("llmrs_linear_recurrence_work_floats")(n, ctx.n_requests, n_heads, dk, dv)) // 4) * 4
     work = torch.empty((n_work + n * n_heads * (dv + 1),), dtype=torch.float32, device=dev)
@@ -1325,9 +1350,9 @@ def ssd(xbc: torch.Tensor, z: torch.Tensor, dt_raw: torch.Tensor, taps: torch.Te
     _need(out, "out", xbc.dtype, contiguous=False)
     empty = lambda width: torch.empty((n, width), dtype=torch.float32, device=xbc.device)
     X, B, Cq, decay, step, y = empty(inner), empty(wk), empty(wk), empty(n_heads), empty(n_heads), empty(inner)
-    turns = walk_from(ctx, n, _walk_blocks(n_heads, vdim), few=1024)
-    tables = torch.empty((int(_lib_ll("llmrs_linear_recurrence_table_floats")(n, ctx.n_requests, n_heads)) if turns else 0,),
-                         dtype=torch.float32, device=xbc.device)
+    turns = walk_from(ctx, n, _walk_blocks(n_heads, vdim), **(LINEAR_CHUNKS if _in_chunks(n_state, vdim) else dict(few=1024)))
+    n_tables = int(_lib_ll("llmrs_linear_recurrence_table_floats")(n, ctx.n_requests, n_heads, n_state, vdim)) if turns else 0
+    tables = torch.empty((n_tables,), dtype=torch.float32, device=xbc.device)
     _check(_lib().llmrs_ssd_prepare(
         _ptr(xbc), _LL(_row_stride(xbc, "xbc")), _ptr(dt_raw), _LL(_row_stride(dt_raw, "dt_raw")), dtype_code(xbc.dtype),
         _ptr(taps), _ptr(conv_bias), _ptr(dt_bias), _ptr(a_log), _ptr(conv_state), _ptr(ctx.token_req), _ptr(ctx.q_start),
@@ -1764,7 +1789,9 @@ def gated_delta(x: torch.Tensor, gate: torch.Tensor, taps: torch.Tensor, ba: Opt
     work = torch.empty((int(_lib_ll("llmrs_gated_delta_work_floats")(n, ctx.n_requests, n_kv_heads, n_heads, dk, dv,
                                                                      int(channel))),),
                        dtype=torch.float32, device=x.device)
-    turns = walk_from(ctx, n, _walk_blocks(n_heads, dv), least=_gated_walk_least(C, dk, channel), per=32)
+    chunks = _in_chunks(dk, dv)
+    rule = _chunk_rule(_gated_chunk_least(C, channel), 1500, 64) if chunks else dict(least=_gated_walk_least(C, dk, channel), per=32)
+    turns = walk_from(ctx, n, _walk_blocks(n_heads, dv), **rule)
     _check(_lib().llmrs_gated_delta(
         _ptr(x), _LL(_row_stride(x, "x")), _ptr(gate), _LL(_row_stride(gate, "gate")), dtype_code(x.dtype), _ptr(taps),
         _ptr(None if channel else ba), _ptr(b), _LL(_row_stride(b, "b") if channel else 0), _ptr(channel_decay),
@@ -1772,7 +1799,7 @@ def gated_delta(x: torch.Tensor, gate: torch.Tensor, taps: torch.Tensor, ba: Opt
         _ptr(ctx.n_new), _ptr(ctx.slot_ids), _ptr(work), _ptr(out), _LL(_row_stride(out, "out")), n, ctx.n_requests,
         n_kv_heads, n_heads, dk, dv, K, ctypes.c_float(key_eps), ctypes.c_float(q_scale), ctypes.c_float(norm_eps),
         ctypes.c_float(out_scale), int(gate_sigmoid), turns, _stream()), "gated_delta",
-        (4 if K > 1 else 3) + (2 if turns > 1 else 0))
+        (4 if K > 1 else 3) + (2 if turns > 1 else 0) + int(bool(turns) and chunks))
     return out
 
 

@@ -56,6 +56,15 @@ def test_convolutions_of_turns(kind, taps, d, dv, lens):
     _compare(kind, d, dv, lens, taps)
 
 
+@pytest.mark.parametrize("kind", ["memory", "retention", "mamba", "gated", "channel", "general"])
+@pytest.mark.parametrize("d,dv,lens", [(64, 64, [16, 17, 15, 1, 33]), (36, 20, [31, 32, 48, 2]), (128, 4, [50]), (4, 16, [16, 5] * 20),
+                                       (100, 132, [35, 0, 64]), (60, 60, [97])])
+def test_chunks_at_their_edges(kind, d, dv, lens):
+    """Heads that chunks of sixteen tokens take (csrc/state_chunks.cuh): whole and broken chunks, requests between others' places,
+    channels and columns that fill no tile."""
+    _compare(kind, d, dv, lens, 4)
+
+
 class _in_turns:
     """The step's requests of at least ``turns`` tokens are walked in turns, whatever the rule says."""
 
