@@ -549,11 +549,17 @@ attn_prefill_tc_kernel(const __grid_constant__ CUtensorMap map_kv, const __grid_
         }
         const bool need_mask = kb + AT_BK - 1 > pos0 || (window > 0 && kb <= pos0 + AT_BQ - 1 - window) || kb < last_lo;
         if (need_mask) {
+          // The row sees the tile's columns a .. b (one comparison of unsigned numbers a column), and with kept keys those below
+          // `kept` too. (Written as the conditions stand, with their shortcuts, a masked tile took 17,000 cycles, an unmasked one
+          // 2,000, and a kernel over windows of 1,024 half its time.)
+          const int a = max(window > 0 ? my_pos - window + 1 : 0, my_lo) - kb, b = my_pos - kb, kept = keep - kb;
+          const unsigned span = b >= a ? (unsigned)(b - a) + 1u : 0u;
+          if (kept > 0) {
 #pragma unroll
-          for (int c = 0; c < AT_BK; ++c) {
-            const int key = kb + c;
-            const bool seen = key <= my_pos && (window <= 0 || key > my_pos - window || key < keep) && key >= my_lo;
-            s[c] = seen ? s[c] : -INFINITY;
+            for (int c = 0; c < AT_BK; ++c) s[c] = ((unsigned)(c - a) < span) | ((c < kept) & (c <= b)) ? s[c] : -INFINITY;
+          } else {
+#pragma unroll
+            for (int c = 0; c < AT_BK; ++c) s[c] = (unsigned)(c - a) < span ? s[c] : -INFINITY;
           }
         }
         // Four running maxima (and sums below): a chain of 128 dependent operations would be the
