@@ -815,7 +815,7 @@ attn_prefill_mma_kernel(const bf16* __restrict__ q, long long q_stride, bf16* __
           for (int e = 0; e < 4; ++e) {
             const int key = kb + n * 8 + tq * 2 + (e & 1);
             const int p = pos_r[e >> 1];
-            const bool seen = key <= p && (window <= 0 || key > p - window);
+            const bool seen = (key <= p) & ((window <= 0) | (key > p - window));
             s[n][e] = seen ? s[n][e] : -INFINITY;
             mx[e >> 1] = fmaxf(mx[e >> 1], s[n][e]);
           }

@@ -776,8 +776,9 @@ scored_prefill_mma_kernel(const bf16* __restrict__ q, long long q_stride, bf16* 
 #pragma unroll
           for (int e = 0; e < 4; ++e) {
             const int key = kb + n * 8 + tq * 2 + (e & 1);
-            const bool seen = key <= pos_r[e >> 1] && (key >= lo_r[e >> 1] || key < opt.keep);
-            s[n][e] = seen ? cap(s[n][e]) : -INFINITY;
+            const bool seen = (key <= pos_r[e >> 1]) & ((key >= lo_r[e >> 1]) | (key < opt.keep));
+            s[n][e] = cap(s[n][e]);
+            s[n][e] = seen ? s[n][e] : -INFINITY;
             mx[e >> 1] = fmaxf(mx[e >> 1], s[n][e]);
           }
       } else {
