@@ -35,6 +35,37 @@ MAX_CLUSTER = 16     # splits that the kernel merges itself
 PREFILL_TILE = 64    # queries per entry of the prefill attention kernels' tile list
 
 
+def prefill_work(step: StepInfo, n_tiles: int) -> tuple:
+    """What a step's prompt portions bring to their attention kernel, for ``tc_pays``: the most keys that a portion sees, blocks of 64
+    queries and the keys of all of them together, the same for blocks of 128."""
+    if n_tiles == 0:
+        return (0, 0, 0, 0, 0)
+    n = np.asarray(step.n_new, np.int64)
+    n, keys = n[n > 1], (np.asarray(step.cached_len, np.int64) + n)[n > 1]
+    few, many = -(-n // 64), -(-n // 128)
+    return int(keys.max()), int(few.sum()), int((few * keys).sum()), int(many.sum()), int((many * keys).sum())
+
+
+# us of the mma.sync and the tcgen05 kernel, by the longest chain of keys (at 0, a key) and by all blocks (at 0, a block, a block's key,
+# both of 16 heads): plain attention, attention with options on the score.
+_PREFILL_US = {False: ((4.6, 0.042, 5.0, 0.13, 0.0023), (6.9, 0.0088, 4.6, 0.45, 0.0009)),
+               True: ((5.5, 0.068, 8.0, 0.14, 0.0037), (8.4, 0.0085, 4.6, 0.45, 0.0009))}
+
+
+def tc_pays(work: tuple, heads: int, window: int, scored: bool) -> bool:
+    """True where the tcgen05 kernel (blocks of 128 queries) is the faster one for portions that fill its blocks less than half. It
+    walks a tile of keys in a fifth of the time, so it pays wherever there are keys to walk; the other starts sooner and holds more
+    blocks. Measured, mma.sync / tcgen05 (us, heads of 128; plain, 16 heads | with a gate, 16 heads): one portion of 20 tokens 5.1 / 7.3 |
+    7.3 / 8.6, of 20 after 500 26.8 / 12.7 | 41 / 14, of 8 after 2,000 90 / 24 | 142 / 25; 64 portions of 30 21 / 33 | 28 / 39, the same
+    after 100 41 / 44 | 59 / 52; 200 portions of 2 after 30 40 / 87 | 56 / 102, after 500 259 / 167 | 419 / 188."""
+    longest, few, few_keys, many, many_keys = work
+    if window > 0:
+        longest, few_keys, many_keys = min(longest, window + 64), min(few_keys, few * (window + 64)), min(many_keys, many * (window + 64))
+    cost = lambda c, blocks, keys: max(c[0] + c[1] * longest, c[2] + heads / 16 * (c[3] * blocks + c[4] * keys))
+    mma, tc = _PREFILL_US[scored]
+    return many > 0 and cost(tc, many, many_keys) <= cost(mma, few, few_keys)
+
+
 # A block of the kernel with the ring of two tiles (three blocks an SM) takes about this much longer than one of the
 # usual kernel (two blocks an SM, two tiles on their way per warp): it pays only where it saves a wave.
 LIGHT_COST = 1.3
@@ -197,7 +228,8 @@ class GQAttention(Mixer):
             max_kv = max(t.shape[1] for t in step.block_tables) * step.page_size
         return Plan(arrays={"prefill_tiles": tiles, "decode_reqs": decode},
                     values={"n_prefill_tiles": int(tiles.shape[0]), "n_decode": int(decode.size),
-                            "max_decode_kv_len": int(max_kv), "long_portions": int(long_portions)})
+                            "max_decode_kv_len": int(max_kv), "long_portions": int(long_portions),
+                            "prefill_work": prefill_work(step, int(tiles.shape[0]))})
 
     def _fuses_rope(self, x, cache, cos_sin) -> bool:
         """True when the q|k|v product can take norms, rotation and cache write as its epilogue."""
@@ -268,7 +300,8 @@ class GQAttention(Mixer):
         if n_tiles:
             ops.attn_prefill(q, out, cache.kv, plan.arrays["prefill_tiles"], n_tiles, ctx.q_start, ctx.n_new,
                              ctx.cached_len, table, nq, nkv, d, cache.page_size, self.window, self.scale,
-                             prefer_tc=bool(plan.values["long_portions"]) and _ATTN_TC)
+                             prefer_tc=_ATTN_TC and (bool(plan.values["long_portions"])
+                                                     or tc_pays(plan.values["prefill_work"], nq, self.window, False)))
         if n_decode:
             split_keys, ring = (self.split_keys, 3) if self.split_keys else self._choose_split(n_decode, max_kv, q)
             max_splits = max(1, -(-max_kv // split_keys))

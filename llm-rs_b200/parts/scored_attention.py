@@ -8,7 +8,7 @@ from typing import Mapping, Optional
 import torch
 
 from .. import host, ops
-from .attention import _ATTN_TC, PREFILL_TILE
+from .attention import _ATTN_TC, PREFILL_TILE, prefill_work, tc_pays
 from .base import Mixer, Plan, Runtime, StepInfo
 from .linear import Linear
 from .position import wavelength_scaled_frequencies
@@ -199,7 +199,8 @@ class ScoredAttention(Mixer):
             max_kv = max(t.shape[1] for t in step.block_tables) * step.page_size
         return Plan(arrays={"prefill_tiles": tiles, "decode_reqs": decode},
                     values={"n_prefill_tiles": int(tiles.shape[0]), "n_decode": int(decode.size),
-                            "max_decode_kv_len": int(max_kv), "long_portions": int(long_portions)})
+                            "max_decode_kv_len": int(max_kv), "long_portions": int(long_portions),
+                            "prefill_work": prefill_work(step, int(tiles.shape[0]))})
 
     def heads(self, x, ctx, cache, out: Optional[torch.Tensor] = None, out_scale: float = 1.0) -> torch.Tensor:
         """The concatenated heads [tokens, n_heads * vdim] before the output projection, times ``out_scale``, written
@@ -244,7 +245,9 @@ class ScoredAttention(Mixer):
         scale = 1.0 if gate is not None else out_scale
         if n_tiles:
             ops.scored_prefill(q, out, pages, plan.arrays["prefill_tiles"], n_tiles, ctx, table, *args,
-                               prefer_tc=bool(plan.values["long_portions"]) and _ATTN_TC, bias=self.bias,
+                               prefer_tc=_ATTN_TC and (bool(plan.values["long_portions"])
+                                                       or tc_pays(plan.values["prefill_work"], self.n_heads, self.mask_size, True)),
+                               bias=self.bias,
                                out_scale=scale, keep=self.keep_first, gate=head_gate)
         if n_decode:
             span = max(1, min(max_kv, self.mask_size + self.keep_first) if self.mask_size else max_kv)   # keys a query can see at most

@@ -85,3 +85,16 @@ def test_without_a_light_kernel_nothing_changes():
         assert cut_keys_and_ring(4096, units, held, lambda cluster: 0) == (cut_keys(4096, units, held), 3)
         assert cut_keys_and_ring(4096, units, held) == (cut_keys(4096, units, held), 3)
     assert LIGHT_COST > 1
+
+
+@pytest.mark.parametrize("lens,cached,heads,window,plain,scored", [
+    ([40], [0], 16, 0, False, False), ([20], [500], 16, 0, True, True), ([8], [2000], 8, 257, True, True),
+    ([30] * 64, [0] * 64, 16, 0, False, False), ([30] * 64, [200] * 64, 16, 0, True, True),
+    ([2] * 200, [30] * 200, 32, 0, False, False), ([2] * 200, [500] * 200, 16, 0, True, True),
+    ([1] * 9, [700] * 9, 16, 0, False, False)])
+def test_prefill_kernel_of_short_portions(lens, cached, heads, window, plain, scored):
+    """The tcgen05 kernel where there are keys to walk, mma.sync for many or short portions over few keys."""
+    from types import SimpleNamespace
+    from llm_rs_b200.parts.attention import prefill_work, tc_pays
+    work = prefill_work(SimpleNamespace(n_new=lens, cached_len=cached), int(max(lens) > 1))
+    assert tc_pays(work, heads, window, False) == plain and tc_pays(work, heads, window, True) == scored
