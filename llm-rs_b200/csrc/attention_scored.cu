@@ -1272,7 +1272,7 @@ scored_decode_grouped_kernel(const T* __restrict__ q, long long q_stride, const 
 }
 
 // The decode kernel for bfloat16 heads of 64 or 128 channels (keys and values alike): one block per (decode request, key head,
-// up to four of the query heads that share it, run of keys), four warps, each with a ring of three tiles of 16 keys that
+// up to four of the query heads that share it, run of keys), four warps, each with a ring of two tiles of 16 keys that
 // asynchronous copies fill, a row's pieces by neighbouring lanes. The products run on the tensor cores (m16n8k16, the
 // bfloat16 products exact, the sums float32). Weights keep their 24 bits: a weight is the sum of three bfloat16 numbers, and
 // the rows of the tile that the heads leave free carry them, heads' first pieces in rows 0-3, second in 4-7, third in 8-11;
@@ -1281,11 +1281,14 @@ scored_decode_grouped_kernel(const T* __restrict__ q, long long q_stride, const 
 //
 // Against the kernel of a lane per key, whose neighbouring lanes read rows 512 bytes apart (both with the merge, us): 64 requests of
 // 2,041 keys, 16 heads over 4 of 128: 128 -> 73 (3.7 TB/s); 8 of 4,096: 50 -> 37; 1 of 4,000: 24 -> 18; 1 of 100: 13.4 -> 9.4;
-// 48 of 2,000 with heads of 64: 77 -> 34. Bound by the latency of three tiles in flight a warp.
-constexpr int SM_KEYS = 16, SM_STAGES = 3;
+// 48 of 2,000 with heads of 64: 77 -> 34. Those with rings of three tiles and two blocks an SM; with two tiles and three blocks 48 of
+// 200 to 4,100 keys take 49 us (4.3 TB/s) where they took 60, 48 of 2,000 47 (57), heads of 64 70 (72): bound by the 700 instructions a
+// tile and warp, each of which waits for the one before, so more warps help and more tiles in flight do not (four blocks of 128
+// registers spill: 55).
+constexpr int SM_KEYS = 16, SM_STAGES = 2;
 template <int D> __host__ __device__ constexpr int sm_ring_bytes() { return SM_STAGES * 2 * SM_KEYS * (D + 8) * 2; }      // of a warp
 template <int D>
-__global__ void __launch_bounds__(SD_THREADS, 2)
+__global__ void __launch_bounds__(SD_THREADS, 3)
 scored_decode_mma_kernel(const bf16* __restrict__ q, long long q_stride, const bf16* __restrict__ cache,
                          const int* __restrict__ dec_reqs, const int* __restrict__ q_start, const int* __restrict__ cached_len,
                          const int* __restrict__ block_table, int table_stride, float* __restrict__ part, int max_splits,
