@@ -13,7 +13,7 @@
 //               widened, as six float32 rows [tokens, heads * d];
 //   (requests that are walked take their rows and the walk of state_chunks.cuh instead of these two, heads of more than 64 channels
 //   `turns` and the walk of state_walk.cuh; 2,048 tokens of 32 heads of 64 x 64: 816 us walked one by one, 246 in turns, 92 in
-//   chunks; their rows 136 us, those of turns 56, where `prepare` takes 38)
+//   chunks; their rows 106 us, those of turns 56, where `prepare` takes 38)
 //   recurrence  one block per (request, head, slice of 16 value columns) walks the request's tokens of the step in
 //               order: a column of S depends on no other column, so the slices run side by side. Four adjacent lanes
 //               share a column, each keeping a quarter of its key channels in registers; u^T S and S^T r are summed
@@ -193,7 +193,8 @@ delta_rows_kernel(const TA* __restrict__ r, const TA* __restrict__ k, const TA* 
   constexpr int GS = CK + 1, DMAX = 64, RS = DMAX + 4, ROW = DMAX + 8;
   extern __shared__ __align__(128) float dr_raw[];
   float* tile = dr_raw;
-  auto ks = reinterpret_cast<float (*)[RS]>(tile + ck_tile(CK_GENERAL, DMAX));
+  float* tile_out = tiles + ((size_t)blockIdx.x * n_heads + blockIdx.y) * ck_tile(CK_GENERAL, DMAX);
+  auto ks = reinterpret_cast<float (*)[RS]>(tile + ck_rows(2, DMAX));      // (two planes of the tile at a time: four blocks an SM)
   auto rs = ks + CK, us = rs + CK, as = us + CK, ws = as + CK;
   __shared__ __align__(16) __nv_bfloat16 E[CK_MATRIX], R[CK_MATRIX], Q[CK_MATRIX], T[CK_MATRIX];
   __shared__ float sums[4][CK][GS];      // u_i . k_j, u_i . a_j, r_i . k_j, r_i . a_j
@@ -297,7 +298,7 @@ delta_rows_kernel(const TA* __restrict__ r, const TA* __restrict__ k, const TA* 
       up *= ws[t][tid];
       rs[t][tid] *= up;
     }
-    tile[ck_rows(CK_GENERAL, DMAX) + tid] = up;
+    tile_out[ck_rows(CK_GENERAL, DMAX) + tid] = up;
   } else if (warp == 3) {
     if (lane < CK) ck_solve(&sums[1][0][0], GS, -1.f, lane, 1.f, T);
   } else {
@@ -318,15 +319,16 @@ delta_rows_kernel(const TA* __restrict__ r, const TA* __restrict__ k, const TA* 
     };
     rows_of(us, x);
     rows_of(rs, f);
-    ck_system_rows(tile, ROW, c0, lane, T, Q, x, f);
+    ck_system_rows(tile, 1, ROW, c0, lane, T, Q, x, f);
     ck_operand(f, a);
-    ck_put(tile, CK_F, ROW, c0, lane, a);
-    rows_of(as, x);
-    ck_operand(x, a);
-    ck_put(tile, CK_B, ROW, c0, lane, a);
-    rows_of(ks, x);
-    ck_operand(x, a);
-    ck_put(tile, CK_C, ROW, c0, lane, a);
+    ck_put(tile, 0, ROW, c0, lane, a);
+    ck_tile_written();
+    __syncthreads();
+    if (tid == 0) {
+      ck_tile_leaves(tile_out + CK_F * ck_rows(1, DMAX), tile, ck_rows(1, DMAX));
+      ck_tile_leaves(tile_out + CK_W * ck_rows(1, DMAX), tile + ck_rows(1, DMAX), ck_rows(1, DMAX));
+      ck_tile_left();
+    }
   }
   {
     float e_v[8], y[8], o[8];
@@ -347,10 +349,21 @@ delta_rows_kernel(const TA* __restrict__ r, const TA* __restrict__ k, const TA* 
       }
     }
   }
+  __syncthreads();      // F and W have left
+#pragma unroll
+  for (int plane = 0; plane < 2; ++plane) {
+    uint32_t a[3][4];
+    float x[8];
+#pragma unroll
+    for (int e = 0; e < 8; ++e) x[e] = (plane ? ks : as)[ck_token(lane, e)][c0 + ck_channel(lane, e)];
+    ck_operand(x, a);
+    ck_put(tile, plane, ROW, c0, lane, a);
+  }
   ck_tile_written();
   __syncthreads();
   if (tid == 0) {
-    ck_tile_leaves(tiles + ((size_t)place * n_heads + h) * ck_tile(CK_GENERAL, DMAX), tile, ck_tile(CK_GENERAL, DMAX));
+    ck_tile_leaves(tile_out + CK_B * ck_rows(1, DMAX), tile, ck_rows(1, DMAX));
+    ck_tile_leaves(tile_out + CK_C * ck_rows(1, DMAX), tile + ck_rows(1, DMAX), ck_rows(1, DMAX));
     ck_tile_left();
   }
 }
@@ -508,7 +521,7 @@ static int launch_delta(int dmax, dim3 grid, cudaStream_t stream, const void* r,
     if (ck_takes(CK_GENERAL, d, d)) {
       const size_t plane = (size_t)rows * d;
       float *u = work + up4((size_t)(DR_ROWS + 1) * rows * d), *g = u + plane, *v_rows = g + plane, *tiles = v_rows + plane;
-      constexpr size_t smem_rows = 4 * (ck_tile(CK_GENERAL, 64) + 5 * CK * 68);
+      constexpr size_t smem_rows = 4 * (ck_rows(2, 64) + 5 * CK * 68);
       cudaError_t e = cudaFuncSetAttribute(delta_rows_kernel<TA>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem_rows);
       if (e != cudaSuccess) return llmrs_fail("delta_rule: shared memory %zu: %s", smem_rows, cudaGetErrorString(e));
       delta_rows_kernel<TA><<<dim3((unsigned)ck_places(n_tokens, n_requests), n_heads), 128, smem_rows, stream>>>(

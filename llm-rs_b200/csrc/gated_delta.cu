@@ -587,7 +587,7 @@ gdr_channel_rows_kernel(const float* __restrict__ pq, const float* __restrict__ 
       f[e] = q[t][c];
       b[e] = g[t][c];
     }
-    ck_system_rows(tile, ROW, c0, lane, T, Q, x, f);
+    ck_system_rows(tile, CK_W, ROW, c0, lane, T, Q, x, f);
     ck_operand(f, a);
     ck_put(tile, CK_F, ROW, c0, lane, a);
     ck_operand(b, a);

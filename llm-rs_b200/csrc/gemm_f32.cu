@@ -470,12 +470,23 @@ gemm_f32_skinny_kernel(const TX* __restrict__ x, const float* __restrict__ w, co
   __shared__ float parts[SK_WARPS][SK_TOKENS];
   TX* xs = reinterpret_cast<TX*>(sk_raw);      // [SK_TOKENS][K]
   const int m0 = blockIdx.x * SK_TOKENS, rows = min(SK_TOKENS, M - m0);
-  for (int i = threadIdx.x; i < SK_TOKENS * K; i += SK_THREADS) {
-    const int r = i / K, k = i - r * K;
-    xs[i] = r < rows ? x[(size_t)(m0 + r) * x_stride + k] : TX(0.f);
+  const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
+  static_assert(SK_WARPS == SK_TOKENS, "a warp a row");
+  // Sixteen bytes at a time, a warp a row, where rows start on such a boundary (value by value with a division each, the rows took
+  // longer than the product: 8 bfloat16 rows of 2,048 into 33 features 9.1 us, 3.7 so).
+  constexpr int PIECE = 16 / (int)sizeof(TX);
+  if (K % PIECE == 0 && x_stride % PIECE == 0 && ((uintptr_t)x & 15) == 0) {
+    const uint4* from = reinterpret_cast<const uint4*>(x + (size_t)(m0 + min(warp, rows - 1)) * x_stride);
+    uint4* to = reinterpret_cast<uint4*>(xs + (size_t)warp * K);
+#pragma unroll 4
+    for (int i = lane; i < K / PIECE; i += 32) to[i] = warp < rows ? __ldg(from + i) : make_uint4(0u, 0u, 0u, 0u);
+  } else {
+    for (int i = threadIdx.x; i < SK_TOKENS * K; i += SK_THREADS) {
+      const int r = i / K, k = i - r * K;
+      xs[i] = r < rows ? x[(size_t)(m0 + r) * x_stride + k] : TX(0.f);
+    }
   }
   __syncthreads();
-  const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
   const int n = SPLIT ? (int)blockIdx.y : (int)blockIdx.y * SK_WARPS + warp;
   const bool live = n < N;
   const float* wr = w + (size_t)(live ? n : 0) * K;
@@ -488,14 +499,14 @@ gemm_f32_skinny_kernel(const TX* __restrict__ x, const float* __restrict__ w, co
   const int k_lo = SPLIT ? warp * piece : 0, k_hi = min(K4, k_lo + piece);
   if (live) {
     for (int k = k_lo + lane * 4; k < k_hi; k += 128) {
-      const float4 wv = *reinterpret_cast<const float4*>(wr + k);
+      const float4 wv = __ldg(reinterpret_cast<const float4*>(wr + k));
 #pragma unroll
       for (int r = 0; r < SK_TOKENS; ++r) {
-        const TX* xr = xs + r * K + k;
-        acc[r] = fmaf(to_float(xr[0]), wv.x, acc[r]);
-        acc[r] = fmaf(to_float(xr[1]), wv.y, acc[r]);
-        acc[r] = fmaf(to_float(xr[2]), wv.z, acc[r]);
-        acc[r] = fmaf(to_float(xr[3]), wv.w, acc[r]);
+        const float4 xv = gf_four(xs + r * K + k);      // (K is a multiple of four)
+        acc[r] = fmaf(xv.x, wv.x, acc[r]);
+        acc[r] = fmaf(xv.y, wv.y, acc[r]);
+        acc[r] = fmaf(xv.z, wv.z, acc[r]);
+        acc[r] = fmaf(xv.w, wv.w, acc[r]);
       }
     }
     if (!SPLIT || warp == SK_WARPS - 1)

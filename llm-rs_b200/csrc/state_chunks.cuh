@@ -439,8 +439,8 @@ __device__ __forceinline__ void ck_put(float* tile, int plane, int row, int c0, 
     asm volatile("stmatrix.sync.aligned.m8n8.x4.trans.shared.b16 [%0], {%1, %2, %3, %4};\n"
                  ::"r"(smem_addr(to + k * CK * row)), "r"(a[k][0]), "r"(a[k][1]), "r"(a[k][2]), "r"(a[k][3]) : "memory");
 }
-// W = T x into its plane, then F = f + Q W into its own.
-__device__ __forceinline__ void ck_system_rows(float* tile, int row, int c0, int lane, const __nv_bfloat16* T, const __nv_bfloat16* Q,
+// W = T x into its plane, then f + Q W, F.
+__device__ __forceinline__ void ck_system_rows(float* tile, int plane, int row, int c0, int lane, const __nv_bfloat16* T, const __nv_bfloat16* Q,
                                                const float (&x)[8], float (&f)[8]) {
   uint32_t a[3][4];
   float w[8];
@@ -448,7 +448,7 @@ __device__ __forceinline__ void ck_system_rows(float* tile, int row, int c0, int
   for (int e = 0; e < 8; ++e) w[e] = 0.f;
   ck_apply(T, x, lane, w);
   ck_operand(w, a);
-  ck_put(tile, CK_W, row, c0, lane, a);
+  ck_put(tile, plane, row, c0, lane, a);
   ck_apply(Q, w, lane, f);
 }
 // Column c of (I + sign M)^-1 diag(scale), M below the diagonal with rows `stride` apart: forward substitution.
@@ -643,7 +643,7 @@ ck_rows_kernel(ChunkRowsArgs p) {
         if constexpr (SYSTEM) {
 #pragma unroll
           for (int e = 0; e < 8; ++e) out[e] = -before[e] * k[e];
-          ck_system_rows(tile, ROW, c0, lane, T[x], Q[x], out, f);
+          ck_system_rows(tile, CK_W, ROW, c0, lane, T[x], Q[x], out, f);
         }
         ck_operand(f, a);
         ck_put(tile, CK_F, ROW, c0, lane, a);
