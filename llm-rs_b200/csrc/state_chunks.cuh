@@ -495,12 +495,12 @@ __device__ __forceinline__ void ck_tile_left() { asm volatile("cp.async.bulk.wai
 // The rows of CK_LINEAR and CK_SYSTEM with a decay per token and head: a block per (place, key head). First the products of the rows
 // on the tensor cores, a quarter of the channels a warp; then, two heads at a time, the coefficients (a warp a head); then head by
 // head the rows, sixteen channels and sixteen columns a warp at a time. Bound by memory latency and the bytes that leave
-// (39 KB a chunk and head of 128 channels): 2,048 tokens of 16 heads over 8 of 128 x 128 55 us (two channels a thread and products on
-// the CUDA cores 61), 16 heads without a system 48.
+// (39 KB a chunk and head of 128 channels): 2,048 tokens of 16 heads over 8 of 128 x 128 54 us (two channels a thread and products on
+// the CUDA cores 61), 16 heads without a system 38. Three blocks an SM: with two, the products apart from the tile, 55 and 48.
 constexpr int CK_ROWS_THREADS = 256;
 __host__ __device__ constexpr int ck_rows_smem(int planes, int dmax) { return 4 * (ck_tile(planes, dmax) + 2 * CK * (dmax + 4)); }
 template <int PLANES, int DMAX>
-__global__ void __launch_bounds__(CK_ROWS_THREADS)
+__global__ void __launch_bounds__(CK_ROWS_THREADS, 3)
 ck_rows_kernel(ChunkRowsArgs p) {
   constexpr int RS = DMAX + 4, GS = CK + 1, ROW = DMAX + 8, THREADS = CK_ROWS_THREADS, HEADS = 2, WARPS = 4;
   constexpr int EACH = (2 * CK * (DMAX / 4) + THREADS - 1) / THREADS;
@@ -508,7 +508,9 @@ ck_rows_kernel(ChunkRowsArgs p) {
   extern __shared__ __align__(128) float ck_rows_raw[];
   float* tile = ck_rows_raw;
   float* rows = tile + ck_tile(PLANES, DMAX);      // k, q: [2][16][RS]
-  __shared__ float part[WARPS][2][CK][CK], gram[2][CK][GS], strengths[HEADS][2][CK], P[HEADS][CK], Z[HEADS][CK];
+  auto part = reinterpret_cast<float (*)[2][CK][CK]>(tile);      // [WARPS]: a warp's share of the products, before there is a tile
+  static_assert(ck_tile(PLANES, DMAX) >= WARPS * 2 * CK * CK, "the products lie where the tile will be");
+  __shared__ float gram[2][CK][GS], strengths[HEADS][2][CK], P[HEADS][CK], Z[HEADS][CK];
   __shared__ float own[HEADS][CK][GS];
   __shared__ __align__(16) __nv_bfloat16 Q[HEADS][CK_MATRIX], T[HEADS][CK_MATRIX];
   const int place = blockIdx.x, group = blockIdx.y, tid = threadIdx.x, lane = tid & 31, warp = tid >> 5, d = p.d;
