@@ -824,7 +824,7 @@ int llmrs_attn_prefill_tc_scored(const void* q, long long q_stride, int n_tokens
 }
 
 // Latent attention of long prompt portions on rows made for the call (portions of 1,700 and 300 tokens, 16 heads of 128 + 64 over
-// a window of 1,024: 62 us, and 25 for the rows; the folded form on mma.sync, with 3.4 times the multiplications, 678 and 77
+// a window of 1,024: 38 us, and 25 for the rows; the folded form on mma.sync, with 3.4 times the multiplications, 678 and 77
 // for its products per head): kv [rows, n_heads * (dn + 128)], every head's own key
 // (dn channels), then every head's value (128); rot [rows, dr], the key part that all heads share; row_of [requests][2], the row
 // of a request's first key and that key's position (a multiple of 128). q: heads of dn + dr channels, q_stride apart; out: heads

@@ -1,5 +1,6 @@
 // The walk of a request's tokens that the recurrences with a matrix state S [key channel, value channel] share, four
-// tokens a turn. With S_0 the state before a turn and i, j the turn's tokens:
+// tokens a turn, for the heads that the chunks of sixteen tokens on the tensor cores (state_chunks.cuh) do not take: a number of
+// channels that four does not divide, or more than 128 key channels (64 under the generalized rule). With S_0 the state before a turn and i, j the turn's tokens:
 //
 //   WALK_LINEAR    y_i = gain_i v_i                                         o_i = P_i (q_i . S_0) + sum_{j<=i} Q_ij y_j
 //   WALK_GATED     y_i = beta_i (v_i - P_i (k_i . S_0) - sum_{j<i} K_ij y_j)        the same o_i
