@@ -36,14 +36,16 @@ PREFILL_TILE = 64    # queries per entry of the prefill attention kernels' tile 
 
 
 def prefill_work(step: StepInfo, n_tiles: int) -> tuple:
-    """What a step's prompt portions bring to their attention kernel, for ``tc_pays``: the most keys that a portion sees, blocks of 64
-    queries and the keys of all of them together, the same for blocks of 128."""
+    """What a step's prompt portions bring to their attention kernel, for ``tc_pays`` (asked only where none is long): the most keys
+    that a portion sees, blocks of 64 queries and the keys of all of them together, the same for blocks of 128."""
     if n_tiles == 0:
         return (0, 0, 0, 0, 0)
-    n = np.asarray(step.n_new, np.int64)
-    n, keys = n[n > 1], (np.asarray(step.cached_len, np.int64) + n)[n > 1]
-    few, many = -(-n // 64), -(-n // 128)
-    return int(keys.max()), int(few.sum()), int((few * keys).sum()), int(many.sum()), int((many * keys).sum())
+    longest = few = few_keys = many = many_keys = 0      # (plain numbers: a dozen small arrays cost a short step more than its requests)
+    for n, cached in zip(np.asarray(step.n_new).tolist(), np.asarray(step.cached_len).tolist()):
+        if n > 1:
+            keys, f, m = cached + n, -(-n // 64), -(-n // 128)
+            longest, few, few_keys, many, many_keys = max(longest, keys), few + f, few_keys + f * keys, many + m, many_keys + m * keys
+    return longest, few, few_keys, many, many_keys
 
 
 # us of the mma.sync and the tcgen05 kernel, by the longest chain of keys (at 0, a key) and by all blocks (at 0, a block, a block's key,
@@ -229,7 +231,7 @@ class GQAttention(Mixer):
         return Plan(arrays={"prefill_tiles": tiles, "decode_reqs": decode},
                     values={"n_prefill_tiles": int(tiles.shape[0]), "n_decode": int(decode.size),
                             "max_decode_kv_len": int(max_kv), "long_portions": int(long_portions),
-                            "prefill_work": prefill_work(step, int(tiles.shape[0]))})
+                            "prefill_work": prefill_work(step, 0 if long_portions else int(tiles.shape[0]))})
 
     def _fuses_rope(self, x, cache, cos_sin) -> bool:
         """True when the q|k|v product can take norms, rotation and cache write as its epilogue."""

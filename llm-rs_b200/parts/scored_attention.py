@@ -200,7 +200,7 @@ class ScoredAttention(Mixer):
         return Plan(arrays={"prefill_tiles": tiles, "decode_reqs": decode},
                     values={"n_prefill_tiles": int(tiles.shape[0]), "n_decode": int(decode.size),
                             "max_decode_kv_len": int(max_kv), "long_portions": int(long_portions),
-                            "prefill_work": prefill_work(step, int(tiles.shape[0]))})
+                            "prefill_work": prefill_work(step, 0 if long_portions else int(tiles.shape[0]))})
 
     def heads(self, x, ctx, cache, out: Optional[torch.Tensor] = None, out_scale: float = 1.0) -> torch.Tensor:
         """The concatenated heads [tokens, n_heads * vdim] before the output projection, times ``out_scale``, written
