@@ -56,6 +56,9 @@ __device__ __forceinline__ void bar_init(uint32_t bar) { asm volatile("mbarrier.
 __device__ __forceinline__ void bar_expect(uint32_t bar, uint32_t bytes) {
   asm volatile("mbarrier.arrive.expect_tx.shared::cta.b64 _, [%0], %1;" ::"r"(bar), "r"(bytes) : "memory");
 }
+__device__ __forceinline__ void bar_expect_only(uint32_t bar, uint32_t bytes) {      // without the arrival
+  asm volatile("mbarrier.expect_tx.relaxed.cta.shared::cta.b64 [%0], %1;" ::"r"(bar), "r"(bytes) : "memory");
+}
 __device__ __forceinline__ bool bar_try(uint32_t bar, uint32_t parity) {
   uint32_t ok;
   asm volatile(
@@ -188,6 +191,18 @@ __device__ __forceinline__ void bar_arrive(uint32_t bar) {
   asm volatile("mbarrier.arrive.shared::cta.b64 _, [%0];" ::"r"(bar) : "memory");
 }
 
+// A box of V by a warp: its rows below `hi` that lie from `floor` on or below `kept`, zeros in the places of the others. (Not inlined:
+// with its loop inside, a tile of keys took 160 cycles more in the other roles; 8 tokens after 2,000 keys, a whole mixer: 64.0 us
+// without it, 64.5 so, 68.3 inlined.)
+__device__ __noinline__ void visible_rows(unsigned char* dst, const bf16* src, int lane, int box_rows, int hi, int floor, int kept) {
+#pragma unroll 8
+  for (int e = lane; e < box_rows * 16; e += 32) {      // row e / 16, 16 bytes e % 16 of it
+    const int r = e >> 4, c = e & 15;
+    const uint4 v = r < hi && (r >= floor || r < kept) ? reinterpret_cast<const uint4*>(src)[e] : make_uint4(0u, 0u, 0u, 0u);
+    *reinterpret_cast<uint4*>(dst + (c >> 3) * HALF_BYTES + r * 128 + (((c & 7) ^ (r & 7)) << 4)) = v;
+  }
+}
+
 // Threads 0..127 (warps 0-3) are the softmax threads: thread r owns query row r. One lane of warp 4
 // issues every MMA, the lanes of warp 5 the TMA copies. Nobody meets at a block-wide barrier inside
 // the loop; the roles talk through mbarriers:
@@ -211,7 +226,7 @@ struct LatentRows {
 template <bool SCORED, int LAT>
 __global__ void __launch_bounds__(AT_THREADS + 96, 1)
 attn_prefill_tc_kernel(const __grid_constant__ CUtensorMap map_kv, const __grid_constant__ CUtensorMap map_rot,
-                       const LatentRows lat, const bf16* __restrict__ q, long long q_stride,
+                       const LatentRows lat, const bf16* __restrict__ cache, int cache_rows, const bf16* __restrict__ q, long long q_stride,
                        bf16* __restrict__ out, long long out_stride, const int* __restrict__ tiles,
                        const int* __restrict__ q_start, const int* __restrict__ n_new,
                        const int* __restrict__ cached_len, const int* __restrict__ block_table, int table_stride,
@@ -373,16 +388,16 @@ attn_prefill_tc_kernel(const __grid_constant__ CUtensorMap map_kv, const __grid_
       if (L < 0) break;
       Item it;
       item_at(L, it);
-      // Page of this lane's box of tile t, or -1 (the lane copies nothing). A box whose keys no query of
-      // the item may see (past the end, or before the window) is filled from the page of the newest key
-      // instead: whatever a slot holds must be finite (it meets a probability of zero), and shared memory
-      // that no copy ever wrote need not be.
-      const int spare_page = LLMRS_CHECKED_PAGE(it.table[(it.kv_hi - 1) / page_size], 6, it.kv_hi - 1);
+      // A weight of zero does not silence a value that is not finite, so no value enters that no query of the item may
+      // see (past the end, before the window): a box without a visible key comes from beyond the map and is all zeros,
+      // and V's boxes that hold both kinds (the newest key's, the window's edge, the kept keys' end: three of an item)
+      // are put together by the warp. K needs no such care: the scores of such keys are replaced, whatever they are.
+      // Page of this lane's box of tile t: -1, the lane copies nothing; -2, no visible key.
       auto page_of = [&](int t) {
         const int key = first_key(it, t) + box_rows * i;
         if (lane >= n_boxes || t >= it.n_tiles) return -1;
         return (key < it.kv_hi && (key + box_rows - 1 >= it.key_floor || key < keep)) ? LLMRS_CHECKED_PAGE(it.table[key / page_size], 6, key)
-                                                                     : spare_page;
+                                                                     : -2;
       };
       int page = page_of(0);                          // looked up one tile ahead of its copy
       for (int t = 0; t < it.n_tiles; ++t) {
@@ -392,16 +407,33 @@ attn_prefill_tc_kernel(const __grid_constant__ CUtensorMap map_kv, const __grid_
         if (g >= AT_STAGES && !wait_all(bar_free + 8 * st, ((g / AT_STAGES) - 1) & 1)) { ok = false; break; }
         copies = g + 1;
         if (!(which == 0 && g == test_skip_tile)) {   // tests only: K of this tile never arrives
-          const unsigned live = __ballot_sync(0xffffffffu, page >= 0);
-          const uint32_t bar = bar_full + 8 * st;
-          if (lane == 0) bar_expect(bar, (uint32_t)__popc(live) * box_bytes);
+          const int key = first_key(it, t) + box_rows * i;
+          const bool mixed = which == 1 && page >= 0 &&
+                             (key + box_rows > it.kv_hi || (key < it.key_floor && key + box_rows > keep && keep < it.key_floor));
+          const unsigned by_hand = __ballot_sync(0xffffffffu, mixed && h == 0);
+          const uint32_t bar = bar_full + 8 * st, by_copy = (uint32_t)(n_boxes - 2 * __popc(by_hand)) * box_bytes;
+          if (lane == 0) {
+            if (by_hand == 0) bar_expect(bar, by_copy);
+            else if (by_copy) bar_expect_only(bar, by_copy);      // (arrives below)
+          }
           __syncwarp();
-          if (page >= 0) {
-            const int key = first_key(it, t) + box_rows * i;
-            const int row = ((page * n_kv_heads + it.kvh) * 2 + which) * page_size + key % page_size;
+          if (page != -1 && !mixed) {
+            const int row = page < 0 ? cache_rows : ((page * n_kv_heads + it.kvh) * 2 + which) * page_size + key % page_size;
             tma_2d(sm(KV) + st * STAGE_BYTES + which * K_BYTES + h * HALF_BYTES + i * box_bytes, &map_kv, bar, h * 64, row);
           }
           __syncwarp();
+          if (by_hand) {
+            for (unsigned left = by_hand; left; left &= left - 1) {
+              const int owner = __ffs(left) - 1, box_key = first_key(it, t) + box_rows * owner;      // (h == 0: lane = box)
+              const int box_page = __shfl_sync(0xffffffffu, page, owner);
+              const size_t row0 = (size_t)((box_page * n_kv_heads + it.kvh) * 2 + 1) * page_size + box_key % page_size;
+              visible_rows(KV + st * STAGE_BYTES + K_BYTES + owner * box_bytes, cache + row0 * AT_D, lane, box_rows,
+                           it.kv_hi - box_key, it.key_floor - box_key, keep - box_key);
+            }
+            asm volatile("fence.proxy.async.shared::cta;" ::: "memory");
+            __syncwarp();
+            if (lane == 0) bar_arrive(bar);
+          }
         }
         page = next;
       }
@@ -719,7 +751,7 @@ int launch_latent_tc(const CUtensorMap& map_kv, const CUtensorMap& map_rot, cons
   const cudaError_t e = cudaFuncSetAttribute(attn_prefill_tc_kernel<true, LAT>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
   if (e != cudaSuccess) return llmrs_fail("latent_attention_tc: shared memory %zu: %s", smem, cudaGetErrorString(e));
   attn_prefill_tc_kernel<true, LAT><<<grid, AT_THREADS + 96, smem, stream>>>(
-      map_kv, map_rot, lat, (const bf16*)q, q_stride, (bf16*)out, out_stride, tiles, q_start, n_new, cached_len, n_new, 0, n_tiles,
+      map_kv, map_rot, lat, nullptr, 0, (const bf16*)q, q_stride, (bf16*)out, out_stride, tiles, q_start, n_new, cached_len, n_new, 0, n_tiles,
       persistent, n_heads, n_heads, 16, 64, window, scale, 0.f, nullptr, 0, 1.0f, 0, (const bf16*)gate, gate_stride, error_flag,
       g_wait_limit, g_test_skip_tile);
   return llmrs_launch_status("latent_attention_tc");
@@ -812,12 +844,12 @@ int llmrs_attn_prefill_tc_scored(const void* q, long long q_stride, int n_tokens
   dim3 grid((unsigned)(persistent ? n_sm : n_lin));
   if (scored)
     attn_prefill_tc_kernel<true, 0><<<grid, AT_THREADS + 96, smem, stream>>>(
-        map_kv, map_kv, LatentRows{}, (const bf16*)q, q_stride, (bf16*)out, out_stride, tiles, q_start, n_new, cached_len, block_table,
+        map_kv, map_kv, LatentRows{}, (const bf16*)cache, (int)cache_rows, (const bf16*)q, q_stride, (bf16*)out, out_stride, tiles, q_start, n_new, cached_len, block_table,
         table_stride, n_tiles, persistent, n_q_heads, n_kv_heads, page_size, box_rows, window, scale, softcap, sink, chunk,
         out_scale, keep, (const bf16*)gate, gate_stride, error_flag, g_wait_limit, g_test_skip_tile);
   else
     attn_prefill_tc_kernel<false, 0><<<grid, AT_THREADS + 96, smem, stream>>>(
-        map_kv, map_kv, LatentRows{}, (const bf16*)q, q_stride, (bf16*)out, out_stride, tiles, q_start, n_new, cached_len, block_table,
+        map_kv, map_kv, LatentRows{}, (const bf16*)cache, (int)cache_rows, (const bf16*)q, q_stride, (bf16*)out, out_stride, tiles, q_start, n_new, cached_len, block_table,
         table_stride, n_tiles, persistent, n_q_heads, n_kv_heads, page_size, box_rows, window, scale, 0.f, nullptr, 0,
         1.0f, 0, nullptr, 0, error_flag, g_wait_limit, g_test_skip_tile);
   return llmrs_launch_status("attn_prefill_tc");
