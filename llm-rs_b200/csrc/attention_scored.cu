@@ -884,7 +884,7 @@ int llmrs_attn_prefill_tc_scored(const void* q, long long q_stride, int n_tokens
                                  const int* q_start, const int* n_new, const int* cached_len, const int* block_table,
                                  int table_stride, int n_q_heads, int n_kv_heads, int page_size, int window, float scale,
                                  float softcap, const float* sink, int chunk, float out_scale, int keep,
-                                 const void* gate, long long gate_stride, int* error_flag, cudaStream_t stream);
+                                 const void* gate, long long gate_stride, int item_rows, int* error_flag, cudaStream_t stream);
 
 // 1: bfloat16 also takes the kernel for any type (tests compare the two).
 LLMRS_API void llmrs_scored_generic_only(int on) { g_scored_generic_only = on; }
@@ -924,8 +924,8 @@ LLMRS_API int llmrs_scored_prefill(const void* q, long long q_stride, void* out,
                                         (long long)n_pages * n_kv_heads * 2 * page_size, tiles, n_tiles, q_start, n_new,
                                         cached_len, block_table, table_stride, n_q_heads, n_kv_heads, page_size,
                                         mask == MASK_WINDOW ? mask_size : 0, scale, softcap, sink,
-                                        mask == MASK_CHUNK ? mask_size : 0, out_scale, keep, gate, gate_stride, nullptr,
-                                        stream);
+                                        mask == MASK_CHUNK ? mask_size : 0, out_scale, keep, gate, gate_stride,
+                                        prefer_tc == 2 ? 64 : 128, nullptr, stream);
   if (dtype == LLMRS_BF16 && !g_scored_generic_only && q_stride % 2 == 0 && out_stride % 2 == 0) {
 #define LLMRS_SM_CASE(K, V)                                                                                     \
   if (dk == 16 * K && dv == 16 * V)                                                                              \

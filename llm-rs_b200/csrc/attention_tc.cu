@@ -230,7 +230,7 @@ attn_prefill_tc_kernel(const __grid_constant__ CUtensorMap map_kv, const __grid_
                        bf16* __restrict__ out, long long out_stride, const int* __restrict__ tiles,
                        const int* __restrict__ q_start, const int* __restrict__ n_new,
                        const int* __restrict__ cached_len, const int* __restrict__ block_table, int table_stride,
-                       int n_list, int persistent, int n_q_heads, int n_kv_heads, int page_size, int box_rows, int window, float scale,
+                       int n_list, int item_rows, int persistent, int n_q_heads, int n_kv_heads, int page_size, int box_rows, int window, float scale,
                        float softcap_, const float* __restrict__ sink_, int chunk_, float out_scale_, int keep_,
                        const bf16* __restrict__ gate_, long long gate_stride, int* __restrict__ error_flag, uint32_t wait_limit, int test_skip_tile) {
   constexpr int AT_STAGES = LAT == 3 ? 2 : 3, KEY_PIECES = LAT > 0 ? LAT : 2;
@@ -255,20 +255,22 @@ attn_prefill_tc_kernel(const __grid_constant__ CUtensorMap map_kv, const __grid_
     if (threadIdx.x == 0) atomicExch(error_flag ? error_flag : &g_attn_tc_error, 3);
     return;
   }
-  // The work: an item is 128 query rows of one request and one query head: those entries of the list of 64-query
-  // tiles whose offset is a multiple of 128 (warp 0 notes them in shared memory first), times the heads. Items are
+  // The work: an item is item_rows = 128 query rows of one request and one query head: those entries of the list of 64-query
+  // tiles whose offset is a multiple of 128 (warp 0 notes them in shared memory first), times the heads; or, for steps of
+  // short portions, 64: every entry, half of the rows empty, so that a query meets the keys that it meets in the kernel on
+  // mma.sync (a value that is not finite, 80 tokens on, would turn its weight of zero into no number). Items are
   // numbered so that later tiles of a prompt, which see more keys, come first, for every head; block b of G walks
   // the numbering like a snake (b, 2G-1-b, 2G+b, 4G-1-b, ...), which gives every block about the same number of
   // key tiles, and keeps tensor memory, barriers and the ring of stages from one item to the next: the copies of an
   // item's first keys run under the end of the item before.
   // With a block per item (persistent == 0) the block's number names an entry and a head, and the block of an entry
   // that starts no 128-row tile leaves at once.
-  if (!persistent && tiles[2 * (n_list - 1 - (int)blockIdx.x / n_q_heads) + 1] % AT_BQ != 0) return;
+  if (!persistent && tiles[2 * (n_list - 1 - (int)blockIdx.x / n_q_heads) + 1] % item_rows != 0) return;
   if (persistent && warp == 0) {
     int n = 0;
     for (int e0 = 0; e0 < n_list; e0 += 32) {
       const int e = e0 + lane;
-      const bool is_item = e < n_list && tiles[2 * e + 1] % AT_BQ == 0;
+      const bool is_item = e < n_list && tiles[2 * e + 1] % item_rows == 0;
       const unsigned m = __ballot_sync(0xffffffffu, is_item);
       if (is_item) valid[n + __popc(m & ((1u << lane) - 1u))] = (uint16_t)e;
       n += __popc(m);
@@ -294,7 +296,7 @@ attn_prefill_tc_kernel(const __grid_constant__ CUtensorMap map_kv, const __grid_
     it.req = req;
     it.head = L % n_q_heads;
     it.kvh = it.head / (n_q_heads / n_kv_heads);
-    it.rows = min(AT_BQ, n_new[req] - q_off);
+    it.rows = min(item_rows, n_new[req] - q_off);
     it.tok0 = q_start[req] + q_off;
     it.pos0 = cached_len[req] + q_off;
     it.kv_hi = it.pos0 + it.rows;
@@ -752,7 +754,7 @@ int launch_latent_tc(const CUtensorMap& map_kv, const CUtensorMap& map_rot, cons
   if (e != cudaSuccess) return llmrs_fail("latent_attention_tc: shared memory %zu: %s", smem, cudaGetErrorString(e));
   attn_prefill_tc_kernel<true, LAT><<<grid, AT_THREADS + 96, smem, stream>>>(
       map_kv, map_rot, lat, nullptr, 0, (const bf16*)q, q_stride, (bf16*)out, out_stride, tiles, q_start, n_new, cached_len, n_new, 0, n_tiles,
-      persistent, n_heads, n_heads, 16, 64, window, scale, 0.f, nullptr, 0, 1.0f, 0, (const bf16*)gate, gate_stride, error_flag,
+      AT_BQ, persistent, n_heads, n_heads, 16, 64, window, scale, 0.f, nullptr, 0, 1.0f, 0, (const bf16*)gate, gate_stride, error_flag,
       g_wait_limit, g_test_skip_tile);
   return llmrs_launch_status("latent_attention_tc");
 }
@@ -787,22 +789,22 @@ bool llmrs_attn_prefill_tc_supported(const void* q, long long q_stride, const vo
 // With options on the score (softcap > 0: cap * tanh(score / cap); sink: one number per query head in the softmax's
 // denominator, or null; chunk > 0: a query sees the keys of its own chunk of that many positions only; out_scale
 // multiplies the output; keep: the first so many keys are seen beside the window's; gate: [tokens, query heads] in
-// bfloat16 or null, the output is multiplied by its sigmoid).
+// bfloat16 or null, the output is multiplied by its sigmoid). item_rows: 128, or 64 for short portions.
 int llmrs_attn_prefill_tc_scored(const void* q, long long q_stride, int n_tokens, void* out, long long out_stride,
                                  const void* cache, long long cache_rows, const int* tiles, int n_tiles,
                                  const int* q_start, const int* n_new, const int* cached_len, const int* block_table,
                                  int table_stride, int n_q_heads, int n_kv_heads, int page_size, int window, float scale,
                                  float softcap, const float* sink, int chunk, float out_scale, int keep,
-                                 const void* gate, long long gate_stride, int* error_flag, cudaStream_t stream);
+                                 const void* gate, long long gate_stride, int item_rows, int* error_flag, cudaStream_t stream);
 
 int llmrs_attn_prefill_tc(const void* q, long long q_stride, int n_tokens, void* out, long long out_stride,
                           const void* cache, long long cache_rows, const int* tiles, int n_tiles, const int* q_start,
                           const int* n_new, const int* cached_len, const int* block_table, int table_stride,
-                          int n_q_heads, int n_kv_heads, int page_size, int window, float scale, int* error_flag,
+                          int n_q_heads, int n_kv_heads, int page_size, int window, float scale, int item_rows, int* error_flag,
                           cudaStream_t stream) {
   return llmrs_attn_prefill_tc_scored(q, q_stride, n_tokens, out, out_stride, cache, cache_rows, tiles, n_tiles, q_start,
                                       n_new, cached_len, block_table, table_stride, n_q_heads, n_kv_heads, page_size,
-                                      window, scale, 0.f, nullptr, 0, 1.0f, 0, nullptr, 0, error_flag, stream);
+                                      window, scale, 0.f, nullptr, 0, 1.0f, 0, nullptr, 0, item_rows, error_flag, stream);
 }
 
 int llmrs_attn_prefill_tc_scored(const void* q, long long q_stride, int n_tokens, void* out, long long out_stride,
@@ -810,7 +812,7 @@ int llmrs_attn_prefill_tc_scored(const void* q, long long q_stride, int n_tokens
                                  const int* q_start, const int* n_new, const int* cached_len, const int* block_table,
                                  int table_stride, int n_q_heads, int n_kv_heads, int page_size, int window, float scale,
                                  float softcap, const float* sink, int chunk, float out_scale, int keep,
-                                 const void* gate, long long gate_stride, int* error_flag, cudaStream_t stream) {
+                                 const void* gate, long long gate_stride, int item_rows, int* error_flag, cudaStream_t stream) {
   CUtensorMap map_kv;
   int rc;
   (void)n_tokens;
@@ -838,19 +840,19 @@ int llmrs_attn_prefill_tc_scored(const void* q, long long q_stride, int n_tokens
     cudaDeviceGetAttribute(&n_sm, cudaDevAttrMultiProcessorCount, dev);
     if (n_sm <= 0) n_sm = 1;
   }
-  // (About every second entry of the list starts a 128-row tile; a block that finds no item leaves at once.)
-  const long long n_lin = (long long)n_q_heads * n_tiles, n_items = (long long)n_q_heads * ((n_tiles + 1) / 2);
+  // (About every second entry of the list starts an item of 128 rows; a block that finds no item leaves at once.)
+  const long long n_lin = (long long)n_q_heads * n_tiles, n_items = item_rows == AT_BQ ? (long long)n_q_heads * ((n_tiles + 1) / 2) : n_lin;
   const int persistent = n_items > n_sm && n_items <= 16LL * n_sm ? 1 : 0;
   dim3 grid((unsigned)(persistent ? n_sm : n_lin));
   if (scored)
     attn_prefill_tc_kernel<true, 0><<<grid, AT_THREADS + 96, smem, stream>>>(
         map_kv, map_kv, LatentRows{}, (const bf16*)cache, (int)cache_rows, (const bf16*)q, q_stride, (bf16*)out, out_stride, tiles, q_start, n_new, cached_len, block_table,
-        table_stride, n_tiles, persistent, n_q_heads, n_kv_heads, page_size, box_rows, window, scale, softcap, sink, chunk,
+        table_stride, n_tiles, item_rows, persistent, n_q_heads, n_kv_heads, page_size, box_rows, window, scale, softcap, sink, chunk,
         out_scale, keep, (const bf16*)gate, gate_stride, error_flag, g_wait_limit, g_test_skip_tile);
   else
     attn_prefill_tc_kernel<false, 0><<<grid, AT_THREADS + 96, smem, stream>>>(
         map_kv, map_kv, LatentRows{}, (const bf16*)cache, (int)cache_rows, (const bf16*)q, q_stride, (bf16*)out, out_stride, tiles, q_start, n_new, cached_len, block_table,
-        table_stride, n_tiles, persistent, n_q_heads, n_kv_heads, page_size, box_rows, window, scale, 0.f, nullptr, 0,
+        table_stride, n_tiles, item_rows, persistent, n_q_heads, n_kv_heads, page_size, box_rows, window, scale, 0.f, nullptr, 0,
         1.0f, 0, nullptr, 0, error_flag, g_wait_limit, g_test_skip_tile);
   return llmrs_launch_status("attn_prefill_tc");
 }

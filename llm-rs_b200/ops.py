@@ -304,9 +304,9 @@ def qk_norm_rope_kvwrite(q: torch.Tensor, k: Optional[torch.Tensor], v: Optional
 def attn_prefill(q: torch.Tensor, out: torch.Tensor, cache: torch.Tensor, tiles: torch.Tensor, n_tiles: int,
                  q_start: torch.Tensor, n_new: torch.Tensor, cached_len: torch.Tensor, block_table: torch.Tensor,
                  n_q_heads: int, n_kv_heads: int, head_dim: int, page_size: int, window: int, scale: float,
-                 prefer_tc: bool = False) -> None:
+                 prefer_tc: int = 0) -> None:
     """Causal attention of prompt portions over the paged cache (their own keys are already written).
-    ``prefer_tc`` asks for the tcgen05 kernel (blocks of 128 queries) where it applies.
+    ``prefer_tc`` asks for the tcgen05 kernel where it applies: 1, blocks of 128 queries; 2, of 64 (short portions).
 
     ``tiles`` is int32 [n_tiles, 2]: (request row, offset of the tile's first query in
     the request's new tokens); a tile covers 64 queries.
@@ -321,7 +321,7 @@ def attn_prefill(q: torch.Tensor, out: torch.Tensor, cache: torch.Tensor, tiles:
         _ptr(q), ctypes.c_longlong(_row_stride(q, "q")), _ptr(out), ctypes.c_longlong(_row_stride(out, "out")),
         _ptr(cache), _ptr(tiles), n_tiles, _ptr(q_start), _ptr(n_new), _ptr(cached_len), _ptr(block_table),
         block_table.size(1), n_q_heads, n_kv_heads, head_dim, page_size, window, ctypes.c_float(scale),
-        dtype_code(q.dtype), q.size(0), cache.size(0), 1 if prefer_tc else 0, _ptr(tc_error_flag(q.device)),
+        dtype_code(q.dtype), q.size(0), cache.size(0), int(prefer_tc), _ptr(tc_error_flag(q.device)),
         _stream()), "attn_prefill")
 
 
@@ -1426,10 +1426,10 @@ def scored_generic_only(on: bool) -> None:
 
 def scored_prefill(q, out, cache, tiles, n_tiles: int, ctx, table, n_q_heads: int, n_kv_heads: int, dk: int, dv: int,
                    page_size: int, scale: float, softcap: float, sink, mask: int, mask_size: int,
-                   prefer_tc: bool = False, bias: Optional[torch.Tensor] = None, out_scale: float = 1.0, keep: int = 0,
+                   prefer_tc: int = 0, bias: Optional[torch.Tensor] = None, out_scale: float = 1.0, keep: int = 0,
                    gate: Optional[torch.Tensor] = None) -> None:
     """Prompt portions (tiles of 64 queries: request, offset) through ``csrc/attention_scored.cu``. ``prefer_tc`` asks
-    for the tcgen05 kernel where it applies (bfloat16, keys and values of 128 channels, pages of a multiple of 16
+    (as in ``attn_prefill``) for the tcgen05 kernel where it applies (bfloat16, keys and values of 128 channels, pages of a multiple of 16
     keys; worth it when the portions are long). ``bias``: float32 [distances, query heads], added to the score of a
     key that many positions behind its query (the last row for every greater distance); ``out_scale`` multiplies
     the output. ``keep`` (with a window): the first so many keys of the sequence are seen too. ``gate`` ([tokens, query

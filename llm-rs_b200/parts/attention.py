@@ -37,15 +37,15 @@ PREFILL_TILE = 64    # queries per entry of the prefill attention kernels' tile 
 
 def prefill_work(step: StepInfo, n_tiles: int) -> tuple:
     """What a step's prompt portions bring to their attention kernel, for ``tc_pays`` (asked only where none is long): the most keys
-    that a portion sees, blocks of 64 queries and the keys of all of them together, the same for blocks of 128."""
+    that a portion sees, blocks of 64 queries and the keys of all of them together."""
     if n_tiles == 0:
-        return (0, 0, 0, 0, 0)
-    longest = few = few_keys = many = many_keys = 0      # (plain numbers: a dozen small arrays cost a short step more than its requests)
+        return (0, 0, 0)
+    longest = blocks = block_keys = 0      # (plain numbers: a dozen small arrays cost a short step more than its requests)
     for n, cached in zip(np.asarray(step.n_new).tolist(), np.asarray(step.cached_len).tolist()):
         if n > 1:
-            keys, f, m = cached + n, -(-n // 64), -(-n // 128)
-            longest, few, few_keys, many, many_keys = max(longest, keys), few + f, few_keys + f * keys, many + m, many_keys + m * keys
-    return longest, few, few_keys, many, many_keys
+            keys, b = cached + n, -(-n // 64)
+            longest, blocks, block_keys = max(longest, keys), blocks + b, block_keys + b * keys
+    return longest, blocks, block_keys
 
 
 # us of the mma.sync and the tcgen05 kernel, by the longest chain of keys (at 0, a key) and by all blocks (at 0, a block, a block's key,
@@ -55,17 +55,23 @@ _PREFILL_US = {False: ((4.6, 0.042, 5.0, 0.13, 0.0023), (6.9, 0.0088, 4.6, 0.45,
 
 
 def tc_pays(work: tuple, heads: int, window: int, scored: bool) -> bool:
-    """True where the tcgen05 kernel (blocks of 128 queries) is the faster one for portions that fill its blocks less than half. It
+    """True where the tcgen05 kernel (with blocks of 64 queries, as mma.sync has them) is the faster one for portions that would fill
+    its blocks of 128 less than half. It
     walks a tile of keys in a fifth of the time, so it pays wherever there are keys to walk; the other starts sooner and holds more
     blocks. Measured, mma.sync / tcgen05 (us, heads of 128; plain, 16 heads | with a gate, 16 heads): one portion of 20 tokens 5.1 / 7.3 |
     7.3 / 8.6, of 20 after 500 26.8 / 12.7 | 41 / 14, of 8 after 2,000 90 / 24 | 142 / 25; 64 portions of 30 21 / 33 | 28 / 39, the same
     after 100 41 / 44 | 59 / 52; 200 portions of 2 after 30 40 / 87 | 56 / 102, after 500 259 / 167 | 419 / 188."""
-    longest, few, few_keys, many, many_keys = work
+    longest, blocks, keys = work
     if window > 0:
-        longest, few_keys, many_keys = min(longest, window + 64), min(few_keys, few * (window + 64)), min(many_keys, many * (window + 64))
-    cost = lambda c, blocks, keys: max(c[0] + c[1] * longest, c[2] + heads / 16 * (c[3] * blocks + c[4] * keys))
+        longest, keys = min(longest, window + 64), min(keys, blocks * (window + 64))
+    cost = lambda c: max(c[0] + c[1] * longest, c[2] + heads / 16 * (c[3] * blocks + c[4] * keys))
     mma, tc = _PREFILL_US[scored]
-    return many > 0 and cost(tc, many, many_keys) <= cost(mma, few, few_keys)
+    return blocks > 0 and cost(tc) <= cost(mma)
+
+
+def prefill_kernel(values, heads: int, window: int, scored: bool) -> int:
+    """``prefer_tc`` of a step's prompt portions, from its plan's values."""
+    return 1 if values["long_portions"] else 2 * tc_pays(values["prefill_work"], heads, window, scored)
 
 
 # A block of the kernel with the ring of two tiles (three blocks an SM) takes about this much longer than one of the
@@ -302,8 +308,7 @@ class GQAttention(Mixer):
         if n_tiles:
             ops.attn_prefill(q, out, cache.kv, plan.arrays["prefill_tiles"], n_tiles, ctx.q_start, ctx.n_new,
                              ctx.cached_len, table, nq, nkv, d, cache.page_size, self.window, self.scale,
-                             prefer_tc=_ATTN_TC and (bool(plan.values["long_portions"])
-                                                     or tc_pays(plan.values["prefill_work"], nq, self.window, False)))
+                             prefer_tc=prefill_kernel(plan.values, nq, self.window, False) if _ATTN_TC else 0)
         if n_decode:
             split_keys, ring = (self.split_keys, 3) if self.split_keys else self._choose_split(n_decode, max_kv, q)
             max_splits = max(1, -(-max_kv // split_keys))

@@ -8,7 +8,7 @@ from typing import Mapping, Optional
 import torch
 
 from .. import host, ops
-from .attention import _ATTN_TC, PREFILL_TILE, prefill_work, tc_pays
+from .attention import _ATTN_TC, PREFILL_TILE, prefill_kernel, prefill_work
 from .base import Mixer, Plan, Runtime, StepInfo
 from .linear import Linear
 from .position import wavelength_scaled_frequencies
@@ -245,8 +245,7 @@ class ScoredAttention(Mixer):
         scale = 1.0 if gate is not None else out_scale
         if n_tiles:
             ops.scored_prefill(q, out, pages, plan.arrays["prefill_tiles"], n_tiles, ctx, table, *args,
-                               prefer_tc=_ATTN_TC and (bool(plan.values["long_portions"])
-                                                       or tc_pays(plan.values["prefill_work"], self.n_heads, self.mask_size, True)),
+                               prefer_tc=prefill_kernel(plan.values, self.n_heads, self.mask_size, True) if _ATTN_TC else 0,
                                bias=self.bias,
                                out_scale=scale, keep=self.keep_first, gate=head_gate)
         if n_decode:

@@ -35,7 +35,7 @@ def _case(lens, cached, page, window, keep, chunk, kv, seed):
     return ctx, torch.from_numpy(tiles.copy()).to(DEV), table.to(DEV), cache.to(DEV), foreign.to(DEV), g
 
 
-@pytest.mark.parametrize("tc", [True, False])
+@pytest.mark.parametrize("tc", [1, 2, 0])
 @pytest.mark.parametrize("page", [16, 48, 64])
 @pytest.mark.parametrize("lens,cached", [([20], [500]), ([8, 3, 64], [0, 77, 2000]), ([200, 129, 5], [45, 128, 127]), ([128, 16], [128, 112])])
 @pytest.mark.parametrize("window,keep,chunk", [(0, 0, 0), (257, 0, 0), (100, 5, 0), (20, 40, 0), (64, 16, 0), (0, 0, 100)])
@@ -62,3 +62,40 @@ def test_cells_that_no_query_sees(tc, page, lens, cached, window, keep, chunk):
     for fill, scored, out in outs:
         assert torch.isfinite(out).all(), (fill, scored)
         assert torch.equal(out, next(o for f, s, o in outs if f == 0.0 and s == scored)), (fill, scored)
+
+
+@pytest.mark.parametrize("tc", [2, 0])
+@pytest.mark.parametrize("scored", [False, True])
+@pytest.mark.parametrize("page,window", [(16, 0), (64, 90)])
+def test_later_blocks_of_a_short_portion(tc, scored, page, window):
+    """A portion of more than 64 tokens beside short ones: the first 64 queries keep their bits whatever the tokens behind them hold,
+    as they do on mma.sync, and the two kernels agree to bfloat16's rounding."""
+    from llm_rs_b200 import ops
+    heads, kv, lens, cached = 4, 2, [100, 2, 2, 127, 3], [500, 500, 30, 61, 500]
+    ctx, tiles, table, cache, _, g = _case(lens, cached, page, window, 0, 0, kv, 5)
+    q = torch.randn(sum(lens), heads * D, generator=g).to(DEV, torch.bfloat16)
+
+    def run(c, how):
+        out = torch.full_like(q, 7.0)
+        if scored:
+            ops.scored_prefill(q, out, c.view(c.size(0), kv, -1), tiles, tiles.size(0), ctx, table, heads, kv, D, D, page, 0.09, 20.0, None,
+                               ops.MASK_WINDOW if window else ops.MASK_CAUSAL, window, prefer_tc=how)
+        else:
+            ops.attn_prefill(q, out, c.view(c.size(0), kv, -1), tiles, tiles.size(0), ctx.q_start, ctx.n_new, ctx.cached_len, table,
+                             heads, kv, D, page, window, 0.09, prefer_tc=how)
+        return out
+
+    want = run(cache, tc)
+    other = run(cache, 2 - tc)
+    assert (want - other).abs().max().item() <= 0.03 * other.abs().max().item()
+    bad = cache.clone()
+    for r, at in ((0, 64), (3, 120)):
+        key = cached[r] + at
+        bad[int(table[r, key // page]), :, :, key % page] = float("nan")
+    got = run(bad, tc)
+    ops.check_attention_error()
+    for r in range(len(lens)):
+        first = sum(lens[:r])
+        n = min(lens[r], 64) if r in (0, 3) else lens[r]
+        assert torch.isfinite(want[first: first + n]).all()
+        assert torch.equal(got[first: first + n], want[first: first + n]), r
