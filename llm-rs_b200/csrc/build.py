@@ -45,7 +45,7 @@ HOST_STAMP_NAME = "host_san_stamp.json" if HOST_SANITIZE else "host_stamp.json"
 HOST_FLAGS = ["-std=c++17", "-fPIC", "-Wall"] + (
     ["-O1", "-g", "-fno-omit-frame-pointer", "-fsanitize=address,undefined", "-fno-sanitize-recover=undefined"]
     if HOST_SANITIZE else ["-O2"])
-HOST_ABI_VERSION = 3
+HOST_ABI_VERSION = 4
 
 _lib: Optional[ctypes.CDLL] = None
 _host_lib: Optional[ctypes.CDLL] = None

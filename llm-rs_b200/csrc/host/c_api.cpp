@@ -34,7 +34,7 @@ T* as(void* handle, const char* what) {
 
 extern "C" {
 
-int llmrs_host_abi_version(void) { return 3; }
+int llmrs_host_abi_version(void) { return 4; }
 const char* llmrs_host_last_error(void) { return g_error.c_str(); }
 
 int llmrs_pool_create(int capacity, void** pool) {
@@ -132,7 +132,7 @@ int llmrs_pack_step(void* cm, int n_entries, const int64_t* ids, const int32_t* 
 
 int llmrs_plan_paged_attention(int n_requests, const int32_t* n_new, const int32_t* cached_len, int tile,
                                int32_t* tiles_out, int64_t tiles_capacity, int32_t* decode_out,
-                               int64_t decode_capacity, int32_t* plan4, int* written) {
+                               int64_t decode_capacity, int32_t* plan4, int64_t* work3, int* written) {
     return guarded([&] {
         AttentionPlan a;
         bool ok = plan_paged_attention(n_requests, n_new, cached_len, tile, tiles_out, tiles_capacity, decode_out,
@@ -141,6 +141,9 @@ int llmrs_plan_paged_attention(int n_requests, const int32_t* n_new, const int32
         plan4[1] = a.n_decode;
         plan4[2] = a.max_decode_kv_len;
         plan4[3] = a.long_portions;
+        work3[0] = a.longest;
+        work3[1] = a.n_tiles;
+        work3[2] = a.tile_keys;
         *written = ok ? 1 : 0;
     });
 }

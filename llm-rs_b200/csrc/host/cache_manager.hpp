@@ -126,6 +126,8 @@ struct AttentionPlan {
     int n_tiles = 0, n_decode = 0;
     int max_decode_kv_len = 0;   // most keys a decoding request sees (its cached length + 1)
     int long_portions = 0;       // blocks of 128 queries would be at least half full on average
+    int longest = 0;             // most keys that a portion of more than one token sees
+    int64_t tile_keys = 0;       // keys of all tiles together, a tile counting its whole portion's
 };
 
 // tiles_out holds 2 * tiles_capacity ints, decode_out decode_capacity ints. Returns false (and only

@@ -51,11 +51,13 @@ int llmrs_pack_step(void* cm, int n_entries, const int64_t* ids, const int32_t* 
 
 /* The plan of paged attention for one step: requests with one new token go to decode_out, longer
  * portions are cut into tiles of `tile` queries, written to tiles_out as (request row, offset)
- * pairs. plan4 receives n_tiles, n_decode, max_decode_kv_len, long_portions. When a capacity
- * (in tiles, in requests) is too small nothing is written and *written is 0. */
+ * pairs. plan4 receives n_tiles, n_decode, max_decode_kv_len, long_portions; work3 what the portions
+ * bring to their attention kernel: the most keys that one of them sees, the tiles, the keys of all
+ * tiles together. When a capacity (in tiles, in requests) is too small nothing is written to tiles_out
+ * and decode_out and *written is 0. */
 int llmrs_plan_paged_attention(int n_requests, const int32_t* n_new, const int32_t* cached_len, int tile,
                                int32_t* tiles_out, int64_t tiles_capacity, int32_t* decode_out,
-                               int64_t decode_capacity, int32_t* plan4, int* written);
+                               int64_t decode_capacity, int32_t* plan4, int64_t* work3, int* written);
 
 /* The scheduler (decisions only; see scheduler.hpp). It reads the cache manager `cm`, which must
  * outlive it, and never changes it: after every call that returns `n_release > 0` ids through

@@ -119,7 +119,10 @@ bool plan_paged_attention(int n_requests, const int32_t* n_new, const int32_t* c
             ++dec;
             max_dec_kv = std::max(max_dec_kv, cached_len[r] + 1);
         } else if (n > 1) {
-            tiles += (n + tile - 1) / tile;
+            const int64_t own = (n + tile - 1) / tile;
+            tiles += own;
+            plan->longest = std::max(plan->longest, cached_len[r] + n);
+            plan->tile_keys += own * (cached_len[r] + n);
             long_blocks += (n + 127) / 128;
             long_tokens += n;
         }

@@ -59,7 +59,7 @@ def lib() -> ctypes.CDLL:
             "llmrs_pack_step": [c_void_p, c_int, c_void_p, c_void_p, c_void_p, c_void_p, c_void_p, c_void_p, c_int,
                                 c_void_p, c_int64, c_void_p, c_void_p, c_void_p, c_void_p, i64p, intp],
             "llmrs_plan_paged_attention": [c_int, c_void_p, c_void_p, c_int, c_void_p, c_int64, c_void_p, c_int64,
-                                           c_void_p, intp],
+                                           c_void_p, i64p, intp],
         }
         for name, argtypes in sigs.items():
             fn = getattr(library, name)
@@ -69,24 +69,33 @@ def lib() -> ctypes.CDLL:
     return library
 
 
-def plan_paged_attention(n_new, cached_len, tile: int):
+_PLAN4, _WORK3 = c_int32 * 4, c_int64 * 3
+
+
+def plan_paged_step(n_new, cached_len, tile: int):
     """The host library's plan of paged attention for a step (int32 numpy arrays of the step's requests in,
-    ``(tiles [n, 2], decode list, max_decode_kv_len, long_portions)`` out)."""
+    ``(tiles [n, 2], decode list, max_decode_kv_len, long_portions, work)`` out; ``work``: the most keys that a portion of more than
+    one token sees, the tiles, the keys of all tiles together)."""
     import numpy as np
     R = int(n_new.shape[0])
     # Requests that bring one token take no tile: n // tile + 1 bounds a longer portion's tiles.
     tiles_cap = int(n_new.sum()) // tile + R
     tiles = np.empty((max(tiles_cap, 1), 2), np.int32)
     decode = np.empty(max(R, 1), np.int32)
-    plan = np.zeros(4, np.int32)
+    plan, work = _PLAN4(), _WORK3()
     written = c_int()
     n_new = np.ascontiguousarray(n_new, np.int32)
     cached_len = np.ascontiguousarray(cached_len, np.int32)
     rc = lib().llmrs_plan_paged_attention(R, n_new.ctypes.data, cached_len.ctypes.data, tile, tiles.ctypes.data,
-                                          tiles_cap, decode.ctypes.data, R, plan.ctypes.data, byref(written))
+                                          tiles_cap, decode.ctypes.data, R, plan, work, byref(written))
     if rc != 0 or not written.value:
         raise RuntimeError(f"attention plan failed: {last_error() if rc else 'capacity'}")
-    return tiles[:plan[0]], decode[:plan[1]], int(plan[2]), bool(plan[3])
+    return tiles[:plan[0]], decode[:plan[1]], plan[2], bool(plan[3]), tuple(work)
+
+
+def plan_paged_attention(n_new, cached_len, tile: int):
+    """``plan_paged_step`` without ``work``."""
+    return plan_paged_step(n_new, cached_len, tile)[:4]
 
 
 def last_error() -> str:

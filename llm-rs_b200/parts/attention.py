@@ -35,17 +35,21 @@ MAX_CLUSTER = 16     # splits that the kernel merges itself
 PREFILL_TILE = 64    # queries per entry of the prefill attention kernels' tile list
 
 
-def prefill_work(step: StepInfo, n_tiles: int) -> tuple:
-    """What a step's prompt portions bring to their attention kernel, for ``tc_pays`` (asked only where none is long): the most keys
-    that a portion sees, blocks of 64 queries and the keys of all of them together."""
-    if n_tiles == 0:
-        return (0, 0, 0)
-    longest = blocks = block_keys = 0      # (plain numbers: a dozen small arrays cost a short step more than its requests)
-    for n, cached in zip(np.asarray(step.n_new).tolist(), np.asarray(step.cached_len).tolist()):
-        if n > 1:
-            keys, b = cached + n, -(-n // 64)
-            longest, blocks, block_keys = max(longest, keys), blocks + b, block_keys + b * keys
-    return longest, blocks, block_keys
+class PrefillWork(tuple):
+    """What a step's prompt portions bring to their attention kernel (``host.plan_paged_step``: the most keys that one sees, blocks of
+    64 queries, the blocks' keys), and which kernel that makes the better one for the heads that have asked: decided once a
+    plan, not once a layer."""
+
+    def __new__(cls, work):
+        self = super().__new__(cls, work)
+        self.kernels = {}
+        return self
+
+
+def prefill_work(step: StepInfo, n_tiles: int) -> PrefillWork:
+    """Of a step's portions of more than one token; zeros where its plan has no tiles."""
+    n_new, cached = (np.asarray(a, np.int32) for a in (step.n_new, step.cached_len))
+    return PrefillWork(host.plan_paged_step(n_new, cached, PREFILL_TILE)[4] if n_tiles else (0, 0, 0))
 
 
 # us of the mma.sync and the tcgen05 kernel, by the longest chain of keys (at 0, a key) and by all blocks (at 0, a block, a block's key,
@@ -71,7 +75,13 @@ def tc_pays(work: tuple, heads: int, window: int, scored: bool) -> bool:
 
 def prefill_kernel(values, heads: int, window: int, scored: bool) -> int:
     """``prefer_tc`` of a step's prompt portions, from its plan's values."""
-    return 1 if values["long_portions"] else 2 * tc_pays(values["prefill_work"], heads, window, scored)
+    if values["long_portions"]:
+        return 1
+    work = values["prefill_work"]
+    kernel = work.kernels.get((heads, window, scored))
+    if kernel is None:
+        kernel = work.kernels[heads, window, scored] = 2 if tc_pays(work, heads, window, scored) else 0
+    return kernel
 
 
 # A block of the kernel with the ring of two tiles (three blocks an SM) takes about this much longer than one of the
@@ -231,13 +241,13 @@ class GQAttention(Mixer):
         queries for the prefill kernel (the host library does it). A step that will be replayed from a CUDA
         graph sizes its decode launch by the block tables' width, which the graph's key holds, instead of the
         longest request."""
-        tiles, decode, max_kv, long_portions = host.plan_paged_attention(step.n_new, step.cached_len, PREFILL_TILE)
+        tiles, decode, max_kv, long_portions, work = host.plan_paged_step(step.n_new, step.cached_len, PREFILL_TILE)
         if step.for_graph and decode.size and step.block_tables:
             max_kv = max(t.shape[1] for t in step.block_tables) * step.page_size
         return Plan(arrays={"prefill_tiles": tiles, "decode_reqs": decode},
                     values={"n_prefill_tiles": int(tiles.shape[0]), "n_decode": int(decode.size),
                             "max_decode_kv_len": int(max_kv), "long_portions": int(long_portions),
-                            "prefill_work": prefill_work(step, 0 if long_portions else int(tiles.shape[0]))})
+                            "prefill_work": PrefillWork(work)})
 
     def _fuses_rope(self, x, cache, cos_sin) -> bool:
         """True when the q|k|v product can take norms, rotation and cache write as its epilogue."""

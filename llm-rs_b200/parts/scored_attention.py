@@ -8,7 +8,7 @@ from typing import Mapping, Optional
 import torch
 
 from .. import host, ops
-from .attention import _ATTN_TC, PREFILL_TILE, prefill_kernel, prefill_work
+from .attention import _ATTN_TC, PREFILL_TILE, PrefillWork, prefill_kernel
 from .base import Mixer, Plan, Runtime, StepInfo
 from .linear import Linear
 from .position import wavelength_scaled_frequencies
@@ -194,13 +194,13 @@ class ScoredAttention(Mixer):
         return ("paged_attention", PREFILL_TILE)
 
     def plan(self, step: StepInfo) -> Plan:
-        tiles, decode, max_kv, long_portions = host.plan_paged_attention(step.n_new, step.cached_len, PREFILL_TILE)
+        tiles, decode, max_kv, long_portions, work = host.plan_paged_step(step.n_new, step.cached_len, PREFILL_TILE)
         if step.for_graph and decode.size and step.block_tables:
             max_kv = max(t.shape[1] for t in step.block_tables) * step.page_size
         return Plan(arrays={"prefill_tiles": tiles, "decode_reqs": decode},
                     values={"n_prefill_tiles": int(tiles.shape[0]), "n_decode": int(decode.size),
                             "max_decode_kv_len": int(max_kv), "long_portions": int(long_portions),
-                            "prefill_work": prefill_work(step, 0 if long_portions else int(tiles.shape[0]))})
+                            "prefill_work": PrefillWork(work)})
 
     def heads(self, x, ctx, cache, out: Optional[torch.Tensor] = None, out_scale: float = 1.0) -> torch.Tensor:
         """The concatenated heads [tokens, n_heads * vdim] before the output projection, times ``out_scale``, written

@@ -148,3 +148,24 @@ def test_refusals():
             pack(m, [("ghost", [1], [], -1)], 8)
         finally:
             del m.requests["ghost"]
+
+
+@pytest.mark.parametrize("lens,cached", [([], []), ([1, 1], [5, 9]), ([1, 20, 0, 64, 1, 65], [3, 500, 7, 0, 9, 100]), ([5000], [60000])])
+def test_work_of_prompt_portions(lens, cached):
+    """What the plan says of its portions, and the kernel that a plan's heads are given: asked once a plan, the same for each layer."""
+    from llm_rs_b200.parts import attention
+    a32 = lambda v: np.array(v, np.int32)
+    tiles, decode, max_kv, long_portions, work = host.plan_paged_step(a32(lens), a32(cached), 64)
+    portions = [(n, c + n) for n, c in zip(lens, cached) if n > 1]
+    assert work == (max((k for _, k in portions), default=0), len(tiles), sum(-(-n // 64) * k for n, k in portions))
+    values = dict(long_portions=long_portions, prefill_work=attention.PrefillWork(work))
+    hash(values["prefill_work"])
+    asked, rule = [], attention.tc_pays
+    try:
+        attention.tc_pays = lambda *a: asked.append(a) or rule(*a)
+        for heads, window, scored in [(16, 0, False), (16, 0, True), (8, 257, True)] * 3:
+            want = 1 if long_portions else (2 if rule(work, heads, window, scored) else 0)
+            assert attention.prefill_kernel(values, heads, window, scored) == want
+    finally:
+        attention.tc_pays = rule
+    assert len(asked) == (0 if long_portions else 3)
