@@ -184,26 +184,42 @@ delta_turns_kernel(const TA* __restrict__ r, const TA* __restrict__ k, const TA*
 // walks a token j through the tokens after it, the decays multiplied on as they go, and then token 15 - j, so that every one has
 // seventeen steps; then a warp makes the rows of sixteen channels, which are sixteen value columns too.
 template <typename TA>
-__global__ void __launch_bounds__(128, 4)
-delta_rows_kernel(const TA* __restrict__ r, const TA* __restrict__ k, const TA* __restrict__ v, const TA* __restrict__ a_raw,
-                  long long in_stride, const float* __restrict__ decay_raw, const float* __restrict__ decay_bias,
-                  const float* __restrict__ a_bias, const int* __restrict__ q_start, const int* __restrict__ n_new,
-                  float* __restrict__ tiles, float* __restrict__ u_out, float* __restrict__ g_out, float* __restrict__ v_out,
-                  int n_requests, int n_heads, int d, float decay_scale, float key_eps, int from) {
+struct DeltaRowsArgs {
+  const TA *r, *k, *v, *a_raw;
+  long long in_stride;
+  const float *decay_raw, *decay_bias, *a_bias;
+  const int *q_start, *n_new;
+  float *tiles, *u_out, *g_out, *v_out;
+  int n_requests, n_heads, d;
+  float decay_scale, key_eps;
+  int from;
+};
+struct DeltaRowsShared {
+  alignas(16) __nv_bfloat16 E[CK_MATRIX], R[CK_MATRIX], Q[CK_MATRIX], T[CK_MATRIX];
+  float sums[4][CK][CK + 1];      // u_i . k_j, u_i . a_j, r_i . k_j, r_i . a_j
+};
+// True where CAREFUL would make something else of it.
+template <typename TA, bool CAREFUL>
+__device__ __forceinline__ bool delta_rows(const DeltaRowsArgs<TA>& p, float* tile, DeltaRowsShared& sh) {
   constexpr int GS = CK + 1, DMAX = 64, RS = DMAX + 4, ROW = DMAX + 8;
-  extern __shared__ __align__(128) float dr_raw[];
-  float* tile = dr_raw;
-  float* tile_out = tiles + ((size_t)blockIdx.x * n_heads + blockIdx.y) * ck_tile(CK_GENERAL, DMAX);
+  const TA *r = p.r, *k = p.k, *v = p.v, *a_raw = p.a_raw;
+  const long long in_stride = p.in_stride;
+  const float *decay_raw = p.decay_raw, *decay_bias = p.decay_bias, *a_bias = p.a_bias;
+  const int *q_start = p.q_start, *n_new = p.n_new;
+  const int n_requests = p.n_requests, n_heads = p.n_heads, d = p.d, from = p.from;
+  const float decay_scale = p.decay_scale, key_eps = p.key_eps;
+  float* tile_out = p.tiles + ((size_t)blockIdx.x * n_heads + blockIdx.y) * ck_tile(CK_GENERAL, DMAX);
   auto ks = reinterpret_cast<float (*)[RS]>(tile + ck_rows(2, DMAX));      // (two planes of the tile at a time: four blocks an SM)
   auto rs = ks + CK, us = rs + CK, as = us + CK, ws = as + CK;
-  __shared__ __align__(16) __nv_bfloat16 E[CK_MATRIX], R[CK_MATRIX], Q[CK_MATRIX], T[CK_MATRIX];
-  __shared__ float sums[4][CK][GS];      // u_i . k_j, u_i . a_j, r_i . k_j, r_i . a_j
+  auto &E = sh.E, &R = sh.R, &Q = sh.Q, &T = sh.T;
+  auto& sums = sh.sums;
+  CkLook look;
   const int h = blockIdx.y, tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
   const int place = blockIdx.x;
   int t_req, n_req;
   const int req = ck_request(q_start, n_new, n_requests, place, t_req, n_req);
   const int first = (place - ck_place(t_req, req)) * CK, have = min(CK, n_req - first);
-  if (first < 0 || have <= 0 || n_req < from) return;
+  if (first < 0 || have <= 0 || n_req < from) return false;
   const size_t t0 = (size_t)(t_req + first), width = (size_t)n_heads * d;
   {
     float kv[CK / 4][2], rv[CK / 4][2], av[CK / 4][2], dec[CK / 4][2], bias_a[2], bias_d[2];      // a warp a token, all on their way together
@@ -300,13 +316,13 @@ delta_rows_kernel(const TA* __restrict__ r, const TA* __restrict__ k, const TA* 
     }
     tile_out[ck_rows(CK_GENERAL, DMAX) + tid] = up;
   } else if (warp == 3) {
-    if (lane < CK) ck_solve(&sums[1][0][0], GS, -1.f, lane, 1.f, T);
+    if (lane < CK) ck_solve<CAREFUL>(&sums[1][0][0], GS, -1.f, lane, 1.f, T);
   } else {
     for (int e = lane; e < CK * CK; e += 32) {
       const int i = e / CK, j = e % CK;
-      ck_set(E, i, j, j < i ? sums[0][i][j] : 0.f);
-      ck_set(R, i, j, j <= i ? sums[2][i][j] : 0.f);
-      ck_set(Q, i, j, j <= i ? sums[3][i][j] : 0.f);
+      ck_set<CAREFUL>(E, i, j, j < i ? sums[0][i][j] : 0.f);
+      ck_set<CAREFUL>(R, i, j, j <= i ? sums[2][i][j] : 0.f);
+      ck_set<CAREFUL>(Q, i, j, j <= i ? sums[3][i][j] : 0.f);
     }
   }
   __syncthreads();
@@ -319,8 +335,8 @@ delta_rows_kernel(const TA* __restrict__ r, const TA* __restrict__ k, const TA* 
     };
     rows_of(us, x);
     rows_of(rs, f);
-    ck_system_rows(tile, 1, ROW, c0, lane, T, Q, x, f);
-    ck_operand(f, a);
+    ck_system_rows<CAREFUL>(tile, 1, ROW, c0, lane, T, Q, x, f, look);
+    ck_operand_of<CAREFUL>(f, a, look);
     ck_put(tile, 0, ROW, c0, lane, a);
     ck_tile_written();
     __syncthreads();
@@ -334,29 +350,30 @@ delta_rows_kernel(const TA* __restrict__ r, const TA* __restrict__ k, const TA* 
     float e_v[8], y[8], o[8];
 #pragma unroll
     for (int e = 0; e < 8; ++e) e_v[e] = y[e] = o[e] = 0.f;
-    ck_apply(R, value, lane, o);
-    ck_apply(E, value, lane, e_v);
-    ck_apply(T, e_v, lane, y);
-    ck_apply(Q, y, lane, o);
+    ck_apply<CAREFUL>(R, value, lane, o, look);
+    ck_apply<CAREFUL>(E, value, lane, e_v, look);
+    ck_apply<CAREFUL>(T, e_v, lane, y, look);
+    ck_apply<CAREFUL>(Q, y, lane, o, look);
 #pragma unroll
     for (int e = 0; e < 8; ++e) {
       const int t = ck_token(lane, e), c = c0 + ck_channel(lane, e);
       if (t < have && c < d) {
         const size_t to = (t0 + t) * width + (size_t)h * d + c;
-        v_out[to] = value[e];
-        u_out[to] = y[e];
-        g_out[to] = o[e];
+        p.v_out[to] = value[e];
+        p.u_out[to] = y[e];
+        p.g_out[to] = o[e];
       }
     }
   }
   __syncthreads();      // F and W have left
+  if (tid == 0) tile[DMAX / 2] = __int_as_float(CAREFUL);      // (B's flag: the place of B is that of F now)
 #pragma unroll
   for (int plane = 0; plane < 2; ++plane) {
     uint32_t a[3][4];
     float x[8];
 #pragma unroll
     for (int e = 0; e < 8; ++e) x[e] = (plane ? ks : as)[ck_token(lane, e)][c0 + ck_channel(lane, e)];
-    ck_operand(x, a);
+    ck_operand_of<CAREFUL>(x, a, look);
     ck_put(tile, plane, ROW, c0, lane, a);
   }
   ck_tile_written();
@@ -364,8 +381,19 @@ delta_rows_kernel(const TA* __restrict__ r, const TA* __restrict__ k, const TA* 
   if (tid == 0) {
     ck_tile_leaves(tile_out + CK_B * ck_rows(1, DMAX), tile, ck_rows(1, DMAX));
     ck_tile_leaves(tile_out + CK_C * ck_rows(1, DMAX), tile + ck_rows(1, DMAX), ck_rows(1, DMAX));
-    ck_tile_left();
+    ck_tile_arrived();
   }
+  return !CAREFUL && look.found();
+}
+template <typename TA>
+__device__ __noinline__ void delta_rows_carefully(const DeltaRowsArgs<TA>& p, float* tile, DeltaRowsShared& sh) {
+  delta_rows<TA, true>(p, tile, sh);
+}
+template <typename TA>
+__global__ void __launch_bounds__(128, 4) delta_rows_kernel(const __grid_constant__ DeltaRowsArgs<TA> p) {
+  extern __shared__ __align__(128) float dr_raw[];
+  __shared__ DeltaRowsShared sh;
+  if (__syncthreads_or(delta_rows<TA, false>(p, dr_raw, sh))) delta_rows_carefully<TA>(p, dr_raw, sh);
 }
 
 // SOME: only requests of fewer than `below` tokens, the others are walked in turns. (A template: with the test in it the kernel
@@ -525,8 +553,8 @@ static int launch_delta(int dmax, dim3 grid, cudaStream_t stream, const void* r,
       cudaError_t e = cudaFuncSetAttribute(delta_rows_kernel<TA>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem_rows);
       if (e != cudaSuccess) return llmrs_fail("delta_rule: shared memory %zu: %s", smem_rows, cudaGetErrorString(e));
       delta_rows_kernel<TA><<<dim3((unsigned)ck_places(n_tokens, n_requests), n_heads), 128, smem_rows, stream>>>(
-          (const TA*)r, (const TA*)k, (const TA*)v, (const TA*)a_raw, in_stride, decay_raw, decay_bias, a_bias, q_start, n_new, tiles,
-          u, g, v_rows, n_requests, n_heads, d, decay_scale, key_eps, walk_from);
+          {(const TA*)r, (const TA*)k, (const TA*)v, (const TA*)a_raw, in_stride, decay_raw, decay_bias, a_bias, q_start, n_new, tiles,
+           u, g, v_rows, n_requests, n_heads, d, decay_scale, key_eps, walk_from});
       rc = llmrs_launch_status("delta_rule (chunks)");
       if (rc != 0) return rc;
       ChunkArgs a = {};

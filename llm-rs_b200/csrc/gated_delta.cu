@@ -465,26 +465,36 @@ gdr_turns_kernel(const TA* __restrict__ x, long long stride, const float* __rest
 // 15 - j, so that every warp has seventeen steps. Then sixteen channels and sixteen columns a warp at a time.
 constexpr int GCR_THREADS = 256;
 __host__ __device__ constexpr int gcr_smem(int dmax) { return 4 * (ck_tile(CK_SYSTEM, dmax) + 3 * CK * (dmax + 4)); }
-template <int DMAX>
-__global__ void __launch_bounds__(GCR_THREADS)
-gdr_channel_rows_kernel(const float* __restrict__ pq, const float* __restrict__ pk, const float* __restrict__ pv,
-                        const float* __restrict__ pbeta, const float* __restrict__ araw, const float* __restrict__ a_log,
-                        const float* __restrict__ dt_bias, const int* __restrict__ q_start, const int* __restrict__ n_new,
-                        float* __restrict__ tiles, float* __restrict__ u, float* __restrict__ g_out, int n_requests, int G, int H,
-                        int d, int dv, int from) {
+struct GcrArgs {
+  const float *pq, *pk, *pv, *pbeta, *araw, *a_log, *dt_bias;
+  const int *q_start, *n_new;
+  float *tiles, *u, *g_out;
+  int n_requests, G, H, d, dv, from;
+};
+struct GcrShared {
+  alignas(16) __nv_bfloat16 Q[CK_MATRIX], T[CK_MATRIX];
+  float sums[2][CK][CK + 1], strength[CK];
+};
+// True where CAREFUL would make something else of it.
+template <int DMAX, bool CAREFUL>
+__device__ __forceinline__ bool gdr_channel_rows(const GcrArgs& p, float* tile, GcrShared& sh) {
   constexpr int GS = CK + 1, RS = DMAX + 4, ROW = DMAX + 8, PER = DMAX / 32;
   constexpr int EACH = (CK * (DMAX / 4) + GCR_THREADS - 1) / GCR_THREADS;
-  extern __shared__ __align__(128) float gcr_raw[];
-  float* tile = gcr_raw;
+  const float *pq = p.pq, *pk = p.pk, *pv = p.pv, *pbeta = p.pbeta, *araw = p.araw, *a_log = p.a_log, *dt_bias = p.dt_bias;
+  const int *q_start = p.q_start, *n_new = p.n_new;
+  const int n_requests = p.n_requests, G = p.G, H = p.H, d = p.d, dv = p.dv, from = p.from;
   auto q = reinterpret_cast<float (*)[RS]>(tile + ck_tile(CK_SYSTEM, DMAX));
   auto k = q + CK, g = k + CK;
-  __shared__ __align__(16) __nv_bfloat16 Q[CK_MATRIX], T[CK_MATRIX];
-  __shared__ float sums[2][CK][GS], strength[CK];
+  auto& Q = sh.Q;
+  auto& T = sh.T;
+  auto& sums = sh.sums;
+  auto& strength = sh.strength;
+  CkLook look;
   const int place = blockIdx.x, h = blockIdx.y, tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
   int t_req, n_req;
   const int req = ck_request(q_start, n_new, n_requests, place, t_req, n_req);
   const int first = (place - ck_place(t_req, req)) * CK, have = min(CK, n_req - first);
-  if (first < 0 || have <= 0 || n_req < from) return;
+  if (first < 0 || have <= 0 || n_req < from) return false;
   const size_t t0 = (size_t)(t_req + first);
   const int kh = h / (H / G);
   {
@@ -568,13 +578,14 @@ gdr_channel_rows_kernel(const float* __restrict__ pq, const float* __restrict__ 
       g[t][tid] = to_end[t];
     }
     tile[ck_rows(CK_SYSTEM, DMAX) + tid] = up;
+    if (tid == 0) tile[ck_flag(DMAX)] = __int_as_float(CAREFUL);
   } else if (warp == 4 && lane < CK) {
 #pragma unroll
     for (int i = 0; i < CK; ++i) sums[1][i][lane] *= strength[i];      // (each lane its own column)
     __syncwarp(0xffffu);
-    ck_solve(&sums[1][0][0], GS, 1.f, lane, strength[lane], T);
+    ck_solve<CAREFUL>(&sums[1][0][0], GS, 1.f, lane, strength[lane], T);
   } else if (warp > 4) {
-    for (int e = tid - 160; e < CK * CK; e += GCR_THREADS - 160) ck_set(Q, e / CK, e % CK, e % CK <= e / CK ? sums[0][e / CK][e % CK] : 0.f);
+    for (int e = tid - 160; e < CK * CK; e += GCR_THREADS - 160) ck_set<CAREFUL>(Q, e / CK, e % CK, e % CK <= e / CK ? sums[0][e / CK][e % CK] : 0.f);
   }
   __syncthreads();
   for (int c0 = 16 * warp; c0 < DMAX; c0 += 16 * (GCR_THREADS / 32)) {
@@ -587,10 +598,10 @@ gdr_channel_rows_kernel(const float* __restrict__ pq, const float* __restrict__ 
       f[e] = q[t][c];
       b[e] = g[t][c];
     }
-    ck_system_rows(tile, CK_W, ROW, c0, lane, T, Q, x, f);
-    ck_operand(f, a);
+    ck_system_rows<CAREFUL>(tile, CK_W, ROW, c0, lane, T, Q, x, f, look);
+    ck_operand_of<CAREFUL>(f, a, look);
     ck_put(tile, CK_F, ROW, c0, lane, a);
-    ck_operand(b, a);
+    ck_operand_of<CAREFUL>(b, a, look);
     ck_put(tile, CK_B, ROW, c0, lane, a);
   }
   ck_tile_written();
@@ -599,32 +610,40 @@ gdr_channel_rows_kernel(const float* __restrict__ pq, const float* __restrict__ 
     float y[8], o[8];
 #pragma unroll
     for (int e = 0; e < 8; ++e) y[e] = o[e] = 0.f;
-    ck_apply(T, v, lane, y);
-    ck_apply(Q, y, lane, o);
+    ck_apply<CAREFUL>(T, v, lane, y, look);
+    ck_apply<CAREFUL>(Q, y, lane, o, look);
 #pragma unroll
     for (int e = 0; e < 8; ++e) {
       const int t = ck_token(lane, e), col = 16 * group + ck_channel(lane, e);
       if (t < have && col < dv) {
-        u[((t0 + t) * H + h) * dv + col] = y[e];
-        g_out[((t0 + t) * H + h) * dv + col] = o[e];
+        p.u[((t0 + t) * H + h) * dv + col] = y[e];
+        p.g_out[((t0 + t) * H + h) * dv + col] = o[e];
       }
     }
   }
   __syncthreads();
   if (tid == 0) {
-    ck_tile_leaves(tiles + ((size_t)place * H + h) * ck_tile(CK_SYSTEM, DMAX), tile, ck_tile(CK_SYSTEM, DMAX));
-    ck_tile_left();
+    ck_tile_leaves(p.tiles + ((size_t)place * H + h) * ck_tile(CK_SYSTEM, DMAX), tile, ck_tile(CK_SYSTEM, DMAX));
+    ck_tile_arrived();
   }
+  return !CAREFUL && look.found();
 }
 template <int DMAX>
-static int launch_channel_rows(dim3 grid, cudaStream_t stream, const float* pq, const float* pk, const float* pv, const float* pbeta,
-                               const float* araw, const float* a_log, const float* dt_bias, const int* q_start, const int* n_new,
-                               float* tiles, float* u, float* g, int n_requests, int G, int H, int d, int dv, int from) {
+__device__ __noinline__ void gdr_channel_rows_carefully(const GcrArgs& p, float* tile, GcrShared& sh) {
+  gdr_channel_rows<DMAX, true>(p, tile, sh);
+}
+template <int DMAX>
+__global__ void __launch_bounds__(GCR_THREADS, 3) gdr_channel_rows_kernel(const __grid_constant__ GcrArgs p) {
+  extern __shared__ __align__(128) float gcr_raw[];
+  __shared__ GcrShared sh;
+  if (__syncthreads_or(gdr_channel_rows<DMAX, false>(p, gcr_raw, sh))) gdr_channel_rows_carefully<DMAX>(p, gcr_raw, sh);
+}
+template <int DMAX>
+static int launch_channel_rows(dim3 grid, cudaStream_t stream, const GcrArgs& p) {
   constexpr size_t smem = gcr_smem(DMAX);
   cudaError_t e = cudaFuncSetAttribute(gdr_channel_rows_kernel<DMAX>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
   if (e != cudaSuccess) return llmrs_fail("gated_delta: shared memory %zu: %s", smem, cudaGetErrorString(e));
-  gdr_channel_rows_kernel<DMAX><<<grid, GCR_THREADS, smem, stream>>>(pq, pk, pv, pbeta, araw, a_log, dt_bias, q_start, n_new, tiles, u,
-                                                                     g, n_requests, G, H, d, dv, from);
+  gdr_channel_rows_kernel<DMAX><<<grid, GCR_THREADS, smem, stream>>>(p);
   return llmrs_launch_status("gated_delta (chunks)");
 }
 
@@ -957,8 +976,8 @@ static int launch_chunk_walk(bool channel, const TurnRows& r, float* work, const
   if (channel) {
     LLMRS_REQUIRE(H <= 65535, "gated_delta: too many heads");
     const dim3 grid((unsigned)ck_places(n_tokens, n_requests), H);
-    rc = (d <= 64 ? launch_channel_rows<64> : launch_channel_rows<128>)(grid, stream, r.pq, r.pk, r.pv, r.pbeta, araw, a_log, dt_bias,
-                                                                        q_start, n_new, tiles, u, g, n_requests, G, H, d, dv, from);
+    const GcrArgs a = {r.pq, r.pk, r.pv, r.pbeta, araw, a_log, dt_bias, q_start, n_new, tiles, u, g, n_requests, G, H, d, dv, from};
+    rc = (d <= 64 ? launch_channel_rows<64> : launch_channel_rows<128>)(grid, stream, a);
   } else {
     ChunkRowsArgs a = {};
     a.q = r.pq; a.k = r.pk; a.stride = (long long)G * d; a.v = r.pv; a.decay = r.pg; a.beta = r.pbeta;

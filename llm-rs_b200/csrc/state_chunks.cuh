@@ -13,7 +13,8 @@
 //   generalized    U = T E V             W = T u                 F = r + Q W           G = R V + Q U         B = a, C = k
 //                  T = (I - A)^-1, the rows decayed from the chunk's start (u, r) or to its end (a, k)
 //
-// Rows are sums over tokens up to their own and nothing else, so a token that is not finite leaves earlier read-outs alone.
+// Rows are sums over tokens up to their own and nothing else, so a token that is not finite leaves earlier read-outs alone. An infinite
+// value or state is one in its own column, as it is token by token, and a finite one stays finite up to the end of the range (CK_LARGE).
 //
 // Nothing is held in fewer than 32 bits. A float32 operand x goes into the tensor cores as three bfloat16 numbers, x = x0 + x1 + x2
 // with x0 = bf16(x), x1 = bf16(x - x0), x2 = bf16(x - x0 - x1): 24 bits, and a product of two such operands is the six products
@@ -47,9 +48,11 @@ enum { CK_F = 0, CK_B = 1, CK_W = 2, CK_C = 3 };
 enum { CK_LINEAR = 2, CK_SYSTEM = 3, CK_GENERAL = 4 };      // the kinds, by their planes
 
 // A chunk's rows of one head, in floats: the planes' pieces [planes][3][16][dmax + 8] bfloat16 (eight numbers beyond a row keep
-// neighbouring rows' reads in different banks), then the chunk's decay D [dmax].
+// neighbouring rows' reads in different banks), then the chunk's decay D [dmax]. (Whole lines of 128 bytes.)
 __host__ __device__ constexpr int ck_rows(int planes, int dmax) { return planes * 3 * CK * (dmax + 8) / 2; }
 __host__ __device__ constexpr int ck_tile(int planes, int dmax) { return ck_rows(planes, dmax) + dmax; }
+// Beyond the first row of B: a word that is not zero where a number that the chunk writes is large or not finite (CK_LARGE).
+__host__ __device__ constexpr int ck_flag(int dmax) { return CK_B * ck_rows(1, dmax) + dmax / 2; }
 __host__ __device__ constexpr int ck_dmax(int d) { return d <= 64 ? 64 : 128; }
 // Places of chunks among all chunks, as walk_place has them for turns.
 __host__ __device__ inline int ck_place(int q_start, int req) { return q_start / CK + req; }
@@ -80,12 +83,52 @@ inline long long ck_work_floats(int planes, int n_tokens, int n_requests, int n_
   return d > 128 ? 0 : ck_places(n_tokens, n_requests) * n_heads * ck_tile(planes, ck_dmax(d)) + 2LL * n_tokens * n_heads * columns + 8;
 }
 
-// The three pieces of two numbers, each pair packed as the operands want it.
+// The three pieces of two numbers, each pair packed as the operands want it. (Subtractions that the compiler does not draw together
+// with the product that made x: the pieces of a number do not depend on what stands around.)
+__device__ __forceinline__ void ck_rest(float x, float y, uint32_t pieces, float& rx, float& ry) {
+  rx = __fsub_rn(x, __uint_as_float(pieces << 16));
+  ry = __fsub_rn(y, __uint_as_float(pieces & 0xffff0000u));
+}
 __device__ __forceinline__ void ck_split(float x, float y, uint32_t& h, uint32_t& m, uint32_t& l) {
   h = pack_bf16(x, y);
-  const float rx = x - __uint_as_float(h << 16), ry = y - __uint_as_float(h & 0xffff0000u);
+  ck_rest(x, y, h, x, y);
+  m = pack_bf16(x, y);
+  ck_rest(x, y, m, x, y);
+  l = pack_bf16(x, y);
+}
+// The same for any numbers. An infinite one, and one that bfloat16 rounds to infinity, has no second piece: a number near the end of
+// the range starts from the largest bfloat16 instead, an infinite one is its first piece and zeros. A product with an infinite
+// operand is then right in its first sum alone (the others hold zero times infinity), which `ck_sum` knows.
+__device__ __forceinline__ void ck_split_any(float x, float y, uint32_t& h, uint32_t& m, uint32_t& l) {
+  auto infinite = [](float v) { return (__float_as_uint(v) & 0x7fffffffu) == 0x7f800000u; };
+  h = pack_bf16(x, y);
+  if ((h & 0x7fffu) == 0x7f80u && !infinite(x)) h -= 1u;
+  if ((h & 0x7fff0000u) == 0x7f800000u && !infinite(y)) h -= 0x10000u;
+  float rx, ry;
+  ck_rest(x, y, h, rx, ry);
+  if (infinite(x)) rx = 0.f;
+  if (infinite(y)) ry = 0.f;
   m = pack_bf16(rx, ry);
-  l = pack_bf16(rx - __uint_as_float(m << 16), ry - __uint_as_float(m & 0xffff0000u));
+  ck_rest(rx, ry, m, rx, ry);
+  l = pack_bf16(rx, ry);
+}
+// Numbers from 2^60 on, and those that are not finite, are looked for where they enter: a product of two smaller ones, and a state
+// that such products are written to sixteen times, stays far from the end of the range. The kernels run as if there were none, and a
+// block that has met one does all of its work once more with CAREFUL, which makes the same of every other number. (Looking costs one
+// to three per cent of a walk; care inside its loop, with a branch for every pair of numbers, cost a fifth.)
+constexpr float CK_LARGE = 1152921504606846976.f;
+struct CkLook {      // first pieces: one instruction a pair
+  __nv_bfloat162 most = __floats2bfloat162_rn(0.f, 0.f);
+  __device__ __forceinline__ void at(const uint32_t (&first)[4]) {
+#pragma unroll
+    for (int i = 0; i < 4; ++i) most = __hmax2_nan(most, __habs2(*reinterpret_cast<const __nv_bfloat162*>(&first[i])));
+  }
+  __device__ __forceinline__ bool found() const { return !(__low2float(most) < CK_LARGE && __high2float(most) < CK_LARGE); }
+};
+// The sum of a product's parts where operands may be infinite.
+__device__ __forceinline__ float ck_sum(float hi, float lo) {
+  const float s = hi + lo;
+  return s == s ? s : hi;
 }
 __device__ __forceinline__ void stmatrix_x4(void* row, const uint32_t (&r)[4]) {
   asm volatile("stmatrix.sync.aligned.m8n8.x4.shared.b16 [%0], {%1, %2, %3, %4};\n"
@@ -108,6 +151,27 @@ __device__ __forceinline__ void ck_zero(float (&x)[N][4]) {
   for (int i = 0; i < N; ++i) x[i][0] = x[i][1] = x[i][2] = x[i][3] = 0.f;
 }
 
+// Entry e of what a lane holds of an operand's sixteen tokens and sixteen channels (columns).
+__device__ __forceinline__ int ck_token(int lane, int e) { return 2 * (lane & 3) + (e & 1) + 8 * (e >> 2); }
+__device__ __forceinline__ int ck_channel(int lane, int e) { return (lane >> 2) + 8 * (e >> 1 & 1); }
+__device__ __forceinline__ void ck_operand(const float (&x)[8], uint32_t (&a)[3][4]) {
+#pragma unroll
+  for (int i = 0; i < 4; ++i) ck_split(x[2 * i], x[2 * i + 1], a[0][i], a[1][i], a[2][i]);
+}
+__device__ __forceinline__ void ck_operand_any(const float (&x)[8], uint32_t (&a)[3][4]) {
+#pragma unroll
+  for (int i = 0; i < 4; ++i) ck_split_any(x[2 * i], x[2 * i + 1], a[0][i], a[1][i], a[2][i]);
+}
+template <bool CAREFUL>
+__device__ __forceinline__ void ck_operand_of(const float (&x)[8], uint32_t (&a)[3][4], CkLook& look) {
+  if (CAREFUL) {
+    ck_operand_any(x, a);
+  } else {
+    ck_operand(x, a);
+    look.at(a[0]);
+  }
+}
+
 struct ChunkArgs {
   const float* tiles;          // [places, heads, ck_tile]
   const float *u, *g;          // [tokens, heads * ck_columns]
@@ -127,12 +191,12 @@ __host__ __device__ constexpr int ck_smem(int planes, int dmax) {
   return 4 * (CK_STAGES * ck_stage(planes, dmax) + 2 * ck_rows(1, dmax) + CK_WARPS * CK_COLS * (24 + 18));
 }
 
-template <int PLANES, int DMAX>
-__global__ void __launch_bounds__(CK_THREADS, 1) state_chunks_kernel(ChunkArgs p, int col_blocks) {
+// True where the block has to do it again, CAREFUL: nothing of the state is written then.
+template <int PLANES, int DMAX, bool CAREFUL>
+__device__ __forceinline__ bool state_chunks_of(const ChunkArgs& p, int col_blocks, float* ck_smem_raw) {
   constexpr int CH = DMAX / CK_WARPS, NT = CH / 8, KS = CH / 16, ROW = DMAX + 8, PLANE = 3 * CK * ROW, HALF = 32 * CK_WARPS;
   constexpr int TILE = ck_tile(PLANES, DMAX), STAGE = ck_stage(PLANES, DMAX), VALUES = PLANES == CK_GENERAL ? 3 : 2;
   constexpr bool SYSTEM = PLANES != CK_LINEAR;
-  extern __shared__ __align__(16) float ck_smem_raw[];
   float* stages = ck_smem_raw;
   __nv_bfloat16* held = reinterpret_cast<__nv_bfloat16*>(stages + CK_STAGES * STAGE);      // the state's pieces
   float* sums = stages + CK_STAGES * STAGE + 2 * ck_rows(1, DMAX);
@@ -141,7 +205,8 @@ __global__ void __launch_bounds__(CK_THREADS, 1) state_chunks_kernel(ChunkArgs p
   const int req = blockIdx.x / (col_blocks * p.n_heads), head = blockIdx.x / col_blocks % p.n_heads;
   const int col0 = blockIdx.x % col_blocks * CK_COLS, tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
   const int n = p.n_new[req], t0 = p.q_start[req], d = p.d, dv = p.dv, columns = p.columns;
-  if (n <= 0 || n < p.from) return;
+  if (n <= 0 || n < p.from) return false;
+  auto sum_of = [](float hi, float lo) { return CAREFUL ? ck_sum(hi, lo) : hi + lo; };
   const int n_chunks = (n + CK - 1) / CK, place0 = ck_place(t0, req);
   for (int e = tid; e < CK_STAGES * VALUES * CK * 20; e += CK_THREADS)      // columns beyond the values stay 0
     stages[e / (VALUES * CK * 20) * STAGE + TILE + e % (VALUES * CK * 20)] = 0.f;
@@ -181,7 +246,8 @@ __global__ void __launch_bounds__(CK_THREADS, 1) state_chunks_kernel(ChunkArgs p
       cp_async_wait<1>();
       __syncthreads();
     }
-    return;
+    cp_async_wait<0>();
+    return !CAREFUL && __syncthreads_or(0);
   }
   if (warp >= CK_WARPS) {
     // The warps that read out.
@@ -211,7 +277,7 @@ __global__ void __launch_bounds__(CK_THREADS, 1) state_chunks_kernel(ChunkArgs p
       for (int i = 0; i < 2; ++i)
 #pragma unroll
         for (int c = 0; c < 2; ++c)
-          *reinterpret_cast<float2*>(to + c * 8 * 18 + i * 8) = make_float2(hi[i][2 * c] + lo[i][2 * c], hi[i][2 * c + 1] + lo[i][2 * c + 1]);
+          *reinterpret_cast<float2*>(to + c * 8 * 18 + i * 8) = make_float2(sum_of(hi[i][2 * c], lo[i][2 * c]), sum_of(hi[i][2 * c + 1], lo[i][2 * c + 1]));
       __syncwarp();
       asm volatile("bar.sync 2, 128;" ::: "memory");      // every reading warp's sums are there
       const int at = ct >> 3, c = 2 * (ct & 7), col = col0 + c;
@@ -236,7 +302,7 @@ __global__ void __launch_bounds__(CK_THREADS, 1) state_chunks_kernel(ChunkArgs p
       __syncthreads();
     }
     read_out(n_chunks - 1);
-    return;
+    return !CAREFUL && __syncthreads_or(0);
   }
 
   // The warps that walk. Lane 4 g + t: columns g and g + 8.
@@ -257,25 +323,28 @@ __global__ void __launch_bounds__(CK_THREADS, 1) state_chunks_kernel(ChunkArgs p
       const float* at = state_at(nt, e);
       S[nt][e] = at ? *at : 0.f;
     }
+  CkLook look;
+  int large = 0;
   __syncthreads();      // chunk 0
 
   for (int chunk = 0; chunk < n_chunks; ++chunk) {
     const float* base = stages + chunk % CK_STAGES * STAGE;
     const __nv_bfloat16* rows = reinterpret_cast<const __nv_bfloat16*>(base);
-    auto operand = [&](const float (&y)[8], uint32_t (&a)[3][4]) {
-#pragma unroll
-      for (int i = 0; i < 4; ++i) ck_split(y[2 * i], y[2 * i + 1], a[0][i], a[1][i], a[2][i]);
-    };
     // The state's pieces, for W S here and for the read-outs.
     uint32_t a[KS][3][4];
 #pragma unroll
     for (int ks = 0; ks < KS; ++ks) {
 #pragma unroll
-      for (int i = 0; i < 4; ++i)
-        ck_split(S[2 * ks + (i >> 1)][2 * (i & 1)], S[2 * ks + (i >> 1)][2 * (i & 1) + 1], a[ks][0][i], a[ks][1][i], a[ks][2][i]);
+      for (int i = 0; i < 4; ++i) {
+        const float s0 = S[2 * ks + (i >> 1)][2 * (i & 1)], s1 = S[2 * ks + (i >> 1)][2 * (i & 1) + 1];
+        if (CAREFUL) ck_split_any(s0, s1, a[ks][0][i], a[ks][1][i], a[ks][2][i]);
+        else ck_split(s0, s1, a[ks][0][i], a[ks][1][i], a[ks][2][i]);
+      }
 #pragma unroll
       for (int x = 0; x < 3; ++x) stmatrix_x4(held + (chunk & 1) * PLANE + (x * CK + row_trans) * ROW + ch0 + 16 * ks + col_trans, a[ks][x]);
+      look.at(a[ks][0]);
     }
+    large |= __float_as_int(base[ck_flag(DMAX)]);
     // Entry e of what a column's tokens bring, in the order of an operand: token 2 t + (e & 1) + 8 (e >> 2) of column
     // g + 8 (e >> 1 & 1).
     auto values = [&](int which, float (&v)[8]) {
@@ -296,7 +365,8 @@ __global__ void __launch_bounds__(CK_THREADS, 1) state_chunks_kernel(ChunkArgs p
     };
     auto write = [&](const float (&what)[8]) {
       uint32_t left[3][4];
-      operand(what, left);
+      if (CAREFUL) ck_operand_any(what, left);
+      else ck_operand(what, left);
       ck_mma<NT / 2>(add, add_lo, left, written);
     };
     if constexpr (PLANES == CK_GENERAL) {
@@ -325,7 +395,7 @@ __global__ void __launch_bounds__(CK_THREADS, 1) state_chunks_kernel(ChunkArgs p
       for (int i = 0; i < 2; ++i)
 #pragma unroll
         for (int c = 0; c < 2; ++c)
-          *reinterpret_cast<float2*>(to + c * 8 * 24 + i * 8) = make_float2(hi[i][2 * c] + lo[i][2 * c], hi[i][2 * c + 1] + lo[i][2 * c + 1]);
+          *reinterpret_cast<float2*>(to + c * 8 * 24 + i * 8) = make_float2(sum_of(hi[i][2 * c], lo[i][2 * c]), sum_of(hi[i][2 * c + 1], lo[i][2 * c + 1]));
       __syncwarp();
       asm volatile("bar.sync 1, 128;" ::: "memory");      // every walking warp's sums are there
 #pragma unroll
@@ -338,15 +408,23 @@ __global__ void __launch_bounds__(CK_THREADS, 1) state_chunks_kernel(ChunkArgs p
         y[2 * i + 1] += (s[0].y + s[1].y) + (s[2].y + s[3].y);
       }
     }
+    if (CAREFUL)      // tokens beyond the last one write nothing (their rows are zeros, and zero times infinity is no number)
+#pragma unroll
+      for (int e = 0; e < 8; ++e)
+        if (chunk * CK + ck_token(lane, e) >= n) y[e] = 0.f;
     write(y);
 #pragma unroll
     for (int i = 0; i < NT; ++i) {
       const float2 decay = *reinterpret_cast<const float2*>(base + ck_rows(PLANES, DMAX) + ch0 + 8 * i + 2 * t);
 #pragma unroll
-      for (int e = 0; e < 4; ++e) S[i][e] = fmaf(e & 1 ? decay.y : decay.x, S[i][e], add[i][e] + add_lo[i][e]);
+      for (int e = 0; e < 4; ++e) {
+        const float written_here = !CAREFUL || ch0 + 8 * i + 2 * t + (e & 1) < d ? sum_of(add[i][e], add_lo[i][e]) : 0.f;      // (nor do channels beyond d)
+        S[i][e] = fmaf(e & 1 ? decay.y : decay.x, S[i][e], written_here);
+      }
     }
     __syncthreads();      // the next chunk is there, and everyone is done with this one
   }
+  if (!CAREFUL && __syncthreads_or(large || look.found())) return true;
 #pragma unroll
   for (int nt = 0; nt < NT; ++nt)
 #pragma unroll
@@ -354,6 +432,17 @@ __global__ void __launch_bounds__(CK_THREADS, 1) state_chunks_kernel(ChunkArgs p
       float* at = state_at(nt, e);
       if (at) *at = S[nt][e];
     }
+  return false;
+}
+template <int PLANES, int DMAX>
+__device__ __noinline__ void state_chunks_carefully(const ChunkArgs& p, int col_blocks, float* smem) {
+  state_chunks_of<PLANES, DMAX, true>(p, col_blocks, smem);
+}
+template <int PLANES, int DMAX>
+__global__ void __launch_bounds__(CK_THREADS, 2 * ck_smem(PLANES, DMAX) <= 226 * 1024 ? 2 : 1)
+state_chunks_kernel(const __grid_constant__ ChunkArgs p, int col_blocks) {
+  extern __shared__ __align__(16) float ck_smem_raw[];
+  if (state_chunks_of<PLANES, DMAX, false>(p, col_blocks, ck_smem_raw)) state_chunks_carefully<PLANES, DMAX>(p, col_blocks, ck_smem_raw);
 }
 
 template <int PLANES, int DMAX>
@@ -376,60 +465,61 @@ static int launch_state_chunks(const ChunkArgs& a, int n_requests, cudaStream_t 
 
 // ---- rows ------------------------------------------------------------------------------------------------------------
 // The products over tokens run transposed on the tensor cores, sixteen channels (or value columns) a warp: entry e of what a lane
-// 4 g + t holds of them is token 2 t + (e & 1) + 8 (e >> 2) of channel g + 8 (e >> 1 & 1), the order of an operand and, as it
-// happens, of the sums that come out.
-__device__ __forceinline__ int ck_token(int lane, int e) { return 2 * (lane & 3) + (e & 1) + 8 * (e >> 2); }
-__device__ __forceinline__ int ck_channel(int lane, int e) { return (lane >> 2) + 8 * (e >> 1 & 1); }
-__device__ __forceinline__ void ck_operand(const float (&x)[8], uint32_t (&a)[3][4]) {
-#pragma unroll
-  for (int i = 0; i < 4; ++i) ck_split(x[2 * i], x[2 * i + 1], a[0][i], a[1][i], a[2][i]);
-}
+// 4 g + t holds of them is token 2 t + (e & 1) + 8 (e >> 2) of channel g + 8 (e >> 1 & 1) (`ck_token`, `ck_channel`), the order of an
+// operand and, as it happens, of the sums that come out.
 // A matrix over the chunk's tokens in shared memory, [3][16][24]: three pieces, rows of 48 bytes (no two of eight on the same banks).
 // What lies above the diagonal must be zero.
 constexpr int CK_MATRIX = 3 * CK * 24;
+template <bool CAREFUL>
 __device__ __forceinline__ void ck_set(__nv_bfloat16* m, int i, int j, float x) {
   uint32_t piece[3];
-  ck_split(x, 0.f, piece[0], piece[1], piece[2]);
+  if (CAREFUL) ck_split_any(x, 0.f, piece[0], piece[1], piece[2]);
+  else ck_split(x, 0.f, piece[0], piece[1], piece[2]);
 #pragma unroll
   for (int k = 0; k < 3; ++k) m[(k * CK + i) * 24 + j] = __ushort_as_bfloat16((unsigned short)piece[k]);
 }
-// out[token i] += sum_j m[i][j] x[token j]. An x that is not finite (or of 2^127 and more, whose first piece would not be) reaches the
-// tokens from its own on and no earlier one: zero times it would be no number, so it goes in as zero and they are set.
-__device__ __forceinline__ void ck_apply(const __nv_bfloat16* m, const float (&x)[8], int lane, float (&out)[8]) {
+// out[token i] += sum_j m[i][j] x[token j]. CAREFUL: an x that is not finite reaches the tokens from its own on and no earlier one:
+// zero times it would be no number, so it goes in as zero and its products are added by themselves.
+template <bool CAREFUL>
+__device__ __forceinline__ void ck_apply(const __nv_bfloat16* m, const float (&x)[8], int lane, float (&out)[8], CkLook& look) {
+  auto finite = [](float v) { return (__float_as_uint(v) & 0x7fffffffu) < 0x7f800000u; };
   float hi[2][4], lo[2][4];
   uint32_t a[3][4], b[1][3][4];
   ck_zero(hi);
   ck_zero(lo);
 #pragma unroll
   for (int k = 0; k < 3; ++k) ldmatrix_x4(b[0][k], m + (k * CK + (lane & 7) + ((lane >> 4) << 3)) * 24 + (lane >> 3 & 1) * 8);
-  unsigned top = 0;
-#pragma unroll
-  for (int e = 0; e < 8; ++e) top = max(top, __float_as_uint(x[e]) & 0x7fffffffu);
-  if (!__any_sync(0xffffffffu, top >= 0x7f000000u)) {
+  if constexpr (!CAREFUL) {
     ck_operand(x, a);
+    look.at(a[0]);
+    look.at(b[0][0]);
     ck_mma<1>(hi, lo, a, b);
 #pragma unroll
     for (int e = 0; e < 8; ++e) out[e] += hi[e >> 2][e & 3] + lo[e >> 2][e & 3];
-    return;
-  }
-  float y[8];
-  int first[2] = {CK, CK};      // of the lane's two channels
+  } else {
+    float y[8];
 #pragma unroll
-  for (int e = 0; e < 8; ++e) {
-    const bool bad = (__float_as_uint(x[e]) & 0x7fffffffu) >= 0x7f000000u;
-    y[e] = bad ? 0.f : x[e];
-    if (bad) first[e >> 1 & 1] = min(first[e >> 1 & 1], ck_token(lane, e));
-  }
+    for (int e = 0; e < 8; ++e) y[e] = finite(x[e]) ? x[e] : 0.f;
+    ck_operand_any(y, a);
+    ck_mma<1>(hi, lo, a, b);
 #pragma unroll
-  for (int c = 0; c < 2; ++c) {
-    first[c] = min(first[c], __shfl_xor_sync(0xffffffffu, first[c], 1));
-    first[c] = min(first[c], __shfl_xor_sync(0xffffffffu, first[c], 2));
-  }
-  ck_operand(y, a);
-  ck_mma<1>(hi, lo, a, b);
+    for (int e = 0; e < 8; ++e) out[e] += ck_sum(hi[e >> 2][e & 3], lo[e >> 2][e & 3]);
 #pragma unroll
-  for (int e = 0; e < 8; ++e)
-    out[e] = ck_token(lane, e) >= first[e >> 1 & 1] ? __int_as_float(0x7fffffff) : out[e] + (hi[e >> 2][e & 3] + lo[e >> 2][e & 3]);
+    for (int j = 0; j < CK; ++j)
+#pragma unroll
+      for (int c = 0; c < 2; ++c) {      // token j of the lane's channel c: lane j % 8 / 2 of its four has it
+        const float xj = __shfl_sync(0xffffffffu, x[(j & 1) + 2 * c + 4 * (j >> 3)], (lane & ~3) | (j & 7) >> 1);
+        if (!finite(xj)) {
+#pragma unroll
+          for (int e = 2 * c; e < 8; e += (e & 1) ? 3 : 1) {
+            const int i = ck_token(lane, e);
+            const __nv_bfloat16* at = m + i * 24 + j;
+            if (i >= j) out[e] = fmaf((__bfloat162float(at[0]) + __bfloat162float(at[CK * 24])) + __bfloat162float(at[2 * CK * 24]), xj, out[e]);
+          }
+        }
+        __syncwarp();
+      }
+  }
 }
 // Rows of a plane, channels c0 .. c0 + 15.
 __device__ __forceinline__ void ck_put(float* tile, int plane, int row, int c0, int lane, const uint32_t (&a)[3][4]) {
@@ -440,18 +530,20 @@ __device__ __forceinline__ void ck_put(float* tile, int plane, int row, int c0, 
                  ::"r"(smem_addr(to + k * CK * row)), "r"(a[k][0]), "r"(a[k][1]), "r"(a[k][2]), "r"(a[k][3]) : "memory");
 }
 // W = T x into its plane, then f + Q W, F.
+template <bool CAREFUL>
 __device__ __forceinline__ void ck_system_rows(float* tile, int plane, int row, int c0, int lane, const __nv_bfloat16* T, const __nv_bfloat16* Q,
-                                               const float (&x)[8], float (&f)[8]) {
+                                               const float (&x)[8], float (&f)[8], CkLook& look) {
   uint32_t a[3][4];
   float w[8];
 #pragma unroll
   for (int e = 0; e < 8; ++e) w[e] = 0.f;
-  ck_apply(T, x, lane, w);
-  ck_operand(w, a);
+  ck_apply<CAREFUL>(T, x, lane, w, look);
+  ck_operand_of<CAREFUL>(w, a, look);
   ck_put(tile, plane, row, c0, lane, a);
-  ck_apply(Q, w, lane, f);
+  ck_apply<CAREFUL>(Q, w, lane, f, look);
 }
 // Column c of (I + sign M)^-1 diag(scale), M below the diagonal with rows `stride` apart: forward substitution.
+template <bool CAREFUL>
 __device__ __forceinline__ void ck_solve(const float* m, int stride, float sign, int c, float scale, __nv_bfloat16* out) {
   float col[CK];
 #pragma unroll
@@ -460,12 +552,12 @@ __device__ __forceinline__ void ck_solve(const float* m, int stride, float sign,
 #pragma unroll
     for (int j = 0; j < i; ++j) acc = fmaf(-sign * m[i * stride + j], col[j], acc);
     col[i] = i >= c ? acc : 0.f;      // (what is no number in a row of M stays in the rows from it on)
-    ck_set(out, i, c, i >= c ? acc * scale : 0.f);
+    ck_set<CAREFUL>(out, i, c, i >= c ? acc * scale : 0.f);
   }
 }
 // hi + lo times x, lo being what rounding took from hi.
 __device__ __forceinline__ void ck_times(float& hi, float& lo, float x) {
-  const float product = hi * x;
+  const float product = __fmul_rn(hi, x);
   lo = fmaf(lo, x, fmaf(hi, x, -product));
   hi = product;
 }
@@ -490,6 +582,7 @@ __device__ __forceinline__ void ck_tile_leaves(float* to, const float* tile, int
   asm volatile("cp.async.bulk.global.shared::cta.bulk_group [%0], [%1], %2;\n\tcp.async.bulk.commit_group;"
                ::"l"(to), "r"(smem_addr(tile)), "r"(floats * 4) : "memory");
 }
+__device__ __forceinline__ void ck_tile_arrived() { asm volatile("cp.async.bulk.wait_group 0;" ::: "memory"); }      // in memory too
 __device__ __forceinline__ void ck_tile_left() { asm volatile("cp.async.bulk.wait_group.read 0;" ::: "memory"); }
 
 // The rows of CK_LINEAR and CK_SYSTEM with a decay per token and head: a block per (place, key head). First the products of the rows
@@ -499,25 +592,32 @@ __device__ __forceinline__ void ck_tile_left() { asm volatile("cp.async.bulk.wai
 // the CUDA cores 61), 16 heads without a system 38. Three blocks an SM: with two, the products apart from the tile, 55 and 48.
 constexpr int CK_ROWS_THREADS = 256;
 __host__ __device__ constexpr int ck_rows_smem(int planes, int dmax) { return 4 * (ck_tile(planes, dmax) + 2 * CK * (dmax + 4)); }
-template <int PLANES, int DMAX>
-__global__ void __launch_bounds__(CK_ROWS_THREADS, 3)
-ck_rows_kernel(ChunkRowsArgs p) {
+struct CkRowsShared {      // beside the tile
+  float gram[2][CK][CK + 1], strengths[2][2][CK], P[2][CK], Z[2][CK], own[2][CK][CK + 1];
+  alignas(16) __nv_bfloat16 Q[2][CK_MATRIX], T[2][CK_MATRIX];
+};
+// True where CAREFUL would make something else of it.
+template <int PLANES, int DMAX, bool CAREFUL>
+__device__ __forceinline__ bool ck_rows_of(const ChunkRowsArgs& p, float* tile, CkRowsShared& sh) {
   constexpr int RS = DMAX + 4, GS = CK + 1, ROW = DMAX + 8, THREADS = CK_ROWS_THREADS, HEADS = 2, WARPS = 4;
   constexpr int EACH = (2 * CK * (DMAX / 4) + THREADS - 1) / THREADS;
   constexpr bool SYSTEM = PLANES == CK_SYSTEM;
-  extern __shared__ __align__(128) float ck_rows_raw[];
-  float* tile = ck_rows_raw;
   float* rows = tile + ck_tile(PLANES, DMAX);      // k, q: [2][16][RS]
   auto part = reinterpret_cast<float (*)[2][CK][CK]>(tile);      // [WARPS]: a warp's share of the products, before there is a tile
   static_assert(ck_tile(PLANES, DMAX) >= WARPS * 2 * CK * CK, "the products lie where the tile will be");
-  __shared__ float gram[2][CK][GS], strengths[HEADS][2][CK], P[HEADS][CK], Z[HEADS][CK];
-  __shared__ float own[HEADS][CK][GS];
-  __shared__ __align__(16) __nv_bfloat16 Q[HEADS][CK_MATRIX], T[HEADS][CK_MATRIX];
+  auto& gram = sh.gram;
+  auto& strengths = sh.strengths;
+  auto& P = sh.P;
+  auto& Z = sh.Z;
+  auto& own = sh.own;
+  auto& Q = sh.Q;
+  auto& T = sh.T;
+  CkLook look;
   const int place = blockIdx.x, group = blockIdx.y, tid = threadIdx.x, lane = tid & 31, warp = tid >> 5, d = p.d;
   int t_req, n_req;
   const int req = ck_request(p.q_start, p.n_new, p.n_requests, place, t_req, n_req);
   const int first = (place - ck_place(t_req, req)) * CK, have = min(CK, n_req - first);
-  if (first < 0 || have <= 0 || n_req < p.from) return;
+  if (first < 0 || have <= 0 || n_req < p.from) return false;
   const size_t t0 = (size_t)(t_req + first);
   const int shared = p.n_heads / p.n_groups;
   float decay_in = 0.f, beta_in = 0.f;      // of token `lane` and this warp's head, the first ones on their way early
@@ -560,8 +660,11 @@ ck_rows_kernel(ChunkRowsArgs p) {
 #pragma unroll
         for (int i = 0; i < 4; ++i) {
           const float2 x = *reinterpret_cast<const float2*>(rows + (a * CK + g + 8 * (i & 1)) * RS + c + 8 * (i >> 1));
-          ck_split(x.x, x.y, left[a][0][i], left[a][1][i], left[a][2][i]);
+          if (CAREFUL) ck_split_any(x.x, x.y, left[a][0][i], left[a][1][i], left[a][2][i]);
+          else ck_split(x.x, x.y, left[a][0][i], left[a][1][i], left[a][2][i]);
         }
+      look.at(left[0][0]);
+      look.at(left[1][0]);
 #pragma unroll
       for (int x = 0; x < 3; ++x) {      // k on the right: tokens g, then g + 8, of both halves of the channels
         right[0][x][0] = left[0][x][0];
@@ -577,7 +680,7 @@ ck_rows_kernel(ChunkRowsArgs p) {
 #pragma unroll
       for (int i = 0; i < 2; ++i)
 #pragma unroll
-        for (int e = 0; e < 4; ++e) part[warp][a][g + 8 * (e >> 1)][8 * i + 2 * t + (e & 1)] = hi[a][i][e] + lo[a][i][e];
+        for (int e = 0; e < 4; ++e) part[warp][a][g + 8 * (e >> 1)][8 * i + 2 * t + (e & 1)] = CAREFUL ? ck_sum(hi[a][i][e], lo[a][i][e]) : hi[a][i][e] + lo[a][i][e];
   }
   __syncthreads();
   for (int e = tid; e < 2 * CK * CK; e += THREADS) {
@@ -599,16 +702,16 @@ ck_rows_kernel(ChunkRowsArgs p) {
         float between = 1.f, between_lo = 0.f, after = 1.f, after_lo = 0.f;
 #pragma unroll
         for (int j = CK - 1; j >= 0; --j) {
-          const float decay = strengths[warp][0][j], w = between + between_lo;
-          ck_set(Q[warp], i, j, j <= i ? gram[1][i][j] * w : 0.f);
+          const float decay = strengths[warp][0][j], w = __fadd_rn(between, between_lo);
+          ck_set<CAREFUL>(Q[warp], i, j, j <= i ? gram[1][i][j] * w : 0.f);
           if (SYSTEM && j < i) own[warp][i][j] = beta_in * (gram[0][i][j] * w);
           if (j <= i) ck_times(between, between_lo, decay);
           if (j > i) ck_times(after, after_lo, decay);
         }
-        P[warp][i] = between + between_lo;
-        Z[warp][i] = after + after_lo;
+        P[warp][i] = __fadd_rn(between, between_lo);
+        Z[warp][i] = __fadd_rn(after, after_lo);
         __syncwarp(0xffffu);
-        if (SYSTEM) ck_solve(&own[warp][0][0], GS, 1.f, i, beta_in, T[warp]);
+        if (SYSTEM) ck_solve<CAREFUL>(&own[warp][0][0], GS, 1.f, i, beta_in, T[warp]);
       }
     }
     for (int x = 0; x < heads; ++x) {
@@ -625,7 +728,10 @@ ck_rows_kernel(ChunkRowsArgs p) {
         }
       };
       if (warp < groups) fetch(warp);
-      if (tid == 0) ck_tile_left();
+      if (tid == 0) {
+        ck_tile_left();
+        tile[ck_flag(DMAX)] = __int_as_float(CAREFUL);
+      }
       __syncthreads();      // the coefficients; the tile before has left
       float before[8], after[8];
 #pragma unroll
@@ -635,23 +741,26 @@ ck_rows_kernel(ChunkRowsArgs p) {
       }
       for (int c0 = 16 * warp; c0 < DMAX; c0 += 16 * (THREADS / 32)) {
         uint32_t a[3][4];
-        float k[8], f[8], out[8];
+        float k[8], q[8], f[8], out[8];
 #pragma unroll
         for (int e = 0; e < 8; ++e) {
           const float* at = rows + ck_token(lane, e) * RS + c0 + ck_channel(lane, e);
           k[e] = at[0];
-          f[e] = before[e] * at[CK * RS];
+          q[e] = at[CK * RS];
+          f[e] = 0.f;
         }
         if constexpr (SYSTEM) {
 #pragma unroll
           for (int e = 0; e < 8; ++e) out[e] = -before[e] * k[e];
-          ck_system_rows(tile, CK_W, ROW, c0, lane, T[x], Q[x], out, f);
+          ck_system_rows<CAREFUL>(tile, CK_W, ROW, c0, lane, T[x], Q[x], out, f, look);
         }
-        ck_operand(f, a);
+#pragma unroll
+        for (int e = 0; e < 8; ++e) f[e] = fmaf(before[e], q[e], f[e]);
+        ck_operand_of<CAREFUL>(f, a, look);
         ck_put(tile, CK_F, ROW, c0, lane, a);
 #pragma unroll
         for (int e = 0; e < 8; ++e) out[e] = after[e] * k[e];
-        ck_operand(out, a);
+        ck_operand_of<CAREFUL>(out, a, look);
         ck_put(tile, CK_B, ROW, c0, lane, a);
         if (lane < 16) tile[ck_rows(PLANES, DMAX) + c0 + lane] = P[x][CK - 1];
       }
@@ -662,18 +771,18 @@ ck_rows_kernel(ChunkRowsArgs p) {
         float u[8], g[8];
 #pragma unroll
         for (int e = 0; e < 8; ++e) {
-          g[e] = skip == 0.f ? 0.f : skip * v[e];
+          g[e] = 0.f;
           u[e] = SYSTEM ? 0.f : strengths[x][1][ck_token(lane, e)] * v[e];
         }
-        if constexpr (SYSTEM) ck_apply(T[x], v, lane, u);
-        ck_apply(Q[x], u, lane, g);
+        if constexpr (SYSTEM) ck_apply<CAREFUL>(T[x], v, lane, u, look);
+        ck_apply<CAREFUL>(Q[x], u, lane, g, look);
 #pragma unroll
         for (int e = 0; e < 8; ++e) {
           const int at = ck_token(lane, e), col = 16 * group + ck_channel(lane, e);
           if (at < have && col < p.columns) {
             const size_t to = ((t0 + at) * p.n_heads + h) * p.columns + col;
             p.u[to] = u[e];
-            p.g[to] = g[e];
+            p.g[to] = skip == 0.f ? g[e] : fmaf(skip, v[e], g[e]);
           }
         }
       }
@@ -681,7 +790,19 @@ ck_rows_kernel(ChunkRowsArgs p) {
       if (tid == 0) ck_tile_leaves(p.tiles + ((size_t)place * p.n_heads + h) * ck_tile(PLANES, DMAX), tile, ck_tile(PLANES, DMAX));
     }
   }
-  if (tid == 0) ck_tile_left();
+  if (tid == 0) ck_tile_arrived();
+  return !CAREFUL && look.found();
+}
+template <int PLANES, int DMAX>
+__device__ __noinline__ void ck_rows_carefully(const ChunkRowsArgs& p, float* tile, CkRowsShared& sh) {
+  ck_rows_of<PLANES, DMAX, true>(p, tile, sh);
+}
+template <int PLANES, int DMAX>
+__global__ void __launch_bounds__(CK_ROWS_THREADS, 3)
+ck_rows_kernel(const __grid_constant__ ChunkRowsArgs p) {
+  extern __shared__ __align__(128) float ck_rows_raw[];
+  __shared__ CkRowsShared sh;
+  if (__syncthreads_or(ck_rows_of<PLANES, DMAX, false>(p, ck_rows_raw, sh))) ck_rows_carefully<PLANES, DMAX>(p, ck_rows_raw, sh);
 }
 
 template <int PLANES, int DMAX>

@@ -128,3 +128,79 @@ def test_tokens_before_one_that_is_not_finite_keep_their_numbers(kind, at, bad):
     assert torch.isfinite(want).all()
     assert torch.equal(got[:at], want[:at])
     assert not torch.isfinite(got[at]).any()
+
+
+def _both_ways(kind, d, dv, lens, change_weights, change_x, change_state):
+    """(outputs, states) walked and token by token, the step's requests all one way."""
+    from llm_rs_b200.parts import Runtime
+    g = torch.Generator().manual_seed(7 * d + dv)
+    D, part = _part(kind, d, dv)
+    w = {s.name: torch.randn(s.shape, generator=g) * (0.5 if len(s.shape) == 1 else s.shape[-1] ** -0.5) for s in part.weight_specs()}
+    change_weights(w)
+    part.bind({k: t.to(DEV) for k, t in w.items()}, Runtime(torch.device(DEV), torch.float32, 4096))
+    x = torch.randn(sum(lens), D, generator=g)
+    change_x(x)
+    start = {name: 0.3 * torch.randn(len(lens), *shape, generator=g) for name, shape in part.state_need().tensors.items()}
+    change_state(start)
+    got = []
+    for turns in (1, 0):
+        state = {k: t.to(DEV) for k, t in start.items()}
+        with _in_turns(turns):
+            got.append((part.forward(x.to(DEV), _ctx(lens, [0] * len(lens)), SimpleNamespace(state=state)).cpu(),
+                        {k: t.cpu() for k, t in state.items()}))
+    return got
+
+
+LINEAR = ("memory", "retention", "mamba")
+
+
+def _same_kinds_of_numbers(kind, walked, single):
+    """Every state finite where it is finite token by token, there the same to float32's rounding (by columns: one of numbers near the
+    largest has neighbours of ordinary ones); under a linear rule infinities where they are, with their signs."""
+    for name in single:
+        a, b = walked[name].double(), single[name].double()
+        assert torch.equal(a.isfinite(), b.isfinite()), name
+        if kind in LINEAR:
+            assert torch.equal(a.isnan(), b.isnan()) and torch.equal(a[a.isinf()], b[b.isinf()]), name
+        a, b = a.nan_to_num(0.0, 0.0, 0.0), b.nan_to_num(0.0, 0.0, 0.0)
+        size = b.abs().amax(-2, keepdim=True) if b.dim() > 3 else b.abs().amax()
+        assert bool(((a - b).abs() <= 3.2e-5 * size.clamp(min=1.0)).all()), name
+
+
+@pytest.mark.parametrize("kind", ["memory", "retention", "mamba", "gated", "channel", "general"])
+@pytest.mark.parametrize("d,dv", [(64, 48), (36, 20), (30, 17)])
+@pytest.mark.parametrize("value", [3.4e38, -1.8e38, float("inf"), float("nan")])
+def test_states_at_the_edge_of_the_range(kind, d, dv, value):
+    """A state that is huge, infinite or no number in one column: its column alone holds it, in whole and broken chunks."""
+    if kind == "general":
+        dv = d
+    def change(state):
+        name = [k for k in state if k.endswith(".state")][0]
+        for slot in range(state[name].size(0)):
+            state[name][slot, 1, 5 + slot, 3 + slot] = value
+    (out, walked), (want, single) = _both_ways(kind, d, dv, [37, 5, 16], lambda w: None, lambda x: None, change)
+    _same_kinds_of_numbers(kind, walked, single)
+    if abs(value) < 1e39 and d % 4 == 0:      # (in turns a product of three numbers near the range's end is taken in another order)
+        assert torch.equal(out.isfinite(), want.isfinite())
+        assert float((out - want).nan_to_num(0.0, 0.0, 0.0).abs().max()) <= 3.2e-5 * max(1.0, float(want.nan_to_num(0.0, 0.0, 0.0).abs().max()))
+
+
+@pytest.mark.parametrize("kind", ["memory", "retention", "gated", "channel", "general"])
+@pytest.mark.parametrize("d,dv", [(64, 48), (36, 20), (30, 17)])
+@pytest.mark.parametrize("at", [0, 3, 15, 16, 36, 38])
+@pytest.mark.parametrize("value", [1.8e38, float("inf")])
+def test_values_at_the_edge_of_the_range(kind, d, dv, at, value):
+    """A token whose value is huge or infinite in one column, at the first and last token of chunks and of requests."""
+    if kind == "general":
+        dv = d
+    def weights(w):
+        w["m.k"] *= 0.2
+        w["m.v"][5] = 0.0
+        w["m.v"][5, 0] = 1e38
+        if "m.v.conv" in w:
+            w["m.v.conv"][5] = 1.0
+    def tokens(x):
+        x[:, 0] = 0.0
+        x[at, 0] = value / 1e38
+    (_, walked), (_, single) = _both_ways(kind, d, dv, [37, 5, 16], weights, tokens, lambda state: None)
+    _same_kinds_of_numbers(kind, walked, single)
