@@ -34,6 +34,8 @@ __device__ __forceinline__ float sigmoidf_(float x) { return 1.0f / (1.0f + expf
 
 constexpr int DR_COLS = 16, DR_LANES = 4, DR_THREADS = DR_COLS * DR_LANES;
 enum { DR_W = 0, DR_AU = 1, DR_U = 2, DR_K = 3, DR_R = 4, DR_V = 5, DR_ROWS = 6 };
+// Planes of rows in the workspace: none where every request is walked in chunks.
+static int dr_prepared(int d, int walk_from) { return walk_from == 1 && ck_takes(CK_GENERAL, d, d) ? 0 : DR_ROWS; }
 
 // prep: float32 [6][tokens][heads * d] in the order of the enum above; of requests of fewer than `below` tokens.
 template <typename TA>
@@ -217,8 +219,8 @@ __device__ __forceinline__ bool delta_rows(const DeltaRowsArgs<TA>& p, float* ti
   const int h = blockIdx.y, tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
   const int place = blockIdx.x;
   int t_req, n_req;
-  const int req = ck_request(q_start, n_new, n_requests, place, t_req, n_req);
-  const int first = (place - ck_place(t_req, req)) * CK, have = min(CK, n_req - first);
+  const int place0 = ck_request(q_start, n_new, n_requests, from, place, t_req, n_req);
+  const int first = (place - place0) * CK, have = min(CK, n_req - first);
   if (first < 0 || have <= 0 || n_req < from) return false;
   const size_t t0 = (size_t)(t_req + first), width = (size_t)n_heads * d;
   {
@@ -542,17 +544,18 @@ static int launch_delta(int dmax, dim3 grid, cudaStream_t stream, const void* r,
                         float norm_eps, int walk_from) {
   const int rows = n_tokens * n_heads;
   float* prep = work;
-  float* o_raw = work + (size_t)DR_ROWS * rows * d;
+  const int prepared = dr_prepared(d, walk_from);      // planes ahead of the read-outs
+  float* o_raw = work + (size_t)prepared * rows * d;
   if (walk_from > 0) {
     auto up4 = [](size_t v) { return (v + 3) & ~(size_t)3; };
     int rc;
     if (ck_takes(CK_GENERAL, d, d)) {
       const size_t plane = (size_t)rows * d;
-      float *u = work + up4((size_t)(DR_ROWS + 1) * rows * d), *g = u + plane, *v_rows = g + plane, *tiles = v_rows + plane;
+      float *u = work + up4((size_t)(prepared + 1) * rows * d), *g = u + plane, *v_rows = g + plane, *tiles = v_rows + plane;
       constexpr size_t smem_rows = 4 * (ck_rows(2, 64) + 5 * CK * 68);
       cudaError_t e = cudaFuncSetAttribute(delta_rows_kernel<TA>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem_rows);
       if (e != cudaSuccess) return llmrs_fail("delta_rule: shared memory %zu: %s", smem_rows, cudaGetErrorString(e));
-      delta_rows_kernel<TA><<<dim3((unsigned)ck_places(n_tokens, n_requests), n_heads), 128, smem_rows, stream>>>(
+      delta_rows_kernel<TA><<<dim3((unsigned)ck_places(n_tokens, n_requests, walk_from), n_heads), 128, smem_rows, stream>>>(
           {(const TA*)r, (const TA*)k, (const TA*)v, (const TA*)a_raw, in_stride, decay_raw, decay_bias, a_bias, q_start, n_new, tiles,
            u, g, v_rows, n_requests, n_heads, d, decay_scale, key_eps, walk_from});
       rc = llmrs_launch_status("delta_rule (chunks)");
@@ -620,12 +623,13 @@ static int launch_delta(int dmax, dim3 grid, cudaStream_t stream, const void* r,
   return launch_delta_out<TA>(o_raw, gate, in_stride, norm_w, out, n_tokens, n_heads, d, norm_eps, stream);
 }
 
-// Float32 workspace the three kernels share, in floats.
-LLMRS_API long long llmrs_delta_rule_work_floats(int n_tokens, int n_requests, int n_heads, int d) {
-  return (long long)(DR_ROWS + 1) * n_tokens * n_heads * d + 16 +
-         std::max(walk_places(n_tokens, n_requests) * n_heads * (d + walk_table(WALK_GENERAL)),
-                  ck_takes(CK_GENERAL, d, d) ? ck_work_floats(CK_GENERAL, n_tokens, n_requests, n_heads, d, d) + (long long)n_tokens * n_heads * d
-                                             : 0);
+// Float32 workspace of the kernels, in floats: the prepared rows, the read-outs and, where requests are walked (walk_from as below), what
+// their walk reads.
+LLMRS_API long long llmrs_delta_rule_work_floats(int n_tokens, int n_requests, int n_heads, int d, int walk_from) {
+  const long long plane = (long long)n_tokens * n_heads * d, base = (dr_prepared(d, walk_from) + 1) * plane + 16;
+  if (walk_from <= 0) return base;
+  if (ck_takes(CK_GENERAL, d, d)) return base + ck_work_floats(CK_GENERAL, n_tokens, n_requests, walk_from, n_heads, d, d) + plane;
+  return base + walk_places(n_tokens, n_requests) * n_heads * (d + walk_table(WALK_GENERAL));
 }
 
 // r, k, v, gate, a_raw: [tokens, ...] of the activation type, rows `in_stride` elements apart, each pointing at its

@@ -492,8 +492,8 @@ __device__ __forceinline__ bool gdr_channel_rows(const GcrArgs& p, float* tile, 
   CkLook look;
   const int place = blockIdx.x, h = blockIdx.y, tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
   int t_req, n_req;
-  const int req = ck_request(q_start, n_new, n_requests, place, t_req, n_req);
-  const int first = (place - ck_place(t_req, req)) * CK, have = min(CK, n_req - first);
+  const int place0 = ck_request(q_start, n_new, n_requests, from, place, t_req, n_req);
+  const int first = (place - place0) * CK, have = min(CK, n_req - first);
   if (first < 0 || have <= 0 || n_req < from) return false;
   const size_t t0 = (size_t)(t_req + first);
   const int kh = h / (H / G);
@@ -975,7 +975,7 @@ static int launch_chunk_walk(bool channel, const TurnRows& r, float* work, const
   int rc;
   if (channel) {
     LLMRS_REQUIRE(H <= 65535, "gated_delta: too many heads");
-    const dim3 grid((unsigned)ck_places(n_tokens, n_requests), H);
+    const dim3 grid((unsigned)ck_places(n_tokens, n_requests, from), H);
     const GcrArgs a = {r.pq, r.pk, r.pv, r.pbeta, araw, a_log, dt_bias, q_start, n_new, tiles, u, g, n_requests, G, H, d, dv, from};
     rc = (d <= 64 ? launch_channel_rows<64> : launch_channel_rows<128>)(grid, stream, a);
   } else {
@@ -993,22 +993,21 @@ static int launch_chunk_walk(bool channel, const TurnRows& r, float* work, const
   return launch_state_chunks<CK_SYSTEM>(a, n_requests, stream);
 }
 
-// Float32 workspace of the kernels, in floats: prepared q, k, v, beta, g and the raw read-outs.
-LLMRS_API long long llmrs_gated_delta_work_floats(int n_tokens, int n_requests, int G, int H, int d, int dv, int channel) {
-  // The walk in turns: coefficients, decays; in chunks: their rows.
-  const long long turns = walk_places(n_tokens, n_requests) * H;
-  const long long sixteens = ck_takes(CK_SYSTEM, d, dv) ? ck_work_floats(CK_SYSTEM, n_tokens, n_requests, H, d, dv) : 0;
-  if (channel)
-    return (long long)n_tokens * (2LL * G * d + 2LL * H * dv + 1LL * H * d + H) + 48 +
-           std::max(3LL * n_tokens * H * d + turns * (d + walk_table(WALK_CHANNEL)), sixteens);
-  const long long chunk_places = n_tokens / GC_C + n_requests + 1;
-  const long long chunks = chunk_places * H * GC_TABLE, tables = std::max(turns * walk_table(WALK_GATED), sixteens);
-  return (long long)n_tokens * (2LL * G * d + 2LL * H * dv + 3LL * H) + 24 + (chunks > tables ? chunks : tables);
-}
-
 static int g_gd_chunked = 0;
 // 1: portions of 64 tokens and more take the chunked form (off by default: it is not ahead yet, see the file's head).
 LLMRS_API void llmrs_gated_delta_chunked(int on) { g_gd_chunked = on; }
+
+// Float32 workspace of the kernels, in floats: prepared q, k, v, beta, g and the raw read-outs; where requests are walked (walk_from as
+// below) their coefficients and decays in turns, their rows in chunks.
+LLMRS_API long long llmrs_gated_delta_work_floats(int n_tokens, int n_requests, int G, int H, int d, int dv, int channel, int walk_from) {
+  const long long prepared = (long long)n_tokens * (2LL * G * d + 2LL * H * dv + (channel ? 1LL * H * d + H : 3LL * H)) + 48;
+  const long long form = g_gd_chunked && !channel ? (n_tokens / GC_C + n_requests + 1LL) * H * GC_TABLE : 0;
+  if (walk_from <= 0) return prepared + form;
+  if (ck_takes(CK_SYSTEM, d, dv)) return prepared + std::max(form, ck_work_floats(CK_SYSTEM, n_tokens, n_requests, walk_from, H, d, dv));
+  const long long turns = walk_places(n_tokens, n_requests) * H;
+  if (channel) return prepared + 3LL * n_tokens * H * d + turns * (d + walk_table(WALK_CHANNEL));
+  return prepared + std::max(form, turns * walk_table(WALK_GATED));
+}
 
 // x: [tokens, >= 2 G d + H dv] of `dtype`, rows `x_stride` apart: the q, k and v channels that enter the convolutions;
 // gate: [tokens, H dv] rows `gate_stride` apart; taps: float32 [2 G d + H dv, K]; state: float32 [slots, H, d, dv];

@@ -470,16 +470,18 @@ LLMRS_API int llmrs_linear_recurrence_planes(const float* Q, const float* K, con
   return llmrs_launch_status("linear_recurrence");
 }
 
-// Floats of the workspace `tables` of llmrs_linear_recurrence_planes: the coefficients of a portion's turns, or the rows of its chunks.
-LLMRS_API long long llmrs_linear_recurrence_table_floats(int n_tokens, int n_requests, int n_heads, int dk, int dv) {
-  if (ck_takes(CK_LINEAR, dk, dv)) return ck_work_floats(CK_LINEAR, n_tokens, n_requests, n_heads, dk, ck_columns(dv, true));
+// Floats of the workspace `tables` of llmrs_linear_recurrence_planes, by its walk_from: the coefficients of a portion's turns, or the
+// rows of its chunks; none where no request is walked.
+LLMRS_API long long llmrs_linear_recurrence_table_floats(int n_tokens, int n_requests, int n_heads, int dk, int dv, int walk_from) {
+  if (walk_from <= 0) return 0;
+  if (ck_takes(CK_LINEAR, dk, dv)) return ck_work_floats(CK_LINEAR, n_tokens, n_requests, walk_from, n_heads, dk, ck_columns(dv, true));
   return walk_places(n_tokens, n_requests) * n_heads * walk_table(WALK_LINEAR);
 }
 
 // Floats of workspace for llmrs_linear_recurrence: the three prepared planes and the tables.
-LLMRS_API long long llmrs_linear_recurrence_work_floats(int n_tokens, int n_requests, int n_heads, int dk, int dv) {
+LLMRS_API long long llmrs_linear_recurrence_work_floats(int n_tokens, int n_requests, int n_heads, int dk, int dv, int walk_from) {
   return (long long)n_tokens * n_heads * (2LL * dk + dv) + 12 +
-         llmrs_linear_recurrence_table_floats(n_tokens, n_requests, n_heads, dk, dv);
+         llmrs_linear_recurrence_table_floats(n_tokens, n_requests, n_heads, dk, dv, walk_from);
 }
 
 // q, k, v: [tokens, ...] of the activation type with their row strides, head h's channels at h * dk (h * dv);

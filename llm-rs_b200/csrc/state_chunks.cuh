@@ -54,33 +54,52 @@ __host__ __device__ constexpr int ck_tile(int planes, int dmax) { return ck_rows
 // Beyond the first row of B: a word that is not zero where a number that the chunk writes is large or not finite (CK_LARGE).
 __host__ __device__ constexpr int ck_flag(int dmax) { return CK_B * ck_rows(1, dmax) + dmax / 2; }
 __host__ __device__ constexpr int ck_dmax(int d) { return d <= 64 ? 64 : 128; }
-// Places of chunks among all chunks, as walk_place has them for turns.
-__host__ __device__ inline int ck_place(int q_start, int req) { return q_start / CK + req; }
-inline long long ck_places(int n_tokens, int n_requests) { return (long long)n_tokens / CK + n_requests + 1; }
-// The request whose chunks place p lies among (the last one that starts at or before it), its start and tokens; all lanes of a warp call it.
-__device__ __forceinline__ int ck_request(const int* __restrict__ q_start, const int* __restrict__ n_new, int n_requests, int p,
+// Places of chunks among all chunks: a walked request's start in sixteens and its rank among the walked ones. Where all requests are
+// walked (from 1) that is its number, with the requests of no tokens; otherwise those with `from` tokens and more are counted, so that
+// a step's short requests take no places.
+__host__ __device__ inline int ck_place(int q_start, int rank) { return q_start / CK + rank; }
+inline long long ck_places(int n_tokens, int n_requests, int from) {
+  return (long long)n_tokens / CK + (from <= 1 ? n_requests : std::min(n_requests, n_tokens / from)) + 1;
+}
+// All lanes of a warp call these two. A request's rank:
+__device__ __forceinline__ int ck_rank(const int* __restrict__ n_new, int req, int from) {
+  if (from <= 1) return req;
+  int rank = 0;
+  for (int base = 0; base < req; base += 32) {
+    const int r = base + (threadIdx.x & 31);
+    rank += __popc(__ballot_sync(0xffffffffu, r < req && n_new[r] >= from));
+  }
+  return rank;
+}
+// The first place, start and tokens of the request whose chunks place p lies among (the last walked one that starts at or before it).
+__device__ __forceinline__ int ck_request(const int* __restrict__ q_start, const int* __restrict__ n_new, int n_requests, int from, int p,
                                           int& start, int& tokens) {
-  int found = 0;
+  int place = 0, rank = 0;
   start = tokens = 0;
   for (int base = 0; base < n_requests; base += 32) {
-    const int r = base + (threadIdx.x & 31);
+    const int lane = threadIdx.x & 31, r = base + lane;
     const int q = r < n_requests ? q_start[r] : 0, n = r < n_requests ? n_new[r] : 0;
-    const unsigned hit = __ballot_sync(0xffffffffu, r < n_requests && ck_place(q, r) <= p);
-    if (hit == 0) break;
-    const int last = 31 - __clz(hit);
-    found = base + last;
-    start = __shfl_sync(0xffffffffu, q, last);
-    tokens = __shfl_sync(0xffffffffu, n, last);
+    const unsigned walked = __ballot_sync(0xffffffffu, r < n_requests && (from <= 1 || n >= from));
+    const int at = ck_place(q, rank + __popc(walked & ((1u << lane) - 1u)));
+    const unsigned hit = __ballot_sync(0xffffffffu, (walked >> lane & 1u) && at <= p);
+    if (hit == 0 && walked != 0) break;
+    if (hit != 0) {
+      const int last = 31 - __clz(hit);
+      place = __shfl_sync(0xffffffffu, at, last);
+      start = __shfl_sync(0xffffffffu, q, last);
+      tokens = __shfl_sync(0xffffffffu, n, last);
+    }
+    rank += __popc(walked);
   }
-  return found;
+  return place;
 }
 // Heads that the chunks take, others go in turns of four tokens: rows by whole 16-byte copies, d within the block's shared memory.
 __host__ inline bool ck_takes(int planes, int d, int dv) { return d % 4 == 0 && dv % 4 == 0 && d <= (planes == CK_GENERAL ? 64 : 128); }
 // Columns that U and G have per head: the values' and, with a normaliser, one whose value is 1 and three to fill up.
 __host__ __device__ inline int ck_columns(int dv, bool norm) { return norm ? dv + 4 : dv; }
 // Floats of the rows, and of U and G, in a workspace.
-inline long long ck_work_floats(int planes, int n_tokens, int n_requests, int n_heads, int d, int columns) {
-  return d > 128 ? 0 : ck_places(n_tokens, n_requests) * n_heads * ck_tile(planes, ck_dmax(d)) + 2LL * n_tokens * n_heads * columns + 8;
+inline long long ck_work_floats(int planes, int n_tokens, int n_requests, int from, int n_heads, int d, int columns) {
+  return d > 128 ? 0 : ck_places(n_tokens, n_requests, from) * n_heads * ck_tile(planes, ck_dmax(d)) + 2LL * n_tokens * n_heads * columns + 8;
 }
 
 // The three pieces of two numbers, each pair packed as the operands want it. (Subtractions that the compiler does not draw together
@@ -207,7 +226,7 @@ __device__ __forceinline__ bool state_chunks_of(const ChunkArgs& p, int col_bloc
   const int n = p.n_new[req], t0 = p.q_start[req], d = p.d, dv = p.dv, columns = p.columns;
   if (n <= 0 || n < p.from) return false;
   auto sum_of = [](float hi, float lo) { return CAREFUL ? ck_sum(hi, lo) : hi + lo; };
-  const int n_chunks = (n + CK - 1) / CK, place0 = ck_place(t0, req);
+  const int n_chunks = (n + CK - 1) / CK;
   for (int e = tid; e < CK_STAGES * VALUES * CK * 20; e += CK_THREADS)      // columns beyond the values stay 0
     stages[e / (VALUES * CK * 20) * STAGE + TILE + e % (VALUES * CK * 20)] = 0.f;
   __syncthreads();
@@ -218,7 +237,7 @@ __device__ __forceinline__ bool state_chunks_of(const ChunkArgs& p, int col_bloc
 
   if (warp >= 2 * CK_WARPS) {
     // The warps that copy.
-    const int ct = tid - 2 * HALF;
+    const int ct = tid - 2 * HALF, place0 = ck_place(t0, ck_rank(p.n_new, req, p.from));
     auto load = [&](int chunk) {
       if (chunk < n_chunks) {
         float* to = stages + chunk % CK_STAGES * STAGE;
@@ -615,8 +634,8 @@ __device__ __forceinline__ bool ck_rows_of(const ChunkRowsArgs& p, float* tile, 
   CkLook look;
   const int place = blockIdx.x, group = blockIdx.y, tid = threadIdx.x, lane = tid & 31, warp = tid >> 5, d = p.d;
   int t_req, n_req;
-  const int req = ck_request(p.q_start, p.n_new, p.n_requests, place, t_req, n_req);
-  const int first = (place - ck_place(t_req, req)) * CK, have = min(CK, n_req - first);
+  const int place0 = ck_request(p.q_start, p.n_new, p.n_requests, p.from, place, t_req, n_req);
+  const int first = (place - place0) * CK, have = min(CK, n_req - first);
   if (first < 0 || have <= 0 || n_req < p.from) return false;
   const size_t t0 = (size_t)(t_req + first);
   const int shared = p.n_heads / p.n_groups;
@@ -817,7 +836,7 @@ static int launch_ck_rows_of(const ChunkRowsArgs& p, dim3 grid, cudaStream_t str
 }
 template <int PLANES>
 static int launch_ck_rows(const ChunkRowsArgs& p, int n_tokens, cudaStream_t stream) {
-  const dim3 grid((unsigned)ck_places(n_tokens, p.n_requests), p.n_groups);
+  const dim3 grid((unsigned)ck_places(n_tokens, p.n_requests, p.from), p.n_groups);
   LLMRS_REQUIRE(grid.y <= 65535, "state chunks: too many heads");
   return p.d <= 64 ? launch_ck_rows_of<PLANES, 64>(p, grid, stream) : launch_ck_rows_of<PLANES, 128>(p, grid, stream);
 }

@@ -1028,11 +1028,11 @@ def delta_rule(r, k, v, gate, a_raw, decay_raw, decay_bias, a_bias, norm_w, stat
     _need(decay_raw, "decay_raw", torch.float32)
     _need(state, "state", torch.float32)
     out = torch.empty((r.size(0), n_heads * d), dtype=r.dtype, device=r.device)
-    work = torch.empty((int(_lib_ll("llmrs_delta_rule_work_floats")(r.size(0), ctx.n_requests, n_heads, d)),),
-                       dtype=torch.float32, device=r.device)
     # (in chunks heads of 32: one portion of 48 tokens 40 / 41 us, 64 tokens 45 / 43; heads of 64: 32 tokens 48 / 46)
     rule = _chunk_rule(64 if d <= 32 else WALK_PORTION, 640, 128) if _in_chunks(d, d, 64) else dict(least=128 if d <= 32 else WALK_PORTION)
     turns = walk_from(ctx, r.size(0), _walk_blocks(n_heads, d), **rule)
+    work = torch.empty((int(_lib_ll("llmrs_delta_rule_work_floats")(r.size(0), ctx.n_requests, n_heads, d, turns)),),
+                       dtype=torch.float32, device=r.device)
     _check(_lib().llmrs_delta_rule(
         _ptr(r), _ptr(k), _ptr(v), _ptr(gate), _ptr(a_raw), _LL(stride), dtype_code(r.dtype), _ptr(decay_raw),
         _ptr(decay_bias), _ptr(a_bias), _ptr(norm_w), _ptr(state), _ptr(ctx.q_start), _ptr(ctx.n_new),
@@ -1305,7 +1305,7 @@ def linear_recurrence(q, k, v, gate, norm_w, state, ctx, n_heads: int, dk: int, 
     turns = walk_from(ctx, n, _walk_blocks(n_heads, dv + (normaliser is not None)),
                       **(LINEAR_CHUNKS if _in_chunks(dk, dv) else dict(few=1024)))
     # One workspace: the kernels' rows, then the raw read-outs and the normaliser's products.
-    n_work = -(-int(_lib_ll("llmrs_linear_recurrence_work_floats")(n, ctx.n_requests, n_heads, dk, dv)) // 4) * 4
+    n_work = -(-int(_lib_ll("llmrs_linear_recurrence_work_floats")(n, ctx.n_requests, n_heads, dk, dv, turns)) // 4) * 4
     work = torch.empty((n_work + n * n_heads * (dv + 1),), dtype=torch.float32, device=dev)
     o_raw = ctypes.c_void_p(work.data_ptr() + 4 * n_work)
     nq = ctypes.c_void_p(work.data_ptr() + 4 * (n_work + n * n_heads * dv) if normaliser is not None else 0)
@@ -1351,7 +1351,7 @@ def ssd(xbc: torch.Tensor, z: torch.Tensor, dt_raw: torch.Tensor, taps: torch.Te
     empty = lambda width: torch.empty((n, width), dtype=torch.float32, device=xbc.device)
     X, B, Cq, decay, step, y = empty(inner), empty(wk), empty(wk), empty(n_heads), empty(n_heads), empty(inner)
     turns = walk_from(ctx, n, _walk_blocks(n_heads, vdim), **(LINEAR_CHUNKS if _in_chunks(n_state, vdim) else dict(few=1024)))
-    n_tables = int(_lib_ll("llmrs_linear_recurrence_table_floats")(n, ctx.n_requests, n_heads, n_state, vdim)) if turns else 0
+    n_tables = int(_lib_ll("llmrs_linear_recurrence_table_floats")(n, ctx.n_requests, n_heads, n_state, vdim, turns))
     tables = torch.empty((n_tables,), dtype=torch.float32, device=xbc.device)
     _check(_lib().llmrs_ssd_prepare(
         _ptr(xbc), _LL(_row_stride(xbc, "xbc")), _ptr(dt_raw), _LL(_row_stride(dt_raw, "dt_raw")), dtype_code(xbc.dtype),
@@ -1786,12 +1786,12 @@ def gated_delta(x: torch.Tensor, gate: torch.Tensor, taps: torch.Tensor, ba: Opt
     if out is None:
         out = torch.empty((n, n_heads * dv), dtype=x.dtype, device=x.device)
     _need(out, "out", x.dtype, contiguous=False)
-    work = torch.empty((int(_lib_ll("llmrs_gated_delta_work_floats")(n, ctx.n_requests, n_kv_heads, n_heads, dk, dv,
-                                                                     int(channel))),),
-                       dtype=torch.float32, device=x.device)
     chunks = _in_chunks(dk, dv)
     rule = _chunk_rule(_gated_chunk_least(C, channel), 1500, 64) if chunks else dict(least=_gated_walk_least(C, dk, channel), per=32)
     turns = walk_from(ctx, n, _walk_blocks(n_heads, dv), **rule)
+    work = torch.empty((int(_lib_ll("llmrs_gated_delta_work_floats")(n, ctx.n_requests, n_kv_heads, n_heads, dk, dv,
+                                                                     int(channel), turns)),),
+                       dtype=torch.float32, device=x.device)
     _check(_lib().llmrs_gated_delta(
         _ptr(x), _LL(_row_stride(x, "x")), _ptr(gate), _LL(_row_stride(gate, "gate")), dtype_code(x.dtype), _ptr(taps),
         _ptr(None if channel else ba), _ptr(b), _LL(_row_stride(b, "b") if channel else 0), _ptr(channel_decay),

@@ -204,3 +204,10 @@ def test_values_at_the_edge_of_the_range(kind, d, dv, at, value):
         x[at, 0] = value / 1e38
     (_, walked), (_, single) = _both_ways(kind, d, dv, [37, 5, 16], weights, tokens, lambda state: None)
     _same_kinds_of_numbers(kind, walked, single)
+
+
+@pytest.mark.parametrize("kind", ["memory", "retention", "mamba", "gated", "channel", "general"])
+@pytest.mark.parametrize("lens", [[1] * 40 + [50] + [1] * 30 + [0, 49, 48] + [1] * 9 + [97], [0, 0, 48, 47, 64, 1], [1] * 33 + [48]])
+def test_walked_requests_among_many_short_ones(kind, lens):
+    """The places of chunks are counted over the walked requests alone, 32 requests at a time."""
+    _compare(kind, 64, 48, lens, 3, 48)
