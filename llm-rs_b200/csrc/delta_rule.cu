@@ -383,12 +383,13 @@ __device__ __forceinline__ bool delta_rows(const DeltaRowsArgs<TA>& p, float* ti
   if (tid == 0) {
     ck_tile_leaves(tile_out + CK_B * ck_rows(1, DMAX), tile, ck_rows(1, DMAX));
     ck_tile_leaves(tile_out + CK_C * ck_rows(1, DMAX), tile + ck_rows(1, DMAX), ck_rows(1, DMAX));
-    ck_tile_arrived();
+    ck_tile_left();
   }
   return !CAREFUL && look.found();
 }
 template <typename TA>
 __device__ __noinline__ void delta_rows_carefully(const DeltaRowsArgs<TA>& p, float* tile, DeltaRowsShared& sh) {
+  ck_tile_again();
   delta_rows<TA, true>(p, tile, sh);
 }
 template <typename TA>

@@ -624,12 +624,13 @@ __device__ __forceinline__ bool gdr_channel_rows(const GcrArgs& p, float* tile, 
   __syncthreads();
   if (tid == 0) {
     ck_tile_leaves(p.tiles + ((size_t)place * H + h) * ck_tile(CK_SYSTEM, DMAX), tile, ck_tile(CK_SYSTEM, DMAX));
-    ck_tile_arrived();
+    ck_tile_left();
   }
   return !CAREFUL && look.found();
 }
 template <int DMAX>
 __device__ __noinline__ void gdr_channel_rows_carefully(const GcrArgs& p, float* tile, GcrShared& sh) {
+  ck_tile_again();
   gdr_channel_rows<DMAX, true>(p, tile, sh);
 }
 template <int DMAX>

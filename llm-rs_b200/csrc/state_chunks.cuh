@@ -591,6 +591,7 @@ struct ChunkRowsArgs {
   const int *q_start, *n_new;
   float *tiles, *u, *g;
   int n_requests, n_heads, n_groups, d, dv, columns, from;
+  int heads_a_block;           // of the heads that share a key head (the launch sets it)
   bool norm;
 };
 
@@ -601,14 +602,20 @@ __device__ __forceinline__ void ck_tile_leaves(float* to, const float* tile, int
   asm volatile("cp.async.bulk.global.shared::cta.bulk_group [%0], [%1], %2;\n\tcp.async.bulk.commit_group;"
                ::"l"(to), "r"(smem_addr(tile)), "r"(floats * 4) : "memory");
 }
-__device__ __forceinline__ void ck_tile_arrived() { asm volatile("cp.async.bulk.wait_group 0;" ::: "memory"); }      // in memory too
 __device__ __forceinline__ void ck_tile_left() { asm volatile("cp.async.bulk.wait_group.read 0;" ::: "memory"); }
+// All threads, before the block's tiles are made once more: the first ones (of thread 0) are in memory.
+__device__ __forceinline__ void ck_tile_again() {
+  if (threadIdx.x == 0) asm volatile("cp.async.bulk.wait_group 0;" ::: "memory");
+  __syncthreads();
+}
 
-// The rows of CK_LINEAR and CK_SYSTEM with a decay per token and head: a block per (place, key head). First the products of the rows
-// on the tensor cores, a quarter of the channels a warp; then, two heads at a time, the coefficients (a warp a head); then head by
-// head the rows, sixteen channels and sixteen columns a warp at a time. Bound by memory latency and the bytes that leave
-// (39 KB a chunk and head of 128 channels): 2,048 tokens of 16 heads over 8 of 128 x 128 54 us (two channels a thread and products on
-// the CUDA cores 61), 16 heads without a system 38. Three blocks an SM: with two, the products apart from the tile, 55 and 48.
+// The rows of CK_LINEAR and CK_SYSTEM with a decay per token and head: a block per (place, key head, some of the heads that share it).
+// First the products of the rows on the tensor cores, a quarter of the channels a warp; then, two heads at a time, the coefficients (a
+// warp a head); then head by head the rows, sixteen channels and sixteen columns a warp at a time. Bound by memory latency and the
+// bytes that leave (39 KB a chunk and head of 128 channels): 2,048 tokens of 16 heads over 8 of 128 x 128 47 us (two channels a thread
+// and products on the CUDA cores 61), 16 heads without a system 39. Three blocks an SM: with two, the products apart from the
+// tile, 55 and 48. Heads that share one key head by a block each pair: a Mamba-2 mixer of 32 heads over one group, 64 tokens
+// 128 us, 186 with all of them in one block; 2,048 tokens 1,628 and 1,645.
 constexpr int CK_ROWS_THREADS = 256;
 __host__ __device__ constexpr int ck_rows_smem(int planes, int dmax) { return 4 * (ck_tile(planes, dmax) + 2 * CK * (dmax + 4)); }
 struct CkRowsShared {      // beside the tile
@@ -632,20 +639,21 @@ __device__ __forceinline__ bool ck_rows_of(const ChunkRowsArgs& p, float* tile, 
   auto& Q = sh.Q;
   auto& T = sh.T;
   CkLook look;
-  const int place = blockIdx.x, group = blockIdx.y, tid = threadIdx.x, lane = tid & 31, warp = tid >> 5, d = p.d;
+  const int place = blockIdx.x, tid = threadIdx.x, lane = tid & 31, warp = tid >> 5, d = p.d;
+  const int shared = p.n_heads / p.n_groups, parts = (shared + p.heads_a_block - 1) / p.heads_a_block, group = blockIdx.y / parts;
+  const int head0 = group * shared + blockIdx.y % parts * p.heads_a_block, head1 = min(head0 + p.heads_a_block, (group + 1) * shared);
   int t_req, n_req;
   const int place0 = ck_request(p.q_start, p.n_new, p.n_requests, p.from, place, t_req, n_req);
   const int first = (place - place0) * CK, have = min(CK, n_req - first);
   if (first < 0 || have <= 0 || n_req < p.from) return false;
   const size_t t0 = (size_t)(t_req + first);
-  const int shared = p.n_heads / p.n_groups;
   float decay_in = 0.f, beta_in = 0.f;      // of token `lane` and this warp's head, the first ones on their way early
   auto fetch_strengths = [&](int h, float& decay, float& beta) {
     const size_t at = (t0 + lane) * p.n_heads + h;
     decay = lane >= have ? 1.f : (p.decay ? p.decay[at] : (p.head_decay ? p.head_decay[h] : 1.f));
     beta = lane >= have ? 0.f : (p.beta ? p.beta[at] : 1.f);
   };
-  if (warp < min(HEADS, shared)) fetch_strengths(group * shared + warp, decay_in, beta_in);
+  if (warp < min(HEADS, head1 - head0)) fetch_strengths(head0 + warp, decay_in, beta_in);
   {
     float4 in[EACH];
 #pragma unroll
@@ -706,11 +714,11 @@ __device__ __forceinline__ bool ck_rows_of(const ChunkRowsArgs& p, float* tile, 
     const int a = e / (CK * CK), i = e / CK % CK, j = e % CK;
     if (SYSTEM || a) gram[a][i][j] = (part[0][a][i][j] + part[1][a][i][j]) + (part[2][a][i][j] + part[3][a][i][j]);
   }
-  for (int h0 = group * shared; h0 < (group + 1) * shared; h0 += HEADS) {
-    const int heads = min(HEADS, (group + 1) * shared - h0);
+  for (int h0 = head0; h0 < head1; h0 += HEADS) {
+    const int heads = min(HEADS, head1 - h0);
     __syncthreads();      // the products; everyone is done with the heads before
     if (warp < heads) {
-      if (h0 > group * shared) fetch_strengths(h0 + warp, decay_in, beta_in);
+      if (h0 > head0) fetch_strengths(h0 + warp, decay_in, beta_in);
       if (lane < CK) {
         const int i = lane;
         strengths[warp][0][i] = decay_in;
@@ -809,11 +817,12 @@ __device__ __forceinline__ bool ck_rows_of(const ChunkRowsArgs& p, float* tile, 
       if (tid == 0) ck_tile_leaves(p.tiles + ((size_t)place * p.n_heads + h) * ck_tile(PLANES, DMAX), tile, ck_tile(PLANES, DMAX));
     }
   }
-  if (tid == 0) ck_tile_arrived();
+  if (tid == 0) ck_tile_left();
   return !CAREFUL && look.found();
 }
 template <int PLANES, int DMAX>
 __device__ __noinline__ void ck_rows_carefully(const ChunkRowsArgs& p, float* tile, CkRowsShared& sh) {
+  ck_tile_again();
   ck_rows_of<PLANES, DMAX, true>(p, tile, sh);
 }
 template <int PLANES, int DMAX>
@@ -835,8 +844,12 @@ static int launch_ck_rows_of(const ChunkRowsArgs& p, dim3 grid, cudaStream_t str
   return llmrs_launch_status("state chunks (rows)");
 }
 template <int PLANES>
-static int launch_ck_rows(const ChunkRowsArgs& p, int n_tokens, cudaStream_t stream) {
-  const dim3 grid((unsigned)ck_places(n_tokens, p.n_requests, p.from), p.n_groups);
+static int launch_ck_rows(ChunkRowsArgs p, int n_tokens, cudaStream_t stream) {
+  // Heads that share a key head go through one block, which makes their products once, as long as there are blocks enough: three for
+  // each of the SMs, two heads (whose coefficients are made together) at least.
+  const long long places = ck_places(n_tokens, p.n_requests, p.from), shared = p.n_heads / p.n_groups, blocks = 3 * 148;
+  p.heads_a_block = (int)std::min(shared, std::max(2ll, places * p.n_heads / blocks / 2 * 2));
+  const dim3 grid((unsigned)places, (unsigned)(p.n_groups * ((shared + p.heads_a_block - 1) / p.heads_a_block)));
   LLMRS_REQUIRE(grid.y <= 65535, "state chunks: too many heads");
   return p.d <= 64 ? launch_ck_rows_of<PLANES, 64>(p, grid, stream) : launch_ck_rows_of<PLANES, 128>(p, grid, stream);
 }

@@ -30,7 +30,10 @@ def _part(kind, d, dv, taps=3):
                "mamba": lambda: Mamba2(D, 4, dv, d, 2, 3, norm_parts=1, prefix="m."),
                "gated": lambda: GatedDelta(D, 4, 2, d, dv, taps, prefix="m."),
                "channel": lambda: ChannelDelta(D, 4, 2, d, dv, taps, 8, 8, prefix="m."),
-               "general": lambda: GeneralDelta(D, 3, d, 8, prefix="m.")}[kind]()
+               "general": lambda: GeneralDelta(D, 3, d, 8, prefix="m."),
+               "mamba of one group": lambda: Mamba2(D, 7, dv, d, 1, 3, norm_parts=1, prefix="m."),
+               "mamba of fives": lambda: Mamba2(D, 10, dv, d, 2, 3, norm_parts=1, prefix="m."),
+               "gated of threes": lambda: GatedDelta(D, 6, 2, d, dv, taps, prefix="m.")}[kind]()
 
 
 @pytest.mark.parametrize("kind", ["memory", "retention", "mamba", "gated", "channel", "general"])
@@ -211,3 +214,10 @@ def test_values_at_the_edge_of_the_range(kind, d, dv, at, value):
 def test_walked_requests_among_many_short_ones(kind, lens):
     """The places of chunks are counted over the walked requests alone, 32 requests at a time."""
     _compare(kind, 64, 48, lens, 3, 48)
+
+
+@pytest.mark.parametrize("kind", ["mamba of one group", "mamba of fives", "gated of threes"])
+@pytest.mark.parametrize("d,dv,lens", [(64, 64, [40, 16, 1]), (128, 20, [33]), (64, 16, [17] * 90), (36, 16, [17] * 170)])
+def test_heads_that_share_a_key_head(kind, d, dv, lens):
+    """Two heads a block of rows, four and all: the last block of a key head has what is left."""
+    _compare(kind, d, dv, lens, 3)
