@@ -379,24 +379,46 @@ static int gf_tiles(const GfArgs<TX>& a) {
                    grid, threads, smem, false, a.stream, a.x, a.w, a.bias, a.out, a.M, a.N, a.K, a.x_stride, a.out_stride);
 }
 
-// Blocks a cluster: as many as the device holds at a time, at most one for every KG segments, at most eight, and no more than
-// leave the last round's blocks with segments (6,144 features of 16 rows, K = 1,024: four blocks 14.3 us, three, the last of which
-// walk a second round alone, 25).
+// Blocks a cluster where `cluster` is 0: as many as the device holds at a time (KG = 1: six an SM, of those that hold 32 rows), at most
+// one for every KG segments, at most eight, and no more than leave the last round's blocks with segments (6,144 features of 16 rows,
+// K = 1,024: four blocks 14.3 us, three, the last of which walk a second round alone, 25).
+static long long gf_cluster(long long tiles, long long turns, int blocks) {
+  const long long most = std::min(8ll, std::max(1ll, blocks / tiles)), rounds = (turns + most - 1) / most;
+  return (turns + rounds - 1) / rounds;
+}
+template <typename TX>
+constexpr size_t gf_seg_smem(int rows, int cols, int kg, int bk, int ns) {
+  return (size_t)(kg + 1) * rows * cols * 4 + (size_t)ns * kg * (cols * (bk + 4) * 4 + rows * (bk * sizeof(TX) + 16));
+}
 template <int RM, int TM, int CN, int TN, int KG, int BK, int NS, typename TX>
-static int gf_segments(const GfArgs<TX>& a) {
-  constexpr int BM = RM * TM, BN = CN * TN, threads = RM * CN * KG, BLOCKS = 148 * (KG > 1 ? 2 : 6);
-  constexpr size_t smem = (size_t)(KG + 1) * BM * BN * 4 + (size_t)NS * KG * (BN * (BK + 4) * 4 + BM * (BK * sizeof(TX) + 16));
+static int gf_segments(const GfArgs<TX>& a, long long cluster = 0) {
+  constexpr int BM = RM * TM, BN = CN * TN, threads = RM * CN * KG;
+  constexpr size_t smem = gf_seg_smem<TX>(BM, BN, KG, BK, NS);
   static_assert(smem <= 227 * 1024, "the block's shared memory");
   const long long tiles_n = (a.N + BN - 1) / BN, tiles_m = (a.M + BM - 1) / BM;
   LLMRS_REQUIRE(tiles_m <= 65535, "gemm_f32: M=%d is too large", a.M);
-  const long long turns = ((a.K + GF_SEG - 1) / GF_SEG + KG - 1) / KG;
-  const long long most = std::min(8ll, std::max(1ll, BLOCKS / (tiles_n * tiles_m))), rounds = (turns + most - 1) / most;
-  const long long cluster = (turns + rounds - 1) / rounds;
+  if (cluster == 0) cluster = gf_cluster(tiles_n * tiles_m, ((a.K + GF_SEG - 1) / GF_SEG + KG - 1) / KG, 148 * (KG > 1 ? 2 : 6));
   const dim3 grid((unsigned)tiles_n, (unsigned)tiles_m, (unsigned)cluster);
   return gf_launch(a.vec ? gemm_f32_seg_kernel<TX, RM, TM, CN, TN, KG, BK, NS, true>
                          : gemm_f32_seg_kernel<TX, RM, TM, CN, TN, KG, BK, NS, false>,
                    grid, threads, smem, true, a.stream, a.x, a.w, a.bias, a.out, a.M, a.N, a.K, a.x_stride, a.out_stride,
                    (int)cluster);
+}
+
+// Estimated us of tiles of `rows` x 32 by segments, clusters of so many blocks, to compare with one another. An SM's
+// blocks share its path from shared memory, rows * (TM + TN) / (TM * TN) a segment; a block by itself waits for its own chain; blocks
+// beyond those that an SM holds wait for a wave. Fitted to 149 products (65 to 576 rows, 512 to 3,072 features, K 768 to 3,072), all
+// tiles and clusters beside one another: the choice below takes 1.05 times as long as the best one on average, 1.28 at worst;
+// by the empty rows alone it was 1.14 and 1.86 (408 rows, K = 1,024 into 1,024: 57 us in tiles of 24, 41 so).
+template <typename TX>
+static double gf_seg_us(int rows, long long cluster, long long M, long long N, long long K) {
+  const long long turns = (K + GF_SEG - 1) / GF_SEG;
+  const double work = rows * (rows / 8 + 4.0) / (rows / 8 * 4);
+  const long long resident = (227 * 1024) / (long long)(gf_seg_smem<TX>(rows, 32, 1, 32, 3) + 1024);
+  const long long blocks = ((M + rows - 1) / rows) * ((N + 31) / 32) * cluster, waves = blocks / (148 * resident), rest = blocks - waves * 148 * resident;
+  auto segment = [&](double an_sm) { return std::max(2.548 + 0.21 * work, 0.075 * work * an_sm); };
+  const double at_once = waves * segment(resident) + (rest ? segment((rest + 147) / 148) : 0.0);
+  return (turns + cluster - 1) / cluster * (at_once + 3.744) + 1.54 * (waves + (rest ? 1 : 0));
 }
 
 // Many rows: the largest tile of which there are enough blocks for the SMs, since larger tiles read the operands less often.
@@ -428,12 +450,25 @@ static int gemm_f32_any(const TX* x, long long x_stride, const float* w, const f
   int rows = 0;      // of a tile: those that leave the fewest empty, of equals the most
   for (int r : {64, 48, 40, 32, 24})
     if (rows == 0 || blocks(r, N) * r < blocks(rows, N) * rows) rows = r;
+  long long cluster = 0;
+  if (M > 64) {      // several tiles of rows: waves weigh more than empty rows do; another choice has to promise an eighth
+    const long long turns = (K + GF_SEG - 1) / GF_SEG;
+    cluster = gf_cluster(blocks(rows, 32), turns, 148 * 6);
+    double best = 0.87 * gf_seg_us<TX>(rows, cluster, M, N, K);
+    for (int r : {24, 32, 40, 48, 64})
+      for (long long c : {1, 2, 3, 4, 6, 8}) {
+        const long long rounds = (turns + c - 1) / c;
+        if (c > turns || (turns + rounds - 1) / rounds != c) continue;
+        const double us = gf_seg_us<TX>(r, c, M, N, K);
+        if (us < best) best = us, rows = r, cluster = c;
+      }
+  }
   switch (rows) {
-    case 24: return gf_segments<8, 3, 8, 4, 1, 32, 3>(a);
-    case 32: return gf_segments<8, 4, 8, 4, 1, 32, 3>(a);
-    case 40: return gf_segments<8, 5, 8, 4, 1, 32, 3>(a);
-    case 48: return gf_segments<8, 6, 8, 4, 1, 32, 3>(a);
-    default: return gf_segments<8, 8, 8, 4, 1, 32, 3>(a);
+    case 24: return gf_segments<8, 3, 8, 4, 1, 32, 3>(a, cluster);
+    case 32: return gf_segments<8, 4, 8, 4, 1, 32, 3>(a, cluster);
+    case 40: return gf_segments<8, 5, 8, 4, 1, 32, 3>(a, cluster);
+    case 48: return gf_segments<8, 6, 8, 4, 1, 32, 3>(a, cluster);
+    default: return gf_segments<8, 8, 8, 4, 1, 32, 3>(a, cluster);
   }
 }
 

@@ -130,6 +130,20 @@ def test_gemm_f32_segments(N, K, pad, rows_dtype):
         assert torch.equal(ops.gemm_f32(x[:M], w, b), whole[:M]), M
 
 
+@pytest.mark.parametrize("rows_dtype", [torch.float32, torch.bfloat16])
+@pytest.mark.parametrize("N,K", [(1024, 1024), (1000, 3072), (530, 2052), (768, 768)])
+def test_gemm_f32_tiles_of_several_hundred_rows(N, K, rows_dtype):
+    """Tiles and clusters are chosen by an estimate: whatever they are, a row has the bits that it has by itself (bound as above)."""
+    ops = _ops()
+    torch.manual_seed(N + K)
+    x, w = torch.randn(576, K, device=DEV).to(rows_dtype), torch.randn(N, K, device=DEV)
+    alone = torch.cat([ops.gemm_f32(x[i:i + 16], w) for i in range(0, 576, 16)])
+    bound = (x.double().abs() @ w.double().abs().t()) * (256 + -(-K // 256)) * 2.0 ** -24
+    assert bool(((alone.double() - x.double() @ w.double().t()).abs() <= bound).all())
+    for M in (66, 97, 121, 161, 216, 240, 264, 300, 336, 385, 408, 456, 481, 505, 528, 553, 576):
+        assert torch.equal(ops.gemm_f32(x[:M], w), alone[:M]), M
+
+
 # -- norm + rotation + cache write ---------------------------------------------------------
 def _paged_setup(lens, new, n_kv, d, page, dtype, seed=0):
     """Random cache with scattered pages; returns tensors for kernels and dense copies for the reference."""
