@@ -447,21 +447,20 @@ static int launch_decode(const void* q, long long q_stride, void* out, long long
   const int groups_per_kv = (G + DC_HG - 1) / DC_HG;
   const int tpr = d / 4;
   const int n_sub = DC_THREADS / tpr;
+  // Queries, scores and sums of the values: at most 200 KB, in which a key of a split takes 32 bytes; its page's id takes four more at
+  // most, 25 KB, so that the two fit the 227 KB that a block can have with pages of any size.
+  constexpr size_t MOST = 200 * 1024, BLOCK = 227 * 1024 - 256;      // (beside the kernel's own few words)
+  static_assert(MOST + (MOST / (DC_HG * sizeof(float)) + 2) * sizeof(int) <= BLOCK, "a page of one key");
   size_t smem = ((size_t)DC_HG * d + (size_t)DC_HG * split_keys + (size_t)n_sub * DC_HG * d) * sizeof(float);
-  LLMRS_REQUIRE(smem <= 200 * 1024, "attn_decode: %zu bytes of shared memory needed (split of %d keys)", smem,
-                split_keys);
+  LLMRS_REQUIRE(smem <= MOST, "attn_decode: %zu bytes of shared memory needed (split of %d keys)", smem, split_keys);
   // Early keys: up to 64 within what is left of some 100 KB (two blocks an SM), where rows start on 16-byte boundaries.
   const size_t page_ids = ((size_t)split_keys / page_size + 2) * sizeof(int), row = 2 * (size_t)(d + VEC) * sizeof(T);
   const size_t room = 100 * 1024 > smem + page_ids ? 100 * 1024 - smem - page_ids : 0;
   const int early = ((uintptr_t)cache & 15) == 0 ? (int)(room / row < 64 ? room / row : 64) : 0;
   smem += early * row + page_ids;
-  static size_t configured = 0;  // per instantiation; raised only when a launch needs more
-  if (smem > configured) {
-    cudaError_t e = cudaFuncSetAttribute(attn_decode_split_kernel<T, VEC>,
-                                         cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
-    if (e != cudaSuccess) return llmrs_fail("attn_decode: shared memory %zu: %s", smem, cudaGetErrorString(e));
-    configured = smem;
-  }
+  // (Asked for once, and all of it: with the size of the call two threads' calls could leave the smaller one's.)
+  static const cudaError_t e = cudaFuncSetAttribute(attn_decode_split_kernel<T, VEC>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)BLOCK);
+  if (e != cudaSuccess) return llmrs_fail("attn_decode: shared memory %zu: %s", BLOCK, cudaGetErrorString(e));
   dim3 grid(n_dec, n_kv_heads * groups_per_kv, max_splits);
   llmrs_launch(attn_decode_split_kernel<T, VEC>, grid, dim3(DC_THREADS), smem, stream, true, (const T*)q, q_stride,
                (const T*)cache, dec_reqs, q_start, cached_len, block_table, table_stride, scratch, max_splits, split_keys,

@@ -313,6 +313,18 @@ def test_decode_attention_merged_by_large_clusters(nq, nkv, d, split_keys, lens)
     assert torch.allclose(got, want, atol=2.5e-2, rtol=2e-2), float((got - want).abs().max())
 
 
+@pytest.mark.parametrize("d,split_keys", [(64, 5312), (16, 5344)])
+def test_decode_attention_with_the_largest_splits_over_pages_of_one_key(d, split_keys):
+    """Scores, sums and page ids at the most shared memory that a block can ask for, in one split and in two."""
+    new, lens = [1, 1, 1], [split_keys - 1, split_keys + 40, 3]
+    torch.manual_seed(d)
+    table, cache = _paged_setup(lens, new, 1, d, 1, torch.float32, seed=2)
+    q = torch.randn(len(lens), 2 * d) * 1.5
+    want = _attention_reference(q, cache, table, lens, new, 2, 1, d, 1, 0, d ** -0.5)
+    got = _run_attention(q, cache, table, lens, new, 2, 1, d, 1, 0, d ** -0.5, split_keys=split_keys, fused_merge=False)
+    assert torch.allclose(got, want, atol=2e-5, rtol=1e-4), float((got - want).abs().max())
+
+
 @pytest.mark.parametrize("nq,nkv,lens,split_keys", [
     (32, 8, [511, 300, 17, 0, 512], 512), (8, 2, [1000, 999], 256), (5, 1, [70], 128), (16, 1, [200, 90], 128)])
 def test_decode_attention_with_the_ring_of_two_tiles(nq, nkv, lens, split_keys):
