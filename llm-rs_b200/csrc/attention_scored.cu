@@ -1284,7 +1284,8 @@ scored_decode_grouped_kernel(const T* __restrict__ q, long long q_stride, const 
 // 48 of 2,000 with heads of 64: 77 -> 34. Those with rings of three tiles and two blocks an SM; with two tiles and three blocks 48 of
 // 200 to 4,100 keys take 49 us (4.3 TB/s) where they took 60, 48 of 2,000 47 (57), heads of 64 70 (72): bound by the 700 instructions a
 // tile and warp, each of which waits for the one before, so more warps help and more tiles in flight do not (four blocks of 128
-// registers spill: 55).
+// registers spill: 55). Nor where the device is not full: a whole mixer of 1 request takes as long with either ring (25 us at 100
+// keys, 33.6 at 4,000), 8 requests of 2,000 and 4,000 keys 43.5 and 51.2 us with two tiles, 46.7 and 55.3 with three.
 constexpr int SM_KEYS = 16, SM_STAGES = 2;
 template <int D> __host__ __device__ constexpr int sm_ring_bytes() { return SM_STAGES * 2 * SM_KEYS * (D + 8) * 2; }      // of a warp
 template <int D>

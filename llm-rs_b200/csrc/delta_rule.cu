@@ -13,7 +13,7 @@
 //               widened, as six float32 rows [tokens, heads * d];
 //   (requests that are walked take their rows and the walk of state_chunks.cuh instead of these two, heads of more than 64 channels
 //   `turns` and the walk of state_walk.cuh; 2,048 tokens of 32 heads of 64 x 64: 816 us walked one by one, 246 in turns, 92 in
-//   chunks; their rows 106 us, those of turns 56, where `prepare` takes 38)
+//   chunks; their rows 104 us, those of turns 56, where `prepare` takes 38)
 //   recurrence  one block per (request, head, slice of 16 value columns) walks the request's tokens of the step in
 //               order: a column of S depends on no other column, so the slices run side by side. Four adjacent lanes
 //               share a column, each keeping a quarter of its key channels in registers; u^T S and S^T r are summed

@@ -41,7 +41,7 @@
 // products per chunk over rows that arrive through two shared-memory buffers, 32 tokens per sequential step instead of
 // one. A chunk's missing tokens (a portion's end) count as k = q = v = 0, beta = 0, g = 1 and change nothing.
 // The chunked form is OFF by default (llmrs_gated_delta_chunked): its products read every operand from shared memory
-// and are bound by that (2,048 tokens of 16 heads of 128 x 128: some 500 us, the walk in turns 265, in chunks on the tensor cores 116).
+// and are bound by that (2,048 tokens of 16 heads of 128 x 128: some 500 us, the walk in turns 265, in chunks on the tensor cores 117).
 #include <limits.h>
 
 #include "common.cuh"

@@ -30,10 +30,11 @@
 // Precision, float32 models of 300 tokens, states against 64 bits (in turns on the CUDA cores -> here): gated 9.7e-7 -> 5.5e-7, channel
 // decays 9.2e-7 -> 5.0e-7, generalized 8.7e-7 -> 4.8e-7, linear with one decay a head 7.3e-7 -> 2.5e-7 (its decays as stored).
 //
-// What bounds it: one warp a scheduler walks, and a chunk is the chain state's pieces -> W S -> exchange -> Y's pieces -> update (some
-// 1,400 cycles of which 48 products issue for 400); the read-outs' products share the tensor cores with it. 2,048 tokens, the walk
-// alone, in turns of four on the CUDA cores -> here: gated, 16 heads of 128 x 128 267 -> 116 us, generalized, 32 heads of 64 x 64
-// 251 -> 92, linear with a normaliser, 1,311 tokens 184 -> 80. (Sixteen tokens with the rows split in here by the copying warps, the
+// What bounds it: one warp a scheduler walks, and a chunk is the chain state's pieces -> W S -> exchange -> Y's pieces -> update (900 ns
+// of which 48 products issue for 200); the read-outs' products share the tensor cores with it, and the copies come just in time: tiles
+// that do not start on lines of 128 bytes cost the gated walk 29 %. 2,048 tokens, the walk
+// alone, in turns of four on the CUDA cores -> here: gated, 16 heads of 128 x 128 267 -> 117 us, generalized, 32 heads of 64 x 64
+// 251 -> 92, linear with a normaliser, 1,311 tokens 184 -> 81. (Sixteen tokens with the rows split in here by the copying warps, the
 // system and the read-outs on the walking warps: 193 us. Read-outs of the chunk that is walked, not of the one before: linear 90
 // against 84.)
 #pragma once
@@ -836,7 +837,7 @@ ck_rows_kernel(const __grid_constant__ ChunkRowsArgs p) {
 template <int PLANES, int DMAX>
 static int launch_ck_rows_of(const ChunkRowsArgs& p, dim3 grid, cudaStream_t stream) {
   constexpr size_t smem = ck_rows_smem(PLANES, DMAX);
-  if (smem > 16 * 1024) {      // (beside the kernel's own 18 KB)
+  if (smem > 32 * 1024) {      // (48 KB need no asking, but the kernel's own 14 KB count too)
     cudaError_t e = cudaFuncSetAttribute(ck_rows_kernel<PLANES, DMAX>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
     if (e != cudaSuccess) return llmrs_fail("state chunks: shared memory %zu: %s", smem, cudaGetErrorString(e));
   }

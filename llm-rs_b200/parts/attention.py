@@ -60,11 +60,11 @@ _PREFILL_US = {False: ((4.6, 0.042, 5.0, 0.13, 0.0023), (6.9, 0.0088, 4.6, 0.45,
 
 def tc_pays(work: tuple, heads: int, window: int, scored: bool) -> bool:
     """True where the tcgen05 kernel (with blocks of 64 queries, as mma.sync has them) is the faster one for portions that would fill
-    its blocks of 128 less than half. It
-    walks a tile of keys in a fifth of the time, so it pays wherever there are keys to walk; the other starts sooner and holds more
-    blocks. Measured, mma.sync / tcgen05 (us, heads of 128; plain, 16 heads | with a gate, 16 heads): one portion of 20 tokens 5.1 / 7.3 |
-    7.3 / 8.6, of 20 after 500 26.8 / 12.7 | 41 / 14, of 8 after 2,000 90 / 24 | 142 / 25; 64 portions of 30 21 / 33 | 28 / 39, the same
-    after 100 41 / 44 | 59 / 52; 200 portions of 2 after 30 40 / 87 | 56 / 102, after 500 259 / 167 | 419 / 188."""
+    its blocks of 128 less than half. It walks a tile of keys in a fifth of the time, so it pays wherever there are keys to walk; the
+    other starts sooner and holds more blocks. Measured, mma.sync / tcgen05 (us, heads of 128; plain, 16 heads | with a gate, 16
+    heads): one portion of 20 tokens 5.1 / 7.3 | 7.3 / 8.6, of 20 after 500 26.8 / 12.7 | 41 / 14, of 8 after 2,000 90 / 24 | 142 / 25;
+    64 portions of 30 21 / 33 | 28 / 39, the same after 100 41 / 44 | 59 / 52; 200 portions of 2 after 30 40 / 87 | 56 / 102, after 500
+    259 / 167 | 419 / 188."""
     longest, blocks, keys = work
     if window > 0:
         longest, keys = min(longest, window + 64), min(keys, blocks * (window + 64))

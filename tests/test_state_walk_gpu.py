@@ -1,5 +1,6 @@
-"""The recurrences with a matrix state walked in turns of four tokens (csrc/state_walk.cuh) and token by token: the same outputs
-and states from either, at the edges of turns, stages and copies, for many requests in one step, with all of a step's requests
+"""The recurrences with a matrix state walked in chunks of sixteen tokens (csrc/state_chunks.cuh) or in turns of four
+(csrc/state_walk.cuh), by their heads, and token by token: the same outputs
+and states from either, at the edges of chunks, turns, stages and copies, for many requests in one step, with all of a step's requests
 in turns or those from some length on. Both are float32 evaluations of one recurrence, each some 1e-6 from 64 bits in the
 2-norm at these sizes; single elements may lie sixteen times that apart."""
 from types import SimpleNamespace
@@ -111,13 +112,15 @@ def _compare(kind, d, dv, lens, taps, turns=1):
 
 
 @pytest.mark.parametrize("kind", ["memory", "retention", "mamba", "gated", "channel", "general"])
-@pytest.mark.parametrize("at", [0, 1, 2, 3, 4, 53, 61])
+@pytest.mark.parametrize("at", [0, 1, 2, 3, 4, 7, 8, 15, 16, 31, 32, 47, 48, 53, 61])
 @pytest.mark.parametrize("bad", [float("inf"), float("nan")])
-def test_tokens_before_one_that_is_not_finite_keep_their_numbers(kind, at, bad):
-    """Wherever the token lies in its turn, earlier outputs keep every bit, and its own is no number."""
+@pytest.mark.parametrize("d,dv", [(64, 48), (30, 17)])
+def test_tokens_before_one_that_is_not_finite_keep_their_numbers(kind, d, dv, at, bad):
+    """Wherever the token lies in its chunk (heads of 64) or in its turn (of 30), earlier outputs keep every bit, and its own is no
+    number."""
     from llm_rs_b200.parts import Runtime
     g = torch.Generator().manual_seed(3)
-    D, part = _part(kind, 64, 48)
+    D, part = _part(kind, d, dv)
     w = {s.name: (torch.randn(s.shape, generator=g) * (0.5 if len(s.shape) == 1 else s.shape[-1] ** -0.5)).to(DEV)
          for s in part.weight_specs()}
     part.bind(w, Runtime(torch.device(DEV), torch.float32, 4096))
